@@ -248,11 +248,11 @@ def kernel_numbers(size: str, T: int, seqs: int, ctx: int, only: str = "") -> li
             return lambda: ops.latent_attention_prefill(qkv, H * a.dim, kv, kr, tl, sink, o, H, a.dim, a.vdim, a.scale)
         k.time("attention", "nubosun latent attention, prefill form", mk_pre, T * H * (2 * a.dim + rot + 2 * a.vdim) * 2,
                2.0 * pairs_causal * H * (a.dim + rot + a.vdim))
-        tiles = ops.prefill_tiles(seq_of_row.cpu(), nq // nkv).to(dev)
+        tiles = ops.prefill_tiles(seq_of_row.cpu(), nq // nkv, ops.prefill_tile_rows(bs)).to(dev)
 
         def mk_lpre(i):
             q, kc, vc, o = _w(T, nq, D), _w(nslots, nkv, D), _w(nslots, nkv, D), torch.empty(T, nq, D, dtype=bf, device=dev)
-            return lambda: ops.prefill_attention(q, kc, vc, tables, ctx_lens, seq_of_row, tiles, o, D ** -0.5, bs)
+            return lambda: ops.prefill_attention(q, kc, vc, tables, ctx_lens, seq_of_row, tiles, o, D ** -0.5, bs, ops.prefill_tile_rows(bs))
         k.time("attention", "llama prefill attention", mk_lpre, T * nq * D * 4 + T * nkv * D * 4, 4.0 * pairs_causal * nq * D)
     return k.rows
 

@@ -16,6 +16,7 @@
 #include <string.h>
 
 #include "../pdl.cuh"
+#include "ops.h"
 
 namespace {
 
@@ -686,15 +687,22 @@ int tbv_op_paged_attention(const void* q, const void* k_cache, const void* v_cac
 }
 
 
-// Causal prefill over the paged cache.  tiles: int32 [ntiles, 2] = (first query row, rows <= 64 / G) with all
-// rows of a tile belonging to one sequence in position order; ctx_lens[row] = keys visible to that row.
+// Causal prefill over the paged cache.  tiles: int32 [ntiles, 2] = (first query row, rows <= tile_rows / G) with all
+// rows of a tile belonging to one sequence in position order; ctx_lens[row] = keys visible to that row.  tile_rows is 64, or up to 128 where
+// the tcgen05 kernel (attn_prefill.cu) takes the call: blocks of a multiple of 16 tokens, 16-byte aligned queries and caches, 32-byte aligned results.
 int tbv_op_prefill_attention(const void* q, const void* k_cache, const void* v_cache, const void* block_tables,
-                             const void* seq_of_query, const void* ctx_lens, const void* tiles, void* out, int ntiles,
+                             const void* seq_of_query, const void* ctx_lens, const void* tiles, void* out, int nq_rows, int ntiles, int tile_rows,
                              int nq_heads, int nkv, int head_dim, int ldq, int ldo, int block_size, int max_blocks, float scale,
                              void* stream) {
   if (ntiles <= 0) return 0;
   if (head_dim != kD || nq_heads % nkv || (ldq % 8) || block_size <= 0) return -2;
   const int G = nq_heads / nkv;
+  if (G != 1 && G != 2 && G != 4 && G != 8) return -2;
+  if (scale > 0.f && tile_rows <= 128 && !(reinterpret_cast<uintptr_t>(v_cache) & 15) && tbvops::attn_prefill_takes(q, k_cache, out, nq_heads, nkv, ldq, ldo, block_size))
+    return tbvops::attn_prefill_split(q, k_cache, v_cache, static_cast<const int*>(block_tables), static_cast<const int*>(seq_of_query),
+                                      static_cast<const int*>(ctx_lens), static_cast<const int*>(tiles), out, nq_rows, ntiles, nq_heads, nkv, ldq, ldo, block_size,
+                                      max_blocks, scale, static_cast<cudaStream_t>(stream));
+  if (tile_rows > 64) return -2;
   PrefillParams pp{};
   AttnParams& p = pp.a;
   p.q = static_cast<const __nv_bfloat16*>(q);

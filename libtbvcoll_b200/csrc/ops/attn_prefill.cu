@@ -1,0 +1,418 @@
+// attn_prefill.cu — attention of prompt rows over a paged cache on tcgen05 tensor cores, heads of 128 channels.
+//
+// A CTA owns 128 MMA rows: the query heads of one key head for up to 128 / heads-per-key-head consecutive tokens of one sequence, so that every cached
+// row is brought in once for all of them.  Scores and sums of a row sit in TMEM and one thread owns a row from end to end: no shuffles, no rescaling
+// through shared memory.  Per tile of 128 keys
+//   S = Q K^T          both operands in shared memory (TMA, 128-byte swizzle), S in 128 TMEM columns
+//   P = 2^(S - m)      warps 0 .. 3; P goes back to TMEM as bf16, over the columns of S
+//   O += P V           P from TMEM, V from shared memory with the channels contiguous
+// K and V have one buffer each: the next K is on its way while the weights are computed, the next V while the next scores are.  A CTA is a chain (product, exponentials,
+// product), so two of them share an SM (99 KB of shared memory and 256 TMEM columns each) and fill each other's gaps.
+// The running maximum is only a reference: sums are rescaled when a row's maximum grew by more than 2^8 over it (fp32 holds what lies between).
+//
+// What bounds it: 16384 exponentials per tile take 1024 clocks of the SM's exponential units (three times that with a soft cap), its two products 1024 clocks of the
+// tensor cores.  Measured (32 query heads, 8 key heads, causal; before: warp-level products, 64 rows per CTA): 8 x 512 tokens 50 us (was 128), 1 x 4096 tokens
+// 155 us (was 868; 0.56 of the tensor peak), rows that hold both 50 and 157 us (were 148 and 848); 1 x 4096, 16 heads, soft cap 50: 4 layers take 0.9 ms less.
+//
+// Two kinds of cache (template PAIR): keys and values in caches of their own, [slots, kv_heads, 128] each (k_prefill_attn_mma in attention.cu is the same for
+// blocks of any size), and rows that hold both, [blocks, kv_heads, block_size, 128 + 128 + pad], with windows, chunks, soft cap and gate (shared_attn.cu, for
+// heads of any size).
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+#include <stdio.h>
+
+#include "../pdl.cuh"
+#include "attn_mma.cuh"
+#include "ops.h"
+#include "sm100.cuh"
+#include "vec.cuh"
+
+using namespace sm100;
+
+namespace {
+
+constexpr int kD = 128, kRows = 128, kKeys = 128;
+constexpr int kHalf = 128 * 128;                   // bytes of 128 rows x 64 channels
+constexpr int kSmem = 6 * kHalf + 1024;            // Q, K, V in halves of 64 channels
+constexpr float kFloor = -1e30f;
+constexpr float kGrow = 8.f;                       // by how much (powers of two) a maximum may exceed the reference
+
+struct Params {
+  const int* tiles;          // [ntiles, 2]: first query row, rows (<= 128 / hpk); PAIR: [ntiles, 4], first row, rows (<= 64), -, keys of the first row
+  const int* seq_of_row;     // table row of a query row (null: the row itself)
+  const int* ctx_lens;       // keys visible to every row (not PAIR)
+  const int* tables;
+  __nv_bfloat16* out;        // [rows, ldo], head h at h * 128
+  const __nv_bfloat16* gate; // [rows, ldg] or null (PAIR)
+  int ntiles, kv_heads, hpk, parts, block_size, max_blocks, ldo, ldg, window, chunk;
+  float scale_log2, softcap;
+  unsigned long long limit_ns;
+  int* err;
+};
+
+struct Smem {
+  unsigned long long q_full, k_full, k_empty, v_full, v_empty, s_full, p_ready;
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, int x, int y, int z, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+               ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem]
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* f) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(f);
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+        "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+               "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// V as the right operand: channels contiguous, 64 of them per 128-byte swizzled row, a token per row; the second 64 channels kHalf bytes further
+__device__ __forceinline__ uint64_t desc_channels_contiguous(uint32_t addr) {
+  uint64_t d = 0;
+  d |= uint64_t((addr & 0x3FFFFu) >> 4);
+  d |= uint64_t(kHalf >> 4) << 16;                 // between groups of 64 channels
+  d |= uint64_t(1024 >> 4) << 32;                  // between groups of 8 tokens
+  d |= uint64_t(1) << 46;
+  d |= uint64_t(2) << 61;                          // 128-byte swizzle
+  return d;
+}
+__device__ __forceinline__ float exp2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ void st_global_32(void* p, const uint32_t* v) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+
+template <bool PAIR, bool CAP>
+__global__ void __launch_bounds__(192, 2)
+k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ Smem s;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t raw = smem_u32(smem_raw), sq = (raw + 1023u) & ~1023u, sk = sq + 2 * kHalf, sv = sk + 2 * kHalf;
+  const uint32_t bq = smem_u32(&s.q_full), bkf = smem_u32(&s.k_full), bke = smem_u32(&s.k_empty), bvf = smem_u32(&s.v_full), bve = smem_u32(&s.v_empty),
+                 bsf = smem_u32(&s.s_full), bpr = smem_u32(&s.p_ready);
+  pdl::launch_dependents();
+  if (threadIdx.x == 0) {
+    mbar_init(bq, 1); mbar_init(bkf, 1); mbar_init(bke, 1); mbar_init(bvf, 1); mbar_init(bve, 1); mbar_init(bsf, 1);
+    mbar_init(bpr, 4);                                            // one arrival per warp of weights
+    s.abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 5) {
+    tmem_alloc(smem_u32(&s.tmem_base), 256);
+    tmem_relinquish();
+  }
+  if (warp == 4 && lane == 0) {
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl::grid_dependency_wait();
+
+  // which rows: a tile of the list and a key head (PAIR: and a part of the tile)
+  const int hpk = p.hpk, per = kRows / hpk;                       // tokens per CTA
+  const int unit = blockIdx.x, head = unit % p.kv_heads, rest = unit / p.kv_heads;
+  const int tile = PAIR ? rest / p.parts : p.ntiles - 1 - rest;   // a prompt's last rows see most keys: they start first (PAIR: the list is in that order)
+  const int t0 = PAIR ? rest % p.parts * per : 0;
+  const int* tl = p.tiles + tile * (PAIR ? 4 : 2);
+  const int row0 = tl[0] + t0, nrows = min(per, tl[1] - t0);
+  const int cap = p.max_blocks * p.block_size;                    // never walk past the block table
+  const bool any = nrows > 0;
+  const int* bt = p.tables + size_t(any ? (p.seq_of_row ? p.seq_of_row[row0] : row0) : 0) * p.max_blocks;
+  // keys that the first and the last row see, and the first key that the first row sees
+  const int see_first = any ? min(PAIR ? tl[3] + t0 : p.ctx_lens[row0], cap) : 0, see_last = any ? min(PAIR ? tl[3] + t0 + nrows - 1 : p.ctx_lens[row0 + nrows - 1], cap) : 0;
+  const int j0 = PAIR ? attn_mma::first_visible(see_first, p.window, p.chunk) / kKeys : 0;
+  const int j1 = (see_last + kKeys - 1) / kKeys, n = any ? max(0, j1 - j0) : 0;
+  const uint32_t tm_s = s.tmem_base, tm_o = tm_s + 128u;
+  volatile int* abortp = &s.abort_flag;
+
+  if (warp == 4) {
+    // ---- copies: lane i takes half i & 1 of the 16 tokens i >> 1 of a tile ----
+    if (n > 0 && lane == 0) {
+      mbar_expect_tx(bq, uint32_t(2 * 128 * hpk * per));
+      tma_load_3d(sq, &tmQ, 0, head * hpk, row0, bq);
+      tma_load_3d(sq + kHalf, &tmQ, 64, head * hpk, row0, bq);
+    }
+    const int piece = lane >> 1, half = lane & 1;
+    int entry = 0;
+    bool ok = true;
+    int k_issued = 0, v_issued = 0;
+    for (int i = 0; i < n && ok; i++) {
+      const int tok = (j0 + i) * kKeys + piece * 16;
+      const int pieces = min(8, (see_last - (j0 + i) * kKeys + 15) >> 4);
+      int x = half * 64, y = 0;
+      if (piece < pieces) {
+        entry = bt[tok / p.block_size];
+        const int in = tok % p.block_size;
+        if (PAIR) y = (entry * p.kv_heads + head) * p.block_size + in;
+        else { y = entry * p.block_size + in; x += head * kD; }
+      }
+      if (i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bke, uint32_t(i - 1) & 1u, abortp, p.limit_ns));
+      if (!ok) break;
+      if (lane == 0) mbar_expect_tx(bkf, uint32_t(pieces) * 4096u);
+      __syncwarp();
+      if (piece < pieces) tma_load_2d(sk + half * kHalf + piece * 2048, &tmK, x, y, bkf);
+      k_issued = i + 1;
+      if (i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bve, uint32_t(i - 1) & 1u, abortp, p.limit_ns));
+      if (!ok) break;
+      if (lane == 0) mbar_expect_tx(bvf, uint32_t(pieces) * 4096u);
+      __syncwarp();
+      if (piece < pieces) tma_load_2d(sv + half * kHalf + piece * 2048, &tmV, PAIR ? x + kD : x, y, bvf);
+      v_issued = i + 1;
+    }
+    if (*abortp && lane == 0) {
+      // gave up: let the copies in flight land before this CTA's shared memory goes away
+      for (int spin = 0; n > 0 && spin < 20000 && !mbar_try_wait(bq, 0); spin++) __nanosleep(50);
+      if (k_issued) for (int spin = 0; spin < 20000 && !mbar_try_wait(bkf, uint32_t(k_issued - 1) & 1u); spin++) __nanosleep(50);
+      if (v_issued) for (int spin = 0; spin < 20000 && !mbar_try_wait(bvf, uint32_t(v_issued - 1) & 1u); spin++) __nanosleep(50);
+    }
+  } else if (warp == 5) {
+    if (lane == 0 && n > 0) {
+      // ---- products ----
+      const uint32_t id_s = umma_idesc_bf16(kRows, kKeys), id_o = umma_idesc_bf16(kRows, kD) | (1u << 16);   // bit 16: channels of V contiguous
+      const uint64_t qd = umma_desc_sw128(sq), kd = umma_desc_sw128(sk), vd = desc_channels_contiguous(sv);
+      bool ok = mbar_wait(bq, 0, abortp, p.limit_ns);
+      for (int i = 0; i < n && ok; i++) {
+        const uint32_t ph = uint32_t(i) & 1u;
+        // the scores replace the weights of the tile before: those must have been used (which also settles the sums before anyone rescales them)
+        if (i > 0 && !mbar_wait(bve, ph ^ 1u, abortp, p.limit_ns)) break;
+        if (!mbar_wait(bkf, ph, abortp, p.limit_ns)) break;
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < kD / 16; k++) {
+          const uint64_t off = uint64_t((k >> 2) * (kHalf >> 4) + (k & 3) * 2);
+          umma_bf16(tm_s, qd + off, kd + off, id_s, k ? 1u : 0u);
+        }
+        umma_commit(bsf);
+        umma_commit(bke);
+        if (!mbar_wait(bvf, ph, abortp, p.limit_ns)) break;
+        if (!mbar_wait(bpr, ph, abortp, p.limit_ns)) break;
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < kKeys / 16; k++) umma_bf16_ts(tm_o, tm_s + uint32_t(8 * k), vd + uint64_t(k * (2048 >> 4)), id_o, (i | k) ? 1u : 0u);
+        umma_commit(bve);
+      }
+    }
+  } else if (n > 0) {
+    // ---- weights: thread = row (token, query head) ----
+    const int r = threadIdx.x, t = r / hpk, g = r - t * hpk;
+    const bool mine = t < nrows;
+    const int see = !mine ? 0 : min(PAIR ? see_first + t : p.ctx_lens[row0 + t], cap);
+    const int lo = PAIR ? attn_mma::first_visible(see, p.window, p.chunk) : 0;
+    const int lo_last = PAIR ? attn_mma::first_visible(see_last, p.window, p.chunk) : 0;
+    const uint32_t lanes = uint32_t(warp * 32) << 16;
+    const float sc = CAP ? 1.f : p.scale_log2;
+    const float cap_a = CAP ? 2.f * attn_mma::kLog2e / p.softcap : 0.f, cap_c = p.softcap * attn_mma::kLog2e, cap_b = -2.f * cap_c;
+    float m = kFloor, l = 0.f;
+    bool ok = true;
+    for (int i = 0; i < n; i++) {
+      const uint32_t ph = uint32_t(i) & 1u;
+      const int key0 = (j0 + i) * kKeys;
+      ok = __all_sync(0xffffffffu, mbar_wait(bsf, ph, abortp, p.limit_ns));
+      if (!ok) break;
+      tc_fence_after();
+      float v[kKeys];
+#pragma unroll
+      for (int c = 0; c < kKeys; c += 32) tmem_ld32(tm_s + lanes + uint32_t(c), v + c);
+      tmem_ld_wait();
+      if (CAP) {                                                  // cap * tanh(v / cap) in powers of two, as attn_mma::capped_log2: c - 2 c / (1 + e^(2 v / cap))
+#pragma unroll
+        for (int c = 0; c < kKeys; c++) v[c] = fmaf(cap_b, rcp_ftz(1.f + exp2_ftz(v[c] * cap_a)), cap_c);
+      }
+      if (key0 + kKeys > see_first || (PAIR && key0 < lo_last)) {
+        const int hi = see - key0, first = lo - key0;
+#pragma unroll
+        for (int c = 0; c < kKeys; c++)
+          if (c >= hi || (PAIR && c < first)) v[c] = -INFINITY;
+      }
+      float x[4] = {v[0], v[1], v[2], v[3]};
+#pragma unroll
+      for (int c = 4; c < kKeys; c += 4) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) x[e] = fmaxf(x[e], v[c + e]);
+      }
+      const float mx = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])) * sc;
+      if (i == 0) {
+        m = fmaxf(mx, kFloor);
+      } else if (__any_sync(0xffffffffu, mx > m + kGrow)) {
+        // the product before is complete (the scores were issued behind it): rescale the sums in place
+        const float to = fmaxf(m, mx), f = exp2_ftz(m - to);
+        m = to;
+        l *= f;
+#pragma unroll 1
+        for (int c = 0; c < kD; c += 16) {
+          uint32_t o[16];
+          tmem_ld16(tm_o + lanes + uint32_t(c), o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; e++) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+          tmem_st16(tm_o + lanes + uint32_t(c), o);
+        }
+      }
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < kKeys; c += 32) {
+        uint32_t w[16];
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) {
+          const float a = exp2_ftz(fmaf(v[c + e], sc, -m)), b = exp2_ftz(fmaf(v[c + e + 1], sc, -m));
+          sum[e & 2] += a;
+          sum[(e & 2) + 1] += b;
+          w[e >> 1] = attn_mma::pack_bf16(a, b);
+        }
+        tmem_st16(tm_s + lanes + uint32_t(c >> 1), w);
+      }
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      if (key0 + kKeys > see_last) {
+        // cached rows behind the last visible one: a weight of zero must not meet a stale bit pattern
+        if (!__all_sync(0xffffffffu, mbar_wait(bvf, ph, abortp, p.limit_ns))) { ok = false; break; }
+        if (key0 + r >= see_last) {
+#pragma unroll
+          for (int c = 0; c < 8; c++) {
+            attn_mma::st_zero16(sv + r * 128 + c * 16);
+            attn_mma::st_zero16(sv + kHalf + r * 128 + c * 16);
+          }
+        }
+        fence_proxy_async_smem();
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bpr);
+    }
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bve, uint32_t(n - 1) & 1u, abortp, p.limit_ns));
+    if (ok) {
+      tc_fence_after();
+      const float f = l > 0.f ? 1.f / l : 0.f;
+      const size_t col = size_t(head * hpk + g) * kD;
+      __nv_bfloat16* dst = p.out + size_t(row0 + (mine ? t : 0)) * p.ldo + col;
+      const __nv_bfloat16* gate = PAIR && p.gate ? p.gate + size_t(row0 + (mine ? t : 0)) * p.ldg + col : nullptr;
+#pragma unroll 1
+      for (int c = 0; c < kD; c += 32) {
+        float o[32];
+        tmem_ld32(tm_o + lanes + uint32_t(c), o);
+        tmem_ld_wait();
+        if (mine) {
+          uint32_t w[16];
+#pragma unroll
+          for (int e = 0; e < 32; e += 8) {
+            float a[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) a[q] = o[e + q] * f;
+            if (gate) {
+              float gt[8];
+              vec::load8(gate + c + e, gt);
+#pragma unroll
+              for (int q = 0; q < 8; q++) a[q] *= vec::sigmoid<__nv_bfloat16>(gt[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q += 2) w[(e + q) >> 1] = attn_mma::pack_bf16(a[q], a[q + 1]);
+          }
+          st_global_32(dst + c, w);                // a whole sector at a time
+          st_global_32(dst + c + 16, w + 8);
+        }
+        __syncwarp();
+      }
+    }
+  } else if (any) {
+    // no visible key at all: nothing to sum
+    const int r = threadIdx.x, t = r / hpk, g = r - t * hpk;
+    if (t < nrows)
+      for (int c = 0; c < kD; c += 8) *reinterpret_cast<uint4*>(p.out + size_t(row0 + t) * p.ldo + size_t(head * hpk + g) * kD + c) = make_uint4(0, 0, 0, 0);
+  }
+
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 5) {
+    tc_fence_after();
+    tmem_dealloc(s.tmem_base, 256);
+  }
+  if (threadIdx.x == 0 && s.abort_flag && p.err) atomicExch(p.err, 1);
+}
+
+template <bool PAIR, bool CAP>
+cudaError_t launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const Params& p, cudaStream_t st) {
+  static const cudaError_t attr = cudaFuncSetAttribute(k_attn_prefill<PAIR, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  if (attr != cudaSuccess) return attr;
+  return pdl::launch(k_attn_prefill<PAIR, CAP>, dim3(unsigned(p.ntiles) * p.parts * p.kv_heads), dim3(192), kSmem, st, 1, q, k, v, p);
+}
+
+int report(cudaError_t e) {
+  if (e != cudaSuccess) fprintf(stderr, "[tbvops] prompt attention launch failed: %s\n", cudaGetErrorString(e));
+  return e == cudaSuccess ? 0 : -1;
+}
+
+// largest number of cached rows that an index can name: blocks come from the block table, so this is no check of what exists
+constexpr unsigned long long kAnyRows = 0x7fffffffull;
+
+}  // namespace
+
+namespace tbvops {
+
+bool attn_prefill_takes(const void* q, const void* kv, const void* out, int heads, int kv_heads, int ldq, int ldo, int block_size) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kv);
+  return heads / kv_heads <= kRows && !(at & 15) && !(reinterpret_cast<uintptr_t>(out) & 31) && !(ldq % 8) && !(ldo % 16) && block_size % 16 == 0;
+}
+
+int attn_prefill_split(const void* q, const void* k_cache, const void* v_cache, const int* tables, const int* seq_of_row, const int* ctx_lens, const int* tiles,
+                       void* out, int rows, int ntiles, int heads, int kv_heads, int ldq, int ldo, int block_size, int max_blocks, float scale, cudaStream_t st) {
+  Params p{};
+  p.tiles = tiles; p.seq_of_row = seq_of_row; p.ctx_lens = ctx_lens; p.tables = tables; p.out = static_cast<__nv_bfloat16*>(out);
+  p.ntiles = ntiles; p.kv_heads = kv_heads; p.hpk = heads / kv_heads; p.parts = 1; p.block_size = block_size; p.max_blocks = max_blocks; p.ldo = ldo;
+  p.scale_log2 = scale * attn_mma::kLog2e; p.limit_ns = 2000000000ull; p.err = gemm_err_flag();
+  CUtensorMap mq, mk, mv;
+  const unsigned long long width = (unsigned long long)kv_heads * kD;
+  if (make_tensor_map_heads(&mq, q, rows, heads, kD, ldq, p.hpk, kRows / p.hpk) != 0 || make_tensor_map_bf16(&mk, k_cache, kAnyRows, width, width, 16) != 0 ||
+      make_tensor_map_bf16(&mv, v_cache, kAnyRows, width, width, 16) != 0) return -3;
+  return report(launch<false, false>(mq, mk, mv, p, st));
+}
+
+int attn_prefill_paired(const void* q, const void* cache, const int* tables, const int* seq_of_row, const int* tiles, const void* gate, void* out, int rows,
+                        int ntiles, int heads, int kv_heads, int ldq, int ldo, int ldg, int row_len, int block_size, int max_blocks, float softcap, int window, int chunk,
+                        cudaStream_t st) {
+  Params p{};
+  p.tiles = tiles; p.seq_of_row = seq_of_row; p.tables = tables; p.out = static_cast<__nv_bfloat16*>(out); p.gate = static_cast<const __nv_bfloat16*>(gate);
+  p.ntiles = ntiles; p.kv_heads = kv_heads; p.hpk = heads / kv_heads; p.block_size = block_size; p.max_blocks = max_blocks; p.ldo = ldo; p.ldg = ldg;
+  p.parts = (64 + kRows / p.hpk - 1) / (kRows / p.hpk);
+  p.window = window; p.chunk = chunk; p.softcap = softcap;
+  p.scale_log2 = attn_mma::kLog2e; p.limit_ns = 2000000000ull; p.err = gemm_err_flag();
+  CUtensorMap mq, mk;
+  if (make_tensor_map_heads(&mq, q, rows, heads, kD, ldq, p.hpk, kRows / p.hpk) != 0 || make_tensor_map_bf16(&mk, cache, kAnyRows, 2 * kD, row_len, 16) != 0) return -3;
+  return report(softcap > 0.f ? launch<true, true>(mq, mk, mk, p, st) : launch<true, false>(mq, mk, mk, p, st));
+}
+
+}  // namespace tbvops

@@ -303,6 +303,17 @@ int make_tensor_map_bf16(CUtensorMap* out, const void* ptr, unsigned long long r
   return 0;
 }
 
+// Heads of `dim` channels side by side, [rows, ld] with head h at h * dim; box = 64 channels x box_heads x box_rows, 128-byte swizzle.
+int make_tensor_map_heads(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned heads, unsigned dim, unsigned long long ld, unsigned box_heads,
+                          unsigned box_rows) {
+  CUtensorMap plain;
+  if (make_tensor_map_bf16(&plain, ptr, rows, (unsigned long long)heads * dim, ld, 1) != 0) return -1;   // also looks up the encoder and checks the alignment
+  const cuuint64_t dims[3] = {dim, heads, rows}, strides[2] = {dim * 2ull, ld * 2ull};
+  const cuuint32_t box[3] = {64, box_heads, box_rows}, estr[3] = {1, 1, 1};
+  return g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -3;
+}
+
 // ---- weights of the GEMM that follows, to be asked into L2 by the kernel launched next ------------------------------
 namespace {
 thread_local const char* t_pf_ptr = nullptr;

@@ -8,6 +8,8 @@ namespace gemm { struct Params; }
 namespace tbvops {
 int make_tensor_map_bf16(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned long long cols,
                          unsigned long long ld, unsigned box_rows, bool cache = true);
+int make_tensor_map_heads(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned heads, unsigned dim, unsigned long long ld, unsigned box_heads,
+                          unsigned box_rows);
 int* gemm_err_flag();
 // The weights announced by tbv_op_gemm_prefetch_next for the next GEMM launch of this host thread: returns the byte count
 // (0 = none or `own_bytes`, the launch's own weight matrix, too small to give cover; capped by TBV_L2_PREFETCH_MB) and forgets
@@ -36,6 +38,13 @@ int shared_attn_rows_any(const void* qa, const void* cache, const int* tables, c
 int paired_attn_rows_any(const void* qa, const void* cache, const int* tables, const int* seq_of_row, const int* ctx_lens, const void* gate, void* out, int rows,
                          int heads, int kv_heads, int Dp, int Vp, int ldg, int block_size, int max_blocks, int splits, float softcap, int window, int chunk, int bf16,
                          cudaStream_t st);
+// attention of prompt rows on tcgen05, heads of 128 channels (attn_prefill.cu): keys and values in caches of their own, or side by side in cached rows
+bool attn_prefill_takes(const void* q, const void* kv, const void* out, int heads, int kv_heads, int ldq, int ldo, int block_size);
+int attn_prefill_split(const void* q, const void* k_cache, const void* v_cache, const int* tables, const int* seq_of_row, const int* ctx_lens, const int* tiles,
+                       void* out, int rows, int ntiles, int heads, int kv_heads, int ldq, int ldo, int block_size, int max_blocks, float scale, cudaStream_t st);
+int attn_prefill_paired(const void* q, const void* cache, const int* tables, const int* seq_of_row, const int* tiles, const void* gate, void* out, int rows,
+                        int ntiles, int heads, int kv_heads, int ldq, int ldo, int ldg, int row_len, int block_size, int max_blocks, float softcap, int window, int chunk,
+                        cudaStream_t st);
 // threads per CTA for the row-normalisation kernels; the fused collective uses the same
 // mapping so that both produce identical bits
 inline int norm_threads(int hidden) {

@@ -881,11 +881,15 @@ int tbv_op_paired_prefill_fits(int Dp, int Vp) { return Vp <= 256 && size_t(64) 
 
 // bf16; q [rows, ldq] with head h at h * Dp, out [rows, ldo] with head h at h * Vp
 int tbv_op_paired_attn_prefill(const void* q, const void* cache, const void* tables, const void* seq_of_row, const void* tiles, const void* gate, void* out,
-                               int ntiles, int ldq, int ldo, int heads, int kv_heads, int Dp, int Vp, int ldg, int block_size, int max_blocks, float softcap, int window,
+                               int rows, int ntiles, int ldq, int ldo, int heads, int kv_heads, int Dp, int Vp, int ldg, int block_size, int max_blocks, float softcap, int window,
                                int chunk, void* stream) {
   if (ntiles <= 0) return 0;
   if ((Dp % 16) || (Vp % 16) || (ldq % 8) || (ldo % 8) || kv_heads <= 0 || heads % kv_heads || ntiles > 65535 || !seq_of_row || (gate && (ldg % 8)) || window < 0 || chunk < 0 ||
       !tbv_op_paired_prefill_fits(Dp, Vp)) return -2;
+  if (Dp == 128 && Vp == 128 && tbvops::attn_prefill_takes(q, cache, out, heads, kv_heads, ldq, ldo, block_size) && !(reinterpret_cast<uintptr_t>(gate) & 15))
+    return tbvops::attn_prefill_paired(q, cache, static_cast<const int*>(tables), static_cast<const int*>(seq_of_row), static_cast<const int*>(tiles), gate, out, rows,
+                                       ntiles, heads, kv_heads, ldq, ldo, ldg, Dp + Vp + kRowPad, block_size, max_blocks, softcap, window, chunk,
+                                       static_cast<cudaStream_t>(stream));
   PrefillParams p{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(cache), static_cast<__nv_bfloat16*>(out),
                   static_cast<const int*>(tiles), static_cast<const int*>(seq_of_row), static_cast<const int*>(tables),
                   ldq, ldo, heads, kv_heads, Dp, Vp, block_size, max_blocks, softcap, window, chunk, static_cast<const __nv_bfloat16*>(gate), ldg};

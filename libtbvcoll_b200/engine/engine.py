@@ -198,7 +198,7 @@ class Engine:
                 if m.expands_context:
                     b.dense_slots = put(hb.dense_slots, np.int64)
         elif self.tiled_prefill_attention:
-            b.tiles = ops.prefill_tiles(torch.from_numpy(hb.seq.astype(np.int32)), m.nq // m.nkv).to(dev)
+            b.tiles = ops.prefill_tiles(torch.from_numpy(hb.seq.astype(np.int32)), m.nq // m.nkv, ops.prefill_tile_rows(self.block_size)).to(dev)
         return b
 
     # ---- one mixed step ---------------------------------------------------------------------------

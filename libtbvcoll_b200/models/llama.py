@@ -147,7 +147,7 @@ class LlamaTP:
                               self.nq, self.nkv, bias=w.get(p + "qkv.bias"))
             if prefill_tiles is not None:
                 ops.prefill_attention(q_view, self.k_cache[l], self.v_cache[l], block_tables, ctx_lens, seq_of_query, prefill_tiles,
-                                      attn_view, self.scale, self.block_size)
+                                      attn_view, self.scale, self.block_size, ops.prefill_tile_rows(self.block_size))
             else:
                 ops.paged_attention(q_view, self.k_cache[l], self.v_cache[l], block_tables, ctx_lens, attn_view, self.scale,
                                     self.block_size, seq_of_query=seq_of_query, splits=attn_splits, workspace=self.attn_ws)
@@ -212,7 +212,7 @@ class LlamaTP:
             ops.rope_kv(qkv, positions, self.cos_sin, slot_mapping, self.k_cache[l], self.v_cache[l], self.nq, self.nkv, self.D)
             if prefill_tiles is not None:
                 ops.prefill_attention(q_view, self.k_cache[l], self.v_cache[l], block_tables, ctx_lens, seq_of_query, prefill_tiles,
-                                      attn_view, self.scale, self.block_size)
+                                      attn_view, self.scale, self.block_size, ops.prefill_tile_rows(self.block_size))
             else:
                 ops.paged_attention(q_view, self.k_cache[l], self.v_cache[l], block_tables, ctx_lens, attn_view, self.scale,
                                     self.block_size, seq_of_query=seq_of_query, splits=1)

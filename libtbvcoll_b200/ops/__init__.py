@@ -45,7 +45,7 @@ def lib():
     l.tbv_op_fixed_decay_sums.argtypes = [I, I, I]
     l.tbv_op_paired_attn_prep.argtypes = [c_vp] * 8 + [I] * 10 + [F, I, c_vp]
     l.tbv_op_paired_attn_rows.argtypes = [c_vp] * 7 + [I] * 9 + [F, I, I, I, c_vp]
-    l.tbv_op_paired_attn_prefill.argtypes = [c_vp] * 7 + [I] * 10 + [F, I, I, c_vp]
+    l.tbv_op_paired_attn_prefill.argtypes = [c_vp] * 7 + [I] * 11 + [F, I, I, c_vp]
     l.tbv_op_paired_prefill_fits.argtypes = [I, I]
     l.tbv_op_decay_scan.argtypes = [c_vp] * 15 + [I, I, c_vp, c_vp, c_vp, c_vp, c_vp] + [I] * 12 + [F, F, F, I, c_vp]
     l.tbv_op_decay_step.argtypes = [c_vp] * 13 + [I] * 9 + [F, F, F, I, c_vp]
@@ -92,7 +92,7 @@ def lib():
     l.tbv_op_gemm_prefetch_next.restype = None
     l.tbv_op_copy_async.argtypes = [c_vp, c_vp, ctypes.c_size_t, c_vp]
     l.tbv_op_copy_async.restype = I
-    l.tbv_op_prefill_attention.argtypes = [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, I, I, I, I, I, I, I, I, F, c_vp]
+    l.tbv_op_prefill_attention.argtypes = [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, I, I, I, I, I, I, I, I, I, I, F, c_vp]
     l.tbv_op_prefill_attention.restype = I
     l.tbv_op_attn_workspace.argtypes = [I, I, I, I]
     l.tbv_op_attn_workspace.restype = SZ
@@ -421,13 +421,19 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     return out
 
 
-def prefill_tiles(seq_of_row, group: int) -> torch.Tensor:
-    """Segments of at most 64 // group consecutive query rows that belong to one sequence, as the
+def prefill_tile_rows(block_size: int) -> int:
+    """(token, head) rows that a tile of ``prefill_attention`` may have: the tcgen05 kernel multiplies 128 at a time, the other form, which takes blocks of
+    any size, 64."""
+    return 128 if block_size % 16 == 0 else 64
+
+
+def prefill_tiles(seq_of_row, group: int, rows: int = 64) -> torch.Tensor:
+    """Segments of at most ``rows`` // group consecutive query rows that belong to one sequence, as the
     int32 [ntiles, 2] (first row, count) list ``prefill_attention`` takes.  ``seq_of_row``: host
     sequence (list / CPU tensor) giving the sequence of every query row, rows grouped by sequence
     in position order."""
     import numpy as np
-    qt = max(1, 64 // group)
+    qt = max(1, rows // group)
     seqs = np.asarray(seq_of_row.numpy() if hasattr(seq_of_row, "numpy") else list(seq_of_row), dtype=np.int64)
     n = int(seqs.size)
     if n == 0:
@@ -443,15 +449,15 @@ def prefill_tiles(seq_of_row, group: int) -> torch.Tensor:
 
 
 def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_tables: torch.Tensor, ctx_lens: torch.Tensor,
-                      seq_of_query: torch.Tensor, tiles: torch.Tensor, out: torch.Tensor, scale: float, block_size: int) -> torch.Tensor:
+                      seq_of_query: torch.Tensor, tiles: torch.Tensor, out: torch.Tensor, scale: float, block_size: int, tile_rows: int = 64) -> torch.Tensor:
     """Causal attention of prompt rows over the paged cache with query tiling on tensor cores: up to
-    64 (token, head) rows share every K/V tile.  Same arguments as ``paged_attention`` plus ``tiles``
-    (device int32 [ntiles, 2] from ``prefill_tiles``)."""
+    ``tile_rows`` (token, head) rows share every K/V tile.  Same arguments as ``paged_attention`` plus ``tiles``
+    (device int32 [ntiles, 2] from ``prefill_tiles``) and the ``tile_rows`` they were made for (``prefill_tile_rows`` or less)."""
     Nq, nq, D = q.shape
     nkv = k_cache.shape[-2]
     assert q.stride(2) == 1 and q.stride(1) == D and out.stride(2) == 1 and out.stride(1) == D and tiles.dtype is torch.int32
     _chk(lib().tbv_op_prefill_attention(_p(q), _p(k_cache), _p(v_cache), _p(block_tables), _p(seq_of_query), _p(ctx_lens), _p(tiles),
-                                        _p(out), tiles.shape[0], nq, nkv, D, q.stride(0), out.stride(0), block_size,
+                                        _p(out), Nq, tiles.shape[0], tile_rows, nq, nkv, D, q.stride(0), out.stride(0), block_size,
                                         block_tables.shape[1], scale, _st()), "tbv_op_prefill_attention")
     _count()
     return out

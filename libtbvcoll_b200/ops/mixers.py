@@ -432,7 +432,7 @@ def paired_attention_prefill(q, cache, tables, seq_of_row, tiles, out, heads: in
     Vp = cache.shape[1] - LATENT_ROW_PAD - dim_p
     assert q.dtype is cache.dtype is out.dtype is torch.bfloat16 and tiles.dtype is torch.int32 and seq_of_row.dtype is torch.int32 and out.shape[1] >= heads * Vp
     assert gate is None or (gate.dtype is q.dtype and gate.shape == (q.shape[0], heads * Vp) and gate.stride(1) == 1)
-    _chk(lib().tbv_op_paired_attn_prefill(_p(q), _p(cache), _p(tables), _p(seq_of_row), _p(tiles), _p(gate), _p(out), tiles.shape[0], q.stride(0), out.stride(0), heads,
+    _chk(lib().tbv_op_paired_attn_prefill(_p(q), _p(cache), _p(tables), _p(seq_of_row), _p(tiles), _p(gate), _p(out), q.shape[0], tiles.shape[0], q.stride(0), out.stride(0), heads,
                                           kv_heads, dim_p, Vp, 0 if gate is None else gate.stride(0), block_size, tables.shape[1], softcap, window, chunk, _st()),
          "tbv_op_paired_attn_prefill")
     _count()

@@ -1,0 +1,141 @@
+"""Attention of prompt rows on tcgen05 (attn_prefill.cu): both kinds of cache against a plain float64 statement, at the edges of its tiles."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+D = 128
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from libtbvcoll_b200 import ops as o
+    return o
+
+
+def rnd(*shape, seed, scale=1.0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return (torch.randn(shape, generator=g, device=DEV) * scale).to(torch.bfloat16)
+
+
+def plain(q, k, v, scale, see, first, cap=0.0):
+    """q [T, H, D], k / v [n, G, D]; row t sees keys first[t] .. see[t] - 1.  Returns the result and the same sum over |v|, which bounds what rounding can do."""
+    T, H = q.shape[:2]
+    rep = H // k.shape[1]
+    q, k, v = q.double(), k.double().repeat_interleave(rep, 1), v.double().repeat_interleave(rep, 1)
+    s = torch.einsum("ihd,jhd->hij", q, k) * scale
+    if cap:
+        s = cap * torch.tanh(s / cap)
+    j = torch.arange(k.shape[0], device=DEV)[None]
+    s = s.masked_fill((j >= see[:, None]) | (j < first[:, None]), float("-inf"))
+    p = torch.softmax(s, -1)
+    return torch.einsum("hij,jhd->ihd", p, v), torch.einsum("hij,jhd->ihd", p, v.abs())
+
+
+def check(got, want, size):
+    # bf16 has 8 significant bits: weights rounded by up to 2^-8 of each, the result by 2^-8, together 2^-7 of the sum over |v|; fp32 sums, scores (below 2^5: they move a
+    # weight by 2^-18) and the approximate exponential are far below
+    assert torch.isfinite(got).all()
+    assert ((got.double() - want).abs() <= size * 2.0 ** -6.95 + 1e-6).all()
+
+
+def layout(lens, starts, bs, seed):
+    """Block tables over shuffled blocks; rows beyond a sequence's last token hold NaN patterns in the caches made by the tests."""
+    need = [(s + n + bs - 1) // bs for n, s in zip(lens, starts)]
+    perm = torch.randperm(sum(need) + 3, generator=torch.Generator().manual_seed(seed)) + 0
+    tables, at = torch.zeros(len(lens), max(need) + 1, dtype=torch.int32), 0
+    for i, n in enumerate(need):
+        tables[i, :n] = perm[at: at + n].to(torch.int32)
+        at += n
+    return tables, sum(need) + 3
+
+
+LENS, STARTS = [129, 1, 31, 128, 300, 33], [0, 127, 128, 129, 5, 700]
+
+
+@pytest.mark.parametrize("nq,nkv,bs,tile_rows", [(8, 2, 16, 128), (8, 2, 16, 64), (4, 4, 48, 128), (8, 1, 32, 128), (4, 2, 16, 100)])
+def test_split_caches(ops, nq, nkv, bs, tile_rows):
+    tables, nblocks = layout(LENS, STARTS, bs, 1)
+    kc, vc = rnd(nblocks * bs, nkv, D, seed=1), rnd(nblocks * bs, nkv, D, seed=2)
+    written = torch.zeros(nblocks * bs, dtype=torch.bool)
+    slots = []
+    for i, (n, s) in enumerate(zip(LENS, STARTS)):
+        pos = torch.arange(n + s)
+        slots.append(tables[i, pos // bs].long() * bs + pos % bs)
+        written[slots[-1]] = True
+    kc[~written.to(DEV)] = float("nan")                     # what nobody wrote must not matter
+    vc[~written.to(DEV)] = float("nan")
+    seqof = torch.tensor(sum(([i] * n for i, n in enumerate(LENS)), []), dtype=torch.int32)
+    ctx = torch.tensor(sum(([s + t + 1 for t in range(n)] for n, s in zip(LENS, STARTS)), []), dtype=torch.int32)
+    T, scale = int(seqof.numel()), 0.2
+    wide = rnd(T, (nq + 2 * nkv) * D, seed=3)
+    q = wide.view(T, -1, D)[:, :nq]                          # as in the model: a view into the projection
+    out = torch.full((T, nq, D), 7.0, dtype=torch.bfloat16, device=DEV)
+    tiles = ops.prefill_tiles(seqof, nq // nkv, tile_rows)
+    assert ops.prefill_tile_rows(bs) == 128
+    ops.prefill_attention(q, kc, vc, tables.to(DEV), ctx.to(DEV), seqof.to(DEV), tiles.to(DEV), out, scale, bs, tile_rows)
+    torch.cuda.synchronize()
+    assert not ops.gemm_error()
+    r0 = 0
+    for i, (n, s) in enumerate(zip(LENS, STARTS)):
+        rows = slots[i].to(DEV)
+        see = torch.arange(s + 1, s + n + 1, device=DEV)
+        check(out[r0: r0 + n], *plain(q[r0: r0 + n], kc[rows], vc[rows], scale, see, torch.zeros_like(see)))
+        r0 += n
+
+
+def test_growing_and_huge_scores(ops):
+    """Keys whose scores grow by more than the rescaling threshold from tile to tile, fall again, and single keys that take all of the weight."""
+    n, bs = 700, 16
+    q, kc, vc = rnd(n, 4, D, seed=5), rnd(n + 16, 1, D, seed=6), rnd(n + 16, 1, D, seed=7)
+    size = torch.ones(n + 16, device=DEV)
+    size[128:256], size[256:384], size[500], size[640:] = 3.0, 0.01, 20.0, 6.0
+    kc = (kc.float() * size[:, None, None]).to(torch.bfloat16)
+    tables = torch.arange(n // bs + 1, dtype=torch.int32)[None].to(DEV)
+    see = torch.arange(1, n + 1, device=DEV)
+    seq = torch.zeros(n, dtype=torch.int32)
+    out = torch.empty_like(q)
+    ops.prefill_attention(q, kc, vc, tables, see.to(torch.int32), seq.to(DEV), ops.prefill_tiles(seq, 4, 128).to(DEV), out, 0.3, bs, 128)
+    want, size = plain(q, kc[:n], vc[:n], 0.3, see, torch.zeros_like(see))
+    assert torch.isfinite(out).all() and not ops.gemm_error()
+    # scores reach 2^9: their 24 bits (and the product with the scale) move a weight by up to 2^-12
+    assert ((out.double() - want).abs() <= size * 2.0 ** -6.8 + 1e-6).all()
+
+
+@pytest.mark.parametrize("H,G,window,chunk,cap,gated", [(8, 2, 0, 0, 0.0, False), (4, 4, 130, 0, 0.0, True), (8, 1, 0, 200, 20.0, False), (12, 2, 1, 0, 50.0, True),
+                                                        (20, 1, 128, 0, 0.0, False)])
+def test_paired_rows(ops, H, G, window, chunk, cap, gated):
+    bs = 16
+    tables, nblocks = layout(LENS, STARTS, bs, 2)
+    row = 2 * D + 8
+    cache = rnd(nblocks * G * bs, row, seed=11)
+    at = []
+    written = torch.zeros(nblocks * G * bs, dtype=torch.bool)
+    for i, (n, s) in enumerate(zip(LENS, STARTS)):
+        pos = torch.arange(n + s)
+        at.append(((tables[i, pos // bs].long() * G)[:, None] + torch.arange(G)[None]) * bs + (pos % bs)[:, None])        # [tokens, G]
+        written[at[-1].reshape(-1)] = True
+    cache[~written.to(DEV)] = float("nan")
+    seqof = torch.tensor(sum(([i] * n for i, n in enumerate(LENS)), []), dtype=torch.int32)
+    T = int(seqof.numel())
+    q, gate = rnd(T, H * D + 64, seed=12, scale=0.3), rnd(T, H * D, seed=13)
+    tiles, r0 = [], 0
+    for n, s in zip(LENS, STARTS):
+        tiles += [(r0 + k, min(64, n - k), 0, s + k + 1) for k in range(0, n, 64)]
+        r0 += n
+    tiles = torch.tensor(tiles, dtype=torch.int32, device=DEV)
+    out = torch.full((T, H * D), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.paired_attention_prefill(q, cache, tables.to(DEV), seqof.to(DEV), tiles, out, H, G, D, bs, cap, window, chunk, gate if gated else None)
+    torch.cuda.synchronize()
+    assert not ops.gemm_error()
+    r0 = 0
+    for i, (n, s) in enumerate(zip(LENS, STARTS)):
+        kv = cache[at[i].to(DEV)]                             # [tokens, G, row]
+        see = torch.arange(s + 1, s + n + 1, device=DEV)
+        first = (see - window).clamp(min=0) if window else (see - 1) // chunk * chunk if chunk else torch.zeros_like(see)
+        want, size = plain(q[r0: r0 + n, : H * D].view(n, H, D), kv[..., :D], kv[..., D: 2 * D], 1.0, see, first, cap)
+        if gated:
+            f = torch.sigmoid(gate[r0: r0 + n].double()).view(n, H, D)
+            want, size = want * f, size * f
+        check(out[r0: r0 + n].view(n, H, D), want, size)
+        r0 += n
