@@ -121,7 +121,6 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   const uint32_t raw = smem_u32(smem_raw), sq = (raw + 1023u) & ~1023u, sk = sq + 2 * kHalf, sv = sk + 2 * kHalf;
   const uint32_t bq = smem_u32(&s.q_full), bkf = smem_u32(&s.k_full), bke = smem_u32(&s.k_empty), bvf = smem_u32(&s.v_full), bve = smem_u32(&s.v_empty),
                  bsf = smem_u32(&s.s_full), bpr = smem_u32(&s.p_ready);
-  pdl::launch_dependents();
   if (threadIdx.x == 0) {
     mbar_init(bq, 1); mbar_init(bkf, 1); mbar_init(bke, 1); mbar_init(bvf, 1); mbar_init(bve, 1); mbar_init(bsf, 1);
     mbar_init(bpr, 4);                                            // one arrival per warp of weights
@@ -140,6 +139,7 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl::launch_dependents();          // behind the allocation: a CTA of the next kernel must not hold TMEM that this one waits for
   pdl::grid_dependency_wait();
 
   // which rows: a tile of the list and a key head (PAIR: and a part of the tile)
