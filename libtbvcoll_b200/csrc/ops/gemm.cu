@@ -394,6 +394,13 @@ void gemm_config(int M, int N, int K, int splits_hint, int* bn_out, int* splits_
 
 }  // namespace tbvops
 
+int tbvops::gemm_persist_mode() {
+  // TBV_GEMM_PERSIST: 0 = never, 1 (default) = where it is estimated to be faster, 2 / 3 = its 128- / 256-token tile
+  // wherever the shape allows; read once, not per launch.
+  if (g_persist_mode == -1) { const char* pe = getenv("TBV_GEMM_PERSIST"); g_persist_mode = pe ? atoi(pe) : 1; }
+  return g_persist_mode;
+}
+
 namespace {
 // Decode-form launch of a filled Params (M, N, K, ldy, output pointers, epilogue arguments, groups).
 int launch_decode_form(const void* w, const void* x, int ldx, Params& p, int epi, int splits_hint, cudaStream_t st) {
@@ -445,12 +452,6 @@ int launch_decode_form(const void* w, const void* x, int ldx, Params& p, int epi
   }
   return 0;
 }
-int persist_mode() {
-  // TBV_GEMM_PERSIST: 0 = never, 1 (default) = where it is estimated to be faster, 2 / 3 = its 128- / 256-token tile
-  // wherever the shape allows; read once, not per launch.
-  if (g_persist_mode == -1) { const char* pe = getenv("TBV_GEMM_PERSIST"); g_persist_mode = pe ? atoi(pe) : 1; }
-  return g_persist_mode;
-}
 }  // namespace
 
 extern "C" {
@@ -470,7 +471,7 @@ int tbv_op_gemm(const void* w, const void* x, void* y, const void* bias, int M, 
   if (M <= 0 || N <= 0 || K <= 0 || (K % 8) || (ldx % 8) || (ldy % 8) || (reinterpret_cast<uintptr_t>(y) & 15u)) return -2;
   if (epi == kEpiSiluMul && (M % 2)) return -2;
   // Hundreds of tokens: the persistent kernel with tokens on the UMMA M axis.
-  const int persist = persist_mode();
+  const int persist = tbvops::gemm_persist_mode();
   if (persist > 0 && splits_hint <= 0) {
     const int th = w_not_constant ? 0 : tbvops::gemm_tok_choose(M, N, K, ldy, epi, persist);   // the many-token kernel always prefetches w
     if (th > 0) return tbvops::gemm_tok_launch(w, x, y, bias, M, N, K, ldx, ldy, epi, th, stream);
@@ -511,8 +512,8 @@ int tbv_op_gemm_ex(const void* w, const void* x, void* y, void* y2, const void* 
   p.pf_ptr = pf_ptr;
   p.pf_bytes = pf_bytes;
   p.groups = groups > 1 ? groups : 1; p.x_group = groups > 1 ? x_group : 0; p.y_group = groups > 1 ? y_group : 0;
-  if (groups <= 1 && persist_mode() > 0 && !(reinterpret_cast<uintptr_t>(y) & 31u)) {   // its fp32 stores are 32 bytes wide
-    const int th = tbvops::gemm_tok_choose(M, N, K, ldy, epi, persist_mode());
+  if (groups <= 1 && tbvops::gemm_persist_mode() > 0 && !(reinterpret_cast<uintptr_t>(y) & 31u)) {   // its fp32 stores are 32 bytes wide
+    const int th = tbvops::gemm_tok_choose(M, N, K, ldy, epi, tbvops::gemm_persist_mode());
     if (th > 0) return tbvops::gemm_tok_launch_p(w, x, p, ldx, epi, th, stream);
   }
   return launch_decode_form(w, x, ldx, p, epi, 0, static_cast<cudaStream_t>(stream));
@@ -529,7 +530,7 @@ int tbv_op_gemm_rows(const void* w, const void* x, void* y, const void* row_off,
   p.y = static_cast<__nv_bfloat16*>(y);
   p.act_a = act_a; p.act_b = act_b; p.act_c = act_c;
   p.groups = groups; p.row_off = static_cast<const int*>(row_off); p.x_rows = x_rows;
-  const int th = persist_mode() > 0 ? tbvops::gemm_tok_rows_choose(M, x_rows, groups) : 0;
+  const int th = tbvops::gemm_persist_mode() > 0 ? tbvops::gemm_tok_rows_choose(M, x_rows, groups) : 0;
   if (th > 0) return tbvops::gemm_tok_launch_p(w, x, p, ldx, epi, th, stream);
   return launch_decode_form(w, x, ldx, p, epi, 0, static_cast<cudaStream_t>(stream));
 }

@@ -24,6 +24,21 @@ constexpr int kMaxStages = 8;
 constexpr int kThreads = 192;   // warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
 constexpr int kATileBytes = kBM * kBK * 2;
 
+// Rotation and cache write behind a qkv projection (gemm_qkv.cu; kEpiRope of the many-token kernel): feature tile h * 128 is head h, queries first, then keys, then values.
+struct Rope {
+  const int* positions;            // [N]
+  const float* cos_sin;            // [max_pos, 128]: cos(0..63), sin(0..63)
+  const long long* slot_mapping;   // [N] cache row per token (< 0: skip) or null
+  __nv_bfloat16* k_cache;          // [slots, nkv, 128]
+  __nv_bfloat16* v_cache;
+  int nq, nkv, max_pos;
+};
+__device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+__device__ __forceinline__ void rotate(float x1, float x2, float c, float s, float& o1, float& o2) {   // HF rotate_half in bf16 arithmetic
+  o1 = bfr(bfr(x1 * c) + bfr(-x2 * s));
+  o2 = bfr(bfr(x2 * c) + bfr(x1 * s));
+}
+
 struct Params {
   int M, N, K;
   int ldy;             // output row stride in elements
@@ -51,11 +66,12 @@ struct Params {
   int x_rows;
   unsigned long long limit_ns;  // bound on every barrier wait
   int* err;                     // device flag: set to 1 if a wait gave up
+  Rope rope;                    // kEpiRope only
   const char* pf_ptr;           // weights of the GEMM that runs next (or null): see the producer's last step
   unsigned long long pf_bytes;  // how much of them to ask into L2 (a multiple of 16), shared out over the CTAs
 };
 
-enum Epi : int { kEpiStore = 0, kEpiSiluMul = 1, kEpiF32 = 2, kEpiClampGlu = 3 };
+enum Epi : int { kEpiStore = 0, kEpiSiluMul = 1, kEpiF32 = 2, kEpiClampGlu = 3, kEpiRope = 4 };   // the last in the many-token kernel only
 enum Act : int { kActNone = 0, kActSoftplus = 1, kActSoftcap = 2, kActSilu = 3, kActGelu = 4 };
 
 // tanh form of gelu: v / 2 * (1 + tanh(s / 2)) = v * sigmoid(s), s = 2 sqrt(2 / pi) (v + 0.044715 v^3)

@@ -66,7 +66,7 @@ struct RowGroups {
 
 // first token row, end of the rows, first feature and its weight row of a tile
 struct At { int n0, nend, f0, w0; };
-template <bool ROWS, int TOK, typename G>
+template <bool ROWS, int TOK, int FEAT, typename G>
 __device__ __forceinline__ At find_tile(const G& groups, int tile, int tok_tiles, int ngroups, int M, int N) {
   if constexpr (ROWS) {
     int lo = 0, hi = ngroups - 1;                  // the last group whose first tile is not beyond `tile`; empty groups are passed over
@@ -76,12 +76,33 @@ __device__ __forceinline__ At find_tile(const G& groups, int tile, int tok_tiles
       else hi = mid - 1;
     }
     const int local = tile - groups.tile[lo], tt = (groups.off[lo + 1] - groups.off[lo] + TOK - 1) / TOK;
-    const int f0 = local / tt * kFeatTile;
+    const int f0 = local / tt * FEAT;
     return At{groups.off[lo] + local % tt * TOK, groups.off[lo + 1], f0, lo * M + f0};
   } else {
-    const int f0 = tile / tok_tiles * kFeatTile;
+    const int f0 = tile / tok_tiles * FEAT;
     return At{tile % tok_tiles * TOK, N, f0, f0};
   }
+}
+
+// Fills the table from the rows' offsets (device memory); whole CTA.
+__device__ __forceinline__ void count_tiles(RowGroups& groups, const gemm::Params& p, int tok, int feat_tiles, int threads) {
+  for (int g = threadIdx.x; g <= p.groups; g += threads) groups.off[g] = p.row_off[g];
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x, per = (p.groups + 31) / 32, a = min(p.groups, lane * per), b = min(p.groups, a + per);
+    auto count = [&](int g) { return (groups.off[g + 1] - groups.off[g] + tok - 1) / tok * feat_tiles; };
+    int sum = 0;
+    for (int g = a; g < b; g++) sum += count(g);
+    int inc = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    int run = inc - sum;
+    for (int g = a; g < b; g++) { groups.tile[g] = run; run += count(g); }
+    if (lane == 31) groups.tile[p.groups] = inc;
+  }
+  __syncthreads();
 }
 
 struct PSmem {
@@ -175,8 +196,95 @@ __device__ __forceinline__ void store16(const gemm::Params& p, int n, int f, con
   }
 }
 
+// One token row, 16 channels d .. of a head and their rotation partners 64 further (`a`, `b`: accumulators): bias, rounding to bf16, rotation, stores to the activations and
+// the cache.  Same arithmetic as k_gemm_qkv_rope.
+__device__ __forceinline__ void store_rope16(const gemm::Params& p, int n, int head, int d, int pos, long long slot, const uint32_t* a, const uint32_t* b) {
+  float lo[16], hi[16];
+#pragma unroll
+  for (int j = 0; j < 16; j++) { lo[j] = __uint_as_float(a[j]); hi[j] = __uint_as_float(b[j]); }
+  if (p.bias) {
+    const __nv_bfloat16* bias = p.bias + head * 128 + d;
+#pragma unroll
+    for (int j = 0; j < 16; j++) { lo[j] += __bfloat162float(bias[j]); hi[j] += __bfloat162float(bias[64 + j]); }
+  }
+  if (head < p.rope.nq + p.rope.nkv) {
+    const float4* c4 = reinterpret_cast<const float4*>(p.rope.cos_sin + size_t(pos) * 128 + d);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const float4 c = c4[q], s = c4[16 + q];
+      const float cs[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const int j = 4 * q + e;
+        gemm::rotate(bf16_round(lo[j]), bf16_round(hi[j]), bf16_round(cs[e]), bf16_round(sn[e]), lo[j], hi[j]);
+      }
+    }
+  }
+  uint4 l0, l1, h0, h1;
+  l0.x = pack_bf16(lo[0], lo[1]);   l0.y = pack_bf16(lo[2], lo[3]);   l0.z = pack_bf16(lo[4], lo[5]);   l0.w = pack_bf16(lo[6], lo[7]);
+  l1.x = pack_bf16(lo[8], lo[9]);   l1.y = pack_bf16(lo[10], lo[11]); l1.z = pack_bf16(lo[12], lo[13]); l1.w = pack_bf16(lo[14], lo[15]);
+  h0.x = pack_bf16(hi[0], hi[1]);   h0.y = pack_bf16(hi[2], hi[3]);   h0.z = pack_bf16(hi[4], hi[5]);   h0.w = pack_bf16(hi[6], hi[7]);
+  h1.x = pack_bf16(hi[8], hi[9]);   h1.y = pack_bf16(hi[10], hi[11]); h1.z = pack_bf16(hi[12], hi[13]); h1.w = pack_bf16(hi[14], hi[15]);
+  auto put = [&](__nv_bfloat16* row) {
+    uint4* x = reinterpret_cast<uint4*>(row + d);
+    uint4* y = reinterpret_cast<uint4*>(row + d + 64);
+    x[0] = l0; x[1] = l1; y[0] = h0; y[1] = h1;
+  };
+  put(p.y + size_t(n) * p.ldy + head * 128);
+  if (slot >= 0 && head >= p.rope.nq) {
+    const bool value = head >= p.rope.nq + p.rope.nkv;
+    put((value ? p.rope.v_cache : p.rope.k_cache) + (size_t(slot) * p.rope.nkv + (head - p.rope.nq - (value ? p.rope.nkv : 0))) * 128);
+  }
+}
+
+// A warp's 32 rows of an accumulator of FEAT columns (`trow`: its TMEM address), token row n of this lane, features f0 ..; release(): called by the whole warp when the
+// accumulator has been read.
+template <int EPI, int FEAT, typename F>
+__device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok, int f0, uint32_t trow, F release) {
+  if constexpr (EPI == gemm::kEpiRope) {
+    // rotation partners lie 64 columns apart: 16 channels of a head and their partners at a time
+    int pos = 0;
+    long long slot = -1;
+    if (row_ok) {
+      pos = p.rope.positions[n];
+      pos = pos < 0 ? 0 : (pos >= p.rope.max_pos ? p.rope.max_pos - 1 : pos);
+      if (p.rope.slot_mapping) slot = p.rope.slot_mapping[n];
+    }
+#pragma unroll 1
+    for (int c = 0; c < FEAT; c += c % 128 == 48 ? 80 : 16) {     // 0 16 32 48 128 144 160 176
+      uint32_t a[16], b[16];
+      __syncwarp();
+      tmem_ld16(trow + uint32_t(c), a);
+      tmem_ld16(trow + uint32_t(c + 64), b);
+      tmem_ld_wait();
+      if (c + 80 == FEAT) {
+        tc_fence_before();
+        __syncwarp();
+        release();
+      }
+      if (row_ok && f0 + c < p.M) store_rope16(p, n, (f0 + c) >> 7, c & 127, pos, slot, a, b);   // M is a multiple of 128
+    }
+  } else {
+    for (int c = 0; c < FEAT; c += 32) {
+      uint32_t r[32];
+      __syncwarp();   // rows past the end skip the stores below: reconverge before the warp-wide load
+      tmem_ld32(trow + uint32_t(c), r);
+      tmem_ld_wait();
+      if (c + 32 == FEAT) {
+        // accumulator fully read by this warp: hand it back to the MMA warp before the last stores go out
+        tc_fence_before();
+        __syncwarp();
+        release();
+      }
+      if (!row_ok) continue;
+      if (f0 + c < p.M) store16<EPI>(p, n, f0 + c, r);               // M is a multiple of 16
+      if (f0 + c + 16 < p.M) store16<EPI>(p, n, f0 + c + 16, r + 16);
+    }
+  }
+}
+
 // EPI 0: store (+bias); 1: SiLU-mul over interleaved gate/up features (output has M / 2 features); 2: fp32 store with
-// an activation; 3: clamped gated unit over interleaved gate/up features.
+// an activation; 3: clamped gated unit over interleaved gate/up features; 4: rotation and cache write of a qkv projection.
 // ROWS: row-grouped problem (p.row_off).
 template <int EPI, int TH, bool ROWS>
 __global__ void __launch_bounds__(Shape<TH>::kThreads, 1)
@@ -219,29 +327,13 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
   if constexpr (ROWS) {
     // the groups' rows were counted on the device by a kernel before this one
     pdl::grid_dependency_wait();
-    for (int g = threadIdx.x; g <= p.groups; g += S::kThreads) groups.off[g] = p.row_off[g];
-    __syncthreads();
-    if (warp == 0) {
-      const int per = (p.groups + 31) / 32, a = min(p.groups, lane * per), b = min(p.groups, a + per);
-      auto count = [&](int g) { return (groups.off[g + 1] - groups.off[g] + S::kTok - 1) / S::kTok * feat_tiles; };
-      int sum = 0;
-      for (int g = a; g < b; g++) sum += count(g);
-      int inc = sum;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += v;
-      }
-      int run = inc - sum;
-      for (int g = a; g < b; g++) { groups.tile[g] = run; run += count(g); }
-      if (lane == 31) groups.tile[p.groups] = inc;
-    }
-    __syncthreads();
+    count_tiles(groups, p, S::kTok, feat_tiles, S::kThreads);
     tiles = groups.tile[p.groups];
   }
   const int my_tiles = int(blockIdx.x) < tiles ? (tiles - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x) : 0;
   const int ngroups = p.groups, feats = p.M, all_rows = p.N;
   // (by value: a capture of the parameter block would put it in local memory)
-  auto locate = [=](int tile) -> At { return find_tile<ROWS, S::kTok>(groups, tile, tok_tiles, ngroups, feats, all_rows); };
+  auto locate = [=](int tile) -> At { return find_tile<ROWS, S::kTok, kFeatTile>(groups, tile, tok_tiles, ngroups, feats, all_rows); };
   const uint32_t tmem0 = s.tmem_base;
   volatile int* abortp = &s.abort_flag;
 
@@ -329,22 +421,9 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
       const int n = at.n0 + half * 128 + quarter * 32 + lane;   // token row
       const int f0 = at.f0;
       const uint32_t trow = tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t((TH == 1 ? buf : half) * kFeatTile);
-      const bool row_ok = n < at.nend;
-      for (int c = 0; c < kFeatTile; c += 32) {
-        uint32_t r[32];
-        __syncwarp();   // rows past the end skip the stores below: reconverge before the warp-wide load
-        tmem_ld32(trow + uint32_t(c), r);
-        tmem_ld_wait();
-        if (c + 32 == kFeatTile) {
-          // accumulator fully read by this warp: hand it back to the MMA warp before the last stores go out
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&s.acc_empty[buf]));
-        }
-        if (!row_ok) continue;
-        if (f0 + c < p.M) store16<EPI>(p, n, f0 + c, r);               // M is a multiple of 16
-        if (f0 + c + 16 < p.M) store16<EPI>(p, n, f0 + c + 16, r + 16);
-      }
+      drain<EPI, kFeatTile>(p, n, n < at.nend, f0, trow, [&] {
+        if (lane == 0) mbar_arrive(smem_u32(&s.acc_empty[buf]));
+      });
     }
   }
 
@@ -425,7 +504,9 @@ int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, in
   p.limit_ns = 2000000000ull;
   p.err = gemm_err_flag();
   if (!g_attr) {
-    cudaError_t a[12] = {cudaFuncSetAttribute(k_gemm_tok<0, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
+    cudaError_t a[14] = {cudaFuncSetAttribute(k_gemm_tok<4, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
+                        cudaFuncSetAttribute(k_gemm_tok<4, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
+                        cudaFuncSetAttribute(k_gemm_tok<0, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
                         cudaFuncSetAttribute(k_gemm_tok<1, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
                         cudaFuncSetAttribute(k_gemm_tok<2, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
                         cudaFuncSetAttribute(k_gemm_tok<3, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
@@ -454,6 +535,8 @@ int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, in
     case 4: e = launch<2, 1>(w, x, p, ldx, st, &map_rc); break;
     case 5: e = launch<2, 2>(w, x, p, ldx, st, &map_rc); break;
     case 6: e = launch<3, 1>(w, x, p, ldx, st, &map_rc); break;
+    case 8: e = launch<4, 1>(w, x, p, ldx, st, &map_rc); break;
+    case 9: e = launch<4, 2>(w, x, p, ldx, st, &map_rc); break;
     case 7: e = launch<3, 2>(w, x, p, ldx, st, &map_rc); break;
     default: e = launch<0, 1>(w, x, p, ldx, st, &map_rc); break;
   }

@@ -6,6 +6,7 @@
 // have stored — applies the HF rotate_half rotation in bf16 arithmetic, writes q / k / v into the
 // qkv activation buffer and scatters the k and v heads into the paged cache.  Results are bit
 // for bit those of `tbv_op_gemm` followed by `tbv_op_rope_kv`; one launch per layer is saved.
+// This kernel serves decode; with hundreds of tokens the many-token kernel runs with the same epilogue (gemm_persist.cu, epilogue kEpiRope).
 // (The reference's engine lists RoPE and the q/k/v -> qkv weight fusion without code:
 // reports/11_custom_engine.md:12,38.)
 #include <cuda.h>
@@ -19,23 +20,11 @@ using namespace sm100;
 
 namespace {
 
-struct RopeArgs {
-  const int* positions;            // [N]
-  const float* cos_sin;            // [max_pos, 128]: cos(0..63), sin(0..63)
-  const long long* slot_mapping;   // [N] cache row per token (< 0: skip) or null
-  __nv_bfloat16* k_cache;          // [slots, nkv, 128]
-  __nv_bfloat16* v_cache;
-  int nq, nkv, max_pos;
-};
-
-__device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-__device__ __forceinline__ void rotate(float x1, float x2, float c, float s, float& o1, float& o2) {
-  o1 = bfr(bfr(x1 * c) + bfr(-x2 * s));
-  o2 = bfr(bfr(x2 * c) + bfr(x1 * s));
-}
+using gemm::bfr;
+using gemm::rotate;
 
 __global__ void __launch_bounds__(gemm::kThreads, 1)
-k_gemm_qkv_rope(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const gemm::Params p, const RopeArgs ra) {
+k_gemm_qkv_rope(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const gemm::Params p, const gemm::Rope ra) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ gemm::Smem s;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -196,6 +185,22 @@ extern "C" int tbv_op_gemm_qkv_rope(const void* w, const void* x, void* qkv, con
   const char* pf_ptr = nullptr;   // an announcement holds for exactly one launch
   const unsigned long long pf_bytes = tbvops::take_next_prefetch(&pf_ptr, (unsigned long long)(M > 0 ? M : 0) * (unsigned long long)(K > 0 ? K : 0) * 2ull);
   if (M != (nq + 2 * nkv) * 128 || N <= 0 || (K % 8) || (ldx % 8) || (ldy % 8)) return -2;
+  const gemm::Rope ra{static_cast<const int*>(positions), static_cast<const float*>(cos_sin), static_cast<const long long*>(slot_mapping),
+                      static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), nq, nkv, max_pos};
+  // Hundreds of tokens: the many-token kernel with this epilogue, wherever it takes the plain product (4096 tokens, 6144 x 4096: 186 us against 226 here, where two CTAs
+  // per SM stage every tile through shared memory).
+  if (splits_hint <= 0 && !((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(cos_sin) | reinterpret_cast<uintptr_t>(k_cache) |
+                             reinterpret_cast<uintptr_t>(v_cache)) & 15u)) {
+    const int persist = tbvops::gemm_persist_mode(), th = persist > 0 ? tbvops::gemm_tok_choose(M, N, K, ldy, gemm::kEpiStore, persist) : 0;
+    if (th > 0) {
+      gemm::Params p{};
+      p.M = M; p.N = N; p.K = K; p.ldy = ldy;
+      p.bias = static_cast<const __nv_bfloat16*>(bias);
+      p.y = static_cast<__nv_bfloat16*>(qkv);
+      p.rope = ra;
+      return tbvops::gemm_tok_launch_p(w, x, p, ldx, gemm::kEpiRope, th, stream);
+    }
+  }
   int bn, splits, stages;
   tbvops::gemm_config(M, N, K, splits_hint, &bn, &splits, &stages);
   CUtensorMap tmA, tmB;
@@ -210,8 +215,6 @@ extern "C" int tbv_op_gemm_qkv_rope(const void* w, const void* x, void* qkv, con
   p.err = tbvops::gemm_err_flag();
   p.pf_ptr = pf_ptr;
   p.pf_bytes = pf_bytes;
-  RopeArgs ra{static_cast<const int*>(positions), static_cast<const float*>(cos_sin), static_cast<const long long*>(slot_mapping),
-              static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), nq, nkv, max_pos};
   if (!g_attr) {
     if (cudaFuncSetAttribute(k_gemm_qkv_rope, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) return -1;
     g_attr = true;

@@ -20,6 +20,7 @@ int sm_count();
 void gemm_config(int M, int N, int K, int splits_hint, int* bn_out, int* splits_out, int* stages_out, int groups = 1,
                  bool f32_out = false);
 // many-token (prefill) persistent kernel, gemm_persist.cu
+int gemm_persist_mode();
 int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode);
 int gemm_tok_launch(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi, int th,
                     void* stream);

@@ -1,0 +1,36 @@
+"""The many-token GEMM (gemm_persist.cu): the epilogue of the qkv projection, in both tile shapes, at remainders of tokens and features."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rnd(*shape, seed, scale=1.0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return (torch.randn(shape, generator=g, device=DEV) * scale).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("mode", [1, 2, 3])
+@pytest.mark.parametrize("T,nq,nkv,K,bias", [(384, 4, 2, 512, False), (401, 3, 1, 1000, True), (1025, 8, 4, 256, True), (384, 1, 0, 64, False)])
+def test_qkv_projection_of_many_tokens_equals_gemm_then_rope(mode, T, nq, nkv, K, bias):
+    """Bit for bit: the same sums in the same order, rounded where the two-kernel form rounds them.  Positions beyond the table, rows without a slot, caches without heads."""
+    from libtbvcoll_b200 import ops
+    D, M = 128, (nq + 2 * nkv) * 128
+    x, w, b = rnd(T, K, seed=1), rnd(M, K, seed=2, scale=0.05), rnd(M, seed=3) if bias else None
+    pos = (torch.arange(T, dtype=torch.int32) * 3 % 260 - 2).to(DEV)
+    cs = ops.rope_cos_sin(D, 256, 5e5, DEV)
+    slots = torch.randperm(T + 40, generator=torch.Generator().manual_seed(4))[:T].to(DEV)
+    slots[::7] = -1
+    kc = [torch.zeros(T + 40, max(nkv, 1), D, dtype=torch.bfloat16, device=DEV) for _ in range(4)]
+    ops.gemm_persist_mode(mode)
+    try:
+        want = ops.gemm(x, w, bias=b)
+        ops.rope_kv(want, pos, cs, slots, kc[0], kc[1], nq, nkv, D)
+        got = torch.zeros(T, M, dtype=torch.bfloat16, device=DEV)
+        ops.gemm_qkv_rope(x, w, got, pos, cs, slots, kc[2], kc[3], nq, nkv, bias=b)
+        torch.cuda.synchronize()
+    finally:
+        ops.gemm_persist_mode(None)
+    assert not ops.gemm_error()
+    assert torch.equal(got, want) and torch.equal(kc[2], kc[0]) and torch.equal(kc[3], kc[1])
