@@ -665,6 +665,8 @@ int tbv_op_paged_attention(const void* q, const void* k_cache, const void* v_cac
     cudaFuncSetAttribute(k_paged_attn_mma<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem);
     cudaFuncSetAttribute(k_paged_attn_mma<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem);
   }
+  if (impl == 1 && (G == 1 || G == 2 || G == 4 || G == 8) && tbvops::attn_rows_takes(q, k_cache, v_cache, out, nq_heads, nkv, ldq, ldo, block_size))
+    return tbvops::attn_rows(q, k_cache, v_cache, p.block_tables, p.seq_of_query, p.ctx_lens, out, nq_rows, nq_heads, nkv, ldq, ldo, block_size, max_blocks, splits, scale, st);
   if (impl == 1) {
     const dim3 blk(kMW * 32);
     switch (G) {

@@ -376,9 +376,6 @@ int report(cudaError_t e) {
   return e == cudaSuccess ? 0 : -1;
 }
 
-// largest number of cached rows that an index can name: blocks come from the block table, so this is no check of what exists
-constexpr unsigned long long kAnyRows = 0x7fffffffull;
-
 }  // namespace
 
 namespace tbvops {
@@ -396,8 +393,8 @@ int attn_prefill_split(const void* q, const void* k_cache, const void* v_cache, 
   p.scale_log2 = scale * attn_mma::kLog2e; p.limit_ns = 2000000000ull; p.err = gemm_err_flag();
   CUtensorMap mq, mk, mv;
   const unsigned long long width = (unsigned long long)kv_heads * kD;
-  if (make_tensor_map_heads(&mq, q, rows, heads, kD, ldq, p.hpk, kRows / p.hpk) != 0 || make_tensor_map_bf16(&mk, k_cache, kAnyRows, width, width, 16) != 0 ||
-      make_tensor_map_bf16(&mv, v_cache, kAnyRows, width, width, 16) != 0) return -3;
+  if (make_tensor_map_heads(&mq, q, rows, heads, kD, ldq, p.hpk, kRows / p.hpk) != 0 || make_tensor_map_bf16(&mk, k_cache, kAnyCacheRows, width, width, 16) != 0 ||
+      make_tensor_map_bf16(&mv, v_cache, kAnyCacheRows, width, width, 16) != 0) return -3;
   return report(launch<false, false>(mq, mk, mv, p, st));
 }
 
@@ -411,7 +408,7 @@ int attn_prefill_paired(const void* q, const void* cache, const int* tables, con
   p.window = window; p.chunk = chunk; p.softcap = softcap;
   p.scale_log2 = attn_mma::kLog2e; p.limit_ns = 2000000000ull; p.err = gemm_err_flag();
   CUtensorMap mq, mk;
-  if (make_tensor_map_heads(&mq, q, rows, heads, kD, ldq, p.hpk, kRows / p.hpk) != 0 || make_tensor_map_bf16(&mk, cache, kAnyRows, 2 * kD, row_len, 16) != 0) return -3;
+  if (make_tensor_map_heads(&mq, q, rows, heads, kD, ldq, p.hpk, kRows / p.hpk) != 0 || make_tensor_map_bf16(&mk, cache, kAnyCacheRows, 2 * kD, row_len, 16) != 0) return -3;
   return report(softcap > 0.f ? launch<true, true>(mq, mk, mk, p, st) : launch<true, false>(mq, mk, mk, p, st));
 }
 

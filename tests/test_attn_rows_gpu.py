@@ -1,0 +1,76 @@
+"""Attention of single rows: paged keys and values (attn_rows.cu) and the fp32 latent form with several heads per CTA, at the edges of their tiles and splits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+D = 128
+
+
+def rnd(*shape, seed, dtype=torch.bfloat16):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return torch.randn(shape, generator=g, device=DEV).to(dtype)
+
+
+@pytest.mark.parametrize("nq,nkv,bs", [(4, 4, 16), (8, 4, 48), (16, 4, 16), (8, 1, 32)])
+@pytest.mark.parametrize("splits", [1, 2, 3, 8])
+def test_paged_rows(nq, nkv, bs, splits):
+    """Contexts around the units of 16 tokens, of warps and of splits; nothing that lies behind a context matters; rows out of order over the sequences."""
+    from libtbvcoll_b200 import ops
+    lens = [1, 15, 16, 17, 63, 64, 65, 127, 129, 800, 1025]
+    need = [(n + bs - 1) // bs for n in lens]
+    perm = torch.randperm(sum(need) + 2, generator=torch.Generator().manual_seed(1))
+    tables, at = torch.zeros(len(lens), max(need) + 1, dtype=torch.int32), 0
+    kc, vc = rnd(len(perm) * bs, nkv, D, seed=1), rnd(len(perm) * bs, nkv, D, seed=2)
+    written, slots = torch.zeros(len(perm) * bs, dtype=torch.bool), []
+    for i, n in enumerate(need):
+        tables[i, :n] = perm[at: at + n].to(torch.int32)
+        at += n
+        pos = torch.arange(lens[i])
+        slots.append(tables[i, pos // bs].long() * bs + pos % bs)
+        written[slots[-1]] = True
+    kc[~written.to(DEV)] = float("nan")
+    vc[~written.to(DEV)] = float("nan")
+    order = list(range(len(lens)))[::-1] + [9, 0]
+    wide = rnd(len(order), (nq + 2 * nkv) * D, seed=3)
+    q = wide.view(len(order), -1, D)[:, :nq]
+    seq = torch.tensor(order, dtype=torch.int32, device=DEV)
+    ctx = torch.tensor([lens[i] for i in order], dtype=torch.int32, device=DEV)
+    out = torch.full((len(order), nq, D), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.paged_attention(q, kc, vc, tables.to(DEV), ctx, out, 0.15, bs, seq_of_query=seq, splits=splits)
+    torch.cuda.synchronize()
+    assert not ops.gemm_error()
+    for j, i in enumerate(order):
+        k, v = (c[slots[i].to(DEV)].double().repeat_interleave(nq // nkv, 1) for c in (kc, vc))
+        p = torch.softmax(torch.einsum("hd,jhd->hj", q[j].double(), k) * 0.15, -1)
+        want, size = torch.einsum("hj,jhd->hd", p, v), torch.einsum("hj,jhd->hd", p, v.abs())
+        # weights and result rounded to 8 significant bits: 2^-8 of the sum over |v| each
+        assert ((out[j].double() - want).abs() <= size * 2.0 ** -6.95 + 1e-6).all()
+
+
+def test_no_visible_key():
+    from libtbvcoll_b200 import ops
+    kc, vc = rnd(32, 1, D, seed=1), rnd(32, 1, D, seed=2)
+    q = rnd(2, 4, D, seed=3)
+    for splits in (1, 4):
+        out = torch.full_like(q, 7.0)
+        ops.paged_attention(q, kc, vc, torch.tensor([[0], [1]], dtype=torch.int32, device=DEV), torch.tensor([0, 3], dtype=torch.int32, device=DEV), out, 0.1, 16, splits=splits)
+        assert not out[0].any() and out[1].any() and torch.isfinite(out).all()
+
+
+def test_fp32_latent_rows_of_many_heads_equal_few():
+    """Enough rows that four heads share a CTA give the same bits as the same rows one at a time."""
+    from libtbvcoll_b200 import ops
+    H, R, rot, bs, n = 8, 80, 16, 16, 300
+    row = ops.latent_row(R, rot)
+    cache = rnd(20 * bs, row, seed=5, dtype=torch.float32)
+    qa = rnd(n, H, row, seed=6, dtype=torch.float32)
+    tables = torch.randperm(20, generator=torch.Generator().manual_seed(7))[None].to(torch.int32).to(DEV)
+    seq, ctx = torch.zeros(n, dtype=torch.int32, device=DEV), torch.arange(1, n + 1, dtype=torch.int32, device=DEV)
+    sink = rnd(H, seed=8, dtype=torch.float32)
+    out = torch.zeros(n, H, R, device=DEV)
+    ops.latent_attention_rows(qa, cache, tables, seq, ctx, sink, out, R, 0.05, bs, window=200)
+    for i in (0, 127, 128, 199, 200, 299):
+        one = torch.zeros(1, H, R, device=DEV)
+        ops.latent_attention_rows(qa[i: i + 1].contiguous(), cache, tables, seq[:1], ctx[i: i + 1], sink, one, R, 0.05, bs, window=200)
+        assert torch.equal(one[0], out[i]) and torch.isfinite(one).all()
