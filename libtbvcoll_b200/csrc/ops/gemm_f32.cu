@@ -3,11 +3,20 @@
 //
 //   y[n, m] = epilogue(sum_k x[n, k] * w[m, k])        x: [N, K], w: [groups * M, K], fp32 row-major
 //
-// 64 tokens x 64 features per CTA, K in steps of 16 through shared memory, 4 x 4 outputs per thread.  The order of
-// the additions for one output depends on K alone, so a row's result does not depend on the batch it is in.
+// k_gemm_f32_tiled: 8 RT tokens x 16 RF features per CTA of 128 threads, RT x RF results per thread.  Operands go to shared memory as they lie in memory
+// (16-byte asynchronous copies, three stages of 32 columns, rows 144 bytes apart so that eight rows fall into different banks), and a thread multiplies PAIRS of
+// neighbouring columns with one packed instruction: neither operand needs a move.  The even and the odd column's sums of 32 columns, sixteen additions each, are
+// kept apart from the running total, so the rounding error grows with 16 + K / 32, not with K.
+// The order of the additions for one output depends on K alone, so a row's result does not depend on the batch it is in.
+// Bound by the fp32 units (74 TFLOP/s at 1.965 GHz).  604 tokens: 8192 x 2048 519 us = 39 TFLOP/s (994 us in the form below),
+// 14336 x 2048 906 (1463), 2048 x 7168 606 (1196); 16 tokens, 8192 x 2048: 41 us (347).
+//
+// k_gemm_f32: any K, stride and alignment; 64 x 64 per CTA, K in steps of 16, sums of one step apart from the total in the same way.
 #include <cuda_runtime.h>
 
+#include "attn_mma.cuh"
 #include "gemm.cuh"
+#include "ops.h"
 
 namespace {
 
@@ -23,18 +32,126 @@ struct F32Params {
   const int* row_off;     // row-grouped form: group g owns rows row_off[g] .. row_off[g + 1] - 1
 };
 
+__device__ __forceinline__ float f32_glu(const F32Params& p, float g, float u) {
+  g = fminf(g, p.act_a);
+  u = fminf(fmaxf(u, -p.act_a), p.act_a);
+  return (isinf(p.act_b) ? fmaxf(g, 0.f) : g / (1.0f + expf(-p.act_b * g))) * (u + p.act_c);
+}
+__device__ __forceinline__ float f32_act(const F32Params& p, float v, int m) {
+  if (!p.act || m >= p.act_m) return v;
+  if (p.act == gemm::kActSilu || p.act == gemm::kActGelu) return v / (1.0f + expf(p.act == gemm::kActSilu ? -v : -gemm::gelu_slope(v)));
+  return p.act == gemm::kActSoftplus ? vec::softplus<float>(v) : gemm::apply_act(v, p.act, p.act_a);
+}
+// Which problem and rows a CTA has: grid (feature tiles of all groups, token tiles).
+struct Where { int grp, m0, M, n0, nend; };
+__device__ __forceinline__ Where f32_where(const F32Params& p, int tok, int feat) {
+  const int mt = (p.M + feat - 1) / feat;
+  Where a;
+  a.grp = min(int(blockIdx.x) / mt, p.m_last ? p.groups : p.groups - 1);
+  a.m0 = (blockIdx.x - a.grp * mt) * feat;
+  a.M = p.m_last && a.grp == p.groups ? p.m_last : p.M;
+  a.n0 = blockIdx.y * tok;
+  a.nend = p.N;
+  if (p.row_off) {
+    a.nend = p.row_off[a.grp + 1];
+    a.n0 += p.row_off[a.grp];
+  }
+  return a;
+}
+
+constexpr int kBlock = 32, kPitch = kBlock + 4, kRing = 3;       // columns of a stage, floats between rows, stages
+template <int RT, int RF>
+__global__ void __launch_bounds__(128) k_gemm_f32_tiled(const F32Params p) {
+  constexpr int TN = 8 * RT, TM = 16 * RF, kStage = (TN + TM) * kPitch;
+  extern __shared__ __align__(16) float ring[];
+  pdl::launch_dependents();
+  pdl::grid_dependency_wait();
+  const Where at = f32_where(p, TN, TM);
+  if (at.n0 >= at.nend) return;
+  const float* w = p.w + (size_t(at.grp) * p.M + at.m0) * p.K;
+  const float* x = p.x + size_t(at.grp) * p.x_group + size_t(at.n0) * p.ldx;
+  float* y = p.y + size_t(at.grp) * p.y_group;
+  const int tid = threadIdx.x, ft = tid & 15, tt = tid >> 4, rows = at.nend - at.n0, feats = at.M - at.m0;
+  const int blocks = (p.K + kBlock - 1) / kBlock;
+  const uint32_t ring0 = attn_mma::smem_addr(ring);
+  // a thread copies 16 bytes of rows tid / 8, + 16, ..; what lies beyond the problem is zeros
+  auto issue = [&](int i) {
+    if (i < blocks) {
+      const int c = (tid & 7) * 4, k = i * kBlock + c;
+      const uint32_t dst = ring0 + uint32_t((i % kRing) * kStage + c) * 4u;
+#pragma unroll
+      for (int r0 = 0; r0 < TN + TM; r0 += 16) {
+        const int r = r0 + (tid >> 3), wr = r - TN;
+        const bool ok = k < p.K && (r0 < TN ? r < rows : wr < feats);
+        const float* src = r0 < TN ? x + size_t(ok ? r : 0) * p.ldx : w + size_t(ok ? wr : 0) * p.K;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + uint32_t(r * kPitch) * 4u), "l"(src + (ok ? k : 0)), "r"(ok ? 16 : 0) : "memory");
+      }
+    }
+    attn_mma::cp_async_commit();
+  };
+  float acc[RT][RF];
+#pragma unroll
+  for (int i = 0; i < RT; i++)
+#pragma unroll
+    for (int j = 0; j < RF; j++) acc[i][j] = 0.f;
+#pragma unroll
+  for (int i = 0; i < kRing - 1; i++) issue(i);
+  for (int b = 0; b < blocks; b++) {
+    attn_mma::cp_async_wait<kRing - 2>();
+    __syncthreads();                                             // the stage is there, and everyone is done with the one before
+    issue(b + kRing - 1);
+    const float* sx = ring + (b % kRing) * kStage + tt * kPitch;
+    const float* sw = ring + (b % kRing) * kStage + (TN + ft) * kPitch;
+    vec::f32x2 part[RT][RF];
+#pragma unroll
+    for (int i = 0; i < RT; i++)
+#pragma unroll
+      for (int j = 0; j < RF; j++) part[i][j] = 0ull;
+#pragma unroll
+    for (int k = 0; k < kBlock; k += 4) {
+      ulonglong2 f[RF];
+#pragma unroll
+      for (int j = 0; j < RF; j++) f[j] = *reinterpret_cast<const ulonglong2*>(sw + j * 16 * kPitch + k);
+#pragma unroll
+      for (int i = 0; i < RT; i++) {
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(sx + i * 8 * kPitch + k);
+#pragma unroll
+        for (int j = 0; j < RF; j++) part[i][j] = vec::fma2(t.y, f[j].y, vec::fma2(t.x, f[j].x, part[i][j]));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RT; i++)
+#pragma unroll
+      for (int j = 0; j < RF; j++) {
+        float even, odd;
+        vec::unpack2(part[i][j], even, odd);
+        acc[i][j] += even + odd;
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < RT; i++) {
+    const int n = at.n0 + tt + 8 * i;
+#pragma unroll
+    for (int j = 0; j < RF; j++) {
+      const int m = at.m0 + ft + 16 * j;
+      float v = acc[i][j] + (p.bias && m < at.M ? p.bias[m] : 0.f);
+      if (p.epi == gemm::kEpiClampGlu) {                         // a gate and its up feature sit in neighbouring threads
+        const float u = __shfl_xor_sync(0xffffffffu, v, 1);
+        if (n < at.nend && m + 1 < at.M && !(ft & 1)) y[size_t(n) * p.ldy + m / 2] = f32_glu(p, v, u);
+      } else if (n < at.nend && m < at.M) {
+        y[size_t(n) * p.ldy + m] = f32_act(p, v, m);
+      }
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256) k_gemm_f32(const F32Params p) {
   __shared__ float sx[kKB][kT + 4], sw[kKB][kT + 4];
   pdl::launch_dependents();
   pdl::grid_dependency_wait();
-  const int mt = (p.M + kT - 1) / kT, grp = min(int(blockIdx.x) / mt, p.m_last ? p.groups : p.groups - 1);
-  const int m0 = (blockIdx.x - grp * mt) * kT, M = p.m_last && grp == p.groups ? p.m_last : p.M;
-  int n0 = blockIdx.y * kT, nend = p.N;
-  if (p.row_off) {
-    nend = p.row_off[grp + 1];
-    n0 += p.row_off[grp];
-    if (n0 >= nend) return;
-  }
+  const Where at = f32_where(p, kT, kT);
+  const int grp = at.grp, m0 = at.m0, M = at.M, n0 = at.n0, nend = at.nend;
+  if (n0 >= nend) return;
   const float* w = p.w + size_t(grp) * p.M * p.K;
   const float* x = p.x + size_t(grp) * p.x_group;
   float* y = p.y + size_t(grp) * p.y_group;
@@ -72,24 +189,45 @@ __global__ void __launch_bounds__(256) k_gemm_f32(const F32Params p) {
     for (int j = 0; j < 4; j++) v[j] = acc[i][j] + ((p.bias && m0 + tm + j < M) ? p.bias[m0 + tm + j] : 0.f);
     if (p.epi == gemm::kEpiClampGlu) {
 #pragma unroll
-      for (int j = 0; j < 4; j += 2) {
-        if (m0 + tm + j + 1 < M) {
-          const float g = fminf(v[j], p.act_a), u = fminf(fmaxf(v[j + 1], -p.act_a), p.act_a);
-          y[size_t(n) * p.ldy + (m0 + tm + j) / 2] = (isinf(p.act_b) ? fmaxf(g, 0.f) : g / (1.0f + expf(-p.act_b * g))) * (u + p.act_c);
-        }
-      }
+      for (int j = 0; j < 4; j += 2)
+        if (m0 + tm + j + 1 < M) y[size_t(n) * p.ldy + (m0 + tm + j) / 2] = f32_glu(p, v[j], v[j + 1]);
     } else {
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        if (m0 + tm + j < M) {
-          if (p.act && m0 + tm + j < p.act_m) {
-            if (p.act == gemm::kActSilu || p.act == gemm::kActGelu) v[j] = v[j] / (1.0f + expf(p.act == gemm::kActSilu ? -v[j] : -gemm::gelu_slope(v[j])));
-            else v[j] = p.act == gemm::kActSoftplus ? vec::softplus<float>(v[j]) : gemm::apply_act(v[j], p.act, p.act_a);
-          }
-          y[size_t(n) * p.ldy + m0 + tm + j] = v[j];
-        }
+        if (m0 + tm + j < M) y[size_t(n) * p.ldy + m0 + tm + j] = f32_act(p, v[j], m0 + tm + j);
     }
   }
+}
+
+template <int RT, int RF>
+cudaError_t launch_tiled(const F32Params& p, cudaStream_t st) {
+  constexpr int TN = 8 * RT, TM = 16 * RF;
+  constexpr size_t smem = size_t(kRing) * (TN + TM) * kPitch * 4;
+  static const cudaError_t attr = cudaFuncSetAttribute(k_gemm_f32_tiled<RT, RF>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (attr != cudaSuccess) return attr;
+  const dim3 grid(p.groups * ((p.M + TM - 1) / TM) + (p.m_last + TM - 1) / TM, (p.N + TN - 1) / TN);
+  return pdl::launch(k_gemm_f32_tiled<RT, RF>, grid, dim3(128), smem, st, 1, p);
+}
+
+int launch_f32(const F32Params& p, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const bool wide = !((reinterpret_cast<uintptr_t>(p.w) | reinterpret_cast<uintptr_t>(p.x)) & 15) && p.K % 4 == 0 && p.ldx % 4 == 0 && p.x_group % 4 == 0;
+  cudaError_t e;
+  if (!wide) {
+    const dim3 grid(p.groups * ((p.M + kT - 1) / kT) + (p.m_last + kT - 1) / kT, (p.N + kT - 1) / kT);
+    e = pdl::launch(k_gemm_f32, grid, dim3(256), 0, st, 1, p);
+  } else {
+    // 64 x 64 tiles do most work per byte and instruction.  Smaller ones where they would leave SMs idle or with one or two CTAs, whose loads nothing hides
+    // (604 tokens, K 4096: 160 features 104 us with 32 x 64, 73 with 16 x 32; 2048 features 369 us with 64 x 64, 347 with 32 x 64), where few
+    // columns leave no time to fill the ring (1000 tokens, 4096 x 128: 50 and 38 us), or where their last round would be emptier.
+    const long sms = tbvops::sm_count(), ft = (long)p.groups * ((p.M + 63) / 64) + (p.m_last + 63) / 64;
+    const long t32 = ft * ((p.N + 31) / 32), r64 = (ft * ((p.N + 63) / 64) + sms - 1) / sms, r32 = (t32 + sms - 1) / sms;
+    if (t32 < sms && p.N <= 16) e = launch_tiled<2, 2>(p, st);
+    else if (t32 < sms) e = p.N <= 32 ? launch_tiled<4, 2>(p, st) : launch_tiled<2, 2>(p, st);
+    else if (p.K < 512 || r64 <= 2 || 23 * r32 < 40 * r64) e = launch_tiled<4, 4>(p, st);
+    else e = launch_tiled<8, 4>(p, st);
+  }
+  return e == cudaSuccess ? 0 : -1;
 }
 
 }  // namespace
@@ -102,8 +240,7 @@ int tbv_op_gemm_f32(const void* w, const void* x, void* y, const void* bias, int
   if (M <= 0 || N <= 0 || K <= 0 || (epi != 0 && epi != 2 && epi != 3) || (epi == 3 && (M % 2)) || (groups > 1 && bias)) return -2;
   F32Params p{static_cast<const float*>(w), static_cast<const float*>(x), static_cast<const float*>(bias), static_cast<float*>(y),
               M, N, K, ldx, ldy, epi, act, groups > 1 ? groups : 1, x_group, y_group, act_a, act_b, act_c, groups > 1 ? m_last : 0, act_m, nullptr};
-  const dim3 grid(p.groups * ((M + kT - 1) / kT) + (p.m_last + kT - 1) / kT, (N + kT - 1) / kT);
-  return pdl::launch(k_gemm_f32, grid, dim3(256), 0, static_cast<cudaStream_t>(stream), 1, p) == cudaSuccess ? 0 : -1;
+  return launch_f32(p, stream);
 }
 
 // Arguments as tbv_op_gemm_rows, everything fp32.
@@ -112,8 +249,7 @@ int tbv_op_gemm_rows_f32(const void* w, const void* x, void* y, const void* row_
   if (M <= 0 || x_rows <= 0 || max_rows <= 0 || K <= 0 || groups <= 0 || (epi != 0 && epi != 3) || (epi == 3 && (M % 2)) || !row_off) return -2;
   F32Params p{static_cast<const float*>(w), static_cast<const float*>(x), nullptr, static_cast<float*>(y),
               M, max_rows, K, ldx, ldy, epi, 0, groups, 0, 0, act_a, act_b, act_c, 0, 0, static_cast<const int*>(row_off)};
-  const dim3 grid(groups * ((M + kT - 1) / kT), (max_rows + kT - 1) / kT);
-  return pdl::launch(k_gemm_f32, grid, dim3(256), 0, static_cast<cudaStream_t>(stream), 1, p) == cudaSuccess ? 0 : -1;
+  return launch_f32(p, stream);
 }
 
 }  // extern "C"

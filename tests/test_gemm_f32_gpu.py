@@ -1,0 +1,72 @@
+"""The fp32 GEMM: every tile form, remainders, grouped and row-grouped problems, operands that only the general form takes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rnd(*shape, seed):
+    return torch.randn(shape, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV)
+
+
+def limit(x, w):
+    # sums of 16 in order, then K / 32 of those in order: (16 + K / 32 + 2) roundings of 2^-24 of the sum of the products' sizes
+    K = x.shape[1]
+    return (x.abs().double() @ w.abs().double().t()) * (18 + K / 32) * 2.0 ** -24 + 1e-30
+
+
+@pytest.mark.parametrize("N", [1, 16, 17, 33, 65, 130, 700])
+@pytest.mark.parametrize("M,K", [(1, 4), (70, 36), (160, 1000), (2050, 516), (300, 130)])     # 130: not a multiple of four columns
+def test_plain(N, M, K):
+    from libtbvcoll_b200 import ops
+    x, w, b = rnd(N, K + 4, seed=1)[:, :K], rnd(M, K, seed=2), rnd(M, seed=3)
+    out = torch.full((N, M + 3), 7.0, device=DEV)
+    ops.linear(x, w, out[:, :M], bias=b)
+    want = x.double() @ w.double().t() + b.double()
+    assert ((out[:, :M].double() - want).abs() <= limit(x, w) + 2.0 ** -23 * want.abs()).all() and (out[:, M:] == 7.0).all()
+    if M % 2 == 0:
+        glu = torch.zeros(N, M // 2, device=DEV)
+        ops.linear(x, w, glu, glu=(2.0, 1.7))
+        y = want - b.double()
+        g, u = y[:, 0::2].clamp(max=2.0), y[:, 1::2].clamp(-2.0, 2.0)
+        e = limit(x, w)
+        # the unit's slope is at most 1.5 in either argument times the other's size (3); 1e-5 for the exponential
+        assert ((glu.double() - g * torch.sigmoid(1.7 * g) * (u + 1)).abs() <= 5 * (e[:, 0::2] + e[:, 1::2]) + 1e-5).all()
+
+
+def test_a_rows_result_does_not_depend_on_its_batch():
+    from libtbvcoll_b200 import ops
+    x, w = rnd(700, 520, seed=1), rnd(1024, 520, seed=2)
+    whole = torch.empty(700, 1024, device=DEV)
+    ops.linear(x, w, whole)
+    for n in (1, 20, 50, 300):
+        part = torch.empty(n, 1024, device=DEV)
+        ops.linear(x[:n], w, part)
+        assert torch.equal(part, whole[:n])
+
+
+@pytest.mark.parametrize("N", [5, 40, 300])
+def test_groups(N):
+    from libtbvcoll_b200 import ops
+    G, M, K, last = 3, 90, 64, 34
+    x, w = rnd(N, G * 68 + K, seed=1), rnd(G * M + last, K, seed=2)
+    out = torch.zeros(N, G * 96 + last, device=DEV)
+    ops.linear(x, w, out, groups=G, x_group=68, y_group=96, last=last)
+    for g in range(G + 1):
+        rows, xs = (slice(g * M, g * M + (M if g < G else last)), x[:, g * 68: g * 68 + K])
+        want = xs.double() @ w[rows].double().t()
+        assert ((out[:, g * 96: g * 96 + want.shape[1]].double() - want).abs() <= limit(xs, w[rows])).all()
+
+
+def test_row_groups():
+    from libtbvcoll_b200 import ops
+    counts, M, K = [0, 70, 1, 0, 129, 33], 48, 100
+    off = torch.tensor([0] + counts).cumsum(0).to(torch.int32).to(DEV)
+    x, w = rnd(sum(counts), K, seed=1), rnd(len(counts) * M, K, seed=2)
+    out = torch.zeros(sum(counts), M, device=DEV)
+    ops.linear_rows(x, w, out, off, len(counts), sum(counts))
+    for g in range(len(counts)):
+        a, b = int(off[g]), int(off[g + 1])
+        want = x[a:b].double() @ w[g * M: (g + 1) * M].double().t()
+        assert ((out[a:b].double() - want).abs() <= limit(x[a:b], w[g * M: (g + 1) * M])).all()
