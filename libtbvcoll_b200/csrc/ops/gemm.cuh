@@ -67,6 +67,7 @@ struct Params {
   unsigned long long limit_ns;  // bound on every barrier wait
   int* err;                     // device flag: set to 1 if a wait gave up
   Rope rope;                    // kEpiRope only
+  int wide;                     // many-token kernels: rows of y are 32-byte aligned
   const char* pf_ptr;           // weights of the GEMM that runs next (or null): see the producer's last step
   unsigned long long pf_bytes;  // how much of them to ask into L2 (a multiple of 16), shared out over the CTAs
 };

@@ -3,24 +3,21 @@
 //   Y[n, m] = epilogue( sum_k X[n, k] * W[m, k] )      X: [N tokens, K], W: [M features, K], both bf16 row-major
 //
 // The decode form (gemm.cu) puts features on the 128-row UMMA M axis because a handful of tokens would
-// waste it.  With hundreds of tokens the natural orientation is the other one: 128 tokens on UMMA M and 256
-// features on UMMA N.  A thread of the epilogue then owns one token row and reads 16 consecutive features
-// per TMEM load, which it stores as 32 contiguous bytes; gate/up pairs of the SiLU-mul epilogue sit in the
-// same thread, so that epilogue needs no shuffles.
+// waste it.  With hundreds of tokens the natural orientation is the other one: tokens on UMMA M and up to 256
+// features on UMMA N.  A thread of the epilogue then owns one token row and reads consecutive features per
+// TMEM load; gate/up pairs of the SiLU-mul epilogue sit in the same thread, so that epilogue needs no shuffles.
 //
-// Two tile shapes (template TH), both filling the 512 TMEM columns of the SM:
-//   TH = 1  128 tokens x 256 features, two accumulators: the epilogue of tile i runs under the MMAs of tile
-//           i + 1.  Every 512 tensor-core clocks consume 48 KB of operands; measured, the tensor pipe is
-//           68 % busy and L2 -> shared memory is the limit.
-//   TH = 2  256 tokens x 256 features as two 128-row MMAs that share one 256-row weight tile: 64 KB of operands
-//           per 1024 tensor-core clocks, a third less traffic per FLOP.  Both accumulators belong to one tile,
-//           so the epilogue (eight warps here, four per half) is exposed once per tile.  Measured at 4096
-//           tokens: down_proj (K 14336) 1450 TFLOP/s against 1144 for TH = 1 and 1560 for cuBLAS.
+// Two tile shapes (template TH), both with all 512 TMEM columns of the SM in use:
+//   TH = 1  128 tokens x 256 features, two accumulator sets: the epilogue of a tile runs under the MMAs of the next.  For epilogues that compute, and where
+//           tiles are few.  4096 tokens: 28672 x 4096 with the SiLU unit 641 us = 1500 TFLOP/s (848 with TH = 2), 6144 x 4096 with rotation 159 (166).
+//   TH = 2  256 tokens x 256 features as two 128-row MMAs that share one 256-row weight tile: a third less traffic per operation, but both accumulators belong
+//           to one tile, so the epilogue (eight warps here, four per half) is exposed once per tile.  For plain stores: 4096 x 4096 97 us (104 with TH = 1), 4096 x 14336 361 (402).
 //
-// The CTAs walk tiles id = blockIdx.x + i * gridDim.x with the token tile fastest: the CTAs running at any
-// moment share a few 256-row weight tiles (streamed from HBM once) and the activations stay in L2.  Warp 0
+// The CTAs walk tiles id = first + i * step with the token tile fastest: the CTAs running at any
+// moment share a few weight tiles (streamed from HBM once) and the activations stay in L2.  Warp 0
 // lane 0 feeds a TMA ring that runs ahead across tile boundaries, warp 1 lane 0 issues tcgen05.mma, warps 2..
-// drain TMEM.  Every wait is bounded; a wait that gives up raises the CTA's abort flag, all roles leave their
+// drain TMEM.  The copying and the issuing thread have some 500 clocks per k-block: stage and phase are counted, a division by the number of
+// stages or k-blocks cost a fifth of the rate.  Every wait is bounded; a wait that gives up raises the CTA's abort flag, all roles leave their
 // loops, TMEM is freed and the host-visible error flag is set.  (The reference has no GEMM; see gemm.cu for
 // what this path replaces.)
 #include <cuda.h>
@@ -48,13 +45,8 @@ template <int TH> struct Shape {
   static constexpr int kStages = TH == 1 ? 4 : 3;              // 192 KB of ring either way
   static constexpr int kBuffers = TH == 1 ? 2 : 1;             // accumulator sets that alternate between tiles
   static constexpr int kEpiWarps = 4 * TH;
-  static constexpr int kThreads = 64 + 32 * kEpiWarps;
+  static constexpr int kThreads = 64 + 32 * kEpiWarps;         // a warp of copies, one of products, the epilogue's
 };
-
-// Fraction of the nominal tensor rate each form sustains (measured; see gemm_tok_choose).
-constexpr double kEffDecode[2] = {0.59, 0.43};   // decode-form kernel: store / SiLU-mul epilogue
-constexpr double kEffTok1 = 0.62;                // 128-token tiles: gate_up 4096 x 28672 x 4096 in 25 rounds, 722 us
-constexpr double kEffTok2 = 0.69;                // 256-token tiles: 0.66 (K 4096, SiLU-mul) .. 0.75 (K 14336) per round
 
 constexpr int kMaxRowGroups = 512;
 
@@ -66,31 +58,25 @@ struct RowGroups {
 
 // first token row, end of the rows, first feature and its weight row of a tile
 struct At { int n0, nend, f0, w0; };
-template <bool ROWS, int TOK, int FEAT, typename G>
-__device__ __forceinline__ At find_tile(const G& groups, int tile, int tok_tiles, int ngroups, int M, int N) {
-  if constexpr (ROWS) {
-    int lo = 0, hi = ngroups - 1;                  // the last group whose first tile is not beyond `tile`; empty groups are passed over
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (groups.tile[mid] <= tile) lo = mid;
-      else hi = mid - 1;
-    }
-    const int local = tile - groups.tile[lo], tt = (groups.off[lo + 1] - groups.off[lo] + TOK - 1) / TOK;
-    const int f0 = local / tt * FEAT;
-    return At{groups.off[lo] + local % tt * TOK, groups.off[lo + 1], f0, lo * M + f0};
-  } else {
-    const int f0 = tile / tok_tiles * FEAT;
-    return At{tile % tok_tiles * TOK, N, f0, f0};
+__device__ __forceinline__ At find_tile(const RowGroups& groups, int tile, int ngroups, int M) {
+  int lo = 0, hi = ngroups - 1;                    // the last group whose first tile is not beyond `tile`; empty groups are passed over
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (groups.tile[mid] <= tile) lo = mid;
+    else hi = mid - 1;
   }
+  const int local = tile - groups.tile[lo], tt = (groups.off[lo + 1] - groups.off[lo] + 127) / 128;
+  const int f0 = local / tt * kFeatTile;
+  return At{groups.off[lo] + local % tt * 128, groups.off[lo + 1], f0, lo * M + f0};
 }
 
 // Fills the table from the rows' offsets (device memory); whole CTA.
-__device__ __forceinline__ void count_tiles(RowGroups& groups, const gemm::Params& p, int tok, int feat_tiles, int threads) {
-  for (int g = threadIdx.x; g <= p.groups; g += threads) groups.off[g] = p.row_off[g];
+__device__ __forceinline__ void count_tiles(RowGroups& groups, const gemm::Params& p, int feat_tiles) {
+  for (int g = threadIdx.x; g <= p.groups; g += Shape<1>::kThreads) groups.off[g] = p.row_off[g];
   __syncthreads();
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x, per = (p.groups + 31) / 32, a = min(p.groups, lane * per), b = min(p.groups, a + per);
-    auto count = [&](int g) { return (groups.off[g + 1] - groups.off[g] + tok - 1) / tok * feat_tiles; };
+    auto count = [&](int g) { return (groups.off[g + 1] - groups.off[g] + 127) / 128 * feat_tiles; };
     int sum = 0;
     for (int g = a; g < b; g++) sum += count(g);
     int inc = sum;
@@ -135,9 +121,13 @@ __device__ __forceinline__ void st_global_f32x8(float* p, const float* v) {
                "f"(v[6]), "f"(v[7]) : "memory");
 }
 
-// One token row, 16 features starting at f: convert, apply the epilogue, store.
+__device__ __forceinline__ void st_global_b32x8(void* p, const uint32_t* v) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+
+// One token row, 16 features starting at f: the bf16 results (8 words, or 4 where gate and up make one) into w, fp32 results to memory.
 template <int EPI>
-__device__ __forceinline__ void store16(const gemm::Params& p, int n, int f, const uint32_t* q) {
+__device__ __forceinline__ void finish16(const gemm::Params& p, int n, int f, const uint32_t* q, uint32_t* w) {
   float v[16];
 #pragma unroll
   for (int j = 0; j < 16; j++) v[j] = __uint_as_float(q[j]);
@@ -162,18 +152,12 @@ __device__ __forceinline__ void store16(const gemm::Params& p, int n, int f, con
       d2[1] = make_uint4(pack_bf16(v[8], v[9]), pack_bf16(v[10], v[11]), pack_bf16(v[12], v[13]), pack_bf16(v[14], v[15]));
     }
   } else if (EPI == gemm::kEpiClampGlu) {
-    float o[8];
 #pragma unroll
-    for (int j = 0; j < 8; j++) o[j] = gemm::clamp_glu(v[2 * j], v[2 * j + 1], p.act_a, p.act_b, p.act_c);
-    *reinterpret_cast<uint4*>(p.y + size_t(n) * p.ldy + (f >> 1)) =
-        make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7]));
-  } else if (EPI == 1) {
-    uint4 o;
-    o.x = pack_bf16(silu_mul_bf16(v[0], v[1]), silu_mul_bf16(v[2], v[3]));
-    o.y = pack_bf16(silu_mul_bf16(v[4], v[5]), silu_mul_bf16(v[6], v[7]));
-    o.z = pack_bf16(silu_mul_bf16(v[8], v[9]), silu_mul_bf16(v[10], v[11]));
-    o.w = pack_bf16(silu_mul_bf16(v[12], v[13]), silu_mul_bf16(v[14], v[15]));
-    *reinterpret_cast<uint4*>(p.y + size_t(n) * p.ldy + (f >> 1)) = o;
+    for (int j = 0; j < 4; j++)
+      w[j] = pack_bf16(gemm::clamp_glu(v[4 * j], v[4 * j + 1], p.act_a, p.act_b, p.act_c), gemm::clamp_glu(v[4 * j + 2], v[4 * j + 3], p.act_a, p.act_b, p.act_c));
+  } else if (EPI == gemm::kEpiSiluMul) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) w[j] = pack_bf16(silu_mul_bf16(v[4 * j], v[4 * j + 1]), silu_mul_bf16(v[4 * j + 2], v[4 * j + 3]));
   } else {
     if (p.act != gemm::kActNone && f < p.act_m) {   // act_m is a multiple of 16
       if (p.act == gemm::kActSilu) {
@@ -187,18 +171,57 @@ __device__ __forceinline__ void store16(const gemm::Params& p, int n, int f, con
         for (int j = 0; j < 16; j++) v[j] = gemm::apply_act(v[j], p.act, p.act_a);
       }
     }
-    uint4 o0, o1;
-    o0.x = pack_bf16(v[0], v[1]);   o0.y = pack_bf16(v[2], v[3]);   o0.z = pack_bf16(v[4], v[5]);   o0.w = pack_bf16(v[6], v[7]);
-    o1.x = pack_bf16(v[8], v[9]);   o1.y = pack_bf16(v[10], v[11]); o1.z = pack_bf16(v[12], v[13]); o1.w = pack_bf16(v[14], v[15]);
-    uint4* dst = reinterpret_cast<uint4*>(p.y + size_t(n) * p.ldy + f);
-    dst[0] = o0;
-    dst[1] = o1;
+#pragma unroll
+    for (int j = 0; j < 8; j++) w[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
+  }
+}
+// 32 features of one token row.  The rows of a warp lie far apart in memory, so the stores cost a pass of the load / store unit per row and instruction: 32 bytes at a time
+// (p.wide: rows and base allow it) are half as many as 16.
+template <int EPI>
+__device__ __forceinline__ void store32(const gemm::Params& p, int n, int f, const uint32_t* q) {
+  uint32_t w[16];
+  constexpr bool kHalf = EPI == gemm::kEpiSiluMul || EPI == gemm::kEpiClampGlu;
+  finish16<EPI>(p, n, f, q, w);
+  const bool second = f + 16 < p.M;                 // M is a multiple of 16
+  if (second) finish16<EPI>(p, n, f + 16, q + 16, w + (kHalf ? 4 : 8));
+  if constexpr (EPI != gemm::kEpiF32) {
+    __nv_bfloat16* dst = p.y + size_t(n) * p.ldy + (kHalf ? f >> 1 : f);
+    if (kHalf) {
+      if (p.wide && second) {
+        st_global_b32x8(dst, w);
+      } else {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        if (second) *reinterpret_cast<uint4*>(dst + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+      }
+    } else if (p.wide) {
+      st_global_b32x8(dst, w);
+      if (second) st_global_b32x8(dst + 16, w + 8);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (j < 2 || second) *reinterpret_cast<uint4*>(dst + 8 * j) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+    }
   }
 }
 
+// cos and sin of 16 channels for a row's position, rounded as the two-kernel form rounds them
+struct Angles { float c[16], s[16]; };
+__device__ __forceinline__ void ld_global_f32x8(const float* p, float* v) {
+  asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
+}
+__device__ __forceinline__ void load_angles(const gemm::Params& p, int pos, int d, Angles& a) {
+  const float* t = p.rope.cos_sin + size_t(pos) * 128 + d;
+  ld_global_f32x8(t, a.c);
+  ld_global_f32x8(t + 8, a.c + 8);
+  ld_global_f32x8(t + 64, a.s);
+  ld_global_f32x8(t + 72, a.s + 8);
+#pragma unroll
+  for (int j = 0; j < 16; j++) { a.c[j] = bf16_round(a.c[j]); a.s[j] = bf16_round(a.s[j]); }
+}
 // One token row, 16 channels d .. of a head and their rotation partners 64 further (`a`, `b`: accumulators): bias, rounding to bf16, rotation, stores to the activations and
 // the cache.  Same arithmetic as k_gemm_qkv_rope.
-__device__ __forceinline__ void store_rope16(const gemm::Params& p, int n, int head, int d, int pos, long long slot, const uint32_t* a, const uint32_t* b) {
+__device__ __forceinline__ void store_rope16(const gemm::Params& p, int n, int head, int d, const Angles& g, long long slot, const uint32_t* a, const uint32_t* b) {
   float lo[16], hi[16];
 #pragma unroll
   for (int j = 0; j < 16; j++) { lo[j] = __uint_as_float(a[j]); hi[j] = __uint_as_float(b[j]); }
@@ -208,27 +231,15 @@ __device__ __forceinline__ void store_rope16(const gemm::Params& p, int n, int h
     for (int j = 0; j < 16; j++) { lo[j] += __bfloat162float(bias[j]); hi[j] += __bfloat162float(bias[64 + j]); }
   }
   if (head < p.rope.nq + p.rope.nkv) {
-    const float4* c4 = reinterpret_cast<const float4*>(p.rope.cos_sin + size_t(pos) * 128 + d);
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const float4 c = c4[q], s = c4[16 + q];
-      const float cs[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const int j = 4 * q + e;
-        gemm::rotate(bf16_round(lo[j]), bf16_round(hi[j]), bf16_round(cs[e]), bf16_round(sn[e]), lo[j], hi[j]);
-      }
-    }
+    for (int j = 0; j < 16; j++) gemm::rotate(bf16_round(lo[j]), bf16_round(hi[j]), g.c[j], g.s[j], lo[j], hi[j]);
   }
-  uint4 l0, l1, h0, h1;
-  l0.x = pack_bf16(lo[0], lo[1]);   l0.y = pack_bf16(lo[2], lo[3]);   l0.z = pack_bf16(lo[4], lo[5]);   l0.w = pack_bf16(lo[6], lo[7]);
-  l1.x = pack_bf16(lo[8], lo[9]);   l1.y = pack_bf16(lo[10], lo[11]); l1.z = pack_bf16(lo[12], lo[13]); l1.w = pack_bf16(lo[14], lo[15]);
-  h0.x = pack_bf16(hi[0], hi[1]);   h0.y = pack_bf16(hi[2], hi[3]);   h0.z = pack_bf16(hi[4], hi[5]);   h0.w = pack_bf16(hi[6], hi[7]);
-  h1.x = pack_bf16(hi[8], hi[9]);   h1.y = pack_bf16(hi[10], hi[11]); h1.z = pack_bf16(hi[12], hi[13]); h1.w = pack_bf16(hi[14], hi[15]);
-  auto put = [&](__nv_bfloat16* row) {
-    uint4* x = reinterpret_cast<uint4*>(row + d);
-    uint4* y = reinterpret_cast<uint4*>(row + d + 64);
-    x[0] = l0; x[1] = l1; y[0] = h0; y[1] = h1;
+  uint32_t w[16];
+#pragma unroll
+  for (int j = 0; j < 8; j++) { w[j] = pack_bf16(lo[2 * j], lo[2 * j + 1]); w[8 + j] = pack_bf16(hi[2 * j], hi[2 * j + 1]); }
+  auto put = [&](__nv_bfloat16* row) {                // 32-byte aligned: see tbv_op_gemm_qkv_rope
+    st_global_b32x8(row + d, w);
+    st_global_b32x8(row + d + 64, w + 8);
   };
   put(p.y + size_t(n) * p.ldy + head * 128);
   if (slot >= 0 && head >= p.rope.nq) {
@@ -242,7 +253,7 @@ __device__ __forceinline__ void store_rope16(const gemm::Params& p, int n, int h
 template <int EPI, int FEAT, typename F>
 __device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok, int f0, uint32_t trow, F release) {
   if constexpr (EPI == gemm::kEpiRope) {
-    // rotation partners lie 64 columns apart: 16 channels of a head and their partners at a time
+    // rotation partners lie 64 columns apart: 16 channels of every head of the tile and their partners at a time, with the angles they share
     int pos = 0;
     long long slot = -1;
     if (row_ok) {
@@ -250,19 +261,25 @@ __device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok,
       pos = pos < 0 ? 0 : (pos >= p.rope.max_pos ? p.rope.max_pos - 1 : pos);
       if (p.rope.slot_mapping) slot = p.rope.slot_mapping[n];
     }
+    const bool turned = (f0 >> 7) < p.rope.nq + p.rope.nkv;       // otherwise the tile holds values only
+    Angles g;
 #pragma unroll 1
-    for (int c = 0; c < FEAT; c += c % 128 == 48 ? 80 : 16) {     // 0 16 32 48 128 144 160 176
-      uint32_t a[16], b[16];
-      __syncwarp();
-      tmem_ld16(trow + uint32_t(c), a);
-      tmem_ld16(trow + uint32_t(c + 64), b);
-      tmem_ld_wait();
-      if (c + 80 == FEAT) {
-        tc_fence_before();
+    for (int d = 0; d < 64; d += 16) {
+      if (turned) load_angles(p, pos, d, g);
+#pragma unroll
+      for (int h = 0; h < FEAT; h += 128) {
+        uint32_t a[16], b[16];
         __syncwarp();
-        release();
+        tmem_ld16(trow + uint32_t(h + d), a);
+        tmem_ld16(trow + uint32_t(h + d + 64), b);
+        tmem_ld_wait();
+        if (d == 48 && h + 128 == FEAT) {
+          tc_fence_before();
+          __syncwarp();
+          release();
+        }
+        if (row_ok && f0 + h < p.M) store_rope16(p, n, (f0 + h) >> 7, d, g, slot, a, b);   // M is a multiple of 128
       }
-      if (row_ok && f0 + c < p.M) store_rope16(p, n, (f0 + c) >> 7, c & 127, pos, slot, a, b);   // M is a multiple of 128
     }
   } else {
     for (int c = 0; c < FEAT; c += 32) {
@@ -276,28 +293,25 @@ __device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok,
         __syncwarp();
         release();
       }
-      if (!row_ok) continue;
-      if (f0 + c < p.M) store16<EPI>(p, n, f0 + c, r);               // M is a multiple of 16
-      if (f0 + c + 16 < p.M) store16<EPI>(p, n, f0 + c + 16, r + 16);
+      if (row_ok && f0 + c < p.M) store32<EPI>(p, n, f0 + c, r);
     }
   }
 }
 
-// EPI 0: store (+bias); 1: SiLU-mul over interleaved gate/up features (output has M / 2 features); 2: fp32 store with
-// an activation; 3: clamped gated unit over interleaved gate/up features; 4: rotation and cache write of a qkv projection.
-// ROWS: row-grouped problem (p.row_off).
+// EPI (gemm::Epi) of all kernels here: 0 store (+bias); 1 SiLU-mul over interleaved gate/up features (output has M / 2 features); 2 fp32 store with
+// an activation; 3 clamped gated unit over interleaved gate/up features; 4 rotation and cache write of a qkv projection.
+// ROWS: row-grouped problem (p.row_off; TH = 1).
 template <int EPI, int TH, bool ROWS>
 __global__ void __launch_bounds__(Shape<TH>::kThreads, 1)
 k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ gemm::Params p) {
   using S = Shape<TH>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ PSmem s;
+  __shared__ typename std::conditional<ROWS, RowGroups, int>::type groups;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
-  const int tok_tiles = (p.N + S::kTok - 1) / S::kTok, feat_tiles = (p.M + kFeatTile - 1) / kFeatTile;
-  const int nkb = p.kb_total;
-  __shared__ typename std::conditional<ROWS, RowGroups, int>::type groups;
+  const int tok_tiles = (p.N + S::kTok - 1) / S::kTok, feat_tiles = (p.M + kFeatTile - 1) / kFeatTile, nkb = p.kb_total;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < S::kStages; i++) {
@@ -325,73 +339,66 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
   pdl::launch_dependents();
   int tiles = tok_tiles * feat_tiles;
   if constexpr (ROWS) {
-    // the groups' rows were counted on the device by a kernel before this one
-    pdl::grid_dependency_wait();
-    count_tiles(groups, p, S::kTok, feat_tiles, S::kThreads);
+    pdl::grid_dependency_wait();                 // the groups' rows were counted on the device by a kernel before this one
+    count_tiles(groups, p, feat_tiles);
     tiles = groups.tile[p.groups];
   }
   const int my_tiles = int(blockIdx.x) < tiles ? (tiles - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x) : 0;
   const int ngroups = p.groups, feats = p.M, all_rows = p.N;
   // (by value: a capture of the parameter block would put it in local memory)
-  auto locate = [=](int tile) -> At { return find_tile<ROWS, S::kTok, kFeatTile>(groups, tile, tok_tiles, ngroups, feats, all_rows); };
+  auto locate = [=](int tile) -> At {
+    if constexpr (ROWS) return find_tile(groups, tile, ngroups, feats);
+    const int f0 = tile / tok_tiles * kFeatTile;
+    return At{tile % tok_tiles * S::kTok, all_rows, f0, f0};
+  };
   const uint32_t tmem0 = s.tmem_base;
   volatile int* abortp = &s.abort_flag;
 
   if (warp == 0 && lane == 0) {
     // ---- TMA producer: one flat sequence of k-blocks over all of this CTA's tiles ----
     const uint64_t pol_x = policy_evict_last();
-    const long total = long(my_tiles) * nkb;
-    long issued = 0;
     // Weights are never written by a kernel: the first ring fill of weight tiles goes out before the
     // preceding kernel has finished; the activations follow once it has.
-    const int pre = total < S::kStages ? int(total) : S::kStages;
+    const int pre = my_tiles ? min(S::kStages, nkb) : 0;
+    At at = my_tiles ? locate(int(blockIdx.x)) : At{};
     for (int i = 0; i < pre; i++) {
-      const int tile = int(blockIdx.x) + (i / nkb) * int(gridDim.x), kb = i % nkb;
       const uint32_t fb = smem_u32(&s.full[i]);
       mbar_expect_tx(fb, S::kStageBytes);
-      tma_load_2d(base + i * S::kStageBytes + S::kXBytes, &tmW, kb * gemm::kBK, locate(tile).w0, fb);
+      tma_load_2d(base + i * S::kStageBytes + S::kXBytes, &tmW, i * gemm::kBK, at.w0, fb);
     }
     pdl::grid_dependency_wait();
-    for (int i = 0; i < pre; i++) {
-      const int tile = int(blockIdx.x) + (i / nkb) * int(gridDim.x), kb = i % nkb;
-      tma_load_2d_hint(base + i * S::kStageBytes, &tmX, kb * gemm::kBK, locate(tile).n0, smem_u32(&s.full[i]), pol_x);
-    }
-    issued = pre;
-    int cur = -1;
-    At at{};
-    for (long i = pre; i < total; i++) {
-      const int st = int(i % S::kStages);
-      const uint32_t ph = uint32_t(i / S::kStages) & 1u;
-      if (!mbar_wait(smem_u32(&s.empty[st]), ph ^ 1u, abortp, p.limit_ns)) break;
-      const int tile = int(blockIdx.x) + int(i / nkb) * int(gridDim.x), kb = int(i % nkb);
-      if (tile != cur) at = locate(cur = tile);
-      const uint32_t fb = smem_u32(&s.full[st]);
-      mbar_expect_tx(fb, S::kStageBytes);
-      tma_load_2d_hint(base + st * S::kStageBytes, &tmX, kb * gemm::kBK, at.n0, fb, pol_x);
-      tma_load_2d(base + st * S::kStageBytes + S::kXBytes, &tmW, kb * gemm::kBK, at.w0, fb);
-      issued = i + 1;
-    }
-    if (*abortp) {
-      // gave up: let the copies already in flight land before this CTA's shared memory goes away
-      for (long i = issued > S::kStages ? issued - S::kStages : 0; i < issued; i++) {
-        const uint32_t fb = smem_u32(&s.full[i % S::kStages]);
-        const uint32_t ph = uint32_t(i / S::kStages) & 1u;
-        for (int spin = 0; spin < 20000 && !mbar_try_wait(fb, ph); spin++) __nanosleep(50);
+    for (int i = 0; i < pre; i++) tma_load_2d_hint(base + i * S::kStageBytes, &tmX, i * gemm::kBK, at.n0, smem_u32(&s.full[i]), pol_x);
+    int st = pre == S::kStages ? 0 : pre;
+    uint32_t ph = pre == S::kStages ? 1u : 0u;   // of the ring's current round
+    bool ok = true;
+    for (int t = 0; t < my_tiles && ok; t++) {
+      if (t) at = locate(int(blockIdx.x) + t * int(gridDim.x));
+      for (int kb = t ? 0 : pre; kb < nkb; kb++) {
+        if (!mbar_wait(smem_u32(&s.empty[st]), ph ^ 1u, abortp, p.limit_ns)) { ok = false; break; }
+        const uint32_t fb = smem_u32(&s.full[st]);
+        mbar_expect_tx(fb, S::kStageBytes);
+        tma_load_2d_hint(base + st * S::kStageBytes, &tmX, kb * gemm::kBK, at.n0, fb, pol_x);
+        tma_load_2d(base + st * S::kStageBytes + S::kXBytes, &tmW, kb * gemm::kBK, at.w0, fb);
+        if (++st == S::kStages) { st = 0; ph ^= 1u; }
       }
+    }
+    if (*abortp && pre) {
+      // gave up: let the copies already in flight land before this CTA's shared memory goes away (a millisecond is many times what a copy takes)
+      const unsigned long long t0 = globaltimer();
+      while (globaltimer() - t0 < 1000000ull) __nanosleep(1000);
     }
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer ----
     const uint32_t idesc = umma_idesc_bf16(128, kFeatTile);
-    long i = 0;
+    int st = 0;
+    uint32_t ph = 0;
     bool ok = true;
     for (int t = 0; t < my_tiles && ok; t++) {
       const int buf = t % S::kBuffers, use = t / S::kBuffers;
       // the epilogue must have drained this accumulator set (kBuffers tiles ago); passes at once on first use
       if (!mbar_wait(smem_u32(&s.acc_empty[buf]), (uint32_t(use) & 1u) ^ 1u, abortp, p.limit_ns)) break;
       tc_fence_after();
-      for (int kb = 0; kb < nkb; kb++, i++) {
-        const int st = int(i % S::kStages);
-        const uint32_t ph = uint32_t(i / S::kStages) & 1u;
+      for (int kb = 0; kb < nkb; kb++) {
         if (!mbar_wait(smem_u32(&s.full[st]), ph, abortp, p.limit_ns)) { ok = false; break; }
         tc_fence_after();
         const uint64_t bd = umma_desc_sw128(base + st * S::kStageBytes + S::kXBytes);
@@ -404,6 +411,7 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
             umma_bf16(tmem_d, ad + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
         }
         umma_commit(smem_u32(&s.empty[st]));
+        if (++st == S::kStages) { st = 0; ph ^= 1u; }
       }
       if (ok) umma_commit(smem_u32(&s.acc_full[buf]));
     }
@@ -412,16 +420,12 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
     const int quarter = warp & 3, half = TH == 1 ? 0 : (warp - 2) >> 2;
     for (int t = 0; t < my_tiles; t++) {
       const int buf = t % S::kBuffers, use = t / S::kBuffers;
-      bool ok = mbar_wait(smem_u32(&s.acc_full[buf]), uint32_t(use) & 1u, abortp, p.limit_ns);
-      ok = __all_sync(0xffffffffu, ok);   // reconverge before the warp-wide TMEM loads
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s.acc_full[buf]), uint32_t(use) & 1u, abortp, p.limit_ns));   // together, before the warp-wide TMEM loads
       if (!ok) break;
       tc_fence_after();
-      const int tile = int(blockIdx.x) + t * int(gridDim.x);
-      const At at = locate(tile);
+      const At at = locate(int(blockIdx.x) + t * int(gridDim.x));
       const int n = at.n0 + half * 128 + quarter * 32 + lane;   // token row
-      const int f0 = at.f0;
-      const uint32_t trow = tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t((TH == 1 ? buf : half) * kFeatTile);
-      drain<EPI, kFeatTile>(p, n, n < at.nend, f0, trow, [&] {
+      drain<EPI, kFeatTile>(p, n, n < at.nend, at.f0, tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t((TH == 1 ? buf : half) * kFeatTile), [&] {
         if (lane == 0) mbar_arrive(smem_u32(&s.acc_empty[buf]));
       });
     }
@@ -438,10 +442,8 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
   if (threadIdx.x == 0 && s.abort_flag && p.err) atomicExch(p.err, 1);
 }
 
-bool g_attr = false;
-
 template <int EPI, int TH, bool ROWS = false>
-cudaError_t launch(const void* w, const void* x, const gemm::Params& p, int ldx, cudaStream_t st, int* map_rc) {
+cudaError_t launch_tok(const void* w, const void* x, const gemm::Params& p, int ldx, cudaStream_t st, int* map_rc) {
   using S = Shape<TH>;
   CUtensorMap tmX, tmW;
   *map_rc = 0;
@@ -450,9 +452,11 @@ cudaError_t launch(const void* w, const void* x, const gemm::Params& p, int ldx,
     *map_rc = -3;
     return cudaSuccess;
   }
-  const int tiles = ((ROWS ? p.x_rows / S::kTok + p.groups : (p.N + S::kTok - 1) / S::kTok)) * ((p.M + kFeatTile - 1) / kFeatTile);   // ROWS: at most
+  constexpr size_t smem = size_t(S::kStages) * S::kStageBytes + 1024;
+  static const cudaError_t attr = cudaFuncSetAttribute(k_gemm_tok<EPI, TH, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (attr != cudaSuccess) return attr;
+  const int tiles = (ROWS ? p.x_rows / S::kTok + p.groups : (p.N + S::kTok - 1) / S::kTok) * ((p.M + kFeatTile - 1) / kFeatTile);   // ROWS: at most
   const int sms = tbvops::sm_count();
-  const size_t smem = size_t(S::kStages) * S::kStageBytes + 1024;
   return pdl::launch(k_gemm_tok<EPI, TH, ROWS>, dim3(tiles < sms ? tiles : sms), dim3(S::kThreads), smem, st, 1, tmX, tmW, p);
 }
 
@@ -460,33 +464,27 @@ cudaError_t launch(const void* w, const void* x, const gemm::Params& p, int ldx,
 
 namespace tbvops {
 
-// Which form takes an [N tokens] x [M features] problem: 0 = the decode-form kernel (gemm.cu), 1 / 2 = this
-// kernel with 128- / 256-token tiles.  `mode`: 1 = choose by estimated time, 2 / 3 = force TH 1 / 2 wherever
-// the shape allows (tests, measurements).
+// Which form takes an [N tokens] x [M features] problem: 0 = the decode-form kernel (gemm.cu), 1 / 2 = k_gemm_tok with 128- / 256-token tiles.  `mode`: 1 = choose,
+// 2 / 3 = force TH 1 / 2 wherever the shape allows (tests, measurements; TH 2 exists for plain stores).
 //
-// Estimated time in units of one 128 x 256 x K tile at full tensor rate.  Tiles are equal-sized and every CTA
-// walks ceil(tiles / SMs) of them, so a persistent schedule costs rounds * tile size / efficiency; the
-// decode-form kernel runs 2 CTAs per SM scheduled by the hardware and costs tiles / SMs / efficiency.
-// Efficiencies are measured on B200 at 4096 tokens (Llama-3-8B shapes).
+// From 384 tokens on k_gemm_tok wins but where few tiles exist, so that most SMs idle while the decode form shares K out over a cluster, and
+// K is not long enough to make up for it (512 tokens, fp32: 2048 x 4096 19 us against 29; 1024 tokens 28.6 against 30; 512 tokens, 4096 x 14336 74 against 88; but
+// 512 tokens, 4096 x 4096 37 against 28, 2048 x 7168 48 against 46).  Plain stores take the wide tiles where those need no more rounds over the SMs than narrow ones,
+// a round of them taking nine tenths of two narrow rounds (1024 tokens, 4096 x 4096: one round either way, 51 us against 31).
 int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode) {
   if (!(N >= 384 && (M % 16) == 0 && (K % 8) == 0 && (ldy % 8) == 0 && epi >= 0 && epi <= 3)) return 0;
-  if (mode == 2) return 1;
-  if (mode == 3) return 2;
-  const double sms = sm_count();
-  const long ft = (M + kFeatTile - 1) / kFeatTile;
-  const long t1 = long((N + 127) / 128) * ft, t2 = long((N + 255) / 256) * ft;
-  const double r1 = double((t1 + long(sms) - 1) / long(sms)), r2 = double((t2 + long(sms) - 1) / long(sms));
-  const double e_dec = double((M + 127) / 128) * ((N + 255) / 256) / sms / kEffDecode[epi & 1];
-  const double e1 = r1 / kEffTok1, e2 = 2.0 * r2 / kEffTok2;
-  if (e_dec <= e1 && e_dec <= e2) return 0;
-  return e1 <= e2 ? 1 : 2;
+  const bool stores = epi == gemm::kEpiStore || epi == gemm::kEpiF32;
+  if (mode >= 2) return mode == 3 && stores ? 2 : 1;
+  const long sms = sm_count(), ft = (M + kFeatTile - 1) / kFeatTile, t1 = (N + 127) / 128 * ft, t2 = (N + 255) / 256 * ft;
+  if (t1 * 4 <= sms && K <= 4096) return 0;
+  return stores && 18 * ((t2 + sms - 1) / sms) <= 10 * ((t1 + sms - 1) / sms) ? 2 : 1;
 }
 
-// Row-grouped: the decode form re-reads a group's weights for every tile of up to 128 rows; this form wastes what a group's last tile lacks.
+// Row-grouped: 0 the decode form, 1 k_gemm_tok.  The decode form re-reads a group's weights for every tile of up to 128 rows; k_gemm_tok wastes what a group's last
+// tile lacks.
 int gemm_tok_rows_choose(int M, int x_rows, int groups) {
   if ((M % 16) || groups > kMaxRowGroups) return 0;
-  const int avg = x_rows / groups;
-  return avg >= 384 ? 2 : (avg >= 64 ? 1 : 0);
+  return x_rows / groups >= 64 ? 1 : 0;
 }
 
 int gemm_tok_launch(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi, int th,
@@ -499,46 +497,22 @@ int gemm_tok_launch(const void* w, const void* x, void* y, const void* bias, int
 }
 
 int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, int epi, int th, void* stream) {
-  p.bn = kFeatTile; p.splits = 1; p.stages = th == 1 ? 4 : 3;
+  p.bn = kFeatTile; p.splits = 1;
   p.kb_total = (p.K + 63) / 64;
+  p.wide = !(reinterpret_cast<uintptr_t>(p.y) & 31) && p.ldy % 16 == 0;
   p.limit_ns = 2000000000ull;
   p.err = gemm_err_flag();
-  if (!g_attr) {
-    cudaError_t a[14] = {cudaFuncSetAttribute(k_gemm_tok<4, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                        cudaFuncSetAttribute(k_gemm_tok<4, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                        cudaFuncSetAttribute(k_gemm_tok<0, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                        cudaFuncSetAttribute(k_gemm_tok<1, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                        cudaFuncSetAttribute(k_gemm_tok<2, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                        cudaFuncSetAttribute(k_gemm_tok<3, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                        cudaFuncSetAttribute(k_gemm_tok<0, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                        cudaFuncSetAttribute(k_gemm_tok<1, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                        cudaFuncSetAttribute(k_gemm_tok<2, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                        cudaFuncSetAttribute(k_gemm_tok<3, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                         cudaFuncSetAttribute(k_gemm_tok<0, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024),
-                         cudaFuncSetAttribute(k_gemm_tok<0, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024),
-                         cudaFuncSetAttribute(k_gemm_tok<3, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024),
-                         cudaFuncSetAttribute(k_gemm_tok<3, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)};
-    for (cudaError_t e : a)
-      if (e != cudaSuccess) return -1;
-    g_attr = true;
-  }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int map_rc = 0;
   cudaError_t e;
   if (p.row_off) {
-    if (epi == gemm::kEpiClampGlu) e = th == 2 ? launch<3, 2, true>(w, x, p, ldx, st, &map_rc) : launch<3, 1, true>(w, x, p, ldx, st, &map_rc);
-    else e = th == 2 ? launch<0, 2, true>(w, x, p, ldx, st, &map_rc) : launch<0, 1, true>(w, x, p, ldx, st, &map_rc);
-  } else switch (epi * 2 + (th == 2 ? 1 : 0)) {
-    case 1: e = launch<0, 2>(w, x, p, ldx, st, &map_rc); break;
-    case 2: e = launch<1, 1>(w, x, p, ldx, st, &map_rc); break;
-    case 3: e = launch<1, 2>(w, x, p, ldx, st, &map_rc); break;
-    case 4: e = launch<2, 1>(w, x, p, ldx, st, &map_rc); break;
-    case 5: e = launch<2, 2>(w, x, p, ldx, st, &map_rc); break;
-    case 6: e = launch<3, 1>(w, x, p, ldx, st, &map_rc); break;
-    case 8: e = launch<4, 1>(w, x, p, ldx, st, &map_rc); break;
-    case 9: e = launch<4, 2>(w, x, p, ldx, st, &map_rc); break;
-    case 7: e = launch<3, 2>(w, x, p, ldx, st, &map_rc); break;
-    default: e = launch<0, 1>(w, x, p, ldx, st, &map_rc); break;
+    e = epi == gemm::kEpiClampGlu ? launch_tok<3, 1, true>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1, true>(w, x, p, ldx, st, &map_rc);
+  } else switch (epi) {
+    case gemm::kEpiSiluMul: e = launch_tok<1, 1>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiF32: e = th == 2 ? launch_tok<2, 2>(w, x, p, ldx, st, &map_rc) : launch_tok<2, 1>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiClampGlu: e = launch_tok<3, 1>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiRope: e = launch_tok<4, 1>(w, x, p, ldx, st, &map_rc); break;
+    default: e = th == 2 ? launch_tok<0, 2>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1>(w, x, p, ldx, st, &map_rc); break;
   }
   if (map_rc != 0) return map_rc;
   if (e != cudaSuccess) {

@@ -187,11 +187,11 @@ extern "C" int tbv_op_gemm_qkv_rope(const void* w, const void* x, void* qkv, con
   if (M != (nq + 2 * nkv) * 128 || N <= 0 || (K % 8) || (ldx % 8) || (ldy % 8)) return -2;
   const gemm::Rope ra{static_cast<const int*>(positions), static_cast<const float*>(cos_sin), static_cast<const long long*>(slot_mapping),
                       static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), nq, nkv, max_pos};
-  // Hundreds of tokens: the many-token kernel with this epilogue, wherever it takes the plain product (4096 tokens, 6144 x 4096: 186 us against 226 here, where two CTAs
+  // Hundreds of tokens: the many-token kernel with this epilogue, wherever it takes the plain product (4096 tokens, 6144 x 4096: 159 us against 226 here, where two CTAs
   // per SM stage every tile through shared memory).
   if (splits_hint <= 0 && !((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(cos_sin) | reinterpret_cast<uintptr_t>(k_cache) |
-                             reinterpret_cast<uintptr_t>(v_cache)) & 15u)) {
-    const int persist = tbvops::gemm_persist_mode(), th = persist > 0 ? tbvops::gemm_tok_choose(M, N, K, ldy, gemm::kEpiStore, persist) : 0;
+                             reinterpret_cast<uintptr_t>(v_cache)) & 31u) && ldy % 16 == 0) {
+    const int persist = tbvops::gemm_persist_mode(), th = persist > 0 ? tbvops::gemm_tok_choose(M, N, K, ldy, gemm::kEpiSiluMul, persist) : 0;   // an epilogue that computes
     if (th > 0) {
       gemm::Params p{};
       p.M = M; p.N = N; p.K = K; p.ldy = ldy;

@@ -34,3 +34,30 @@ def test_qkv_projection_of_many_tokens_equals_gemm_then_rope(mode, T, nq, nkv, K
         ops.gemm_persist_mode(None)
     assert not ops.gemm_error()
     assert torch.equal(got, want) and torch.equal(kc[2], kc[0]) and torch.equal(kc[3], kc[1])
+
+
+@pytest.mark.parametrize("N,M,K", [(384, 16, 64), (513, 272, 72), (1000, 640, 1000), (1025, 2064, 520), (2300, 4096, 136)])
+def test_tile_shapes_give_the_same_bits(N, M, K):
+    """Every epilogue, remainders of tokens, features and k-blocks: one accumulator per result, summed in the order of k in all forms."""
+    from libtbvcoll_b200 import ops
+    x, w, b = rnd(N, K, seed=1), rnd(M, K, seed=2, scale=0.1), rnd(M, seed=3)
+
+    def run():
+        f32, copy = torch.zeros(N, M, device=DEV), torch.zeros(N, M, dtype=torch.bfloat16, device=DEV)
+        ops.linear(x, w, f32, bias=b, act=ops.ACT_SOFTCAP, act_arg=3.0, copy=copy)
+        out = torch.zeros(N, M, dtype=torch.bfloat16, device=DEV)
+        ops.linear(x, w, out, act=ops.ACT_SILU, act_cols=16)
+        glu = torch.zeros(N, M // 2, dtype=torch.bfloat16, device=DEV)
+        ops.linear(x, w, glu, glu=(2.0, 1.7))
+        return [f32, copy, out, glu, ops.gemm(x, w, bias=b), ops.gemm(x, w, epi=ops.EPI_SILU_MUL)]
+    try:
+        ops.gemm_persist_mode(2)
+        want = run()
+        ops.gemm_persist_mode(3)
+        got = run()
+        torch.cuda.synchronize()
+    finally:
+        ops.gemm_persist_mode(None)
+    assert not ops.gemm_error()
+    for a, c in zip(got, want):
+        assert torch.equal(a, c)
