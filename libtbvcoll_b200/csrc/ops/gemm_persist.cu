@@ -7,7 +7,9 @@
 // features on UMMA N.  A thread of the epilogue then owns one token row and reads consecutive features per
 // TMEM load; gate/up pairs of the SiLU-mul epilogue sit in the same thread, so that epilogue needs no shuffles.
 //
-// Two tile shapes (template TH), both with all 512 TMEM columns of the SM in use:
+// Tile shapes (templates TH, FEAT); an SM takes in some 70 bytes per clock through TMA (measured with three quarters of the MMAs left out, 133 GB/s), which bounds the smaller ones:
+//   TH = 1, FEAT = 128  128 tokens x 128 features: a quarter less work per byte than 256 features, for problems whose wider tiles would leave SMs idle
+//           (1024 tokens, 2048 x 7168 37 us against 45, 512 tokens, 3072 x 2048 with rotation 20 against 23).
 //   TH = 1  128 tokens x 256 features, two accumulator sets: the epilogue of a tile runs under the MMAs of the next.  For epilogues that compute, and where
 //           tiles are few.  4096 tokens: 28672 x 4096 with the SiLU unit 641 us = 1500 TFLOP/s (848 with TH = 2), 6144 x 4096 with rotation 159 (166).
 //   TH = 2  256 tokens x 256 features as two 128-row MMAs that share one 256-row weight tile: a third less traffic per operation, but both accumulators belong
@@ -33,17 +35,16 @@ using namespace sm100;
 
 namespace {
 
-constexpr int kFeatTile = 256;                    // UMMA N
 constexpr int kHalfBytes = 128 * gemm::kBK * 2;      // one 128-token operand tile: 16 KB
-constexpr int kWBytes = kFeatTile * gemm::kBK * 2;   // 32 KB
-constexpr int kMaxStages = 4;
+constexpr int kMaxStages = 6;
 
-template <int TH> struct Shape {
+template <int TH, int FEAT> struct Shape {
   static constexpr int kTok = 128 * TH;                        // tokens per tile
   static constexpr int kXBytes = kHalfBytes * TH;
-  static constexpr int kStageBytes = kXBytes + kWBytes;        // 48 KB / 64 KB
-  static constexpr int kStages = TH == 1 ? 4 : 3;              // 192 KB of ring either way
+  static constexpr int kStageBytes = kXBytes + FEAT * gemm::kBK * 2;        // 48 / 32 / 64 KB
+  static constexpr int kStages = 192 * 1024 / kStageBytes;     // 4 / 6 / 3
   static constexpr int kBuffers = TH == 1 ? 2 : 1;             // accumulator sets that alternate between tiles
+  static constexpr int kCols = 2 * FEAT;                       // TMEM columns of two sets, or of two halves
   static constexpr int kEpiWarps = 4 * TH;
   static constexpr int kThreads = 64 + 32 * kEpiWarps;         // a warp of copies, one of products, the epilogue's
 };
@@ -55,6 +56,7 @@ struct RowGroups {
   int off[kMaxRowGroups + 1];      // first row of every group
   int tile[kMaxRowGroups + 1];     // first tile of every group
 };
+constexpr int kFeatTile = 256;     // of row-grouped problems
 
 // first token row, end of the rows, first feature and its weight row of a tile
 struct At { int n0, nend, f0, w0; };
@@ -72,7 +74,7 @@ __device__ __forceinline__ At find_tile(const RowGroups& groups, int tile, int n
 
 // Fills the table from the rows' offsets (device memory); whole CTA.
 __device__ __forceinline__ void count_tiles(RowGroups& groups, const gemm::Params& p, int feat_tiles) {
-  for (int g = threadIdx.x; g <= p.groups; g += Shape<1>::kThreads) groups.off[g] = p.row_off[g];
+  for (int g = threadIdx.x; g <= p.groups; g += 192) groups.off[g] = p.row_off[g];
   __syncthreads();
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x, per = (p.groups + 31) / 32, a = min(p.groups, lane * per), b = min(p.groups, a + per);
@@ -300,18 +302,18 @@ __device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok,
 
 // EPI (gemm::Epi) of all kernels here: 0 store (+bias); 1 SiLU-mul over interleaved gate/up features (output has M / 2 features); 2 fp32 store with
 // an activation; 3 clamped gated unit over interleaved gate/up features; 4 rotation and cache write of a qkv projection.
-// ROWS: row-grouped problem (p.row_off; TH = 1).
-template <int EPI, int TH, bool ROWS>
-__global__ void __launch_bounds__(Shape<TH>::kThreads, 1)
+// ROWS: row-grouped problem (p.row_off; TH = 1, FEAT = 256).
+template <int EPI, int TH, int FEAT, bool ROWS>
+__global__ void __launch_bounds__(Shape<TH, FEAT>::kThreads, 1)
 k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ gemm::Params p) {
-  using S = Shape<TH>;
+  using S = Shape<TH, FEAT>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ PSmem s;
   __shared__ typename std::conditional<ROWS, RowGroups, int>::type groups;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
-  const int tok_tiles = (p.N + S::kTok - 1) / S::kTok, feat_tiles = (p.M + kFeatTile - 1) / kFeatTile, nkb = p.kb_total;
+  const int tok_tiles = (p.N + S::kTok - 1) / S::kTok, feat_tiles = (p.M + FEAT - 1) / FEAT, nkb = p.kb_total;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < S::kStages; i++) {
@@ -326,7 +328,7 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&s.tmem_base), 512);
+    tmem_alloc(smem_u32(&s.tmem_base), S::kCols);
     tmem_relinquish();
   }
   if (warp == 0 && lane == 0) {
@@ -348,7 +350,7 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
   // (by value: a capture of the parameter block would put it in local memory)
   auto locate = [=](int tile) -> At {
     if constexpr (ROWS) return find_tile(groups, tile, ngroups, feats);
-    const int f0 = tile / tok_tiles * kFeatTile;
+    const int f0 = tile / tok_tiles * FEAT;
     return At{tile % tok_tiles * S::kTok, all_rows, f0, f0};
   };
   const uint32_t tmem0 = s.tmem_base;
@@ -389,7 +391,7 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
     }
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer ----
-    const uint32_t idesc = umma_idesc_bf16(128, kFeatTile);
+    const uint32_t idesc = umma_idesc_bf16(128, FEAT);
     int st = 0;
     uint32_t ph = 0;
     bool ok = true;
@@ -405,7 +407,7 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
 #pragma unroll
         for (int h = 0; h < TH; h++) {           // the 128-token halves share the weight tile
           const uint64_t ad = umma_desc_sw128(base + st * S::kStageBytes + h * kHalfBytes);
-          const uint32_t tmem_d = tmem0 + uint32_t((TH == 1 ? buf : h) * kFeatTile);
+          const uint32_t tmem_d = tmem0 + uint32_t((TH == 1 ? buf : h) * FEAT);
 #pragma unroll
           for (int k = 0; k < gemm::kBK / 16; k++)
             umma_bf16(tmem_d, ad + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
@@ -425,7 +427,7 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
       tc_fence_after();
       const At at = locate(int(blockIdx.x) + t * int(gridDim.x));
       const int n = at.n0 + half * 128 + quarter * 32 + lane;   // token row
-      drain<EPI, kFeatTile>(p, n, n < at.nend, at.f0, tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t((TH == 1 ? buf : half) * kFeatTile), [&] {
+      drain<EPI, FEAT>(p, n, n < at.nend, at.f0, tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t((TH == 1 ? buf : half) * FEAT), [&] {
         if (lane == 0) mbar_arrive(smem_u32(&s.acc_empty[buf]));
       });
     }
@@ -437,47 +439,50 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(s.tmem_base, 512);
+    tmem_dealloc(s.tmem_base, S::kCols);
   }
   if (threadIdx.x == 0 && s.abort_flag && p.err) atomicExch(p.err, 1);
 }
 
-template <int EPI, int TH, bool ROWS = false>
+template <int EPI, int TH, int FEAT, bool ROWS = false>
 cudaError_t launch_tok(const void* w, const void* x, const gemm::Params& p, int ldx, cudaStream_t st, int* map_rc) {
-  using S = Shape<TH>;
+  using S = Shape<TH, FEAT>;
   CUtensorMap tmX, tmW;
   *map_rc = 0;
   if (tbvops::make_tensor_map_bf16(&tmX, x, ROWS ? p.x_rows : p.N, p.K, ldx, S::kTok) != 0 ||
-      tbvops::make_tensor_map_bf16(&tmW, w, (unsigned long long)(ROWS ? p.groups : 1) * p.M, p.K, p.K, kFeatTile) != 0) {
+      tbvops::make_tensor_map_bf16(&tmW, w, (unsigned long long)(ROWS ? p.groups : 1) * p.M, p.K, p.K, FEAT) != 0) {
     *map_rc = -3;
     return cudaSuccess;
   }
   constexpr size_t smem = size_t(S::kStages) * S::kStageBytes + 1024;
-  static const cudaError_t attr = cudaFuncSetAttribute(k_gemm_tok<EPI, TH, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  static const cudaError_t attr = cudaFuncSetAttribute(k_gemm_tok<EPI, TH, FEAT, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (attr != cudaSuccess) return attr;
-  const int tiles = (ROWS ? p.x_rows / S::kTok + p.groups : (p.N + S::kTok - 1) / S::kTok) * ((p.M + kFeatTile - 1) / kFeatTile);   // ROWS: at most
+  const int tiles = (ROWS ? p.x_rows / S::kTok + p.groups : (p.N + S::kTok - 1) / S::kTok) * ((p.M + FEAT - 1) / FEAT);   // ROWS: at most
   const int sms = tbvops::sm_count();
-  return pdl::launch(k_gemm_tok<EPI, TH, ROWS>, dim3(tiles < sms ? tiles : sms), dim3(S::kThreads), smem, st, 1, tmX, tmW, p);
+  return pdl::launch(k_gemm_tok<EPI, TH, FEAT, ROWS>, dim3(tiles < sms ? tiles : sms), dim3(S::kThreads), smem, st, 1, tmX, tmW, p);
 }
 
 }  // namespace
 
 namespace tbvops {
 
-// Which form takes an [N tokens] x [M features] problem: 0 = the decode-form kernel (gemm.cu), 1 / 2 = k_gemm_tok with 128- / 256-token tiles.  `mode`: 1 = choose,
-// 2 / 3 = force TH 1 / 2 wherever the shape allows (tests, measurements; TH 2 exists for plain stores).
+// Which form takes an [N tokens] x [M features] problem: 0 = the decode-form kernel (gemm.cu), k_gemm_tok with 1 / 2 = 128- / 256-token tiles of 256 features, 3 = 128 x 128
+// tiles.  `mode`: 1 = choose, 2 / 3 / 4 = force the first / second / third tile wherever the shape allows (tests, measurements; 256-token tiles exist for plain stores).
 //
-// From 384 tokens on k_gemm_tok wins but where few tiles exist, so that most SMs idle while the decode form shares K out over a cluster, and
-// K is not long enough to make up for it (512 tokens, fp32: 2048 x 4096 19 us against 29; 1024 tokens 28.6 against 30; 512 tokens, 4096 x 14336 74 against 88; but
-// 512 tokens, 4096 x 4096 37 against 28, 2048 x 7168 48 against 46).  Plain stores take the wide tiles where those need no more rounds over the SMs than narrow ones,
-// a round of them taking nine tenths of two narrow rounds (1024 tokens, 4096 x 4096: one round either way, 51 us against 31).
+// Every CTA walks ceil(tiles / SMs) tiles.  A k-block of a 128 x 128 tile takes two thirds of the time of a 128 x 256 one (both bound by what TMA brings in), and one of
+// 256 x 256 nine tenths of two of those.  512 tokens, 4096 x 4096 24 / 28 / 45 us with 128 x 128 / 128 x 256 / 256 x 256 tiles,
+// 1024 tokens, 14336 x 2048 with the SiLU unit 75 / 61.
+// Fewer than 384 tokens, and problems of few tiles and not too long K, go to the decode form, which shares K out over clusters (512 tokens, fp32, 2048 x 4096: 19 us
+// against 24; 1024 tokens 28 against 24; 512 tokens, 2048 x 2048 15.3 against 13.5, 2048 x 7168 49 against 36).
 int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode) {
   if (!(N >= 384 && (M % 16) == 0 && (K % 8) == 0 && (ldy % 8) == 0 && epi >= 0 && epi <= 3)) return 0;
   const bool stores = epi == gemm::kEpiStore || epi == gemm::kEpiF32;
-  if (mode >= 2) return mode == 3 && stores ? 2 : 1;
-  const long sms = sm_count(), ft = (M + kFeatTile - 1) / kFeatTile, t1 = (N + 127) / 128 * ft, t2 = (N + 255) / 256 * ft;
-  if (t1 * 4 <= sms && K <= 4096) return 0;
-  return stores && 18 * ((t2 + sms - 1) / sms) <= 10 * ((t1 + sms - 1) / sms) ? 2 : 1;
+  if (mode >= 2) return mode == 4 ? 3 : (mode == 3 && stores ? 2 : 1);
+  const long sms = sm_count(), f256 = (M + 255) / 256, f128 = (M + 127) / 128, n128 = (N + 127) / 128, n256 = (N + 255) / 256;
+  auto rounds = [&](long tiles) { return (tiles + sms - 1) / sms; };
+  if (n128 * f128 * (K > 2048 ? 2 : 4) <= sms && K <= 4096) return 0;
+  if (2 * rounds(n128 * f128) < 3 * rounds(n128 * f256)) return 3;
+  return stores && 18 * rounds(n256 * f256) <= 10 * rounds(n128 * f256) ? 2 : 1;
 }
 
 // Row-grouped: 0 the decode form, 1 k_gemm_tok.  The decode form re-reads a group's weights for every tile of up to 128 rows; k_gemm_tok wastes what a group's last
@@ -497,7 +502,7 @@ int gemm_tok_launch(const void* w, const void* x, void* y, const void* bias, int
 }
 
 int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, int epi, int th, void* stream) {
-  p.bn = kFeatTile; p.splits = 1;
+  p.bn = 256; p.splits = 1;
   p.kb_total = (p.K + 63) / 64;
   p.wide = !(reinterpret_cast<uintptr_t>(p.y) & 31) && p.ldy % 16 == 0;
   p.limit_ns = 2000000000ull;
@@ -506,17 +511,21 @@ int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, in
   int map_rc = 0;
   cudaError_t e;
   if (p.row_off) {
-    e = epi == gemm::kEpiClampGlu ? launch_tok<3, 1, true>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1, true>(w, x, p, ldx, st, &map_rc);
+    e = epi == gemm::kEpiClampGlu ? launch_tok<3, 1, 256, true>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1, 256, true>(w, x, p, ldx, st, &map_rc);
   } else switch (epi) {
-    case gemm::kEpiSiluMul: e = launch_tok<1, 1>(w, x, p, ldx, st, &map_rc); break;
-    case gemm::kEpiF32: e = th == 2 ? launch_tok<2, 2>(w, x, p, ldx, st, &map_rc) : launch_tok<2, 1>(w, x, p, ldx, st, &map_rc); break;
-    case gemm::kEpiClampGlu: e = launch_tok<3, 1>(w, x, p, ldx, st, &map_rc); break;
-    case gemm::kEpiRope: e = launch_tok<4, 1>(w, x, p, ldx, st, &map_rc); break;
-    default: e = th == 2 ? launch_tok<0, 2>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiSiluMul: e = th == 3 ? launch_tok<1, 1, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<1, 1, 256>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiF32:
+      e = th == 3 ? launch_tok<2, 1, 128>(w, x, p, ldx, st, &map_rc) : th == 2 ? launch_tok<2, 2, 256>(w, x, p, ldx, st, &map_rc) : launch_tok<2, 1, 256>(w, x, p, ldx, st, &map_rc);
+      break;
+    case gemm::kEpiClampGlu: e = th == 3 ? launch_tok<3, 1, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<3, 1, 256>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiRope: e = th == 3 ? launch_tok<4, 1, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<4, 1, 256>(w, x, p, ldx, st, &map_rc); break;
+    default:
+      e = th == 3 ? launch_tok<0, 1, 128>(w, x, p, ldx, st, &map_rc) : th == 2 ? launch_tok<0, 2, 256>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1, 256>(w, x, p, ldx, st, &map_rc);
+      break;
   }
   if (map_rc != 0) return map_rc;
   if (e != cudaSuccess) {
-    fprintf(stderr, "[tbvops] many-token gemm launch failed: %s (M=%d N=%d K=%d tile %dx256)\n", cudaGetErrorString(e), p.M, p.N, p.K, 128 * th);
+    fprintf(stderr, "[tbvops] many-token gemm launch failed: %s (M=%d N=%d K=%d tile %d)\n", cudaGetErrorString(e), p.M, p.N, p.K, th);
     return -1;
   }
   return 0;
