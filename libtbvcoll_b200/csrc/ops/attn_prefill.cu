@@ -366,7 +366,8 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
 template <bool PAIR, bool CAP>
 cudaError_t launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const Params& p, cudaStream_t st) {
-  static const cudaError_t attr = cudaFuncSetAttribute(k_attn_prefill<PAIR, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  static std::atomic<unsigned> done{0};
+  const cudaError_t attr = pdl::allow_smem(k_attn_prefill<PAIR, CAP>, kSmem, done);
   if (attr != cudaSuccess) return attr;
   return pdl::launch(k_attn_prefill<PAIR, CAP>, dim3(unsigned(p.ntiles) * p.parts * p.kv_heads), dim3(192), kSmem, st, 1, q, k, v, p);
 }

@@ -263,8 +263,8 @@ bool attn_rows_takes(const void* q, const void* k_cache, const void* v_cache, co
 
 int attn_rows(const void* q, const void* k_cache, const void* v_cache, const int* tables, const int* seq_of_row, const int* ctx_lens, void* out, int rows, int heads,
               int kv_heads, int ldq, int ldo, int block_size, int max_blocks, int splits, float scale, cudaStream_t st) {
-  static const cudaError_t attr = cudaFuncSetAttribute(k_attn_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-  if (attr != cudaSuccess) return -1;
+  static std::atomic<unsigned> done{0};
+  if (pdl::allow_smem(k_attn_rows, kSmem, done) != cudaSuccess) return -1;
   const unsigned long long width = (unsigned long long)kv_heads * kD;
   CUtensorMap mk, mv;
   if (make_tensor_map_bf16(&mk, k_cache, kAnyCacheRows, width, width, kTok) != 0 || make_tensor_map_bf16(&mv, v_cache, kAnyCacheRows, width, width, kTok) != 0) return -3;

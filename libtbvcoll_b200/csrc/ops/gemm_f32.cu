@@ -203,7 +203,8 @@ template <int RT, int RF>
 cudaError_t launch_tiled(const F32Params& p, cudaStream_t st) {
   constexpr int TN = 8 * RT, TM = 16 * RF;
   constexpr size_t smem = size_t(kRing) * (TN + TM) * kPitch * 4;
-  static const cudaError_t attr = cudaFuncSetAttribute(k_gemm_f32_tiled<RT, RF>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  static std::atomic<unsigned> done{0};
+  const cudaError_t attr = pdl::allow_smem(k_gemm_f32_tiled<RT, RF>, smem, done);
   if (attr != cudaSuccess) return attr;
   const dim3 grid(p.groups * ((p.M + TM - 1) / TM) + (p.m_last + TM - 1) / TM, (p.N + TN - 1) / TN);
   return pdl::launch(k_gemm_f32_tiled<RT, RF>, grid, dim3(128), smem, st, 1, p);

@@ -455,7 +455,8 @@ cudaError_t launch_tok(const void* w, const void* x, const gemm::Params& p, int 
     return cudaSuccess;
   }
   constexpr size_t smem = size_t(S::kStages) * S::kStageBytes + 1024;
-  static const cudaError_t attr = cudaFuncSetAttribute(k_gemm_tok<EPI, TH, FEAT, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  static std::atomic<unsigned> done{0};
+  const cudaError_t attr = pdl::allow_smem(k_gemm_tok<EPI, TH, FEAT, ROWS>, smem, done);
   if (attr != cudaSuccess) return attr;
   const int tiles = (ROWS ? p.x_rows / S::kTok + p.groups : (p.N + S::kTok - 1) / S::kTok) * ((p.M + FEAT - 1) / FEAT);   // ROWS: at most
   const int sms = tbvops::sm_count();

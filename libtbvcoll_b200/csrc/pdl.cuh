@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 namespace pdl {
 
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -25,6 +27,18 @@ inline bool enabled() {
     v = (e && e[0] == '0') ? 0 : 1;
   }
   return v == 1;
+}
+
+// Opt-in to `bytes` of dynamic shared memory, once per device; `done`: the devices that have it, a mask per kernel.
+template <typename K>
+inline cudaError_t allow_smem(K kernel, size_t bytes, std::atomic<unsigned>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const unsigned bit = 1u << (dev & 31);
+  if (e != cudaSuccess || (done.load(std::memory_order_acquire) & bit)) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
 }
 
 // cudaLaunchKernelEx with the PDL attribute (and an optional cluster size along z).
