@@ -8,7 +8,8 @@
 //   O += P V           P from TMEM, V from shared memory with the channels contiguous
 // K and V have one buffer each: the next K is on its way while the weights are computed, the next V while the next scores are.  A CTA is a chain (product, exponentials,
 // product), so two of them share an SM (99 KB of shared memory and 256 TMEM columns each) and fill each other's gaps.
-// The running maximum is only a reference: sums are rescaled when a row's maximum grew by more than 2^8 over it (fp32 holds what lies between).
+// The running maximum is only a reference: sums are rescaled when a row's maximum grew by more than 2^8 over it (fp32 holds what lies between).  Each row decides for
+// itself (the warp only skips the loop when none has to), so a row's bits do not depend on the rows beside it.
 //
 // What bounds it: 16384 exponentials per tile take 1024 clocks of the SM's exponential units (three times that with a soft cap), its two products 1024 clocks of the
 // tensor cores.  Measured (32 query heads, 8 key heads, causal; before: warp-level products, 64 rows per CTA): 8 x 512 tokens 50 us (was 128), 1 x 4096 tokens
@@ -265,12 +266,13 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         for (int e = 0; e < 4; e++) x[e] = fmaxf(x[e], v[c + e]);
       }
       const float mx = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])) * sc;
+      const bool grew = mine && mx > m + kGrow;                   // the row's own business: rows that no query fills hold anything
       if (i == 0) {
         m = fmaxf(mx, kFloor);
-      } else if (__any_sync(0xffffffffu, mx > m + kGrow)) {
-        // the product before is complete (the scores were issued behind it): rescale the sums in place
-        const float to = fmaxf(m, mx), f = exp2_ftz(m - to);
-        m = to;
+      } else if (__any_sync(0xffffffffu, grew)) {
+        // the product before is complete (the scores were issued behind it): rescale the sums in place, those of the other rows of the warp by one
+        const float f = grew ? exp2_ftz(m - mx) : 1.f;
+        if (grew) m = mx;
         l *= f;
 #pragma unroll 1
         for (int c = 0; c < kD; c += 16) {

@@ -139,3 +139,48 @@ def test_paired_rows(ops, H, G, window, chunk, cap, gated):
             want, size = want * f, size * f
         check(out[r0: r0 + n].view(n, H, D), want, size)
         r0 += n
+
+
+@pytest.mark.parametrize("paired,hpk", [(False, 4), (False, 1), (True, 4), (True, 6)])
+def test_a_rows_bits_are_its_own(ops, paired, hpk):
+    """The bits of a row depend on its own query, keys and values: not on the rows of the next sequence that the same MMA holds, not on a neighbour whose scores grow from
+    tile to tile, and not on what an earlier kernel left in the rows of shared memory that no query fills (128 is no multiple of six heads)."""
+    bs, G, start, n = 16, 2, 500, 13
+    H, keys = G * hpk, start + n + 3
+    k, v = rnd(keys // bs * bs + bs, G, D, seed=21), rnd(keys // bs * bs + bs, G, D, seed=22)
+    k = (k.float() * (1 + torch.arange(k.shape[0], device=DEV) // 128)[:, None, None]).to(torch.bfloat16)
+    cache = torch.zeros(k.shape[0] // bs, G, bs, 2 * D + 8, dtype=torch.bfloat16, device=DEV)
+    cache[..., :D], cache[..., D: 2 * D] = k.view(-1, bs, G, D).transpose(1, 2), v.view(-1, bs, G, D).transpose(1, 2)
+    cache = cache.view(-1, 2 * D + 8)
+
+    def run(q, counts, heads=H):
+        T = q.shape[0]
+        tables = torch.arange(k.shape[0] // bs, dtype=torch.int32, device=DEV)[None].expand(len(counts), -1).contiguous()
+        seq = torch.tensor(sum(([i] * c for i, c in enumerate(counts)), []), dtype=torch.int32)
+        out = torch.empty(T, heads * D, dtype=torch.bfloat16, device=DEV)
+        if paired:
+            tiles = [(sum(counts[:i]) + a, min(64, c - a), 0, start + a + 1) for i, c in enumerate(counts) for a in range(0, c, 64)]
+            ops.paired_attention_prefill(q, cache, tables, seq.to(DEV), torch.tensor(tiles, dtype=torch.int32, device=DEV), out, heads, G, D, bs, 0.0, 0, 0, None)
+        else:
+            see = torch.cat([torch.arange(start + 1, start + c + 1) for c in counts]).to(torch.int32).to(DEV)
+            tiles = ops.prefill_tiles(seq, heads // G, 128).to(DEV)
+            ops.prefill_attention(q.view(T, heads, D), k, v, tables, see, seq.to(DEV), tiles, out.view(T, heads, D), 1.0, bs, 128)
+        torch.cuda.synchronize()
+        return out.view(T, heads, D)
+
+    def dirty(size):                       # leaves queries of this size in shared memory of every SM
+        run(rnd(6400, 8 * D, seed=23, scale=size), [13] * 492 + [4], heads=8)
+
+    q = rnd(n, H * D, seed=24, scale=0.1)
+    dirty(0.0)
+    alone = run(q, [n])
+    assert torch.isfinite(alone).all()
+    beside = run(torch.cat((q, rnd(40, H * D, seed=25, scale=30.0))), [n, 40])
+    assert torch.equal(beside[:n], alone)
+    other = q.clone()
+    other[5, :D] *= 300.0
+    got = run(other, [n])
+    got[5, 0] = alone[5, 0]
+    assert torch.equal(got, alone)
+    dirty(30.0)
+    assert torch.equal(run(q, [n]), alone)
