@@ -530,7 +530,7 @@ int tbv_op_gemm_rows(const void* w, const void* x, void* y, const void* row_off,
   p.y = static_cast<__nv_bfloat16*>(y);
   p.act_a = act_a; p.act_b = act_b; p.act_c = act_c;
   p.groups = groups; p.row_off = static_cast<const int*>(row_off); p.x_rows = x_rows;
-  const int th = tbvops::gemm_persist_mode() > 0 ? tbvops::gemm_tok_rows_choose(M, x_rows, groups) : 0;
+  const int persist = tbvops::gemm_persist_mode(), th = persist > 0 ? tbvops::gemm_tok_rows_choose(M, x_rows, groups, K, epi, persist, tbvops::sm_count()) : 0;
   if (th > 0) return tbvops::gemm_tok_launch_p(w, x, p, ldx, epi, th, stream);
   return launch_decode_form(w, x, ldx, p, epi, 0, static_cast<cudaStream_t>(stream));
 }
@@ -549,6 +549,9 @@ int tbv_op_gemm_error(void) {
   cudaMemcpy(&v, tbvops::gemm_err_flag(), sizeof(int), cudaMemcpyDeviceToHost);
   return v;
 }
+
+// Which form a row-grouped product of that shape takes on a GPU of `sms` SMs (see gemm_tok_rows_choose); needs no device.
+int tbv_op_gemm_rows_form(int M, int x_rows, int groups, int K, int epi, int sms) { return tbvops::gemm_tok_rows_choose(M, x_rows, groups, K, epi, 1, sms); }
 
 void tbv_op_gemm_config(int M, int N, int K, int splits_hint, int* bn, int* splits, int* stages) {
   tbvops::gemm_config(M, N, K, splits_hint, bn, splits, stages);

@@ -60,6 +60,7 @@ constexpr int kFeatTile = 256;     // of row-grouped problems
 
 // first token row, end of the rows, first feature and its weight row of a tile
 struct At { int n0, nend, f0, w0; };
+template <int TOK>
 __device__ __forceinline__ At find_tile(const RowGroups& groups, int tile, int ngroups, int M) {
   int lo = 0, hi = ngroups - 1;                    // the last group whose first tile is not beyond `tile`; empty groups are passed over
   while (lo < hi) {
@@ -67,18 +68,19 @@ __device__ __forceinline__ At find_tile(const RowGroups& groups, int tile, int n
     if (groups.tile[mid] <= tile) lo = mid;
     else hi = mid - 1;
   }
-  const int local = tile - groups.tile[lo], tt = (groups.off[lo + 1] - groups.off[lo] + 127) / 128;
+  const int local = tile - groups.tile[lo], tt = (groups.off[lo + 1] - groups.off[lo] + TOK - 1) / TOK;
   const int f0 = local / tt * kFeatTile;
-  return At{groups.off[lo] + local % tt * 128, groups.off[lo + 1], f0, lo * M + f0};
+  return At{groups.off[lo] + local % tt * TOK, groups.off[lo + 1], f0, lo * M + f0};
 }
 
-// Fills the table from the rows' offsets (device memory); whole CTA.
+// Fills the table from the rows' offsets (device memory); whole CTA of THREADS.
+template <int TOK, int THREADS>
 __device__ __forceinline__ void count_tiles(RowGroups& groups, const gemm::Params& p, int feat_tiles) {
-  for (int g = threadIdx.x; g <= p.groups; g += 192) groups.off[g] = p.row_off[g];
+  for (int g = threadIdx.x; g <= p.groups; g += THREADS) groups.off[g] = p.row_off[g];
   __syncthreads();
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x, per = (p.groups + 31) / 32, a = min(p.groups, lane * per), b = min(p.groups, a + per);
-    auto count = [&](int g) { return (groups.off[g + 1] - groups.off[g] + 127) / 128 * feat_tiles; };
+    auto count = [&](int g) { return (groups.off[g + 1] - groups.off[g] + TOK - 1) / TOK * feat_tiles; };
     int sum = 0;
     for (int g = a; g < b; g++) sum += count(g);
     int inc = sum;
@@ -302,7 +304,7 @@ __device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok,
 
 // EPI (gemm::Epi) of all kernels here: 0 store (+bias); 1 SiLU-mul over interleaved gate/up features (output has M / 2 features); 2 fp32 store with
 // an activation; 3 clamped gated unit over interleaved gate/up features; 4 rotation and cache write of a qkv projection.
-// ROWS: row-grouped problem (p.row_off; TH = 1, FEAT = 256).
+// ROWS: row-grouped problem (p.row_off; FEAT = 256).
 template <int EPI, int TH, int FEAT, bool ROWS>
 __global__ void __launch_bounds__(Shape<TH, FEAT>::kThreads, 1)
 k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ gemm::Params p) {
@@ -342,14 +344,14 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
   int tiles = tok_tiles * feat_tiles;
   if constexpr (ROWS) {
     pdl::grid_dependency_wait();                 // the groups' rows were counted on the device by a kernel before this one
-    count_tiles(groups, p, feat_tiles);
+    count_tiles<S::kTok, S::kThreads>(groups, p, feat_tiles);
     tiles = groups.tile[p.groups];
   }
   const int my_tiles = int(blockIdx.x) < tiles ? (tiles - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x) : 0;
   const int ngroups = p.groups, feats = p.M, all_rows = p.N;
   // (by value: a capture of the parameter block would put it in local memory)
   auto locate = [=](int tile) -> At {
-    if constexpr (ROWS) return find_tile(groups, tile, ngroups, feats);
+    if constexpr (ROWS) return find_tile<S::kTok>(groups, tile, ngroups, feats);
     const int f0 = tile / tok_tiles * FEAT;
     return At{tile % tok_tiles * S::kTok, all_rows, f0, f0};
   };
@@ -486,11 +488,18 @@ int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode) {
   return stores && 18 * rounds(n256 * f256) <= 10 * rounds(n128 * f256) ? 2 : 1;
 }
 
-// Row-grouped: 0 the decode form, 1 k_gemm_tok.  The decode form re-reads a group's weights for every tile of up to 128 rows; k_gemm_tok wastes what a group's last
-// tile lacks.
-int gemm_tok_rows_choose(int M, int x_rows, int groups) {
-  if ((M % 16) || groups > kMaxRowGroups) return 0;
-  return x_rows / groups >= 64 ? 1 : 0;
+// Row-grouped: 0 the decode form, 1 / 2 k_gemm_tok with 128- / 256-token tiles of 256 features (`mode` 2 and 4 / 3 force them).  The decode form re-reads a group's weights
+// for every tile of up to 128 rows; k_gemm_tok wastes what a group's last tile lacks, on average half a tile.
+//
+// How the rows spread over the groups is not known here, and 256-token tiles lose up to half where they need a round more (8 x 513 rows, 2048 x 3584: 89 us against 59).
+// They pay for plain stores where K is long (their epilogue is exposed), groups are large against a tile and rounds are many: 4096 x 7168, 8 groups of 768 / 1000 /
+// 2048 rows 259 / 338 / 601 us against 282 / 367 / 664, 16 of 1500 1031 against 1040; but 16 of 500 428 against 398; with K 3584 8 of 2000 340 against 330.
+int gemm_tok_rows_choose(int M, int x_rows, int groups, int K, int epi, int mode, int sms) {
+  if ((M % 16) || groups > kMaxRowGroups || x_rows / groups < 64) return 0;
+  if (epi != gemm::kEpiStore || mode == 2 || mode == 4) return 1;
+  if (mode == 3) return 2;
+  const long tiles = (x_rows / 256 + groups / 2) * (long)((M + 255) / 256);
+  return K > 4096 && x_rows / groups >= 768 && tiles >= 3l * sms ? 2 : 1;
 }
 
 int gemm_tok_launch(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi, int th,
@@ -512,7 +521,8 @@ int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, in
   int map_rc = 0;
   cudaError_t e;
   if (p.row_off) {
-    e = epi == gemm::kEpiClampGlu ? launch_tok<3, 1, 256, true>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1, 256, true>(w, x, p, ldx, st, &map_rc);
+    e = epi == gemm::kEpiClampGlu ? launch_tok<3, 1, 256, true>(w, x, p, ldx, st, &map_rc) :
+        th == 2 ? launch_tok<0, 2, 256, true>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1, 256, true>(w, x, p, ldx, st, &map_rc);
   } else switch (epi) {
     case gemm::kEpiSiluMul: e = th == 3 ? launch_tok<1, 1, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<1, 1, 256>(w, x, p, ldx, st, &map_rc); break;
     case gemm::kEpiF32:

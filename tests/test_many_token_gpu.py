@@ -1,4 +1,4 @@
-"""The many-token GEMM (gemm_persist.cu): the epilogue of the qkv projection, in both tile shapes, at remainders of tokens and features."""
+"""The many-token GEMM (gemm_persist.cu): the epilogue of the qkv projection and row-grouped products, in every tile shape, at remainders of tokens and features."""
 import pytest
 import torch
 
@@ -62,3 +62,27 @@ def test_tile_shapes_give_the_same_bits(mode, N, M, K):
     assert not ops.gemm_error()
     for a, c in zip(got, want):
         assert torch.equal(a, c)
+
+
+@pytest.mark.parametrize("counts", [[0, 300, 1, 0, 513, 256], [64, 64, 64], [700, 0, 0, 255]])
+@pytest.mark.parametrize("M,K", [(272, 72), (2064, 520)])
+def test_row_groups_in_both_tile_shapes_give_the_same_bits(counts, M, K):
+    from libtbvcoll_b200 import ops
+    off = torch.tensor([0] + counts).cumsum(0).to(torch.int32).to(DEV)
+    x, w = rnd(sum(counts), K, seed=1), rnd(len(counts) * M, K, seed=2, scale=0.1)
+    got = []
+    try:
+        for mode in (2, 3):
+            ops.gemm_persist_mode(mode)
+            got.append(torch.full((sum(counts), M), 7.0, dtype=torch.bfloat16, device=DEV))
+            ops.linear_rows(x, w, got[-1], off, len(counts), sum(counts))
+        torch.cuda.synchronize()
+    finally:
+        ops.gemm_persist_mode(None)
+    assert not ops.gemm_error() and torch.equal(*got)
+    for g in range(len(counts)):
+        a, b = int(off[g]), int(off[g + 1])
+        want = x[a:b].double() @ w[g * M: (g + 1) * M].double().t()
+        size = x[a:b].double().abs() @ w[g * M: (g + 1) * M].double().abs().t()
+        # one rounding to bf16 and K fp32 additions
+        assert ((got[0][a:b].double() - want).abs() <= want.abs() * 2.0 ** -8 + size * K * 2.0 ** -23).all()
