@@ -402,6 +402,13 @@ int tbvops::gemm_persist_mode() {
 }
 
 namespace {
+// Which form tbv_op_gemm_ex takes (0: the decode form).  The many-token kernel stores fp32 results 32 bytes at a time and their bf16 copy 16; the decode form's copy-out
+// of a copy is 8 bytes wide, all that the entry asks of it.
+int ex_form(const void* y, const void* y2, int M, int N, int K, int ldy, int epi, int groups, int mode, int sms) {
+  if (groups > 1 || mode <= 0 || (reinterpret_cast<uintptr_t>(y) & 31u) || (reinterpret_cast<uintptr_t>(y2) & 15u)) return 0;
+  return tbvops::gemm_tok_choose(M, N, K, ldy, epi, mode, sms);
+}
+
 // Decode-form launch of a filled Params (M, N, K, ldy, output pointers, epilogue arguments, groups).
 int launch_decode_form(const void* w, const void* x, int ldx, Params& p, int epi, int splits_hint, cudaStream_t st) {
   const int M = p.M, N = p.N, K = p.K, G = p.groups > 1 ? p.groups : 1;
@@ -473,7 +480,7 @@ int tbv_op_gemm(const void* w, const void* x, void* y, const void* bias, int M, 
   // Hundreds of tokens: the persistent kernel with tokens on the UMMA M axis.
   const int persist = tbvops::gemm_persist_mode();
   if (persist > 0 && splits_hint <= 0) {
-    const int th = w_not_constant ? 0 : tbvops::gemm_tok_choose(M, N, K, ldy, epi, persist);   // the many-token kernel always prefetches w
+    const int th = w_not_constant ? 0 : tbvops::gemm_tok_choose(M, N, K, ldy, epi, persist, tbvops::sm_count());   // the many-token kernel always prefetches w
     if (th > 0) return tbvops::gemm_tok_launch(w, x, y, bias, M, N, K, ldx, ldy, epi, th, stream);
   }
   // Large weight matrices at decode batch sizes: the persistent kernel that splits the work evenly over the SMs.
@@ -512,10 +519,8 @@ int tbv_op_gemm_ex(const void* w, const void* x, void* y, void* y2, const void* 
   p.pf_ptr = pf_ptr;
   p.pf_bytes = pf_bytes;
   p.groups = groups > 1 ? groups : 1; p.x_group = groups > 1 ? x_group : 0; p.y_group = groups > 1 ? y_group : 0;
-  if (groups <= 1 && tbvops::gemm_persist_mode() > 0 && !(reinterpret_cast<uintptr_t>(y) & 31u)) {   // its fp32 stores are 32 bytes wide
-    const int th = tbvops::gemm_tok_choose(M, N, K, ldy, epi, tbvops::gemm_persist_mode());
-    if (th > 0) return tbvops::gemm_tok_launch_p(w, x, p, ldx, epi, th, stream);
-  }
+  const int th = ex_form(y, y2, M, N, K, ldy, epi, groups, tbvops::gemm_persist_mode(), tbvops::sm_count());
+  if (th > 0) return tbvops::gemm_tok_launch_p(w, x, p, ldx, epi, th, stream);
   return launch_decode_form(w, x, ldx, p, epi, 0, static_cast<cudaStream_t>(stream));
 }
 
@@ -550,6 +555,10 @@ int tbv_op_gemm_error(void) {
   return v;
 }
 
+// Which form tbv_op_gemm_ex takes for these results, copy (or null) and sizes on a GPU of `sms` SMs; needs no device and touches no memory.
+int tbv_op_gemm_ex_form(const void* y, const void* y2, int M, int N, int K, int ldy, int epi, int groups, int sms) {
+  return ex_form(y, y2, M, N, K, ldy, epi, groups, 1, sms);
+}
 // Which form a row-grouped product of that shape takes on a GPU of `sms` SMs (see gemm_tok_rows_choose); needs no device.
 int tbv_op_gemm_rows_form(int M, int x_rows, int groups, int K, int epi, int sms) { return tbvops::gemm_tok_rows_choose(M, x_rows, groups, K, epi, 1, sms); }
 

@@ -477,11 +477,11 @@ namespace tbvops {
 // 1024 tokens, 14336 x 2048 with the SiLU unit 75 / 61.
 // Fewer than 384 tokens, and problems of few tiles and not too long K, go to the decode form, which shares K out over clusters (512 tokens, fp32, 2048 x 4096: 19 us
 // against 24; 1024 tokens 28 against 24; 512 tokens, 2048 x 2048 15.3 against 13.5, 2048 x 7168 49 against 36).
-int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode) {
+int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode, int sms) {
   if (!(N >= 384 && (M % 16) == 0 && (K % 8) == 0 && (ldy % 8) == 0 && epi >= 0 && epi <= 3)) return 0;
   const bool stores = epi == gemm::kEpiStore || epi == gemm::kEpiF32;
   if (mode >= 2) return mode == 4 ? 3 : (mode == 3 && stores ? 2 : 1);
-  const long sms = sm_count(), f256 = (M + 255) / 256, f128 = (M + 127) / 128, n128 = (N + 127) / 128, n256 = (N + 255) / 256;
+  const long f256 = (M + 255) / 256, f128 = (M + 127) / 128, n128 = (N + 127) / 128, n256 = (N + 255) / 256;
   auto rounds = [&](long tiles) { return (tiles + sms - 1) / sms; };
   if (n128 * f128 * (K > 2048 ? 2 : 4) <= sms && K <= 4096) return 0;
   if (2 * rounds(n128 * f128) < 3 * rounds(n128 * f256)) return 3;

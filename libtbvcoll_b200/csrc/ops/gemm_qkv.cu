@@ -191,7 +191,7 @@ extern "C" int tbv_op_gemm_qkv_rope(const void* w, const void* x, void* qkv, con
   // per SM stage every tile through shared memory).
   if (splits_hint <= 0 && !((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(cos_sin) | reinterpret_cast<uintptr_t>(k_cache) |
                              reinterpret_cast<uintptr_t>(v_cache)) & 31u) && ldy % 16 == 0) {
-    const int persist = tbvops::gemm_persist_mode(), th = persist > 0 ? tbvops::gemm_tok_choose(M, N, K, ldy, gemm::kEpiSiluMul, persist) : 0;   // an epilogue that computes
+    const int persist = tbvops::gemm_persist_mode(), th = persist > 0 ? tbvops::gemm_tok_choose(M, N, K, ldy, gemm::kEpiSiluMul, persist, tbvops::sm_count()) : 0;   // an epilogue that computes
     if (th > 0) {
       gemm::Params p{};
       p.M = M; p.N = N; p.K = K; p.ldy = ldy;

@@ -21,7 +21,7 @@ void gemm_config(int M, int N, int K, int splits_hint, int* bn_out, int* splits_
                  bool f32_out = false);
 // many-token (prefill) persistent kernel, gemm_persist.cu
 int gemm_persist_mode();
-int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode);
+int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode, int sms);
 int gemm_tok_launch(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi, int th,
                     void* stream);
 // the same for a filled parameter block (M, N, K, ldy, outputs, epilogue arguments)

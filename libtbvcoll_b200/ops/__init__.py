@@ -74,6 +74,7 @@ def lib():
     l.tbv_op_gemm_streamk_min_bytes.restype = None
     l.tbv_op_gemm_qkv_rope.argtypes = [c_vp, c_vp, c_vp, c_vp, I, I, I, I, I, c_vp, c_vp, c_vp, c_vp, c_vp, I, I, I, I, c_vp]
     l.tbv_op_gemm_qkv_rope.restype = I
+    l.tbv_op_gemm_ex_form.argtypes = [c_vp, c_vp] + [I] * 7
     l.tbv_op_gemm_config.argtypes = [I, I, I, I, ctypes.POINTER(I), ctypes.POINTER(I), ctypes.POINTER(I)]
     l.tbv_op_rmsnorm.argtypes = [c_vp, c_vp, c_vp, I, I, F, c_vp]
     l.tbv_op_add_rmsnorm.argtypes = [c_vp, c_vp, c_vp, c_vp, c_vp, I, I, F, c_vp]

@@ -86,3 +86,20 @@ def test_row_groups_in_both_tile_shapes_give_the_same_bits(counts, M, K):
         size = x[a:b].double().abs() @ w[g * M: (g + 1) * M].double().abs().t()
         # one rounding to bf16 and K fp32 additions
         assert ((got[0][a:b].double() - want).abs() <= want.abs() * 2.0 ** -8 + size * K * 2.0 ** -23).all()
+
+
+@pytest.mark.parametrize("offset", [0, 4, 8, 12])
+def test_copies_that_are_column_slices(offset):
+    """A bf16 copy of fp32 results at any 8-byte offset, with more rows than the decode form takes by itself; what lies around it stays."""
+    from libtbvcoll_b200 import ops
+    N, M, K = 513, 2064, 264
+    x, w = rnd(N, K, seed=1), rnd(M, K, seed=2, scale=0.1)
+    out = torch.zeros(N, M + 16, device=DEV)[:, :M]
+    around = torch.full((N, M + 16), 7.0, dtype=torch.bfloat16, device=DEV)
+    copy = around[:, offset: offset + M]
+    ops.linear(x, w, out, copy=copy)
+    torch.cuda.synchronize()
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert not ops.gemm_error() and torch.equal(copy, out.to(torch.bfloat16))
+    assert ((out.double() - want).abs() <= size * K * 2.0 ** -23).all()                      # K fp32 additions
+    assert (around[:, :offset] == 7).all() and (around[:, offset + M:] == 7).all()
