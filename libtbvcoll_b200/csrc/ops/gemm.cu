@@ -11,6 +11,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
 #include <mutex>
 #include <unordered_map>
 
@@ -240,6 +241,14 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn g_encode = nullptr;
 std::once_flag g_encode_once;
+CUresult encode(CUtensorMap* out, unsigned rank, const void* ptr, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
+  // the encoder wants the device's context to be current, which in a thread that has made no CUDA call yet it is not
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return CUDA_ERROR_INVALID_CONTEXT;
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+}
 
 struct MapKey {
   const void* ptr;
@@ -257,8 +266,10 @@ struct MapKeyHash {
 std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;
 std::mutex g_maps_mu;
 int g_persist_mode = -1;   // TBV_GEMM_PERSIST, read on first use; tbv_op_gemm_persist_mode overrides it
-int* g_err_flag[16] = {nullptr};
-int g_sm_count[16] = {0};
+__device__ int g_err_word;                         // the flag of tbv_op_gemm_error, one per device
+constexpr int kMaxDevices = 64;
+std::atomic<int*> g_err_flag[kMaxDevices];         // its address
+std::atomic<int> g_sm_count[kMaxDevices];
 bool g_attr_done = false;
 
 }  // namespace
@@ -288,12 +299,8 @@ int make_tensor_map_bf16(CUtensorMap* out, const void* ptr, unsigned long long r
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {ld * 2};
   cuuint32_t box[2] = {64, box_rows};
-  cuuint32_t estr[2] = {1, 1};
   CUtensorMap m;
-  CUresult r = g_encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return -3;
+  if (encode(&m, 2, ptr, dims, strides, box) != CUDA_SUCCESS) return -3;
   if (cache) {
     std::lock_guard<std::mutex> g(g_maps_mu);
     if (g_maps.size() > 65536) g_maps.clear();
@@ -309,9 +316,8 @@ int make_tensor_map_heads(CUtensorMap* out, const void* ptr, unsigned long long 
   CUtensorMap plain;
   if (make_tensor_map_bf16(&plain, ptr, rows, (unsigned long long)heads * dim, ld, 1) != 0) return -1;   // also looks up the encoder and checks the alignment
   const cuuint64_t dims[3] = {dim, heads, rows}, strides[2] = {dim * 2ull, ld * 2ull};
-  const cuuint32_t box[3] = {64, box_heads, box_rows}, estr[3] = {1, 1, 1};
-  return g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -3;
+  const cuuint32_t box[3] = {64, box_heads, box_rows};
+  return encode(out, 3, ptr, dims, strides, box) == CUDA_SUCCESS ? 0 : -3;
 }
 
 // ---- weights of the GEMM that follows, to be asked into L2 by the kernel launched next ------------------------------
@@ -346,24 +352,29 @@ void set_next_prefetch(const void* ptr, unsigned long long bytes) {
   t_pf_bytes = bytes;
 }
 
+// Both are looked up on a device's first call, by any thread, also in the midst of a stream capture: nothing is allocated, copied or waited for, and threads that come
+// at the same time find the same values.
 int* gemm_err_flag() {
   int dev = 0;
-  cudaGetDevice(&dev);
-  dev &= 15;
-  if (!g_err_flag[dev]) {
-    cudaMalloc(&g_err_flag[dev], sizeof(int));
-    cudaMemset(g_err_flag[dev], 0, sizeof(int));
-    cudaDeviceProp prop;
-    cudaGetDeviceProperties(&prop, dev);
-    g_sm_count[dev] = prop.multiProcessorCount;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kMaxDevices) return nullptr;
+  int* at = g_err_flag[dev].load(std::memory_order_acquire);
+  if (!at) {
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_err_word) != cudaSuccess) return nullptr;
+    at = static_cast<int*>(p);
+    g_err_flag[dev].store(at, std::memory_order_release);
   }
-  return g_err_flag[dev];
+  return at;
 }
 int sm_count() {
   int dev = 0;
-  cudaGetDevice(&dev);
-  gemm_err_flag();
-  return g_sm_count[dev & 15];
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kMaxDevices) return 1;
+  int n = g_sm_count[dev].load(std::memory_order_acquire);
+  if (!n) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 1;
+    g_sm_count[dev].store(n, std::memory_order_release);
+  }
+  return n;
 }
 
 void gemm_config(int M, int N, int K, int splits_hint, int* bn_out, int* splits_out, int* stages_out, int groups, bool f32_out) {
@@ -551,7 +562,8 @@ void tbv_op_gemm_persist_mode(int mode) { g_persist_mode = mode < -1 ? -1 : mode
 // 1 if any GEMM wait ever gave up on the current device (synchronises the device).
 int tbv_op_gemm_error(void) {
   int v = 0;
-  cudaMemcpy(&v, tbvops::gemm_err_flag(), sizeof(int), cudaMemcpyDeviceToHost);
+  const int* at = tbvops::gemm_err_flag();
+  if (at) cudaMemcpy(&v, at, sizeof(int), cudaMemcpyDeviceToHost);
   return v;
 }
 

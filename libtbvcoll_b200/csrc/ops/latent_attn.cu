@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kRW * 32 + 32, 1) k_latent_rows_mma(const Rows
     // gave up: let the copies in flight land before this memory goes away, and report
     for (int k = 0; k < 2; k++)
       for (int spin = 0; spin < 20000 && ntiles > k && !sm100::mbar_try_wait(smem_addr(&full[k]), uint32_t((ntiles - 1 - k) >> 1) & 1u); spin++) __nanosleep(50);
-    atomicExch(p.err, 1);
+    if (p.err) atomicExch(p.err, 1);
   }
   l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
   l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);

@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_shared_rows(const RowsParams
     // gave up: let the copies in flight land before this memory goes away, and report
     for (int i = done; i < mine && i < done + kStages; i++)
       for (int spin = 0; spin < 20000 && !sm100::mbar_try_wait(smem_addr(&full[warp][i % kStages]), uint32_t(i / kStages) & 1u); spin++) __nanosleep(50);
-    if (lane == 0) atomicExch(p.err, 1);
+    if (lane == 0 && p.err) atomicExch(p.err, 1);
   }
 #pragma unroll
   for (int t = 0; t < NH; t++)

@@ -1,0 +1,68 @@
+"""The first call of a process: inside a stream capture, and by several threads at the same time.  Every case is a process of its own."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SETUP = """
+import torch
+from libtbvcoll_b200 import ops
+dev, bf = "cuda:0", torch.bfloat16
+g = torch.Generator(device=dev).manual_seed(1)
+rnd = lambda *s, dtype=bf: torch.randn(s, generator=g, device=dev).to(dtype)
+q, kc, vc = rnd(33, 8, 128), rnd(64, 2, 128), rnd(64, 2, 128)
+tables = torch.arange(4, dtype=torch.int32, device=dev).repeat(33, 1)
+ctx, seq = torch.arange(1, 34, dtype=torch.int32, device=dev), torch.zeros(33, dtype=torch.int32, device=dev)
+tiles = ops.prefill_tiles(torch.zeros(33, dtype=torch.int32), 4, 128).to(dev)
+x, w = rnd(33, 64, dtype=torch.float32), rnd(70, 64, dtype=torch.float32)
+xb, wb = rnd(33, 64), rnd(72, 64)
+calls = {
+    "rows": (lambda out: ops.paged_attention(q, kc, vc, tables, ctx, out, 0.1, 16), lambda: torch.zeros_like(q)),
+    "prompt": (lambda out: ops.prefill_attention(q, kc, vc, tables, ctx, seq, tiles, out, 0.1, 16, 128), lambda: torch.zeros_like(q)),
+    "fp32": (lambda out: ops.linear(x, w, out), lambda: torch.zeros(33, 70, device=dev)),
+    "bf16": (lambda out: ops.gemm(xb, wb, out), lambda: torch.zeros(33, 72, dtype=bf, device=dev)),
+}
+torch.cuda.synchronize()
+"""
+
+CAPTURE = SETUP + """
+call, make = calls[CASE]
+captured, eager = make(), make()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    call(captured)
+graph.replay()
+call(eager)
+torch.cuda.synchronize()
+assert captured.any() and torch.equal(captured, eager) and not ops.gemm_error()
+print("passed")
+"""
+
+THREADS = SETUP + """
+import threading
+call, make = calls[CASE]
+outs, gate = [make() for _ in range(16)], threading.Barrier(16)
+streams = [torch.cuda.Stream() for _ in range(16)]
+torch.cuda.synchronize()
+def work(i):
+    with torch.cuda.stream(streams[i]):
+        gate.wait()
+        call(outs[i])
+ts = [threading.Thread(target=work, args=(i,)) for i in range(16)]
+[t.start() for t in ts]
+[t.join() for t in ts]
+torch.cuda.synchronize()
+assert outs[0].any() and all(torch.equal(o, outs[0]) for o in outs) and not ops.gemm_error()
+print("passed")
+"""
+
+
+@pytest.mark.parametrize("case", ["rows", "prompt", "fp32", "bf16"])
+@pytest.mark.parametrize("form", [CAPTURE, THREADS], ids=["captured", "threads"])
+def test_first_call(form, case):
+    r = subprocess.run([sys.executable, "-c", f"CASE = {case!r}\n" + form], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("passed"), r.stdout + r.stderr
