@@ -10,10 +10,10 @@
 // Tile shapes (templates TH, FEAT); an SM takes in some 70 bytes per clock through TMA (measured with three quarters of the MMAs left out, 133 GB/s), which bounds the smaller ones:
 //   TH = 1, FEAT = 128  128 tokens x 128 features: a quarter less work per byte than 256 features, for problems whose wider tiles would leave SMs idle
 //           (1024 tokens, 2048 x 7168 37 us against 45, 512 tokens, 3072 x 2048 with rotation 20 against 23).
-//   TH = 1  128 tokens x 256 features, two accumulator sets: the epilogue of a tile runs under the MMAs of the next.  For epilogues that compute, and where
+//   TH = 1  128 tokens x 256 features, two accumulator sets: the epilogue of a tile runs under the MMAs of the next.  For gated units, the rotation, and where
 //           tiles are few.  4096 tokens: 28672 x 4096 with the SiLU unit 641 us = 1500 TFLOP/s (848 with TH = 2), 6144 x 4096 with rotation 159 (166).
 //   TH = 2  256 tokens x 256 features as two 128-row MMAs that share one 256-row weight tile: a third less traffic per operation, but both accumulators belong
-//           to one tile, so the epilogue (eight warps here, four per half) is exposed once per tile.  For plain stores: 4096 x 4096 97 us (104 with TH = 1), 4096 x 14336 361 (402).
+//           to one tile, so the epilogue (eight warps here, four per half) is exposed once per tile.  For stores, bf16 or fp32 (the choice does not look at an activation): 4096 x 4096 97 us (104 with TH = 1), 4096 x 14336 361 (402).
 //
 // The CTAs walk tiles id = first + i * step with the token tile fastest: the CTAs running at any
 // moment share a few weight tiles (streamed from HBM once) and the activations stay in L2.  Warp 0
@@ -470,20 +470,25 @@ cudaError_t launch_tok(const void* w, const void* x, const gemm::Params& p, int 
 namespace tbvops {
 
 // Which form takes an [N tokens] x [M features] problem: 0 = the decode-form kernel (gemm.cu), k_gemm_tok with 1 / 2 = 128- / 256-token tiles of 256 features, 3 = 128 x 128
-// tiles.  `mode`: 1 = choose, 2 / 3 / 4 = force the first / second / third tile wherever the shape allows (tests, measurements; 256-token tiles exist for plain stores).
+// tiles.  `mode`: 1 = choose, 2 / 3 / 4 = force the first / second / third tile wherever the shape allows (tests, measurements; 256-token tiles exist for stores).
 //
 // Every CTA walks ceil(tiles / SMs) tiles.  A k-block of a 128 x 128 tile takes two thirds of the time of a 128 x 256 one (both bound by what TMA brings in), and one of
 // 256 x 256 nine tenths of two of those.  512 tokens, 4096 x 4096 24 / 28 / 45 us with 128 x 128 / 128 x 256 / 256 x 256 tiles,
 // 1024 tokens, 14336 x 2048 with the SiLU unit 75 / 61.
-// Fewer than 384 tokens, and problems of few tiles and not too long K, go to the decode form, which shares K out over clusters (512 tokens, fp32, 2048 x 4096: 19 us
-// against 24; 1024 tokens 28 against 24; 512 tokens, 2048 x 2048 15.3 against 13.5, 2048 x 7168 49 against 36).
+// Fewer than 384 tokens, and problems of few tiles, go to the decode form, which shares K out over clusters (512 tokens, fp32, 2048 x 4096: 19 us
+// against 24; 1024 tokens 28 against 24; 512 tokens, 2048 x 2048 15.3 against 13.5).  With long K a CTA here walks all of it (0.3 us per k-block of a 128 x 128 tile, one after
+// another) while the decode form takes some 1.6 us per 128 x 256 tile of its own, and per k-block only a little: it wins while it has fewer tiles than a fifth of the k-blocks
+// (us, decode form / here: 512 tokens, 288 x 8192 17 / 38, 1280 x 8192 34 / 39, 1024 x 14336 43 / 67, 512 x 28672 32 / 126; 2048 tokens, 288 x 8192 33 / 39,
+// 1024 x 28672 143 / 156; the other side: 512 tokens, 1024 x 5120 28 / 26, 2048 x 7168 48 / 36, 1024 tokens, 1280 x 8192 47 / 41, 2048 tokens, 2048 x 28672 247 / 185).  With fp32
+// results the decode form keeps to a CTA per SM and wins further (2048 tokens, 512 x 8192 24 / 41, 1024 x 14336 58 / 68; the other side: 1536 tokens, 1024 x 5120 31 / 28).
 int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode, int sms) {
   if (!(N >= 384 && (M % 16) == 0 && (K % 8) == 0 && (ldy % 8) == 0 && epi >= 0 && epi <= 3)) return 0;
   const bool stores = epi == gemm::kEpiStore || epi == gemm::kEpiF32;
   if (mode >= 2) return mode == 4 ? 3 : (mode == 3 && stores ? 2 : 1);
   const long f256 = (M + 255) / 256, f128 = (M + 127) / 128, n128 = (N + 127) / 128, n256 = (N + 255) / 256;
   auto rounds = [&](long tiles) { return (tiles + sms - 1) / sms; };
-  if (n128 * f128 * (K > 2048 ? 2 : 4) <= sms && K <= 4096) return 0;
+  const long kb = (K + 63) / 64, decode = f128 * n256;
+  if (K <= 4096 ? n128 * f128 * (K > 2048 ? 2 : 4) <= sms : epi == gemm::kEpiF32 ? decode <= 32 || 7 * decode <= 2 * kb : 5 * decode < kb) return 0;
   if (2 * rounds(n128 * f128) < 3 * rounds(n128 * f256)) return 3;
   return stores && 18 * rounds(n256 * f256) <= 10 * rounds(n128 * f256) ? 2 : 1;
 }

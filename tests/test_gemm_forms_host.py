@@ -26,3 +26,25 @@ def test_row_grouped_products(lib, M, rows, groups, K, epi, form):
 def test_results_and_copies_that_the_wide_stores_cannot_take(lib, y, copy, many):
     """fp32 results are stored 32 bytes at a time and their bf16 copy 16: a copy that is only 8-byte aligned (a slice of columns) goes to the form that stores 8."""
     assert (lib.tbv_op_gemm_ex_form(y, copy, 4096, 1024, 2048, 4096, 2, 1, SMS) > 0) == many
+
+
+# 0 decode form, 1 / 2 / 3 tiles of 128 x 256 / 256 x 256 / 128 x 128; results in bf16, with a rotation or a gated unit (epi 1), in fp32 (epi 2)
+@pytest.mark.parametrize("M,N,K,epi,forms", [
+    (288, 512, 8192, 0, [0]), (288, 2048, 8192, 0, [0]), (288, 4096, 8192, 0, [1, 3]),          # nubosun-8b: step size, B and C of its scan
+    (1280, 512, 8192, 1, [0]), (1280, 1024, 8192, 1, [1, 3]), (2560, 384, 8192, 1, [1, 3]),      # llama3-70b: qkv on 8 and 4 ranks
+    (512, 2048, 28672, 0, [0]), (1024, 2048, 28672, 0, [0]), (2048, 2048, 28672, 0, [1, 2, 3]),
+    (1024, 384, 14336, 0, [0]), (2048, 1024, 14336, 0, [1, 2, 3]), (512, 384, 5120, 0, [0]), (1024, 512, 5120, 0, [1, 3]),
+    (512, 2048, 8192, 2, [0]), (1024, 2048, 14336, 2, [0]), (1024, 1536, 5120, 2, [1, 2, 3]), (4096, 4096, 8192, 2, [1, 2, 3]),
+    (2048, 512, 7168, 0, [3]), (2048, 1024, 7168, 0, [3]), (4096, 512, 4096, 0, [1, 3]),         # llama3-2k down, llama3-8b out
+    (2048, 512, 4096, 0, [0]), (2048, 512, 2048, 0, [3]), (3072, 383, 2048, 0, [0]),
+    (28672, 4096, 4096, 1, [1]), (4096, 4096, 14336, 0, [2]), (6144, 4096, 4096, 1, [1])])        # llama3-8b at 4096 tokens
+def test_products_of_many_tokens(lib, M, N, K, epi, forms):
+    assert lib.tbv_op_gemm_ex_form(None, None, M, N, K, M, epi, 1, SMS) in forms
+
+
+@pytest.mark.parametrize("N", [384, 512, 1000, 2048, 4097])
+@pytest.mark.parametrize("M", [128, 1280, 6144])
+@pytest.mark.parametrize("K", [512, 4096, 8192, 28672])
+def test_qkv_projection_goes_with_the_plain_product(lib, N, M, K):
+    """``gemm_qkv_rope`` promises the bits of ``gemm`` and ``rope_kv``: both take the decode form (whose sums over K are split) or neither does."""
+    assert (lib.tbv_op_gemm_ex_form(None, None, M, N, K, M, 1, 1, SMS) > 0) == (lib.tbv_op_gemm_ex_form(None, None, M, N, K, M, 0, 1, SMS) > 0)
