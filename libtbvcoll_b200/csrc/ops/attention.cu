@@ -691,7 +691,7 @@ int tbv_op_paged_attention(const void* q, const void* k_cache, const void* v_cac
 
 // Causal prefill over the paged cache.  tiles: int32 [ntiles, 2] = (first query row, rows <= tile_rows / G) with all
 // rows of a tile belonging to one sequence in position order; ctx_lens[row] = keys visible to that row.  tile_rows is 64, or up to 128 where
-// the tcgen05 kernel (attn_prefill.cu) takes the call: blocks of a multiple of 16 tokens, 16-byte aligned queries and caches, 32-byte aligned results.
+// the tcgen05 kernel (attn_prefill.cu) takes the call: blocks of a multiple of 16 tokens, a positive scale, 16-byte aligned queries, caches and results, query rows that do not overlap.
 int tbv_op_prefill_attention(const void* q, const void* k_cache, const void* v_cache, const void* block_tables,
                              const void* seq_of_query, const void* ctx_lens, const void* tiles, void* out, int nq_rows, int ntiles, int tile_rows,
                              int nq_heads, int nkv, int head_dim, int ldq, int ldo, int block_size, int max_blocks, float scale,

@@ -48,6 +48,7 @@ struct Params {
   __nv_bfloat16* out;        // [rows, ldo], head h at h * 128
   const __nv_bfloat16* gate; // [rows, ldg] or null (PAIR)
   int ntiles, kv_heads, hpk, parts, block_size, max_blocks, ldo, ldg, window, chunk;
+  int wide;                  // rows of out are 32-byte aligned
   float scale_log2, softcap;
   unsigned long long limit_ns;
   int* err;
@@ -343,8 +344,13 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
             for (int q = 0; q < 8; q += 2) w[(e + q) >> 1] = attn_mma::pack_bf16(a[q], a[q + 1]);
           }
-          st_global_32(dst + c, w);                // a whole sector at a time
-          st_global_32(dst + c + 16, w + 8);
+          if (p.wide) {                            // a whole sector at a time
+            st_global_32(dst + c, w);
+            st_global_32(dst + c + 16, w + 8);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 4; q++) *reinterpret_cast<uint4*>(dst + c + 8 * q) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+          }
         }
         __syncwarp();
       }
@@ -384,8 +390,8 @@ int report(cudaError_t e) {
 namespace tbvops {
 
 bool attn_prefill_takes(const void* q, const void* kv, const void* out, int heads, int kv_heads, int ldq, int ldo, int block_size) {
-  const uintptr_t at = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kv);
-  return heads / kv_heads <= kRows && !(at & 15) && !(reinterpret_cast<uintptr_t>(out) & 31) && !(ldq % 8) && !(ldo % 16) && block_size % 16 == 0;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kv) | reinterpret_cast<uintptr_t>(out);
+  return heads / kv_heads <= kRows && !(at & 15) && ldq >= heads * kD && !(ldq % 8) && !(ldo % 8) && block_size % 16 == 0;
 }
 
 int attn_prefill_split(const void* q, const void* k_cache, const void* v_cache, const int* tables, const int* seq_of_row, const int* ctx_lens, const int* tiles,
@@ -393,6 +399,7 @@ int attn_prefill_split(const void* q, const void* k_cache, const void* v_cache, 
   Params p{};
   p.tiles = tiles; p.seq_of_row = seq_of_row; p.ctx_lens = ctx_lens; p.tables = tables; p.out = static_cast<__nv_bfloat16*>(out);
   p.ntiles = ntiles; p.kv_heads = kv_heads; p.hpk = heads / kv_heads; p.parts = 1; p.block_size = block_size; p.max_blocks = max_blocks; p.ldo = ldo;
+  p.wide = !(reinterpret_cast<uintptr_t>(out) & 31) && ldo % 16 == 0;
   p.scale_log2 = scale * attn_mma::kLog2e; p.limit_ns = 2000000000ull; p.err = gemm_err_flag();
   CUtensorMap mq, mk, mv;
   const unsigned long long width = (unsigned long long)kv_heads * kD;
@@ -409,6 +416,7 @@ int attn_prefill_paired(const void* q, const void* cache, const int* tables, con
   p.ntiles = ntiles; p.kv_heads = kv_heads; p.hpk = heads / kv_heads; p.block_size = block_size; p.max_blocks = max_blocks; p.ldo = ldo; p.ldg = ldg;
   p.parts = (64 + kRows / p.hpk - 1) / (kRows / p.hpk);
   p.window = window; p.chunk = chunk; p.softcap = softcap;
+  p.wide = !(reinterpret_cast<uintptr_t>(out) & 31) && ldo % 16 == 0;
   p.scale_log2 = attn_mma::kLog2e; p.limit_ns = 2000000000ull; p.err = gemm_err_flag();
   CUtensorMap mq, mk;
   if (make_tensor_map_heads(&mq, q, rows, heads, kD, ldq, p.hpk, kRows / p.hpk) != 0 || make_tensor_map_bf16(&mk, cache, kAnyCacheRows, 2 * kD, row_len, 16) != 0) return -3;

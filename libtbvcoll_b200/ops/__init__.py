@@ -453,7 +453,8 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
                       seq_of_query: torch.Tensor, tiles: torch.Tensor, out: torch.Tensor, scale: float, block_size: int, tile_rows: int = 64) -> torch.Tensor:
     """Causal attention of prompt rows over the paged cache with query tiling on tensor cores: up to
     ``tile_rows`` (token, head) rows share every K/V tile.  Same arguments as ``paged_attention`` plus ``tiles``
-    (device int32 [ntiles, 2] from ``prefill_tiles``) and the ``tile_rows`` they were made for (``prefill_tile_rows`` or less)."""
+    (device int32 [ntiles, 2] from ``prefill_tiles``) and the ``tile_rows`` they were made for (``prefill_tile_rows`` or less; more than 64 also need a
+    positive ``scale``, 16-byte aligned rows and query rows that do not overlap)."""
     Nq, nq, D = q.shape
     nkv = k_cache.shape[-2]
     assert q.stride(2) == 1 and q.stride(1) == D and out.stride(2) == 1 and out.stride(1) == D and tiles.dtype is torch.int32

@@ -53,8 +53,10 @@ def layout(lens, starts, bs, seed):
 LENS, STARTS = [129, 1, 31, 128, 300, 33], [0, 127, 128, 129, 5, 700]
 
 
-@pytest.mark.parametrize("nq,nkv,bs,tile_rows", [(8, 2, 16, 128), (8, 2, 16, 64), (4, 4, 48, 128), (8, 1, 32, 128), (4, 2, 16, 100)])
-def test_split_caches(ops, nq, nkv, bs, tile_rows):
+# the last column: channels by which the results lie beside a 32-byte boundary (rows then are no multiple of 32 bytes either)
+@pytest.mark.parametrize("nq,nkv,bs,tile_rows,off", [(8, 2, 16, 128, 0), (8, 2, 16, 64, 0), (4, 4, 48, 128, 0), (8, 1, 32, 128, 0), (4, 2, 16, 100, 0), (8, 2, 16, 128, 8), (4, 4, 16, 64, 8),
+                                                     (8, 2, 16, 64, 4), (8, 2, 8, 64, 0), (4, 4, 24, 64, 2), (8, 1, 8, 64, 0), (4, 2, 40, 64, 0)])
+def test_split_caches(ops, nq, nkv, bs, tile_rows, off):
     tables, nblocks = layout(LENS, STARTS, bs, 1)
     kc, vc = rnd(nblocks * bs, nkv, D, seed=1), rnd(nblocks * bs, nkv, D, seed=2)
     written = torch.zeros(nblocks * bs, dtype=torch.bool)
@@ -70,9 +72,10 @@ def test_split_caches(ops, nq, nkv, bs, tile_rows):
     T, scale = int(seqof.numel()), 0.2
     wide = rnd(T, (nq + 2 * nkv) * D, seed=3)
     q = wide.view(T, -1, D)[:, :nq]                          # as in the model: a view into the projection
-    out = torch.full((T, nq, D), 7.0, dtype=torch.bfloat16, device=DEV)
+    around = torch.full((T, nq * D + off), 7.0, dtype=torch.bfloat16, device=DEV)
+    out = around[:, off:].unflatten(1, (nq, D))
     tiles = ops.prefill_tiles(seqof, nq // nkv, tile_rows)
-    assert ops.prefill_tile_rows(bs) == 128
+    assert ops.prefill_tile_rows(bs) == (64 if bs % 16 else 128)
     ops.prefill_attention(q, kc, vc, tables.to(DEV), ctx.to(DEV), seqof.to(DEV), tiles.to(DEV), out, scale, bs, tile_rows)
     torch.cuda.synchronize()
     assert not ops.gemm_error()
@@ -82,6 +85,7 @@ def test_split_caches(ops, nq, nkv, bs, tile_rows):
         see = torch.arange(s + 1, s + n + 1, device=DEV)
         check(out[r0: r0 + n], *plain(q[r0: r0 + n], kc[rows], vc[rows], scale, see, torch.zeros_like(see)))
         r0 += n
+    assert (around[:, :off] == 7).all()
 
 
 def test_growing_and_huge_scores(ops):
@@ -102,10 +106,10 @@ def test_growing_and_huge_scores(ops):
     assert ((out.double() - want).abs() <= size * 2.0 ** -6.8 + 1e-6).all()
 
 
-@pytest.mark.parametrize("H,G,window,chunk,cap,gated", [(8, 2, 0, 0, 0.0, False), (4, 4, 130, 0, 0.0, True), (8, 1, 0, 200, 20.0, False), (12, 2, 1, 0, 50.0, True),
-                                                        (20, 1, 128, 0, 0.0, False)])
-def test_paired_rows(ops, H, G, window, chunk, cap, gated):
-    bs = 16
+@pytest.mark.parametrize("H,G,window,chunk,cap,gated,bs,off", [(8, 2, 0, 0, 0.0, False, 16, 0), (4, 4, 130, 0, 0.0, True, 16, 0), (8, 1, 0, 200, 20.0, False, 16, 0),
+                                                               (12, 2, 1, 0, 50.0, True, 16, 0), (20, 1, 128, 0, 0.0, False, 16, 0), (8, 2, 130, 0, 0.0, True, 16, 8),
+                                                               (8, 2, 0, 0, 0.0, True, 8, 0), (12, 2, 130, 0, 50.0, False, 24, 8), (4, 4, 0, 200, 0.0, False, 8, 0)])
+def test_paired_rows(ops, H, G, window, chunk, cap, gated, bs, off):
     tables, nblocks = layout(LENS, STARTS, bs, 2)
     row = 2 * D + 8
     cache = rnd(nblocks * G * bs, row, seed=11)
@@ -124,7 +128,8 @@ def test_paired_rows(ops, H, G, window, chunk, cap, gated):
         tiles += [(r0 + k, min(64, n - k), 0, s + k + 1) for k in range(0, n, 64)]
         r0 += n
     tiles = torch.tensor(tiles, dtype=torch.int32, device=DEV)
-    out = torch.full((T, H * D), 7.0, dtype=torch.bfloat16, device=DEV)
+    around = torch.full((T, H * D + off), 7.0, dtype=torch.bfloat16, device=DEV)
+    out = around[:, off:]
     ops.paired_attention_prefill(q, cache, tables.to(DEV), seqof.to(DEV), tiles, out, H, G, D, bs, cap, window, chunk, gate if gated else None)
     torch.cuda.synchronize()
     assert not ops.gemm_error()
@@ -137,8 +142,9 @@ def test_paired_rows(ops, H, G, window, chunk, cap, gated):
         if gated:
             f = torch.sigmoid(gate[r0: r0 + n].double()).view(n, H, D)
             want, size = want * f, size * f
-        check(out[r0: r0 + n].view(n, H, D), want, size)
+        check(out[r0: r0 + n].unflatten(1, (H, D)), want, size)
         r0 += n
+    assert (around[:, :off] == 7).all()
 
 
 @pytest.mark.parametrize("paired,hpk", [(False, 4), (False, 1), (True, 4), (True, 6)])

@@ -12,7 +12,8 @@ def rnd(*shape, seed, dtype=torch.bfloat16):
     return torch.randn(shape, generator=g, device=DEV).to(dtype)
 
 
-@pytest.mark.parametrize("nq,nkv,bs", [(4, 4, 16), (8, 4, 48), (16, 4, 16), (8, 1, 32)])
+# blocks of 8, 24 and 40 tokens: the form for any block size (k_paged_attn_mma)
+@pytest.mark.parametrize("nq,nkv,bs", [(4, 4, 16), (8, 4, 48), (16, 4, 16), (8, 1, 32), (4, 4, 8), (8, 4, 24), (16, 4, 40), (8, 1, 8)])
 @pytest.mark.parametrize("splits", [1, 2, 3, 8])
 def test_paged_rows(nq, nkv, bs, splits):
     """Contexts around the units of 16 tokens, of warps and of splits; nothing that lies behind a context matters; rows out of order over the sequences."""
