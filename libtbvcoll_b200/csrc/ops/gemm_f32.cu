@@ -210,6 +210,17 @@ cudaError_t launch_tiled(const F32Params& p, cudaStream_t st) {
   return pdl::launch(k_gemm_f32_tiled<RT, RF>, grid, dim3(128), smem, st, 1, p);
 }
 
+// Tile of the tiled form: results per thread, 10 * tokens + features.
+// 64 x 64 tiles do most work per byte and instruction.  Smaller ones where they would leave SMs idle or with one or two CTAs, whose loads nothing hides
+// (604 tokens, K 4096: 160 features 104 us with 32 x 64, 73 with 16 x 32; 2048 features 369 us with 64 x 64, 347 with 32 x 64), where few
+// columns leave no time to fill the ring (1000 tokens, 4096 x 128: 50 and 38 us), or where their last round would be emptier.  A grid has at most 65535 rows of tiles.
+int f32_tile(int M, int N, int K, int groups, int m_last, long sms) {
+  const long ft = (long)groups * ((M + 63) / 64) + (m_last + 63) / 64;
+  const long t32 = ft * ((N + 31l) / 32), r64 = (ft * ((N + 63l) / 64) + sms - 1) / sms, r32 = (t32 + sms - 1) / sms;
+  if (t32 < sms) return N > 16 && N <= 32 ? 42 : 22;
+  return (N + 31l) / 32 <= 65535 && (K < 512 || r64 <= 2 || 23 * r32 < 40 * r64) ? 44 : 84;
+}
+
 int launch_f32(const F32Params& p, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool wide = !((reinterpret_cast<uintptr_t>(p.w) | reinterpret_cast<uintptr_t>(p.x)) & 15) && p.K % 4 == 0 && p.ldx % 4 == 0 && p.x_group % 4 == 0;
@@ -218,15 +229,12 @@ int launch_f32(const F32Params& p, void* stream) {
     const dim3 grid(p.groups * ((p.M + kT - 1) / kT) + (p.m_last + kT - 1) / kT, (p.N + kT - 1) / kT);
     e = pdl::launch(k_gemm_f32, grid, dim3(256), 0, st, 1, p);
   } else {
-    // 64 x 64 tiles do most work per byte and instruction.  Smaller ones where they would leave SMs idle or with one or two CTAs, whose loads nothing hides
-    // (604 tokens, K 4096: 160 features 104 us with 32 x 64, 73 with 16 x 32; 2048 features 369 us with 64 x 64, 347 with 32 x 64), where few
-    // columns leave no time to fill the ring (1000 tokens, 4096 x 128: 50 and 38 us), or where their last round would be emptier.
-    const long sms = tbvops::sm_count(), ft = (long)p.groups * ((p.M + 63) / 64) + (p.m_last + 63) / 64;
-    const long t32 = ft * ((p.N + 31) / 32), r64 = (ft * ((p.N + 63) / 64) + sms - 1) / sms, r32 = (t32 + sms - 1) / sms;
-    if (t32 < sms && p.N <= 16) e = launch_tiled<2, 2>(p, st);
-    else if (t32 < sms) e = p.N <= 32 ? launch_tiled<4, 2>(p, st) : launch_tiled<2, 2>(p, st);
-    else if (p.K < 512 || r64 <= 2 || 23 * r32 < 40 * r64) e = launch_tiled<4, 4>(p, st);
-    else e = launch_tiled<8, 4>(p, st);
+    switch (f32_tile(p.M, p.N, p.K, p.groups, p.m_last, tbvops::sm_count())) {
+      case 22: e = launch_tiled<2, 2>(p, st); break;
+      case 42: e = launch_tiled<4, 2>(p, st); break;
+      case 44: e = launch_tiled<4, 4>(p, st); break;
+      default: e = launch_tiled<8, 4>(p, st); break;
+    }
   }
   return e == cudaSuccess ? 0 : -1;
 }
@@ -243,6 +251,9 @@ int tbv_op_gemm_f32(const void* w, const void* x, void* y, const void* bias, int
               M, N, K, ldx, ldy, epi, act, groups > 1 ? groups : 1, x_group, y_group, act_a, act_b, act_c, groups > 1 ? m_last : 0, act_m, nullptr};
   return launch_f32(p, stream);
 }
+
+// Tile that the tiled form takes for a shape on a GPU of `sms` SMs (results per thread, 10 * tokens + features); needs no device.
+int tbv_op_gemm_f32_tile(int M, int N, int K, int groups, int m_last, int sms) { return f32_tile(M, N, K, groups, m_last, sms); }
 
 // Arguments as tbv_op_gemm_rows, everything fp32.
 int tbv_op_gemm_rows_f32(const void* w, const void* x, void* y, const void* row_off, int groups, int M, int x_rows, int max_rows, int K, int ldx,

@@ -1,4 +1,4 @@
-"""The fp32 GEMM: every tile form, remainders, grouped and row-grouped problems, operands that only the general form takes."""
+"""The fp32 GEMM: every tile, remainders, grouped and row-grouped problems, operands that only the general form takes."""
 import pytest
 import torch
 
@@ -70,3 +70,13 @@ def test_row_groups():
         a, b = int(off[g]), int(off[g + 1])
         want = x[a:b].double() @ w[g * M: (g + 1) * M].double().t()
         assert ((out[a:b].double() - want).abs() <= limit(x[a:b], w[g * M: (g + 1) * M])).all()
+
+
+def test_more_rows_than_a_grid_has_small_tiles():
+    from libtbvcoll_b200 import ops
+    N, M, K = 32 * 65535 + 33, 3, 4
+    x, w = rnd(N, K, seed=1), rnd(M, K, seed=2)
+    out = torch.zeros(N, M, device=DEV)
+    ops.linear(x, w, out)
+    want = x.double() @ w.double().t()
+    assert ((out.double() - want).abs() <= limit(x, w)).all()

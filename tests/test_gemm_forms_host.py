@@ -48,3 +48,11 @@ def test_products_of_many_tokens(lib, M, N, K, epi, forms):
 def test_qkv_projection_goes_with_the_plain_product(lib, N, M, K):
     """``gemm_qkv_rope`` promises the bits of ``gemm`` and ``rope_kv``: both take the decode form (whose sums over K are split) or neither does."""
     assert (lib.tbv_op_gemm_ex_form(None, None, M, N, K, M, 1, 1, SMS) > 0) == (lib.tbv_op_gemm_ex_form(None, None, M, N, K, M, 0, 1, SMS) > 0)
+
+
+def test_every_fp32_call_fits_the_grid(lib):
+    """A grid has at most 65535 rows of tiles, 8 tokens per result of a thread: up to 64 x 65535 rows are taken, as the general form takes them."""
+    for N in (1, 17, 33, 5000, 32 * 65535, 32 * 65535 + 1, 64 * 65535):
+        for M, K in ((1, 4), (4096, 128), (64, 4096), (7168, 2048)):
+            tile = lib.tbv_op_gemm_f32_tile(M, N, K, 1, 0, SMS)
+            assert tile in (22, 42, 44, 84) and (N + 8 * (tile // 10) - 1) // (8 * (tile // 10)) <= 65535
