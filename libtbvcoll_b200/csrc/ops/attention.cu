@@ -692,15 +692,19 @@ int tbv_op_paged_attention(const void* q, const void* k_cache, const void* v_cac
 // Causal prefill over the paged cache.  tiles: int32 [ntiles, 2] = (first query row, rows <= tile_rows / G) with all
 // rows of a tile belonging to one sequence in position order; ctx_lens[row] = keys visible to that row.  tile_rows is 64, or up to 128 where
 // the tcgen05 kernel (attn_prefill.cu) takes the call: blocks of a multiple of 16 tokens, a positive scale, 16-byte aligned queries, caches and results, query rows that do not overlap.
+// keys: the most keys that any row sees, as far as the caller knows (0: it does not).  A CTA of the tcgen05 kernel has some 7 us of set-up and one tile of 128 keys behind it
+// whatever it has to do; with up to 64 keys the 64-row form is through before (us, 64-row form / tcgen05, 16 query and 4 key heads: 1 x 32 tokens 4.0 / 6.9, 256 x 16 14.6 / 29.5,
+// 1 x 64 5.6 / 7.0, 64 x 64 19.3 / 17.7; the other side: 1 x 96 7.1 / 7.1, 8 x 96 10.7 / 8.5).
 int tbv_op_prefill_attention(const void* q, const void* k_cache, const void* v_cache, const void* block_tables,
-                             const void* seq_of_query, const void* ctx_lens, const void* tiles, void* out, int nq_rows, int ntiles, int tile_rows,
+                             const void* seq_of_query, const void* ctx_lens, const void* tiles, void* out, int nq_rows, int ntiles, int tile_rows, int keys,
                              int nq_heads, int nkv, int head_dim, int ldq, int ldo, int block_size, int max_blocks, float scale,
                              void* stream) {
   if (ntiles <= 0) return 0;
   if (head_dim != kD || nq_heads % nkv || (ldq % 8) || block_size <= 0) return -2;
   const int G = nq_heads / nkv;
   if (G != 1 && G != 2 && G != 4 && G != 8) return -2;
-  if (scale > 0.f && tile_rows <= 128 && !(reinterpret_cast<uintptr_t>(v_cache) & 15) && tbvops::attn_prefill_takes(q, k_cache, out, nq_heads, nkv, ldq, ldo, block_size))
+  const bool few = keys > 0 && keys <= 64 && tile_rows <= 64;
+  if (!few && scale > 0.f && tile_rows <= 128 && !(reinterpret_cast<uintptr_t>(v_cache) & 15) && tbvops::attn_prefill_takes(q, k_cache, out, nq_heads, nkv, ldq, ldo, block_size))
     return tbvops::attn_prefill_split(q, k_cache, v_cache, static_cast<const int*>(block_tables), static_cast<const int*>(seq_of_query),
                                       static_cast<const int*>(ctx_lens), static_cast<const int*>(tiles), out, nq_rows, ntiles, nq_heads, nkv, ldq, ldo, block_size,
                                       max_blocks, scale, static_cast<cudaStream_t>(stream));

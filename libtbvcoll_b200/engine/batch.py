@@ -35,8 +35,9 @@ class StepBatch:
     out_tokens: Optional[torch.Tensor] = None      # int64: greedy tokens of the logit rows (None: no sampling)
     logits_out: Optional[torch.Tensor] = None      # fp32 [n_logits, vocab]: the logits themselves
     attn_splits: int = 1
-    # paged-attention query tiles (ops.prefill_tiles)
+    # paged-attention query tiles (ops.prefill_tiles) and the most keys that a row of the pass sees
     tiles: Optional[torch.Tensor] = None
+    tile_keys: int = 0
     # models with carried state: int32 [nseg, 4] (first row, rows, state slot, 0) and the segment of every row (None: identity)
     segs: Optional[torch.Tensor] = None
     seg_of_row: Optional[torch.Tensor] = None

@@ -148,7 +148,7 @@ class Engine:
             if self.sp_prefill and hasattr(self.model, "sp_ok") and self.model.sp_ok(batch.T):
                 sel = batch.logit_rows if rows else torch.zeros(1, dtype=torch.int64, device=self.device)
                 self.model.forward_sp(batch.T, batch.ids, batch.positions, batch.slots, self.bm.tables, batch.ctx, batch.seq_of_row, sel,
-                                      max(len(rows), 1), out, prefill_tiles=batch.tiles)
+                                      max(len(rows), 1), out, prefill_tiles=batch.tiles, prefill_keys=batch.tile_keys)
                 self.sp_chunks += 1
             else:
                 self.model.forward_batch(batch)
@@ -198,7 +198,8 @@ class Engine:
                 if m.expands_context:
                     b.dense_slots = put(hb.dense_slots, np.int64)
         elif self.tiled_prefill_attention:
-            b.tiles = ops.prefill_tiles(torch.from_numpy(hb.seq.astype(np.int32)), m.nq // m.nkv, ops.prefill_tile_rows(self.block_size)).to(dev)
+            b.tile_keys = int(hb.pos.max()) + 1
+            b.tiles = ops.prefill_tiles(torch.from_numpy(hb.seq.astype(np.int32)), m.nq // m.nkv, ops.prefill_tile_rows(self.block_size, b.tile_keys)).to(dev)
         return b
 
     # ---- one mixed step ---------------------------------------------------------------------------

@@ -95,13 +95,13 @@ class LlamaTP:
                 rows = torch.zeros(1, dtype=torch.int64, device=self.device)
             out = b.out_tokens if b.out_tokens is not None and b.n_logits else torch.empty(1, dtype=torch.int64, device=self.device)
             self.forward(b.T, b.ids, b.positions, b.slots, b.tables, b.ctx, b.seq_of_row, rows, max(b.n_logits, 1), out,
-                         attn_splits=b.attn_splits, prefill_tiles=b.tiles, layer_begin=layer_begin, layer_end=layer_end)
+                         attn_splits=b.attn_splits, prefill_tiles=b.tiles, prefill_keys=b.tile_keys, layer_begin=layer_begin, layer_end=layer_end)
             return
         n0 = min(b.n_logits, self.max_batch)
         out = b.out_tokens if b.out_tokens is not None else torch.empty(n0, dtype=torch.int64, device=self.device)
         assert b.out_tokens is None or b.n_logits <= self.max_batch
         self.forward(b.T, b.ids, b.positions, b.slots, b.tables, b.ctx, b.seq_of_row, b.logit_rows[:n0], n0, out, attn_splits=b.attn_splits,
-                     prefill_tiles=b.tiles)
+                     prefill_tiles=b.tiles, prefill_keys=b.tile_keys)
         for c0 in range(0, b.n_logits, self.max_batch):
             n = min(self.max_batch, b.n_logits - c0)
             if c0:
@@ -118,9 +118,10 @@ class LlamaTP:
     def forward(self, T: int, ids: torch.Tensor, positions: torch.Tensor, slot_mapping: torch.Tensor, block_tables: torch.Tensor,
                 ctx_lens: torch.Tensor, seq_of_query: Optional[torch.Tensor], logit_rows: Optional[torch.Tensor], n_logits: int,
                 out_tokens: torch.Tensor, attn_splits: int = 1, prefill_tiles: Optional[torch.Tensor] = None,
-                layer_begin: int = 0, layer_end: Optional[int] = None) -> Optional[torch.Tensor]:
+                layer_begin: int = 0, layer_end: Optional[int] = None, prefill_keys: int = 0) -> Optional[torch.Tensor]:
         """ids/positions/slot_mapping/ctx_lens: [T]; logit_rows: int64 [n_logits] rows whose next
         token is wanted (None = all T rows, decode).  Writes greedy tokens to out_tokens[:n_logits].
+        ``prefill_tiles``: query tiles (``ops.prefill_tiles`` with ``ops.prefill_tile_rows`` of the block size and ``prefill_keys``, the most keys that a row sees).
         ``layer_begin`` / ``layer_end`` run a slice of the model (the state between slices lives in this object's
         static buffers): the embedding and first norm belong to the slice that starts at layer 0, the LM head and
         the sampling to the slice that ends at the last layer; other slices return None."""
@@ -147,7 +148,7 @@ class LlamaTP:
                               self.nq, self.nkv, bias=w.get(p + "qkv.bias"))
             if prefill_tiles is not None:
                 ops.prefill_attention(q_view, self.k_cache[l], self.v_cache[l], block_tables, ctx_lens, seq_of_query, prefill_tiles,
-                                      attn_view, self.scale, self.block_size, ops.prefill_tile_rows(self.block_size))
+                                      attn_view, self.scale, self.block_size, ops.prefill_tile_rows(self.block_size, prefill_keys), prefill_keys)
             else:
                 ops.paged_attention(q_view, self.k_cache[l], self.v_cache[l], block_tables, ctx_lens, attn_view, self.scale,
                                     self.block_size, seq_of_query=seq_of_query, splits=attn_splits, workspace=self.attn_ws)
@@ -183,7 +184,7 @@ class LlamaTP:
         return bool(bn) and T * H * 2 <= tp.comm.cap and (rpr // bn) * (H // 128) <= 256
 
     def forward_sp(self, T: int, ids, positions, slot_mapping, block_tables, ctx_lens, seq_of_query, logit_rows, n_logits, out_tokens,
-                   prefill_tiles=None):
+                   prefill_tiles=None, prefill_keys: int = 0):
         """Prefill with the token dimension sharded between the collectives (Megatron-style
         sequence parallelism): residual stream and norms live on T/tp rows; each column-parallel GEMM
         is all-gather -> GEMM, each row-parallel GEMM is GEMM -> reduce-scatter (+ residual + RMSNorm
@@ -212,7 +213,7 @@ class LlamaTP:
             ops.rope_kv(qkv, positions, self.cos_sin, slot_mapping, self.k_cache[l], self.v_cache[l], self.nq, self.nkv, self.D)
             if prefill_tiles is not None:
                 ops.prefill_attention(q_view, self.k_cache[l], self.v_cache[l], block_tables, ctx_lens, seq_of_query, prefill_tiles,
-                                      attn_view, self.scale, self.block_size, ops.prefill_tile_rows(self.block_size))
+                                      attn_view, self.scale, self.block_size, ops.prefill_tile_rows(self.block_size, prefill_keys), prefill_keys)
             else:
                 ops.paged_attention(q_view, self.k_cache[l], self.v_cache[l], block_tables, ctx_lens, attn_view, self.scale,
                                     self.block_size, seq_of_query=seq_of_query, splits=1)

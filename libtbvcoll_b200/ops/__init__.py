@@ -93,7 +93,7 @@ def lib():
     l.tbv_op_gemm_prefetch_next.restype = None
     l.tbv_op_copy_async.argtypes = [c_vp, c_vp, ctypes.c_size_t, c_vp]
     l.tbv_op_copy_async.restype = I
-    l.tbv_op_prefill_attention.argtypes = [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, I, I, I, I, I, I, I, I, I, I, F, c_vp]
+    l.tbv_op_prefill_attention.argtypes = [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, I, I, I, I, I, I, I, I, I, I, I, F, c_vp]
     l.tbv_op_prefill_attention.restype = I
     l.tbv_op_attn_workspace.argtypes = [I, I, I, I]
     l.tbv_op_attn_workspace.restype = SZ
@@ -422,10 +422,10 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     return out
 
 
-def prefill_tile_rows(block_size: int) -> int:
-    """(token, head) rows that a tile of ``prefill_attention`` may have: the tcgen05 kernel multiplies 128 at a time, the other form, which takes blocks of
-    any size, 64."""
-    return 128 if block_size % 16 == 0 else 64
+def prefill_tile_rows(block_size: int, keys: int = 0) -> int:
+    """(token, head) rows that a tile of ``prefill_attention`` should have: the tcgen05 kernel multiplies 128 at a time, the other form, which takes blocks of
+    any size and is faster where no row sees more than 64 keys, 64.  ``keys``: the most keys that any row sees (0: not known)."""
+    return 64 if block_size % 16 or 0 < keys <= 64 else 128
 
 
 def prefill_tiles(seq_of_row, group: int, rows: int = 64) -> torch.Tensor:
@@ -450,16 +450,18 @@ def prefill_tiles(seq_of_row, group: int, rows: int = 64) -> torch.Tensor:
 
 
 def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_tables: torch.Tensor, ctx_lens: torch.Tensor,
-                      seq_of_query: torch.Tensor, tiles: torch.Tensor, out: torch.Tensor, scale: float, block_size: int, tile_rows: int = 64) -> torch.Tensor:
+                      seq_of_query: torch.Tensor, tiles: torch.Tensor, out: torch.Tensor, scale: float, block_size: int, tile_rows: int = 64,
+                      keys: int = 0) -> torch.Tensor:
     """Causal attention of prompt rows over the paged cache with query tiling on tensor cores: up to
     ``tile_rows`` (token, head) rows share every K/V tile.  Same arguments as ``paged_attention`` plus ``tiles``
     (device int32 [ntiles, 2] from ``prefill_tiles``) and the ``tile_rows`` they were made for (``prefill_tile_rows`` or less; more than 64 also need a
-    positive ``scale``, 16-byte aligned rows and query rows that do not overlap)."""
+    positive ``scale``, 16-byte aligned rows and query rows that do not overlap).  ``keys``: the most keys that any row sees, 0 if that is not known; it takes part in the
+    choice of the kernel and nothing else."""
     Nq, nq, D = q.shape
     nkv = k_cache.shape[-2]
     assert q.stride(2) == 1 and q.stride(1) == D and out.stride(2) == 1 and out.stride(1) == D and tiles.dtype is torch.int32
     _chk(lib().tbv_op_prefill_attention(_p(q), _p(k_cache), _p(v_cache), _p(block_tables), _p(seq_of_query), _p(ctx_lens), _p(tiles),
-                                        _p(out), Nq, tiles.shape[0], tile_rows, nq, nkv, D, q.stride(0), out.stride(0), block_size,
+                                        _p(out), Nq, tiles.shape[0], tile_rows, keys, nq, nkv, D, q.stride(0), out.stride(0), block_size,
                                         block_tables.shape[1], scale, _st()), "tbv_op_prefill_attention")
     _count()
     return out

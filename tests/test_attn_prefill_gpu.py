@@ -53,10 +53,11 @@ def layout(lens, starts, bs, seed):
 LENS, STARTS = [129, 1, 31, 128, 300, 33], [0, 127, 128, 129, 5, 700]
 
 
-# the last column: channels by which the results lie beside a 32-byte boundary (rows then are no multiple of 32 bytes either)
-@pytest.mark.parametrize("nq,nkv,bs,tile_rows,off", [(8, 2, 16, 128, 0), (8, 2, 16, 64, 0), (4, 4, 48, 128, 0), (8, 1, 32, 128, 0), (4, 2, 16, 100, 0), (8, 2, 16, 128, 8), (4, 4, 16, 64, 8),
-                                                     (8, 2, 16, 64, 4), (8, 2, 8, 64, 0), (4, 4, 24, 64, 2), (8, 1, 8, 64, 0), (4, 2, 40, 64, 0)])
-def test_split_caches(ops, nq, nkv, bs, tile_rows, off):
+# keys: what the caller says of the longest context (64 or less: the 64-row form); off: channels by which the results lie beside a 32-byte boundary (rows then are no multiple of 32 bytes either)
+@pytest.mark.parametrize("nq,nkv,bs,tile_rows,off,keys", [(8, 2, 16, 128, 0, 0), (8, 2, 16, 64, 0, 0), (4, 4, 48, 128, 0, 0), (8, 1, 32, 128, 0, 64), (4, 2, 16, 100, 0, 64), (8, 2, 16, 128, 8, 0), (4, 4, 16, 64, 8, 0),
+                                                     (8, 2, 16, 64, 4, 0), (8, 2, 8, 64, 0, 0), (4, 4, 24, 64, 2, 0), (8, 1, 8, 64, 0, 0), (4, 2, 40, 64, 0, 0),
+                                                          (8, 2, 16, 64, 0, 64), (4, 4, 48, 64, 0, 1), (8, 2, 16, 64, 0, 65)])
+def test_split_caches(ops, nq, nkv, bs, tile_rows, off, keys):
     tables, nblocks = layout(LENS, STARTS, bs, 1)
     kc, vc = rnd(nblocks * bs, nkv, D, seed=1), rnd(nblocks * bs, nkv, D, seed=2)
     written = torch.zeros(nblocks * bs, dtype=torch.bool)
@@ -76,7 +77,7 @@ def test_split_caches(ops, nq, nkv, bs, tile_rows, off):
     out = around[:, off:].unflatten(1, (nq, D))
     tiles = ops.prefill_tiles(seqof, nq // nkv, tile_rows)
     assert ops.prefill_tile_rows(bs) == (64 if bs % 16 else 128)
-    ops.prefill_attention(q, kc, vc, tables.to(DEV), ctx.to(DEV), seqof.to(DEV), tiles.to(DEV), out, scale, bs, tile_rows)
+    ops.prefill_attention(q, kc, vc, tables.to(DEV), ctx.to(DEV), seqof.to(DEV), tiles.to(DEV), out, scale, bs, tile_rows, keys)
     torch.cuda.synchronize()
     assert not ops.gemm_error()
     r0 = 0

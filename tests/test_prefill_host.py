@@ -49,3 +49,11 @@ def test_prefill_tiles_equal_greedy_segmentation():
             got = ops.prefill_tiles(chunk, g)
             assert got.dtype is torch.int32 and got.tolist() == [list(t) for t in greedy(chunk.tolist(), g)]
     assert ops.prefill_tiles(torch.zeros(0, dtype=torch.int32), 4).shape == (0, 2)
+
+
+def test_tiles_fit_the_kernel_that_takes_them():
+    """128 rows for the tcgen05 kernel, 64 where another form runs: blocks of other than a multiple of 16 tokens, or no context longer than 64 keys."""
+    from libtbvcoll_b200 import ops
+    assert [ops.prefill_tile_rows(b) for b in (8, 16, 24, 32, 48, 64)] == [64, 128, 64, 128, 128, 128]
+    assert [ops.prefill_tile_rows(16, k) for k in (0, 1, 63, 64, 65, 8000)] == [128, 64, 64, 64, 128, 128]
+    assert ops.prefill_tile_rows(8, 8000) == 64
