@@ -75,3 +75,26 @@ def test_fp32_latent_rows_of_many_heads_equal_few():
         one = torch.zeros(1, H, R, device=DEV)
         ops.latent_attention_rows(qa[i: i + 1].contiguous(), cache, tables, seq[:1], ctx[i: i + 1], sink, one, R, 0.05, bs, window=200)
         assert torch.equal(one[0], out[i]) and torch.isfinite(one).all()
+
+
+@pytest.mark.parametrize("paired,H,G,window,chunk,cap", [(False, 8, 2, 0, 0, 30.0), (False, 16, 1, 0, 0, 0.0), (True, 8, 2, 150, 0, 20.0), (True, 8, 1, 0, 140, 0.0)])
+def test_fp32_rows_of_many_heads_equal_few(paired, H, G, window, chunk, cap):
+    """The same for the other two kinds of cached rows: heads of one key head side by side in a CTA, against a row at a time."""
+    from libtbvcoll_b200 import ops
+    D, V, bs, n = 48, 144, 16, 300
+    cache = rnd(20 * G * bs, D + (V if paired else 0) + 8, seed=5, dtype=torch.float32)
+    qa, gate = rnd(n, H, D + 8, seed=6, dtype=torch.float32), rnd(n, H * V, seed=7, dtype=torch.float32)
+    tables = torch.randperm(20, generator=torch.Generator().manual_seed(7))[None].to(torch.int32).to(DEV)
+    seq, ctx = torch.zeros(n, dtype=torch.int32, device=DEV), torch.arange(1, n + 1, dtype=torch.int32, device=DEV)
+
+    def run(i0, i1):
+        out = torch.zeros(i1 - i0, H, V if paired else D, device=DEV)
+        a = (qa[i0:i1].contiguous(), cache, tables, seq[i0:i1], ctx[i0:i1], out, G, bs, cap)
+        if paired:
+            ops.paired_attention_rows(*a, window=window, chunk=chunk, gate=gate[i0:i1])
+        else:
+            ops.shared_attention_rows(*a)
+        return out
+    whole = run(0, n)
+    for i in (0, 127, 128, 139, 140, 150, 299):
+        assert torch.equal(run(i, i + 1)[0], whole[i]) and torch.isfinite(whole[i]).all() and whole[i].any()
