@@ -253,13 +253,15 @@ CUresult encode(CUtensorMap* out, unsigned rank, const void* ptr, const cuuint64
 struct MapKey {
   const void* ptr;
   unsigned long long rows, cols, ld;
-  unsigned box_rows;
-  bool operator==(const MapKey& o) const { return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows; }
+  unsigned box_rows, dim, box_heads;               // the last two: maps of heads (0 otherwise)
+  bool operator==(const MapKey& o) const {
+    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && dim == o.dim && box_heads == o.box_heads;
+  }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
     size_t h = reinterpret_cast<size_t>(k.ptr);
-    h = h * 1000003u ^ k.rows; h = h * 1000003u ^ k.cols; h = h * 1000003u ^ k.ld; h = h * 1000003u ^ k.box_rows;
+    h = h * 1000003u ^ k.rows; h = h * 1000003u ^ k.cols; h = h * 1000003u ^ k.ld; h = h * 1000003u ^ k.box_rows; h = h * 1000003u ^ (k.dim * 512u + k.box_heads);
     return h;
   }
 };
@@ -276,12 +278,11 @@ bool g_attr_done = false;
 
 namespace tbvops {
 
-// [rows, cols] bf16 row-major with row stride ld (elements); box = box_rows x 64, 128-byte swizzle.
-// The encoded map is a pure function of the arguments (it names addresses, it holds no
-// reference), so the memo below can never go stale; `cache = false` skips it for maps that a
+namespace {
+// The encoded map is a pure function of the key (it names addresses, it holds no
+// reference), so the memo can never go stale; `cache = false` skips it for maps that a
 // caller keeps itself.
-int make_tensor_map_bf16(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned long long cols,
-                         unsigned long long ld, unsigned box_rows, bool cache) {
+int make_tensor_map(CUtensorMap* out, const MapKey& key, bool cache) {
   std::call_once(g_encode_once, [] {
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult q;
@@ -289,18 +290,24 @@ int make_tensor_map_bf16(CUtensorMap* out, const void* ptr, unsigned long long r
       g_encode = reinterpret_cast<EncodeTiledFn>(fn);
   });
   if (!g_encode) return -1;
-  MapKey key{ptr, rows, cols, ld, box_rows};
   if (cache) {
     std::lock_guard<std::mutex> g(g_maps_mu);
     auto it = g_maps.find(key);
     if (it != g_maps.end()) { *out = it->second; return 0; }
   }
-  if ((reinterpret_cast<uintptr_t>(ptr) & 15u) || (ld * 2) % 16 || box_rows > 256 || box_rows == 0) return -2;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {ld * 2};
-  cuuint32_t box[2] = {64, box_rows};
+  if ((reinterpret_cast<uintptr_t>(key.ptr) & 15u) || (key.ld * 2) % 16 || key.box_rows > 256 || key.box_rows == 0) return -2;
   CUtensorMap m;
-  if (encode(&m, 2, ptr, dims, strides, box) != CUDA_SUCCESS) return -3;
+  CUresult r;
+  if (key.dim) {
+    const cuuint64_t dims[3] = {key.dim, key.cols / key.dim, key.rows}, strides[2] = {key.dim * 2ull, key.ld * 2};
+    const cuuint32_t box[3] = {64, key.box_heads, key.box_rows};
+    r = encode(&m, 3, key.ptr, dims, strides, box);
+  } else {
+    const cuuint64_t dims[2] = {key.cols, key.rows}, strides[1] = {key.ld * 2};
+    const cuuint32_t box[2] = {64, key.box_rows};
+    r = encode(&m, 2, key.ptr, dims, strides, box);
+  }
+  if (r != CUDA_SUCCESS) return -3;
   if (cache) {
     std::lock_guard<std::mutex> g(g_maps_mu);
     if (g_maps.size() > 65536) g_maps.clear();
@@ -309,15 +316,16 @@ int make_tensor_map_bf16(CUtensorMap* out, const void* ptr, unsigned long long r
   *out = m;
   return 0;
 }
+}  // namespace
 
+// [rows, cols] bf16 row-major with row stride ld (elements); box = box_rows x 64, 128-byte swizzle.
+int make_tensor_map_bf16(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld, unsigned box_rows, bool cache) {
+  return make_tensor_map(out, MapKey{ptr, rows, cols, ld, box_rows, 0, 0}, cache);
+}
 // Heads of `dim` channels side by side, [rows, ld] with head h at h * dim; box = 64 channels x box_heads x box_rows, 128-byte swizzle.
 int make_tensor_map_heads(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned heads, unsigned dim, unsigned long long ld, unsigned box_heads,
                           unsigned box_rows) {
-  CUtensorMap plain;
-  if (make_tensor_map_bf16(&plain, ptr, rows, (unsigned long long)heads * dim, ld, 1) != 0) return -1;   // also looks up the encoder and checks the alignment
-  const cuuint64_t dims[3] = {dim, heads, rows}, strides[2] = {dim * 2ull, ld * 2ull};
-  const cuuint32_t box[3] = {64, box_heads, box_rows};
-  return encode(out, 3, ptr, dims, strides, box) == CUDA_SUCCESS ? 0 : -3;
+  return make_tensor_map(out, MapKey{ptr, rows, (unsigned long long)heads * dim, ld, box_rows, dim, box_heads}, true);
 }
 
 // ---- weights of the GEMM that follows, to be asked into L2 by the kernel launched next ------------------------------
