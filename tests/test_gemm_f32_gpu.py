@@ -11,13 +11,24 @@ def rnd(*shape, seed):
 
 
 def limit(x, w):
-    # sums of 16 in order, then K / 32 of those in order: (16 + K / 32 + 2) roundings of 2^-24 of the sum of the products' sizes
+    # sums of 16 in order, then those in order into a total: (16 + blocks + 2) roundings of 2^-24 of the sum of the products' sizes, with a block of 32 columns (even and odd
+    # ones apart) where rows of four columns can be copied, of 16 in the general form
     K = x.shape[1]
-    return (x.abs().double() @ w.abs().double().t()) * (18 + K / 32) * 2.0 ** -24 + 1e-30
+    block = 32 if K % 4 == 0 and x.stride(0) % 4 == 0 else 16
+    return (x.abs().double() @ w.abs().double().t()) * (18 + -(-K // block)) * 2.0 ** -24 + 1e-30
 
 
-@pytest.mark.parametrize("N", [1, 16, 17, 33, 65, 130, 700])
-@pytest.mark.parametrize("M,K", [(1, 4), (70, 36), (160, 1000), (2050, 516), (300, 130)])     # 130: not a multiple of four columns
+ROWS, SHAPES = [1, 16, 17, 33, 65, 130, 700, 1000], [(1, 4), (70, 36), (160, 1000), (2050, 516), (300, 130)]     # 130: not a multiple of four columns
+
+
+def test_the_cases_here_reach_every_tile():
+    from libtbvcoll_b200 import ops
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert {ops.lib().tbv_op_gemm_f32_tile(M, N, K, 1, 0, sms) for N in ROWS for M, K in SHAPES if K % 4 == 0} == {22, 42, 44, 84}
+
+
+@pytest.mark.parametrize("N", ROWS)
+@pytest.mark.parametrize("M,K", SHAPES)
 def test_plain(N, M, K):
     from libtbvcoll_b200 import ops
     x, w, b = rnd(N, K + 4, seed=1)[:, :K], rnd(M, K, seed=2), rnd(M, seed=3)
