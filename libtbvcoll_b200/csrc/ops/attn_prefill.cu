@@ -13,7 +13,9 @@
 //
 // What bounds it: 16384 exponentials per tile take 1024 clocks of the SM's exponential units (three times that with a soft cap), its two products 1024 clocks of the
 // tensor cores.  Measured (32 query heads, 8 key heads, causal; before: warp-level products, 64 rows per CTA): 8 x 512 tokens 50 us (was 128), 1 x 4096 tokens
-// 155 us (was 868; 0.56 of the tensor peak), rows that hold both 50 and 157 us (were 148 and 848); 1 x 4096, 16 heads, soft cap 50: 4 layers take 0.9 ms less.
+// 155 us (was 868; 0.53 of the measured bf16 burst rate), rows that hold both 50 and 157 us (were 148 and 848); 1 x 4096, 16 heads, soft cap 50: 4 layers take 0.9 ms less.
+// Set-up and one tile take some 7 us, so few keys are better served elsewhere: tbv_op_prefill_attention sends up to 64 of them to the 64-row form.  Rows that hold both
+// stay here: one token 7.1 us (7.2 before), 64 tokens 7.3 (8.1), but 5 tokens with a soft cap 8.5 (7.4).
 //
 // Two kinds of cache (template PAIR): keys and values in caches of their own, [slots, kv_heads, 128] each (k_prefill_attn_mma in attention.cu is the same for
 // blocks of any size), and rows that hold both, [blocks, kv_heads, block_size, 128 + 128 + pad], with windows, chunks, soft cap and gate (shared_attn.cu, for

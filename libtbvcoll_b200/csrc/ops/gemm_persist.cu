@@ -11,7 +11,7 @@
 //   TH = 1, FEAT = 128  128 tokens x 128 features: a quarter less work per byte than 256 features, for problems whose wider tiles would leave SMs idle
 //           (1024 tokens, 2048 x 7168 37 us against 45, 512 tokens, 3072 x 2048 with rotation 20 against 23).
 //   TH = 1  128 tokens x 256 features, two accumulator sets: the epilogue of a tile runs under the MMAs of the next.  For gated units, the rotation, and where
-//           tiles are few.  4096 tokens: 28672 x 4096 with the SiLU unit 641 us = 1500 TFLOP/s (848 with TH = 2), 6144 x 4096 with rotation 159 (166).
+//           tiles are few.  4096 tokens: 28672 x 4096 with the SiLU unit 641 us = 1500 TFLOP/s (848 with TH = 2, which these epilogues had once), 6144 x 4096 with rotation 159 (166).
 //   TH = 2  256 tokens x 256 features as two 128-row MMAs that share one 256-row weight tile: a third less traffic per operation, but both accumulators belong
 //           to one tile, so the epilogue (eight warps here, four per half) is exposed once per tile.  For stores, bf16 or fp32 (the choice does not look at an activation): 4096 x 4096 97 us (104 with TH = 1), 4096 x 14336 361 (402).
 //
