@@ -480,7 +480,8 @@ namespace tbvops {
 // another) while the decode form takes some 1.6 us per 128 x 256 tile of its own, and per k-block only a little: it wins while it has fewer tiles than a fifth of the k-blocks
 // (us, decode form / here: 512 tokens, 288 x 8192 17 / 38, 1280 x 8192 34 / 39, 1024 x 14336 43 / 67, 512 x 28672 32 / 126; 2048 tokens, 288 x 8192 33 / 39,
 // 1024 x 28672 143 / 156; the other side: 512 tokens, 1024 x 5120 28 / 26, 2048 x 7168 48 / 36, 1024 tokens, 1280 x 8192 47 / 41, 2048 tokens, 2048 x 28672 247 / 185).  With fp32
-// results the decode form keeps to a CTA per SM and wins further (2048 tokens, 512 x 8192 24 / 41, 1024 x 14336 58 / 68; the other side: 1536 tokens, 1024 x 5120 31 / 28).
+// results the decode form keeps to a CTA per SM and wins further (2048 tokens, 512 x 8192 24 / 41, 1024 x 14336 58 / 68; 512 tokens, 2560 x 8192 39 / 42; the other side: 1536 tokens, 1024 x 5120 31 / 28,
+// 2048 tokens, 2048 x 28672 212 / 208).
 int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode, int sms) {
   if (!(N >= 384 && (M % 16) == 0 && (K % 8) == 0 && (ldy % 8) == 0 && epi >= 0 && epi <= 3)) return 0;
   const bool stores = epi == gemm::kEpiStore || epi == gemm::kEpiF32;
@@ -488,7 +489,7 @@ int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode, int sms) {
   const long f256 = (M + 255) / 256, f128 = (M + 127) / 128, n128 = (N + 127) / 128, n256 = (N + 255) / 256;
   auto rounds = [&](long tiles) { return (tiles + sms - 1) / sms; };
   const long kb = (K + 63) / 64, decode = f128 * n256;
-  if (K <= 4096 ? n128 * f128 * (K > 2048 ? 2 : 4) <= sms : epi == gemm::kEpiF32 ? decode <= 32 || 7 * decode <= 2 * kb : 5 * decode < kb) return 0;
+  if (K <= 4096 ? n128 * f128 * (K > 2048 ? 2 : 4) <= sms : epi == gemm::kEpiF32 ? decode <= 32 || (decode <= 96 && 5 * decode <= 2 * kb) : 5 * decode < kb) return 0;
   if (2 * rounds(n128 * f128) < 3 * rounds(n128 * f256)) return 3;
   return stores && 18 * rounds(n256 * f256) <= 10 * rounds(n128 * f256) ? 2 : 1;
 }

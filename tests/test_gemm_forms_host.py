@@ -34,7 +34,7 @@ def test_results_and_copies_that_the_wide_stores_cannot_take(lib, y, copy, many)
     (1280, 512, 8192, 1, [0]), (1280, 1024, 8192, 1, [1, 3]), (2560, 384, 8192, 1, [1, 3]),      # llama3-70b: qkv on 8 and 4 ranks
     (512, 2048, 28672, 0, [0]), (1024, 2048, 28672, 0, [0]), (2048, 2048, 28672, 0, [1, 2, 3]),
     (1024, 384, 14336, 0, [0]), (2048, 1024, 14336, 0, [1, 2, 3]), (512, 384, 5120, 0, [0]), (1024, 512, 5120, 0, [1, 3]),
-    (512, 2048, 8192, 2, [0]), (1024, 2048, 14336, 2, [0]), (1024, 1536, 5120, 2, [1, 2, 3]), (4096, 4096, 8192, 2, [1, 2, 3]),
+    (512, 2048, 8192, 2, [0]), (1024, 2048, 14336, 2, [0]), (2560, 512, 8192, 2, [0]), (288, 4096, 8192, 2, [0]), (2048, 2048, 28672, 2, [1, 2, 3]), (1024, 1536, 5120, 2, [1, 2, 3]), (4096, 4096, 8192, 2, [1, 2, 3]),
     (2048, 512, 7168, 0, [3]), (2048, 1024, 7168, 0, [3]), (4096, 512, 4096, 0, [1, 3]),         # llama3-2k down, llama3-8b out
     (2048, 512, 4096, 0, [0]), (2048, 512, 2048, 0, [3]), (3072, 383, 2048, 0, [0]),
     (28672, 4096, 4096, 1, [1]), (4096, 4096, 14336, 0, [2]), (6144, 4096, 4096, 1, [1])])        # llama3-8b at 4096 tokens
