@@ -414,7 +414,7 @@ void gemm_config(int M, int N, int K, int splits_hint, int* bn_out, int* splits_
 }  // namespace tbvops
 
 int tbvops::gemm_persist_mode() {
-  // TBV_GEMM_PERSIST: 0 = never, 1 (default) = where it is estimated to be faster, 2 / 3 / 4 = its 128 x 256 / 256 x 256 (stores only) / 128 x 128
+  // TBV_GEMM_PERSIST: 0 = never, 1 (default) = where it is estimated to be faster, 2 / 3 / 4 = its 128 x 256 / 256 x 256 / 128 x 128
   // tile wherever the shape allows; read once, not per launch.
   if (g_persist_mode == -1) { const char* pe = getenv("TBV_GEMM_PERSIST"); g_persist_mode = pe ? atoi(pe) : 1; }
   return g_persist_mode;

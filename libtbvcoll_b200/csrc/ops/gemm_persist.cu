@@ -11,9 +11,9 @@
 //   TH = 1, FEAT = 128  128 tokens x 128 features: a quarter less work per byte than 256 features, for problems whose wider tiles would leave SMs idle
 //           (1024 tokens, 2048 x 7168 37 us against 45, 512 tokens, 3072 x 2048 with rotation 20 against 23).
 //   TH = 1  128 tokens x 256 features, two accumulator sets: the epilogue of a tile runs under the MMAs of the next.  For gated units, the rotation, and where
-//           tiles are few.  4096 tokens: 28672 x 4096 with the SiLU unit 641 us = 1500 TFLOP/s (848 with TH = 2, which these epilogues had once), 6144 x 4096 with rotation 159 (166).
+//           tiles are few.  4096 tokens: 28672 x 4096 with the SiLU unit 641 us = 1500 TFLOP/s (793 .. 848 with TH = 2), 6144 x 4096 with rotation 159 (166 with a TH = 2 that is gone).
 //   TH = 2  256 tokens x 256 features as two 128-row MMAs that share one 256-row weight tile: a third less traffic per operation, but both accumulators belong
-//           to one tile, so the epilogue (eight warps here, four per half) is exposed once per tile.  For stores, bf16 or fp32 (the choice does not look at an activation): 4096 x 4096 97 us (104 with TH = 1), 4096 x 14336 361 (402).
+//           to one tile, so the epilogue (eight warps here, four per half) is exposed once per tile.  For stores, bf16 or fp32 (the choice does not look at an activation), and gated units of one or two rounds: 4096 x 4096 97 us (104 with TH = 1), 4096 x 14336 361 (402).
 //
 // The CTAs walk tiles id = first + i * step with the token tile fastest: the CTAs running at any
 // moment share a few weight tiles (streamed from HBM once) and the activations stay in L2.  Warp 0
@@ -470,11 +470,13 @@ cudaError_t launch_tok(const void* w, const void* x, const gemm::Params& p, int 
 namespace tbvops {
 
 // Which form takes an [N tokens] x [M features] problem: 0 = the decode-form kernel (gemm.cu), k_gemm_tok with 1 / 2 = 128- / 256-token tiles of 256 features, 3 = 128 x 128
-// tiles.  `mode`: 1 = choose, 2 / 3 / 4 = force the first / second / third tile wherever the shape allows (tests, measurements; 256-token tiles exist for stores).
+// tiles.  `mode`: 1 = choose, 2 / 3 / 4 = force the first / second / third tile wherever the shape allows (tests, measurements; the qkv projection, which asks for epilogue 1, has no 256-token tile and takes 128 x 256 instead).
 //
 // Every CTA walks ceil(tiles / SMs) tiles.  A k-block of a 128 x 128 tile takes two thirds of the time of a 128 x 256 one (both bound by what TMA brings in), and one of
 // 256 x 256 nine tenths of two of those.  512 tokens, 4096 x 4096 24 / 28 / 45 us with 128 x 128 / 128 x 256 / 256 x 256 tiles,
-// 1024 tokens, 14336 x 2048 with the SiLU unit 75 / 61.
+// 1024 tokens, 14336 x 2048 with the SiLU unit 75 / 61.  A gated unit's epilogue is long (10 us for 128 rows) and exposed in 256-token tiles: they pay where all of the problem is
+// one round of them instead of two, or two instead of four of long K, and with short K, where the epilogue is all there is and they have twice the warps for it (us, 128 x 256 / 256 x 256 with the SiLU unit: 512 tokens, 14336 x 4096 62 / 56, 2048 tokens, 4096 x 14336
+// 189 / 165, 4096 x 1792 35 / 32, 1024 tokens, 7168 x 8192 107 / 95; 4096 tokens, 4096 x 8192 217 / 197, 14336 x 128 143 / 85, 14336 x 1024 158 / 144; but 14336 x 2048 on 1000 60 / 64, 8192 x 4096 on 3000 150 / 162).
 // Fewer than 384 tokens, and problems of few tiles, go to the decode form, which shares K out over clusters (512 tokens, fp32, 2048 x 4096: 19 us
 // against 24; 1024 tokens 28 against 24; 512 tokens, 2048 x 2048 15.3 against 13.5).  With long K a CTA here walks all of it (0.3 us per k-block of a 128 x 128 tile, one after
 // another) while the decode form takes some 1.6 us per 128 x 256 tile of its own, and per k-block only a little: it wins while it has fewer tiles than a fifth of the k-blocks
@@ -485,13 +487,16 @@ namespace tbvops {
 int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode, int sms) {
   if (!(N >= 384 && (M % 16) == 0 && (K % 8) == 0 && (ldy % 8) == 0 && epi >= 0 && epi <= 3)) return 0;
   const bool stores = epi == gemm::kEpiStore || epi == gemm::kEpiF32;
-  if (mode >= 2) return mode == 4 ? 3 : (mode == 3 && stores ? 2 : 1);
+  if (mode >= 2) return mode == 4 ? 3 : (mode == 3 ? 2 : 1);
   const long f256 = (M + 255) / 256, f128 = (M + 127) / 128, n128 = (N + 127) / 128, n256 = (N + 255) / 256;
   auto rounds = [&](long tiles) { return (tiles + sms - 1) / sms; };
   const long kb = (K + 63) / 64, decode = f128 * n256;
   if (K <= 4096 ? n128 * f128 * (K > 2048 ? 2 : 4) <= sms : epi == gemm::kEpiF32 ? decode <= 32 || (decode <= 96 && 5 * decode <= 2 * kb) : 5 * decode < kb) return 0;
-  if (2 * rounds(n128 * f128) < 3 * rounds(n128 * f256)) return 3;
-  return stores && 18 * rounds(n256 * f256) <= 10 * rounds(n128 * f256) ? 2 : 1;
+  const long r1 = rounds(n128 * f256), r2 = rounds(n256 * f256);
+  if (2 * rounds(n128 * f128) < 3 * r1) return 3;
+  if (stores) return 18 * r2 <= 10 * r1 ? 2 : 1;
+  if (K <= 1024) return 3 * r2 <= 2 * r1 ? 2 : 1;
+  return 2 * r2 <= r1 && (r2 == 1 || (r2 == 2 && K > 4096)) ? 2 : 1;
 }
 
 // Row-grouped: 0 the decode form, 1 / 2 k_gemm_tok with 128- / 256-token tiles of 256 features (`mode` 2 and 4 / 3 force them).  The decode form re-reads a group's weights
@@ -530,12 +535,17 @@ int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, in
     e = epi == gemm::kEpiClampGlu ? launch_tok<3, 1, 256, true>(w, x, p, ldx, st, &map_rc) :
         th == 2 ? launch_tok<0, 2, 256, true>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1, 256, true>(w, x, p, ldx, st, &map_rc);
   } else switch (epi) {
-    case gemm::kEpiSiluMul: e = th == 3 ? launch_tok<1, 1, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<1, 1, 256>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiSiluMul:
+      e = th == 3 ? launch_tok<1, 1, 128>(w, x, p, ldx, st, &map_rc) : th == 2 ? launch_tok<1, 2, 256>(w, x, p, ldx, st, &map_rc) : launch_tok<1, 1, 256>(w, x, p, ldx, st, &map_rc);
+      break;
     case gemm::kEpiF32:
       e = th == 3 ? launch_tok<2, 1, 128>(w, x, p, ldx, st, &map_rc) : th == 2 ? launch_tok<2, 2, 256>(w, x, p, ldx, st, &map_rc) : launch_tok<2, 1, 256>(w, x, p, ldx, st, &map_rc);
       break;
-    case gemm::kEpiClampGlu: e = th == 3 ? launch_tok<3, 1, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<3, 1, 256>(w, x, p, ldx, st, &map_rc); break;
-    case gemm::kEpiRope: e = th == 3 ? launch_tok<4, 1, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<4, 1, 256>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiClampGlu:
+      e = th == 3 ? launch_tok<3, 1, 128>(w, x, p, ldx, st, &map_rc) : th == 2 ? launch_tok<3, 2, 256>(w, x, p, ldx, st, &map_rc) : launch_tok<3, 1, 256>(w, x, p, ldx, st, &map_rc);
+      break;
+    case gemm::kEpiRope:   // no 256-token form
+      e = th == 3 ? launch_tok<4, 1, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<4, 1, 256>(w, x, p, ldx, st, &map_rc); break;
     default:
       e = th == 3 ? launch_tok<0, 1, 128>(w, x, p, ldx, st, &map_rc) : th == 2 ? launch_tok<0, 2, 256>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1, 256>(w, x, p, ldx, st, &map_rc);
       break;

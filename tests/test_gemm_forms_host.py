@@ -37,6 +37,8 @@ def test_results_and_copies_that_the_wide_stores_cannot_take(lib, y, copy, many)
     (512, 2048, 8192, 2, [0]), (1024, 2048, 14336, 2, [0]), (2560, 512, 8192, 2, [0]), (288, 4096, 8192, 2, [0]), (2048, 2048, 28672, 2, [1, 2, 3]), (1024, 1536, 5120, 2, [1, 2, 3]), (4096, 4096, 8192, 2, [1, 2, 3]),
     (2048, 512, 7168, 0, [3]), (2048, 1024, 7168, 0, [3]), (4096, 512, 4096, 0, [1, 3]),         # llama3-2k down, llama3-8b out
     (2048, 512, 4096, 0, [0]), (2048, 512, 2048, 0, [3]), (3072, 383, 2048, 0, [0]),
+    (7168, 1024, 8192, 1, [2]), (14336, 512, 4096, 3, [2]), (4096, 2048, 14336, 1, [2]), (4096, 4096, 8192, 3, [2]),        # gated units in one or two rounds
+    (14336, 4096, 1024, 1, [2]), (14336, 4096, 128, 3, [2]), (7168, 400, 1024, 1, [1]), (14336, 4096, 1792, 1, [1]),    (14336, 1000, 4096, 1, [1]), (8192, 3000, 4096, 1, [1]), (14336, 768, 4096, 3, [1]), (14336, 1536, 8192, 1, [1]),
     (28672, 4096, 4096, 1, [1]), (4096, 4096, 14336, 0, [2]), (6144, 4096, 4096, 1, [1])])        # llama3-8b at 4096 tokens
 def test_products_of_many_tokens(lib, M, N, K, epi, forms):
     assert lib.tbv_op_gemm_ex_form(None, None, M, N, K, M, epi, 1, SMS) in forms
