@@ -1,0 +1,258 @@
+// gemm_pair.cu — the many-token (prefill) bf16 GEMM on pairs of SMs: a persistent kernel, one CTA per SM, the two CTAs of a cluster on one tile.
+//
+//   Y[n, m] = epilogue( sum_k X[n, k] * W[m, k] )      X: [N tokens, K], W: [M features, K], both bf16 row-major
+//
+// tcgen05.mma.cta_group::2 multiplies 256 token rows, 128 in each CTA's shared memory and TMEM, with kFeat features, half of them in each CTA's shared memory.  So a CTA takes
+// in 128 rows of X and kFeat / 2 rows of W per k-block for 128 x kFeat results: 32 KB where a CTA by itself with a 128 x 256 tile (gemm_persist.cu) takes 48.
+//
+// Warp 0 lane 0 of each CTA feeds its own ring by TMA and reports to the full barriers of the first CTA; warp 1 lane 0 of the FIRST CTA issues the products of both and
+// commits to the barriers of both; warps 2.. of each CTA drain its 128 rows, one tile behind the products (two accumulators of kFeat columns).  Every wait is bounded; who gives
+// up raises its CTA's abort flag, the other CTA's waits then run out too, all roles leave their loops, the pair meets at the cluster barrier and frees its TMEM.
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <stdio.h>
+
+#include <type_traits>
+
+#include "gemm_tok.cuh"
+#include "ops.h"
+
+using namespace sm100;
+using namespace gemm_tok;
+
+namespace {
+
+constexpr int kXBytes = 128 * gemm::kBK * 2;                   // a CTA's token rows of a k-block
+
+constexpr int kTok = 256, kFeat = 256;
+constexpr int kStageBytes = kXBytes + kFeat / 2 * gemm::kBK * 2;               // 32 KB
+constexpr int kStages = 6;
+constexpr int kCols = 2 * kFeat;                               // TMEM columns of two accumulators
+constexpr int kEpiWarps = 8, kSide = kFeat / 2;                // four per half of the features (a head of a qkv projection)
+constexpr int kThreads = 64 + 32 * kEpiWarps;
+
+struct PSmem {
+  unsigned long long full[kStages], empty[kStages], acc_full[2], acc_empty[2];
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+__device__ __forceinline__ void tmem_alloc2(uint32_t smem_dst, uint32_t ncols) {       // a warp of each CTA of the pair
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void umma2_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// one arrival at the barrier of that offset in both CTAs, when the products issued so far have finished
+__device__ __forceinline__ void umma2_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)3) : "memory");
+}
+// into this CTA's shared memory; `bar` (shared::cluster) may be the other CTA's
+__device__ __forceinline__ void tma2_load(uint32_t smem_dst, const CUtensorMap* m, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+               ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma2_load_hint(uint32_t smem_dst, const CUtensorMap* m, int x, int y, uint32_t bar, uint64_t policy) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
+               ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(bar), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// mbar_wait for a barrier at which threads of the other CTA arrive
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned long long limit_ns) {
+  if (!mbar_wait(bar, parity, abort_flag, limit_ns)) return false;
+  asm volatile("fence.acq_rel.cluster;" ::: "memory");
+  return true;
+}
+
+template <int EPI, bool ROWS>
+__global__ void __launch_bounds__(kThreads, 1)
+k_gemm_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ gemm::Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ PSmem s;
+  __shared__ typename std::conditional<ROWS, RowGroups, int>::type groups;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = int(cluster_ctarank()), pair = int(blockIdx.x) >> 1, pairs = int(gridDim.x) >> 1;
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;                  // the same offset in both CTAs
+  const int tok_tiles = (p.N + kTok - 1) / kTok, feat_tiles = (p.M + kFeat - 1) / kFeat, nkb = p.kb_total;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; i++) {
+      mbar_init(smem_u32(&s.full[i]), 1);
+      mbar_init(smem_u32(&s.empty[i]), 1);
+    }
+    for (int i = 0; i < 2; i++) {
+      mbar_init(smem_u32(&s.acc_full[i]), 1);
+      mbar_init(smem_u32(&s.acc_empty[i]), 2 * kEpiWarps);    // one arrival per epilogue warp of both CTAs
+    }
+    s.abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc2(smem_u32(&s.tmem_base), kCols);
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmX);
+    tma_prefetch_desc(&tmW);
+  }
+  __syncwarp();
+  tc_fence_before();
+  cluster_sync_all();                            // the other CTA's barriers stand before anything arrives there
+  tc_fence_after();
+  pdl::launch_dependents();
+  int tiles = tok_tiles * feat_tiles;
+  if constexpr (ROWS) {
+    pdl::grid_dependency_wait();                 // the groups' rows were counted on the device by a kernel before this one
+    count_tiles<kTok, kThreads>(groups, p, feat_tiles);
+    tiles = groups.tile[p.groups];
+  }
+  const int my_tiles = pair < tiles ? (tiles - pair + pairs - 1) / pairs : 0;
+  const int ngroups = p.groups, feats = p.M, all_rows = p.N;
+  // (by value: a capture of the parameter block would put it in local memory)
+  auto locate = [=](int tile) -> At {
+    if constexpr (ROWS) return find_tile<kTok>(groups, tile, ngroups, feats);
+    const int f0 = tile / tok_tiles * kFeat;
+    return At{tile % tok_tiles * kTok, all_rows, f0, f0};
+  };
+  const uint32_t tmem0 = s.tmem_base;
+  volatile int* abortp = &s.abort_flag;
+
+  if (warp == 0 && lane == 0) {
+    // ---- TMA producer of this CTA: one flat sequence of k-blocks over all of the pair's tiles ----
+    const uint64_t pol_x = policy_evict_last();
+    const uint32_t full0 = mapa_shared(smem_u32(&s.full[0]), 0);              // barriers of the first CTA
+    // Weights are never written by a kernel: the first ring fill of weight tiles goes out before the
+    // preceding kernel has finished; the activations follow once it has.
+    const int pre = my_tiles ? min(kStages, nkb) : 0;
+    At at = my_tiles ? locate(pair) : At{};
+    for (int i = 0; i < pre; i++) {
+      if (rank == 0) mbar_expect_tx(smem_u32(&s.full[i]), 2 * kStageBytes);
+      tma2_load(base + i * kStageBytes + kXBytes, &tmW, i * gemm::kBK, at.w0 + rank * kFeat / 2, full0 + 8u * i);
+    }
+    pdl::grid_dependency_wait();
+    for (int i = 0; i < pre; i++) tma2_load_hint(base + i * kStageBytes, &tmX, i * gemm::kBK, at.n0 + rank * 128, full0 + 8u * i, pol_x);
+    int st = pre == kStages ? 0 : pre;
+    uint32_t ph = pre == kStages ? 1u : 0u;   // of the ring's current round
+    bool ok = true;
+    for (int t = 0; t < my_tiles && ok; t++) {
+      if (t) at = locate(pair + t * pairs);
+      for (int kb = t ? 0 : pre; kb < nkb; kb++) {
+        // (the first CTA's wait for this round stands behind the products that read the stage, so the other CTA's bytes cannot meet an older round's count)
+        if (!mbar_wait(smem_u32(&s.empty[st]), ph ^ 1u, abortp, p.limit_ns)) { ok = false; break; }
+        if (rank == 0) mbar_expect_tx(smem_u32(&s.full[st]), 2 * kStageBytes);
+        tma2_load_hint(base + st * kStageBytes, &tmX, kb * gemm::kBK, at.n0 + rank * 128, full0 + 8u * st, pol_x);
+        tma2_load(base + st * kStageBytes + kXBytes, &tmW, kb * gemm::kBK, at.w0 + rank * kFeat / 2, full0 + 8u * st);
+        if (++st == kStages) { st = 0; ph ^= 1u; }
+      }
+    }
+    if (*abortp && pre) {
+      // gave up: let the copies already in flight land before this CTA's shared memory goes away (a millisecond is many times what a copy takes)
+      const unsigned long long t0 = globaltimer();
+      while (globaltimer() - t0 < 1000000ull) __nanosleep(1000);
+    }
+  } else if (warp == 1 && lane == 0 && rank == 0) {
+    // ---- MMA issuer for both CTAs ----
+    const uint32_t idesc = umma_idesc_bf16(256, kFeat);
+    int st = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int t = 0; t < my_tiles && ok; t++) {
+      const int buf = t & 1, use = t >> 1;
+      // the epilogues must have drained this accumulator (two tiles ago); passes at once on first use
+      if (!mbar_wait_cluster(smem_u32(&s.acc_empty[buf]), (uint32_t(use) & 1u) ^ 1u, abortp, p.limit_ns)) break;
+      tc_fence_after();
+      const uint32_t tmem_d = tmem0 + uint32_t(buf * kFeat);
+      for (int kb = 0; kb < nkb; kb++) {
+        if (!mbar_wait(smem_u32(&s.full[st]), ph, abortp, p.limit_ns)) { ok = false; break; }
+        tc_fence_after();
+        const uint64_t ad = umma_desc_sw128(base + st * kStageBytes), bd = umma_desc_sw128(base + st * kStageBytes + kXBytes);
+#pragma unroll
+        for (int k = 0; k < gemm::kBK / 16; k++) umma2_bf16(tmem_d, ad + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
+        umma2_commit(smem_u32(&s.empty[st]));
+        if (++st == kStages) { st = 0; ph ^= 1u; }
+      }
+      if (ok) umma2_commit(smem_u32(&s.acc_full[buf]));
+    }
+  } else if (warp >= 2) {
+    // ---- epilogue: thread = one token row of this CTA's 128, on one side of the features ----
+    const int quarter = warp & 3, side = (warp - 2) >> 2;
+    const uint32_t free0 = mapa_shared(smem_u32(&s.acc_empty[0]), 0);
+    for (int t = 0; t < my_tiles; t++) {
+      const int buf = t & 1, use = t >> 1;
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s.acc_full[buf]), uint32_t(use) & 1u, abortp, p.limit_ns));   // together, before the warp-wide TMEM loads
+      if (!ok) break;
+      tc_fence_after();
+      const At at = locate(pair + t * pairs);
+      const int n = at.n0 + rank * 128 + quarter * 32 + lane;   // token row
+      drain<EPI, kSide>(p, n, n < at.nend, at.f0 + side * kSide, tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t(buf * kFeat + side * kSide), [&] {
+        if (lane == 0) mbar_arrive_cluster(free0 + 8u * buf);
+      });
+    }
+  }
+
+  // ---- teardown: both CTAs are done with TMEM, with each other's barriers and shared memory ----
+  __syncwarp();
+  tc_fence_before();
+  cluster_sync_all();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc2(s.tmem_base, kCols);
+  }
+  if (threadIdx.x == 0 && s.abort_flag && p.err) atomicExch(p.err, 1);
+}
+
+template <int EPI, bool ROWS = false>
+cudaError_t launch(const void* w, const void* x, const gemm::Params& p, int ldx, cudaStream_t st, int* map_rc) {
+  CUtensorMap tmX, tmW;
+  *map_rc = 0;
+  if (tbvops::make_tensor_map_bf16(&tmX, x, ROWS ? p.x_rows : p.N, p.K, ldx, 128) != 0 ||
+      tbvops::make_tensor_map_bf16(&tmW, w, (unsigned long long)(ROWS ? p.groups : 1) * p.M, p.K, p.K, kFeat / 2) != 0) {
+    *map_rc = -3;
+    return cudaSuccess;
+  }
+  constexpr size_t smem = size_t(kStages) * kStageBytes + 1024;
+  static std::atomic<unsigned> done{0};
+  const cudaError_t attr = pdl::allow_smem(k_gemm_pair<EPI, ROWS>, smem, done);
+  if (attr != cudaSuccess) return attr;
+  const int tiles = (ROWS ? p.x_rows / 256 + p.groups : (p.N + 255) / 256) * ((p.M + kFeat - 1) / kFeat);   // ROWS: at most
+  const int pairs = tbvops::sm_count() / 2;
+  return pdl::launch_clusters(k_gemm_pair<EPI, ROWS>, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kThreads), smem, st, dim3(2), tmX, tmW, p);   // (pairs lie along x)
+}
+
+}  // namespace
+
+namespace tbvops {
+
+// p is filled (gemm_tok_launch_p)
+int gemm_pair_launch(const void* w, const void* x, const gemm::Params& p, int ldx, int epi, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  int map_rc = 0;
+  cudaError_t e;
+  if (p.row_off) {
+    e = epi == gemm::kEpiClampGlu ? launch<3, true>(w, x, p, ldx, st, &map_rc) : launch<0, true>(w, x, p, ldx, st, &map_rc);
+  } else switch (epi) {
+    case gemm::kEpiSiluMul: e = launch<1>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiF32: e = launch<2>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiClampGlu: e = launch<3>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiRope: e = launch<4>(w, x, p, ldx, st, &map_rc); break;
+    default: e = launch<0>(w, x, p, ldx, st, &map_rc); break;
+  }
+  if (map_rc != 0) return map_rc;
+  if (e != cudaSuccess) {
+    fprintf(stderr, "[tbvops] paired many-token gemm launch failed: %s (M=%d N=%d K=%d)\n", cudaGetErrorString(e), p.M, p.N, p.K);
+    return -1;
+  }
+  return 0;
+}
+
+}  // namespace tbvops

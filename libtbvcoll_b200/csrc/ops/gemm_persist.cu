@@ -7,13 +7,12 @@
 // features on UMMA N.  A thread of the epilogue then owns one token row and reads consecutive features per
 // TMEM load; gate/up pairs of the SiLU-mul epilogue sit in the same thread, so that epilogue needs no shuffles.
 //
-// Tile shapes (templates TH, FEAT); an SM takes in some 70 bytes per clock through TMA (measured with three quarters of the MMAs left out, 133 GB/s), which bounds the smaller ones:
-//   TH = 1, FEAT = 128  128 tokens x 128 features: a quarter less work per byte than 256 features, for problems whose wider tiles would leave SMs idle
-//           (1024 tokens, 2048 x 7168 37 us against 45, 512 tokens, 3072 x 2048 with rotation 20 against 23).
-//   TH = 1  128 tokens x 256 features, two accumulator sets: the epilogue of a tile runs under the MMAs of the next.  For gated units, the rotation, and where
-//           tiles are few.  4096 tokens: 28672 x 4096 with the SiLU unit 641 us = 1500 TFLOP/s (793 .. 848 with TH = 2), 6144 x 4096 with rotation 159 (166 with a TH = 2 that is gone).
-//   TH = 2  256 tokens x 256 features as two 128-row MMAs that share one 256-row weight tile: a third less traffic per operation, but both accumulators belong
-//           to one tile, so the epilogue (eight warps here, four per half) is exposed once per tile.  For stores, bf16 or fp32 (the choice does not look at an activation), and gated units of one or two rounds: 4096 x 4096 97 us (104 with TH = 1), 4096 x 14336 361 (402).
+// Tile shapes: shared memory moves 128 bytes per clock, for what TMA writes and for what the products read of it, so a k-block of 128 tokens x FEAT features costs
+// (16 KB + FEAT * 128 bytes) * 2 / 128 clocks, half again what its products cost at 256 features and twice that at 128:
+//   FEAT = 128  a quarter less work per byte, for problems whose wider tiles would leave SMs idle (1024 tokens, 2048 x 7168 37 us against 45, 512 tokens,
+//           3072 x 2048 with rotation 20 against 23).
+//   FEAT = 256  for few tiles and short K; otherwise pairs of SMs share the operands of 256 x 256 tiles (gemm_pair.cu).
+// Two accumulators: the epilogue of a tile runs under the products of the next.
 //
 // The CTAs walk tiles id = first + i * step with the token tile fastest: the CTAs running at any
 // moment share a few weight tiles (streamed from HBM once) and the activations stay in L2.  Warp 0
@@ -28,72 +27,25 @@
 
 #include <type_traits>
 
-#include "gemm.cuh"
+#include "gemm_tok.cuh"
 #include "ops.h"
 
 using namespace sm100;
+using namespace gemm_tok;
 
 namespace {
 
-constexpr int kHalfBytes = 128 * gemm::kBK * 2;      // one 128-token operand tile: 16 KB
+constexpr int kTok = 128;                             // tokens per tile
+constexpr int kXBytes = kTok * gemm::kBK * 2;
 constexpr int kMaxStages = 6;
 
-template <int TH, int FEAT> struct Shape {
-  static constexpr int kTok = 128 * TH;                        // tokens per tile
-  static constexpr int kXBytes = kHalfBytes * TH;
-  static constexpr int kStageBytes = kXBytes + FEAT * gemm::kBK * 2;        // 48 / 32 / 64 KB
-  static constexpr int kStages = 192 * 1024 / kStageBytes;     // 4 / 6 / 3
-  static constexpr int kBuffers = TH == 1 ? 2 : 1;             // accumulator sets that alternate between tiles
-  static constexpr int kCols = 2 * FEAT;                       // TMEM columns of two sets, or of two halves
-  static constexpr int kEpiWarps = 4 * TH;
-  static constexpr int kThreads = 64 + 32 * kEpiWarps;         // a warp of copies, one of products, the epilogue's
+constexpr int kEpiWarps = 4, kThreads = 64 + 32 * kEpiWarps;      // a warp of copies, one of products, the epilogue's
+
+template <int FEAT> struct Shape {
+  static constexpr int kStageBytes = kXBytes + FEAT * gemm::kBK * 2;        // 48 / 32 KB
+  static constexpr int kStages = 192 * 1024 / kStageBytes;     // 4 / 6
+  static constexpr int kCols = 2 * FEAT;                       // TMEM columns of two accumulators
 };
-
-constexpr int kMaxRowGroups = 512;
-
-// Where a tile of a row-grouped problem lies: tiles are numbered group after group, inside a group token tile fastest.
-struct RowGroups {
-  int off[kMaxRowGroups + 1];      // first row of every group
-  int tile[kMaxRowGroups + 1];     // first tile of every group
-};
-constexpr int kFeatTile = 256;     // of row-grouped problems
-
-// first token row, end of the rows, first feature and its weight row of a tile
-struct At { int n0, nend, f0, w0; };
-template <int TOK>
-__device__ __forceinline__ At find_tile(const RowGroups& groups, int tile, int ngroups, int M) {
-  int lo = 0, hi = ngroups - 1;                    // the last group whose first tile is not beyond `tile`; empty groups are passed over
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (groups.tile[mid] <= tile) lo = mid;
-    else hi = mid - 1;
-  }
-  const int local = tile - groups.tile[lo], tt = (groups.off[lo + 1] - groups.off[lo] + TOK - 1) / TOK;
-  const int f0 = local / tt * kFeatTile;
-  return At{groups.off[lo] + local % tt * TOK, groups.off[lo + 1], f0, lo * M + f0};
-}
-
-// Fills the table from the rows' offsets (device memory); whole CTA of THREADS.
-template <int TOK, int THREADS>
-__device__ __forceinline__ void count_tiles(RowGroups& groups, const gemm::Params& p, int feat_tiles) {
-  for (int g = threadIdx.x; g <= p.groups; g += THREADS) groups.off[g] = p.row_off[g];
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x, per = (p.groups + 31) / 32, a = min(p.groups, lane * per), b = min(p.groups, a + per);
-    auto count = [&](int g) { return (groups.off[g + 1] - groups.off[g] + TOK - 1) / TOK * feat_tiles; };
-    int sum = 0;
-    for (int g = a; g < b; g++) sum += count(g);
-    int inc = sum;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += v;
-    }
-    int run = inc - sum;
-    for (int g = a; g < b; g++) { groups.tile[g] = run; run += count(g); }
-    if (lane == 31) groups.tile[p.groups] = inc;
-  }
-  __syncthreads();
-}
 
 struct PSmem {
   unsigned long long full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2];
@@ -101,221 +53,20 @@ struct PSmem {
   int abort_flag;
 };
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {  // 32 lanes x 32 consecutive fp32 columns
-  tmem_ld16(taddr, r);
-  tmem_ld16(taddr + 16u, r + 16);
-}
-__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-// Same arithmetic as the decode kernel's SiLU-mul: every intermediate an unfused bf16 pipeline would
-// have stored is rounded to bf16.
-__device__ __forceinline__ float silu_mul_bf16(float g, float u) {
-  g = bf16_round(g);
-  u = bf16_round(u);
-  const float s = bf16_round(g / (1.0f + __expf(-g)));
-  return s * u;
-}
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-
-// One 32-byte store: a whole sector per thread, where rows of different tokens sit in neighbouring threads.
-__device__ __forceinline__ void st_global_f32x8(float* p, const float* v) {
-  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]),
-               "f"(v[6]), "f"(v[7]) : "memory");
-}
-
-__device__ __forceinline__ void st_global_b32x8(void* p, const uint32_t* v) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
-}
-
-// One token row, 16 features starting at f: the bf16 results (8 words, or 4 where gate and up make one) into w, fp32 results to memory.
-template <int EPI>
-__device__ __forceinline__ void finish16(const gemm::Params& p, int n, int f, const uint32_t* q, uint32_t* w) {
-  float v[16];
-#pragma unroll
-  for (int j = 0; j < 16; j++) v[j] = __uint_as_float(q[j]);
-  if (p.bias) {
-#pragma unroll
-    for (int j = 0; j < 16; j++) v[j] += __bfloat162float(p.bias[f + j]);
-  }
-  if (EPI == gemm::kEpiF32) {
-    if (p.act == gemm::kActSoftplus) {              // one branch, not one per value
-#pragma unroll
-      for (int j = 0; j < 16; j++) v[j] = gemm::apply_act(v[j], gemm::kActSoftplus, 0.f);
-    } else if (p.act != gemm::kActNone) {
-#pragma unroll
-      for (int j = 0; j < 16; j++) v[j] = gemm::apply_act(v[j], p.act, p.act_a);
-    }
-    float* dst = p.yf + size_t(n) * p.ldy + f;      // 64-byte aligned rows: M and ldy are multiples of 16 and 8
-    st_global_f32x8(dst, v);
-    st_global_f32x8(dst + 8, v + 8);
-    if (p.y2) {
-      uint4* d2 = reinterpret_cast<uint4*>(p.y2 + size_t(n) * p.ldy + f);
-      d2[0] = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-      d2[1] = make_uint4(pack_bf16(v[8], v[9]), pack_bf16(v[10], v[11]), pack_bf16(v[12], v[13]), pack_bf16(v[14], v[15]));
-    }
-  } else if (EPI == gemm::kEpiClampGlu) {
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-      w[j] = pack_bf16(gemm::clamp_glu(v[4 * j], v[4 * j + 1], p.act_a, p.act_b, p.act_c), gemm::clamp_glu(v[4 * j + 2], v[4 * j + 3], p.act_a, p.act_b, p.act_c));
-  } else if (EPI == gemm::kEpiSiluMul) {
-#pragma unroll
-    for (int j = 0; j < 4; j++) w[j] = pack_bf16(silu_mul_bf16(v[4 * j], v[4 * j + 1]), silu_mul_bf16(v[4 * j + 2], v[4 * j + 3]));
-  } else {
-    if (p.act != gemm::kActNone && f < p.act_m) {   // act_m is a multiple of 16
-      if (p.act == gemm::kActSilu) {
-#pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = gemm::apply_act(v[j], gemm::kActSilu, 0.f);
-      } else if (p.act == gemm::kActGelu) {
-#pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = gemm::apply_act(v[j], gemm::kActGelu, 0.f);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = gemm::apply_act(v[j], p.act, p.act_a);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 8; j++) w[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
-  }
-}
-// 32 features of one token row.  The rows of a warp lie far apart in memory, so the stores cost a pass of the load / store unit per row and instruction: 32 bytes at a time
-// (p.wide: rows and base allow it) are half as many as 16.
-template <int EPI>
-__device__ __forceinline__ void store32(const gemm::Params& p, int n, int f, const uint32_t* q) {
-  uint32_t w[16];
-  constexpr bool kHalf = EPI == gemm::kEpiSiluMul || EPI == gemm::kEpiClampGlu;
-  finish16<EPI>(p, n, f, q, w);
-  const bool second = f + 16 < p.M;                 // M is a multiple of 16
-  if (second) finish16<EPI>(p, n, f + 16, q + 16, w + (kHalf ? 4 : 8));
-  if constexpr (EPI != gemm::kEpiF32) {
-    __nv_bfloat16* dst = p.y + size_t(n) * p.ldy + (kHalf ? f >> 1 : f);
-    if (kHalf) {
-      if (p.wide && second) {
-        st_global_b32x8(dst, w);
-      } else {
-        *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-        if (second) *reinterpret_cast<uint4*>(dst + 8) = make_uint4(w[4], w[5], w[6], w[7]);
-      }
-    } else if (p.wide) {
-      st_global_b32x8(dst, w);
-      if (second) st_global_b32x8(dst + 16, w + 8);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (j < 2 || second) *reinterpret_cast<uint4*>(dst + 8 * j) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
-    }
-  }
-}
-
-// cos and sin of 16 channels for a row's position, rounded as the two-kernel form rounds them
-struct Angles { float c[16], s[16]; };
-__device__ __forceinline__ void ld_global_f32x8(const float* p, float* v) {
-  asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
-}
-__device__ __forceinline__ void load_angles(const gemm::Params& p, int pos, int d, Angles& a) {
-  const float* t = p.rope.cos_sin + size_t(pos) * 128 + d;
-  ld_global_f32x8(t, a.c);
-  ld_global_f32x8(t + 8, a.c + 8);
-  ld_global_f32x8(t + 64, a.s);
-  ld_global_f32x8(t + 72, a.s + 8);
-#pragma unroll
-  for (int j = 0; j < 16; j++) { a.c[j] = bf16_round(a.c[j]); a.s[j] = bf16_round(a.s[j]); }
-}
-// One token row, 16 channels d .. of a head and their rotation partners 64 further (`a`, `b`: accumulators): bias, rounding to bf16, rotation, stores to the activations and
-// the cache.  Same arithmetic as k_gemm_qkv_rope.
-__device__ __forceinline__ void store_rope16(const gemm::Params& p, int n, int head, int d, const Angles& g, long long slot, const uint32_t* a, const uint32_t* b) {
-  float lo[16], hi[16];
-#pragma unroll
-  for (int j = 0; j < 16; j++) { lo[j] = __uint_as_float(a[j]); hi[j] = __uint_as_float(b[j]); }
-  if (p.bias) {
-    const __nv_bfloat16* bias = p.bias + head * 128 + d;
-#pragma unroll
-    for (int j = 0; j < 16; j++) { lo[j] += __bfloat162float(bias[j]); hi[j] += __bfloat162float(bias[64 + j]); }
-  }
-  if (head < p.rope.nq + p.rope.nkv) {
-#pragma unroll
-    for (int j = 0; j < 16; j++) gemm::rotate(bf16_round(lo[j]), bf16_round(hi[j]), g.c[j], g.s[j], lo[j], hi[j]);
-  }
-  uint32_t w[16];
-#pragma unroll
-  for (int j = 0; j < 8; j++) { w[j] = pack_bf16(lo[2 * j], lo[2 * j + 1]); w[8 + j] = pack_bf16(hi[2 * j], hi[2 * j + 1]); }
-  auto put = [&](__nv_bfloat16* row) {                // 32-byte aligned: see tbv_op_gemm_qkv_rope
-    st_global_b32x8(row + d, w);
-    st_global_b32x8(row + d + 64, w + 8);
-  };
-  put(p.y + size_t(n) * p.ldy + head * 128);
-  if (slot >= 0 && head >= p.rope.nq) {
-    const bool value = head >= p.rope.nq + p.rope.nkv;
-    put((value ? p.rope.v_cache : p.rope.k_cache) + (size_t(slot) * p.rope.nkv + (head - p.rope.nq - (value ? p.rope.nkv : 0))) * 128);
-  }
-}
-
-// A warp's 32 rows of an accumulator of FEAT columns (`trow`: its TMEM address), token row n of this lane, features f0 ..; release(): called by the whole warp when the
-// accumulator has been read.
-template <int EPI, int FEAT, typename F>
-__device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok, int f0, uint32_t trow, F release) {
-  if constexpr (EPI == gemm::kEpiRope) {
-    // rotation partners lie 64 columns apart: 16 channels of every head of the tile and their partners at a time, with the angles they share
-    int pos = 0;
-    long long slot = -1;
-    if (row_ok) {
-      pos = p.rope.positions[n];
-      pos = pos < 0 ? 0 : (pos >= p.rope.max_pos ? p.rope.max_pos - 1 : pos);
-      if (p.rope.slot_mapping) slot = p.rope.slot_mapping[n];
-    }
-    const bool turned = (f0 >> 7) < p.rope.nq + p.rope.nkv;       // otherwise the tile holds values only
-    Angles g;
-#pragma unroll 1
-    for (int d = 0; d < 64; d += 16) {
-      if (turned) load_angles(p, pos, d, g);
-#pragma unroll
-      for (int h = 0; h < FEAT; h += 128) {
-        uint32_t a[16], b[16];
-        __syncwarp();
-        tmem_ld16(trow + uint32_t(h + d), a);
-        tmem_ld16(trow + uint32_t(h + d + 64), b);
-        tmem_ld_wait();
-        if (d == 48 && h + 128 == FEAT) {
-          tc_fence_before();
-          __syncwarp();
-          release();
-        }
-        if (row_ok && f0 + h < p.M) store_rope16(p, n, (f0 + h) >> 7, d, g, slot, a, b);   // M is a multiple of 128
-      }
-    }
-  } else {
-    for (int c = 0; c < FEAT; c += 32) {
-      uint32_t r[32];
-      __syncwarp();   // rows past the end skip the stores below: reconverge before the warp-wide load
-      tmem_ld32(trow + uint32_t(c), r);
-      tmem_ld_wait();
-      if (c + 32 == FEAT) {
-        // accumulator fully read by this warp: hand it back to the MMA warp before the last stores go out
-        tc_fence_before();
-        __syncwarp();
-        release();
-      }
-      if (row_ok && f0 + c < p.M) store32<EPI>(p, n, f0 + c, r);
-    }
-  }
-}
-
 // EPI (gemm::Epi) of all kernels here: 0 store (+bias); 1 SiLU-mul over interleaved gate/up features (output has M / 2 features); 2 fp32 store with
 // an activation; 3 clamped gated unit over interleaved gate/up features; 4 rotation and cache write of a qkv projection.
 // ROWS: row-grouped problem (p.row_off; FEAT = 256).
-template <int EPI, int TH, int FEAT, bool ROWS>
-__global__ void __launch_bounds__(Shape<TH, FEAT>::kThreads, 1)
+template <int EPI, int FEAT, bool ROWS>
+__global__ void __launch_bounds__(kThreads, 1)
 k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ gemm::Params p) {
-  using S = Shape<TH, FEAT>;
+  using S = Shape<FEAT>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ PSmem s;
   __shared__ typename std::conditional<ROWS, RowGroups, int>::type groups;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
-  const int tok_tiles = (p.N + S::kTok - 1) / S::kTok, feat_tiles = (p.M + FEAT - 1) / FEAT, nkb = p.kb_total;
+  const int tok_tiles = (p.N + kTok - 1) / kTok, feat_tiles = (p.M + FEAT - 1) / FEAT, nkb = p.kb_total;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < S::kStages; i++) {
@@ -324,7 +75,7 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
     }
     for (int i = 0; i < 2; i++) {
       mbar_init(smem_u32(&s.acc_full[i]), 1);
-      mbar_init(smem_u32(&s.acc_empty[i]), S::kEpiWarps);   // one arrival per epilogue warp
+      mbar_init(smem_u32(&s.acc_empty[i]), kEpiWarps);   // one arrival per epilogue warp
     }
     s.abort_flag = 0;
     mbar_fence_init();
@@ -344,16 +95,16 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
   int tiles = tok_tiles * feat_tiles;
   if constexpr (ROWS) {
     pdl::grid_dependency_wait();                 // the groups' rows were counted on the device by a kernel before this one
-    count_tiles<S::kTok, S::kThreads>(groups, p, feat_tiles);
+    count_tiles<kTok, kThreads>(groups, p, feat_tiles);
     tiles = groups.tile[p.groups];
   }
   const int my_tiles = int(blockIdx.x) < tiles ? (tiles - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x) : 0;
   const int ngroups = p.groups, feats = p.M, all_rows = p.N;
   // (by value: a capture of the parameter block would put it in local memory)
   auto locate = [=](int tile) -> At {
-    if constexpr (ROWS) return find_tile<S::kTok>(groups, tile, ngroups, feats);
+    if constexpr (ROWS) return find_tile<kTok>(groups, tile, ngroups, feats);
     const int f0 = tile / tok_tiles * FEAT;
-    return At{tile % tok_tiles * S::kTok, all_rows, f0, f0};
+    return At{tile % tok_tiles * kTok, all_rows, f0, f0};
   };
   const uint32_t tmem0 = s.tmem_base;
   volatile int* abortp = &s.abort_flag;
@@ -368,7 +119,7 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
     for (int i = 0; i < pre; i++) {
       const uint32_t fb = smem_u32(&s.full[i]);
       mbar_expect_tx(fb, S::kStageBytes);
-      tma_load_2d(base + i * S::kStageBytes + S::kXBytes, &tmW, i * gemm::kBK, at.w0, fb);
+      tma_load_2d(base + i * S::kStageBytes + kXBytes, &tmW, i * gemm::kBK, at.w0, fb);
     }
     pdl::grid_dependency_wait();
     for (int i = 0; i < pre; i++) tma_load_2d_hint(base + i * S::kStageBytes, &tmX, i * gemm::kBK, at.n0, smem_u32(&s.full[i]), pol_x);
@@ -382,7 +133,7 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
         const uint32_t fb = smem_u32(&s.full[st]);
         mbar_expect_tx(fb, S::kStageBytes);
         tma_load_2d_hint(base + st * S::kStageBytes, &tmX, kb * gemm::kBK, at.n0, fb, pol_x);
-        tma_load_2d(base + st * S::kStageBytes + S::kXBytes, &tmW, kb * gemm::kBK, at.w0, fb);
+        tma_load_2d(base + st * S::kStageBytes + kXBytes, &tmW, kb * gemm::kBK, at.w0, fb);
         if (++st == S::kStages) { st = 0; ph ^= 1u; }
       }
     }
@@ -398,38 +149,35 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
     uint32_t ph = 0;
     bool ok = true;
     for (int t = 0; t < my_tiles && ok; t++) {
-      const int buf = t % S::kBuffers, use = t / S::kBuffers;
-      // the epilogue must have drained this accumulator set (kBuffers tiles ago); passes at once on first use
+      const int buf = t & 1, use = t >> 1;
+      // the epilogue must have drained this accumulator (two tiles ago); passes at once on first use
       if (!mbar_wait(smem_u32(&s.acc_empty[buf]), (uint32_t(use) & 1u) ^ 1u, abortp, p.limit_ns)) break;
       tc_fence_after();
       for (int kb = 0; kb < nkb; kb++) {
         if (!mbar_wait(smem_u32(&s.full[st]), ph, abortp, p.limit_ns)) { ok = false; break; }
         tc_fence_after();
-        const uint64_t bd = umma_desc_sw128(base + st * S::kStageBytes + S::kXBytes);
+        const uint64_t bd = umma_desc_sw128(base + st * S::kStageBytes + kXBytes);
+        const uint64_t ad = umma_desc_sw128(base + st * S::kStageBytes);
+        const uint32_t tmem_d = tmem0 + uint32_t(buf * FEAT);
 #pragma unroll
-        for (int h = 0; h < TH; h++) {           // the 128-token halves share the weight tile
-          const uint64_t ad = umma_desc_sw128(base + st * S::kStageBytes + h * kHalfBytes);
-          const uint32_t tmem_d = tmem0 + uint32_t((TH == 1 ? buf : h) * FEAT);
-#pragma unroll
-          for (int k = 0; k < gemm::kBK / 16; k++)
-            umma_bf16(tmem_d, ad + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < gemm::kBK / 16; k++)
+          umma_bf16(tmem_d, ad + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
         umma_commit(smem_u32(&s.empty[st]));
         if (++st == S::kStages) { st = 0; ph ^= 1u; }
       }
       if (ok) umma_commit(smem_u32(&s.acc_full[buf]));
     }
   } else if (warp >= 2) {
-    // ---- epilogue: thread = one token row of the tile (TH = 2: warps 2..5 first half, 6..9 second half) ----
-    const int quarter = warp & 3, half = TH == 1 ? 0 : (warp - 2) >> 2;
+    // ---- epilogue: thread = one token row of the tile ----
+    const int quarter = warp & 3;
     for (int t = 0; t < my_tiles; t++) {
-      const int buf = t % S::kBuffers, use = t / S::kBuffers;
+      const int buf = t & 1, use = t >> 1;
       const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s.acc_full[buf]), uint32_t(use) & 1u, abortp, p.limit_ns));   // together, before the warp-wide TMEM loads
       if (!ok) break;
       tc_fence_after();
       const At at = locate(int(blockIdx.x) + t * int(gridDim.x));
-      const int n = at.n0 + half * 128 + quarter * 32 + lane;   // token row
-      drain<EPI, FEAT>(p, n, n < at.nend, at.f0, tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t((TH == 1 ? buf : half) * FEAT), [&] {
+      const int n = at.n0 + quarter * 32 + lane;   // token row
+      drain<EPI, FEAT>(p, n, n < at.nend, at.f0, tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t(buf * FEAT), [&] {
         if (lane == 0) mbar_arrive(smem_u32(&s.acc_empty[buf]));
       });
     }
@@ -446,31 +194,32 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
   if (threadIdx.x == 0 && s.abort_flag && p.err) atomicExch(p.err, 1);
 }
 
-template <int EPI, int TH, int FEAT, bool ROWS = false>
+template <int EPI, int FEAT, bool ROWS = false>
 cudaError_t launch_tok(const void* w, const void* x, const gemm::Params& p, int ldx, cudaStream_t st, int* map_rc) {
-  using S = Shape<TH, FEAT>;
+  using S = Shape<FEAT>;
   CUtensorMap tmX, tmW;
   *map_rc = 0;
-  if (tbvops::make_tensor_map_bf16(&tmX, x, ROWS ? p.x_rows : p.N, p.K, ldx, S::kTok) != 0 ||
+  if (tbvops::make_tensor_map_bf16(&tmX, x, ROWS ? p.x_rows : p.N, p.K, ldx, kTok) != 0 ||
       tbvops::make_tensor_map_bf16(&tmW, w, (unsigned long long)(ROWS ? p.groups : 1) * p.M, p.K, p.K, FEAT) != 0) {
     *map_rc = -3;
     return cudaSuccess;
   }
   constexpr size_t smem = size_t(S::kStages) * S::kStageBytes + 1024;
   static std::atomic<unsigned> done{0};
-  const cudaError_t attr = pdl::allow_smem(k_gemm_tok<EPI, TH, FEAT, ROWS>, smem, done);
+  const cudaError_t attr = pdl::allow_smem(k_gemm_tok<EPI, FEAT, ROWS>, smem, done);
   if (attr != cudaSuccess) return attr;
-  const int tiles = (ROWS ? p.x_rows / S::kTok + p.groups : (p.N + S::kTok - 1) / S::kTok) * ((p.M + FEAT - 1) / FEAT);   // ROWS: at most
+  const int tiles = (ROWS ? p.x_rows / kTok + p.groups : (p.N + kTok - 1) / kTok) * ((p.M + FEAT - 1) / FEAT);   // ROWS: at most
   const int sms = tbvops::sm_count();
-  return pdl::launch(k_gemm_tok<EPI, TH, FEAT, ROWS>, dim3(tiles < sms ? tiles : sms), dim3(S::kThreads), smem, st, 1, tmX, tmW, p);
+  return pdl::launch(k_gemm_tok<EPI, FEAT, ROWS>, dim3(tiles < sms ? tiles : sms), dim3(kThreads), smem, st, 1, tmX, tmW, p);
 }
 
 }  // namespace
 
 namespace tbvops {
 
-// Which form takes an [N tokens] x [M features] problem: 0 = the decode-form kernel (gemm.cu), k_gemm_tok with 1 / 2 = 128- / 256-token tiles of 256 features, 3 = 128 x 128
-// tiles.  `mode`: 1 = choose, 2 / 3 / 4 = force the first / second / third tile wherever the shape allows (tests, measurements; the qkv projection, which asks for epilogue 1, has no 256-token tile and takes 128 x 256 instead).
+// Which form takes an [N tokens] x [M features] problem: 0 = the decode-form kernel (gemm.cu); otherwise by the work that a tile has, 1 / 2 = 128 / 256 tokens x 256 features
+// (the tiles of both go to pairs of SMs where takes_pairs says so), 3 = 128 x 128.  `mode`: 1 = choose, 2 / 3 / 4 = force 128 x 256 / 256 x 256 on pairs / 128 x 128 wherever the
+// shape allows (tests, measurements).
 //
 // Every CTA walks ceil(tiles / SMs) tiles.  A k-block of a 128 x 128 tile takes two thirds of the time of a 128 x 256 one (both bound by what TMA brings in), and one of
 // 256 x 256 nine tenths of two of those.  512 tokens, 4096 x 4096 24 / 28 / 45 us with 128 x 128 / 128 x 256 / 256 x 256 tiles,
@@ -499,7 +248,7 @@ int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode, int sms) {
   return 2 * r2 <= r1 && (r2 == 1 || (r2 == 2 && K > 4096)) ? 2 : 1;
 }
 
-// Row-grouped: 0 the decode form, 1 / 2 k_gemm_tok with 128- / 256-token tiles of 256 features (`mode` 2 and 4 / 3 force them).  The decode form re-reads a group's weights
+// Row-grouped: 0 the decode form, 1 / 2 tiles of 128 / 256 tokens as above (`mode` 2 and 4 / 3 force them alone / in pairs).  The decode form re-reads a group's weights
 // for every tile of up to 128 rows; k_gemm_tok wastes what a group's last tile lacks, on average half a tile.
 //
 // How the rows spread over the groups is not known here, and 256-token tiles lose up to half where they need a round more (8 x 513 rows, 2048 x 3584: 89 us against 59).
@@ -507,10 +256,23 @@ int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode, int sms) {
 // 2048 rows 259 / 338 / 601 us against 282 / 367 / 664, 16 of 1500 1031 against 1040; but 16 of 500 428 against 398; with K 3584 8 of 2000 340 against 330.
 int gemm_tok_rows_choose(int M, int x_rows, int groups, int K, int epi, int mode, int sms) {
   if ((M % 16) || groups > kMaxRowGroups || x_rows / groups < 64) return 0;
-  if (epi != gemm::kEpiStore || mode == 2 || mode == 4) return 1;
   if (mode == 3) return 2;
+  if (epi != gemm::kEpiStore || mode >= 2) return 1;
   const long tiles = (x_rows / 256 + groups / 2) * (long)((M + 255) / 256);
   return K > 4096 && x_rows / groups >= 768 && tiles >= 3l * sms ? 2 : 1;
+}
+
+// Whether the 256-feature tiles of a problem go to pairs of SMs (gemm_pair.cu): where that needs no more rounds and the pair's start and end (a cluster's launch, two barriers: some
+// 2 us) are small beside them.  A gated unit's long epilogue gains by the pair's twice as many warps in any case.
+// us, alone / in pairs: 4096 tokens, 6144 x 4096 with rotation 158 / 148, 4096 x 4096 102 / 94, 14336 x 2048 with the SiLU unit 186 / 165, 2048 x 7168 101 / 91, 8192 x 2048 98 / 92;
+// 1024 tokens, 14336 x 2048 with the SiLU unit 68 / 58, 28672 x 4096 190 / 172, 4096 x 14336 99 / 87; the other side: 1024 tokens, 3072 x 2048 27 / 28, 2048 x 2048 17.6 / 18.4,
+// 2048 tokens, 2048 x 2048 20 / 22, 4096 tokens, 4096 x 128 26 / 30.  Groups of rows, whose last tiles are half empty on average: 8 groups of about 700, 7168 x 2048 gated 174 / 153,
+// 2048 x 3584 87 / 78, of about 1024 206 / 197 and 114 / 102; of about 512 137 / 135 and 67 / 84.
+static bool takes_pairs(const gemm::Params& p, int epi, int sms) {
+  if (sms < 2) return false;
+  if (p.row_off) return p.x_rows / p.groups >= 640;
+  const long f256 = (p.M + 255) / 256, single = ((p.N + 127l) / 128 * f256 + sms - 1) / sms, pairs = ((p.N + 255l) / 256 * f256 + sms / 2 - 1) / (sms / 2);
+  return pairs <= single && (epi == gemm::kEpiSiluMul || epi == gemm::kEpiClampGlu || single * p.kb_total >= 48);
 }
 
 int gemm_tok_launch(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi, int th,
@@ -528,26 +290,28 @@ int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, in
   p.wide = !(reinterpret_cast<uintptr_t>(p.y) & 31) && p.ldy % 16 == 0;
   p.limit_ns = 2000000000ull;
   p.err = gemm_err_flag();
+  const int mode = gemm_persist_mode();
+  if (mode == 1 && th == 2 && p.kb_total <= 4 && epi == gemm::kEpiF32) th = 3;    // all epilogue: more CTAs for it (4096 tokens, 4096 x 128 23.6 us against 26)
+  if (mode == 1 ? th != 3 && takes_pairs(p, epi, sm_count()) : th == 2) return gemm_pair_launch(w, x, p, ldx, epi, stream);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int map_rc = 0;
   cudaError_t e;
   if (p.row_off) {
-    e = epi == gemm::kEpiClampGlu ? launch_tok<3, 1, 256, true>(w, x, p, ldx, st, &map_rc) :
-        th == 2 ? launch_tok<0, 2, 256, true>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1, 256, true>(w, x, p, ldx, st, &map_rc);
+    e = epi == gemm::kEpiClampGlu ? launch_tok<3, 256, true>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 256, true>(w, x, p, ldx, st, &map_rc);
   } else switch (epi) {
     case gemm::kEpiSiluMul:
-      e = th == 3 ? launch_tok<1, 1, 128>(w, x, p, ldx, st, &map_rc) : th == 2 ? launch_tok<1, 2, 256>(w, x, p, ldx, st, &map_rc) : launch_tok<1, 1, 256>(w, x, p, ldx, st, &map_rc);
+      e = th == 3 ? launch_tok<1, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<1, 256>(w, x, p, ldx, st, &map_rc);
       break;
     case gemm::kEpiF32:
-      e = th == 3 ? launch_tok<2, 1, 128>(w, x, p, ldx, st, &map_rc) : th == 2 ? launch_tok<2, 2, 256>(w, x, p, ldx, st, &map_rc) : launch_tok<2, 1, 256>(w, x, p, ldx, st, &map_rc);
+      e = th == 3 ? launch_tok<2, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<2, 256>(w, x, p, ldx, st, &map_rc);
       break;
     case gemm::kEpiClampGlu:
-      e = th == 3 ? launch_tok<3, 1, 128>(w, x, p, ldx, st, &map_rc) : th == 2 ? launch_tok<3, 2, 256>(w, x, p, ldx, st, &map_rc) : launch_tok<3, 1, 256>(w, x, p, ldx, st, &map_rc);
+      e = th == 3 ? launch_tok<3, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<3, 256>(w, x, p, ldx, st, &map_rc);
       break;
-    case gemm::kEpiRope:   // no 256-token form
-      e = th == 3 ? launch_tok<4, 1, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<4, 1, 256>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiRope:
+      e = th == 3 ? launch_tok<4, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<4, 256>(w, x, p, ldx, st, &map_rc); break;
     default:
-      e = th == 3 ? launch_tok<0, 1, 128>(w, x, p, ldx, st, &map_rc) : th == 2 ? launch_tok<0, 2, 256>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 1, 256>(w, x, p, ldx, st, &map_rc);
+      e = th == 3 ? launch_tok<0, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<0, 256>(w, x, p, ldx, st, &map_rc);
       break;
   }
   if (map_rc != 0) return map_rc;

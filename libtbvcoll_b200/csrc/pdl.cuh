@@ -41,10 +41,9 @@ inline cudaError_t allow_smem(K kernel, size_t bytes, std::atomic<unsigned>& don
   return e;
 }
 
-// cudaLaunchKernelEx with the PDL attribute (and an optional cluster size along z).
+// cudaLaunchKernelEx with the PDL attribute and an optional cluster.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster_z,
-                          Args&&... args) {
+inline cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, dim3 cluster, Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -52,11 +51,11 @@ inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   unsigned n = 0;
-  if (cluster_z > 1) {
+  if (cluster.x * cluster.y * cluster.z > 1) {
     attr[n].id = cudaLaunchAttributeClusterDimension;
-    attr[n].val.clusterDim.x = 1;
-    attr[n].val.clusterDim.y = 1;
-    attr[n].val.clusterDim.z = unsigned(cluster_z);
+    attr[n].val.clusterDim.x = cluster.x;
+    attr[n].val.clusterDim.y = cluster.y;
+    attr[n].val.clusterDim.z = cluster.z;
     n++;
   }
   if (enabled()) {
@@ -67,6 +66,11 @@ inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
   cfg.attrs = attr;
   cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+// the same as launch_clusters with a cluster size along z
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster_z, Args&&... args) {
+  return launch_clusters(kernel, grid, block, smem, stream, dim3(1, 1, cluster_z), static_cast<Args&&>(args)...);
 }
 
 }  // namespace pdl

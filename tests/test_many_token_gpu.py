@@ -103,3 +103,44 @@ def test_copies_that_are_column_slices(offset):
     assert not ops.gemm_error() and torch.equal(copy, out.to(torch.bfloat16))
     assert ((out.double() - want).abs() <= size * K * 2.0 ** -23).all()                      # K fp32 additions
     assert (around[:, :offset] == 7).all() and (around[:, offset + M:] == 7).all()
+
+
+@pytest.mark.parametrize("T,nq,nkv,K,bias", [(384, 4, 2, 512, False), (401, 3, 1, 1000, True), (1025, 8, 4, 256, True), (384, 1, 0, 64, False), (5001, 8, 4, 72, False)])
+def test_qkv_projection_on_pairs_of_sms(T, nq, nkv, K, bias):
+    """Bit for bit the 128-token form: second CTAs without rows, tiles whose second head lies beyond the features, more tiles than accumulators."""
+    from libtbvcoll_b200 import ops
+    D, M = 128, (nq + 2 * nkv) * 128
+    x, w, b = rnd(T, K, seed=1), rnd(M, K, seed=2, scale=0.05), rnd(M, seed=3) if bias else None
+    pos, cs = (torch.arange(T, dtype=torch.int32) * 3 % 260 - 2).to(DEV), ops.rope_cos_sin(D, 256, 5e5, DEV)
+    slots = torch.randperm(T + 40, generator=torch.Generator().manual_seed(4))[:T].to(DEV)
+    slots[::7] = -1
+    got = []
+    try:
+        for mode in (2, 3):
+            ops.gemm_persist_mode(mode)
+            got.append([torch.zeros(T, M, dtype=torch.bfloat16, device=DEV)] + [torch.zeros(T + 40, max(nkv, 1), D, dtype=torch.bfloat16, device=DEV) for _ in range(2)])
+            ops.gemm_qkv_rope(x, w, got[-1][0], pos, cs, slots, *got[-1][1:], nq, nkv, bias=b)
+        torch.cuda.synchronize()
+    finally:
+        ops.gemm_persist_mode(None)
+    assert not ops.gemm_error()
+    for a, c in zip(*got):
+        assert torch.equal(a, c)
+
+
+@pytest.mark.parametrize("counts", [[0, 300, 1, 0, 513, 256], [700, 0, 0, 255]])
+@pytest.mark.parametrize("M,K", [(272, 72), (2064, 520)])
+def test_gated_row_groups_on_pairs_of_sms(counts, M, K):
+    from libtbvcoll_b200 import ops
+    off = torch.tensor([0] + counts).cumsum(0).to(torch.int32).to(DEV)
+    x, w = rnd(sum(counts), K, seed=1), rnd(len(counts) * M, K, seed=2, scale=0.1)
+    got = []
+    try:
+        for mode in (2, 3):
+            ops.gemm_persist_mode(mode)
+            got.append(torch.full((sum(counts), M // 2), 7.0, dtype=torch.bfloat16, device=DEV))
+            ops.linear_rows(x, w, got[-1], off, len(counts), sum(counts), glu=(2.0, 1.7))
+        torch.cuda.synchronize()
+    finally:
+        ops.gemm_persist_mode(None)
+    assert not ops.gemm_error() and torch.equal(*got)
