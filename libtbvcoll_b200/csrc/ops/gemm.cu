@@ -241,12 +241,12 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn g_encode = nullptr;
 std::once_flag g_encode_once;
-CUresult encode(CUtensorMap* out, unsigned rank, const void* ptr, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
+CUresult encode(CUtensorMap* out, CUtensorMapDataType type, unsigned rank, const void* ptr, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
   // the encoder wants the device's context to be current, which in a thread that has made no CUDA call yet it is not
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return CUDA_ERROR_INVALID_CONTEXT;
   const cuuint32_t estr[3] = {1, 1, 1};
-  return g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  return g_encode(out, type, rank, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
@@ -254,14 +254,15 @@ struct MapKey {
   const void* ptr;
   unsigned long long rows, cols, ld;
   unsigned box_rows, dim, box_heads;               // the last two: maps of heads (0 otherwise)
+  bool f32 = false;
   bool operator==(const MapKey& o) const {
-    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && dim == o.dim && box_heads == o.box_heads;
+    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && dim == o.dim && box_heads == o.box_heads && f32 == o.f32;
   }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
     size_t h = reinterpret_cast<size_t>(k.ptr);
-    h = h * 1000003u ^ k.rows; h = h * 1000003u ^ k.cols; h = h * 1000003u ^ k.ld; h = h * 1000003u ^ k.box_rows; h = h * 1000003u ^ (k.dim * 512u + k.box_heads);
+    h = h * 1000003u ^ k.rows; h = h * 1000003u ^ k.cols; h = h * 1000003u ^ k.ld; h = h * 1000003u ^ k.box_rows; h = h * 1000003u ^ (k.dim * 1024u + k.box_heads * 2u + k.f32);
     return h;
   }
 };
@@ -295,17 +296,18 @@ int make_tensor_map(CUtensorMap* out, const MapKey& key, bool cache) {
     auto it = g_maps.find(key);
     if (it != g_maps.end()) { *out = it->second; return 0; }
   }
-  if ((reinterpret_cast<uintptr_t>(key.ptr) & 15u) || (key.ld * 2) % 16 || key.box_rows > 256 || key.box_rows == 0) return -2;
+  const unsigned size = key.f32 ? 4 : 2;
+  if ((reinterpret_cast<uintptr_t>(key.ptr) & 15u) || (key.ld * size) % 16 || key.box_rows > 256 || key.box_rows == 0) return -2;
   CUtensorMap m;
   CUresult r;
   if (key.dim) {
     const cuuint64_t dims[3] = {key.dim, key.cols / key.dim, key.rows}, strides[2] = {key.dim * 2ull, key.ld * 2};
     const cuuint32_t box[3] = {64, key.box_heads, key.box_rows};
-    r = encode(&m, 3, key.ptr, dims, strides, box);
+    r = encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, key.ptr, dims, strides, box);
   } else {
-    const cuuint64_t dims[2] = {key.cols, key.rows}, strides[1] = {key.ld * 2};
-    const cuuint32_t box[2] = {64, key.box_rows};
-    r = encode(&m, 2, key.ptr, dims, strides, box);
+    const cuuint64_t dims[2] = {key.cols, key.rows}, strides[1] = {key.ld * size};
+    const cuuint32_t box[2] = {128 / size, key.box_rows};
+    r = encode(&m, key.f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, key.ptr, dims, strides, box);
   }
   if (r != CUDA_SUCCESS) return -3;
   if (cache) {
@@ -321,6 +323,10 @@ int make_tensor_map(CUtensorMap* out, const MapKey& key, bool cache) {
 // [rows, cols] bf16 row-major with row stride ld (elements); box = box_rows x 64, 128-byte swizzle.
 int make_tensor_map_bf16(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld, unsigned box_rows, bool cache) {
   return make_tensor_map(out, MapKey{ptr, rows, cols, ld, box_rows, 0, 0}, cache);
+}
+// The same of fp32 rows; box = box_rows x 32.
+int make_tensor_map_f32(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld, unsigned box_rows) {
+  return make_tensor_map(out, MapKey{ptr, rows, cols, ld, box_rows, 0, 0, true}, true);
 }
 // Heads of `dim` channels side by side, [rows, ld] with head h at h * dim; box = 64 channels x box_heads x box_rows, 128-byte swizzle.
 int make_tensor_map_heads(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned heads, unsigned dim, unsigned long long ld, unsigned box_heads,

@@ -1,5 +1,5 @@
-// gemm_f32.cu — full 32-bit GEMM on the CUDA cores, for models run with fp32 weights and activations (numerics
-// checks; tensor cores have no full-fp32 mode).  Same epilogues and grouped form as the tcgen05 GEMM's extended entry.
+// gemm_f32.cu — full 32-bit GEMM, for models run with fp32 weights and activations (numerics checks): the choice of its form, and the forms on the CUDA cores, which take
+// short K, few features and any stride and alignment (weights of some size and K go to gemm_f32_split.cu).  Same epilogues and grouped form as the tcgen05 GEMM's extended entry.
 //
 //   y[n, m] = epilogue(sum_k x[n, k] * w[m, k])        x: [N, K], w: [groups * M, K], fp32 row-major
 //
@@ -15,49 +15,14 @@
 #include <cuda_runtime.h>
 
 #include "attn_mma.cuh"
-#include "gemm.cuh"
+#include "gemm_f32.cuh"
 #include "ops.h"
 
 namespace {
 
+using namespace gemm_f32;
+
 constexpr int kT = 64, kKB = 16;
-
-struct F32Params {
-  const float *w, *x, *bias;
-  float* y;
-  int M, N, K, ldx, ldy, epi, act, groups, x_group, y_group;
-  float act_a, act_b, act_c;
-  int m_last;             // > 0: one more group with this many features
-  int act_m;              // the activation acts on the first act_m features
-  const int* row_off;     // row-grouped form: group g owns rows row_off[g] .. row_off[g + 1] - 1
-};
-
-__device__ __forceinline__ float f32_glu(const F32Params& p, float g, float u) {
-  g = fminf(g, p.act_a);
-  u = fminf(fmaxf(u, -p.act_a), p.act_a);
-  return (isinf(p.act_b) ? fmaxf(g, 0.f) : g / (1.0f + expf(-p.act_b * g))) * (u + p.act_c);
-}
-__device__ __forceinline__ float f32_act(const F32Params& p, float v, int m) {
-  if (!p.act || m >= p.act_m) return v;
-  if (p.act == gemm::kActSilu || p.act == gemm::kActGelu) return v / (1.0f + expf(p.act == gemm::kActSilu ? -v : -gemm::gelu_slope(v)));
-  return p.act == gemm::kActSoftplus ? vec::softplus<float>(v) : gemm::apply_act(v, p.act, p.act_a);
-}
-// Which problem and rows a CTA has: grid (feature tiles of all groups, token tiles).
-struct Where { int grp, m0, M, n0, nend; };
-__device__ __forceinline__ Where f32_where(const F32Params& p, int tok, int feat) {
-  const int mt = (p.M + feat - 1) / feat;
-  Where a;
-  a.grp = min(int(blockIdx.x) / mt, p.m_last ? p.groups : p.groups - 1);
-  a.m0 = (blockIdx.x - a.grp * mt) * feat;
-  a.M = p.m_last && a.grp == p.groups ? p.m_last : p.M;
-  a.n0 = blockIdx.y * tok;
-  a.nend = p.N;
-  if (p.row_off) {
-    a.nend = p.row_off[a.grp + 1];
-    a.n0 += p.row_off[a.grp];
-  }
-  return a;
-}
 
 constexpr int kBlock = 32, kPitch = kBlock + 4, kRing = 3;       // columns of a stage, floats between rows, stages
 template <int RT, int RF>
@@ -221,9 +186,10 @@ int f32_tile(int M, int N, int K, int groups, int m_last, long sms) {
   return (N + 31l) / 32 <= 65535 && (K < 512 || r64 <= 2 || 23 * r32 < 40 * r64) ? 44 : 84;
 }
 
-int launch_f32(const F32Params& p, void* stream) {
+int launch_f32(const F32Params& p, int x_rows, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool wide = !((reinterpret_cast<uintptr_t>(p.w) | reinterpret_cast<uintptr_t>(p.x)) & 15) && p.K % 4 == 0 && p.ldx % 4 == 0 && p.x_group % 4 == 0;
+  if (wide && tbvops::gemm_f32_split_takes(p.M, p.K, p.groups, p.m_last)) return tbvops::gemm_f32_split_launch(p, x_rows, stream);
   cudaError_t e;
   if (!wide) {
     const dim3 grid(p.groups * ((p.M + kT - 1) / kT) + (p.m_last + kT - 1) / kT, (p.N + kT - 1) / kT);
@@ -249,7 +215,7 @@ int tbv_op_gemm_f32(const void* w, const void* x, void* y, const void* bias, int
   if (M <= 0 || N <= 0 || K <= 0 || (epi != 0 && epi != 2 && epi != 3) || (epi == 3 && (M % 2)) || (groups > 1 && bias)) return -2;
   F32Params p{static_cast<const float*>(w), static_cast<const float*>(x), static_cast<const float*>(bias), static_cast<float*>(y),
               M, N, K, ldx, ldy, epi, act, groups > 1 ? groups : 1, x_group, y_group, act_a, act_b, act_c, groups > 1 ? m_last : 0, act_m, nullptr};
-  return launch_f32(p, stream);
+  return launch_f32(p, N, stream);
 }
 
 // Tile that the tiled form takes for a shape on a GPU of `sms` SMs (results per thread, 10 * tokens + features); needs no device.
@@ -261,7 +227,7 @@ int tbv_op_gemm_rows_f32(const void* w, const void* x, void* y, const void* row_
   if (M <= 0 || x_rows <= 0 || max_rows <= 0 || K <= 0 || groups <= 0 || (epi != 0 && epi != 3) || (epi == 3 && (M % 2)) || !row_off) return -2;
   F32Params p{static_cast<const float*>(w), static_cast<const float*>(x), nullptr, static_cast<float*>(y),
               M, max_rows, K, ldx, ldy, epi, 0, groups, 0, 0, act_a, act_b, act_c, 0, 0, static_cast<const int*>(row_off)};
-  return launch_f32(p, stream);
+  return launch_f32(p, x_rows, stream);
 }
 
 }  // extern "C"

@@ -1,0 +1,50 @@
+// gemm_f32.cuh — what the full 32-bit GEMM kernels (gemm_f32.cu, gemm_f32_split.cu) share: arguments, epilogue arithmetic, which problem and rows a CTA has.
+#pragma once
+#include "gemm.cuh"
+
+namespace gemm_f32 {
+
+struct F32Params {
+  const float *w, *x, *bias;
+  float* y;
+  int M, N, K, ldx, ldy, epi, act, groups, x_group, y_group;
+  float act_a, act_b, act_c;
+  int m_last;             // > 0: one more group with this many features
+  int act_m;              // the activation acts on the first act_m features
+  const int* row_off;     // row-grouped form: group g owns rows row_off[g] .. row_off[g + 1] - 1
+};
+
+__device__ __forceinline__ float f32_glu(const F32Params& p, float g, float u) {
+  g = fminf(g, p.act_a);
+  u = fminf(fmaxf(u, -p.act_a), p.act_a);
+  return (isinf(p.act_b) ? fmaxf(g, 0.f) : g / (1.0f + expf(-p.act_b * g))) * (u + p.act_c);
+}
+__device__ __forceinline__ float f32_act(const F32Params& p, float v, int m) {
+  if (!p.act || m >= p.act_m) return v;
+  if (p.act == gemm::kActSilu || p.act == gemm::kActGelu) return v / (1.0f + expf(p.act == gemm::kActSilu ? -v : -gemm::gelu_slope(v)));
+  return p.act == gemm::kActSoftplus ? vec::softplus<float>(v) : gemm::apply_act(v, p.act, p.act_a);
+}
+// Which problem and rows a CTA has: grid (feature tiles of all groups, token tiles).
+struct Where { int grp, m0, M, n0, nend; };
+__device__ __forceinline__ Where f32_where(const F32Params& p, int tok, int feat) {
+  const int mt = (p.M + feat - 1) / feat;
+  Where a;
+  a.grp = min(int(blockIdx.x) / mt, p.m_last ? p.groups : p.groups - 1);
+  a.m0 = (blockIdx.x - a.grp * mt) * feat;
+  a.M = p.m_last && a.grp == p.groups ? p.m_last : p.M;
+  a.n0 = blockIdx.y * tok;
+  a.nend = p.N;
+  if (p.row_off) {
+    a.nend = p.row_off[a.grp + 1];
+    a.n0 += p.row_off[a.grp];
+  }
+  return a;
+}
+
+}  // namespace gemm_f32
+
+namespace tbvops {
+// the form on tensor cores (gemm_f32_split.cu); whether it takes a shape (operands of the wide form) depends on the weights alone
+bool gemm_f32_split_takes(int M, int K, int groups, int m_last);
+int gemm_f32_split_launch(const gemm_f32::F32Params& p, int x_rows, void* stream);
+}  // namespace tbvops

@@ -1,0 +1,368 @@
+// gemm_f32_split.cu — full 32-bit GEMM on the tensor cores: every operand as a sum of three bf16 pieces.
+//
+//   y[n, m] = epilogue(sum_k x[n, k] * w[m, k])        x: [N, K], w: [groups * M, K], fp32 row-major
+//
+// A float is the exact sum of its rounding to bf16 (8 bits), of the rest's rounding (8 bits) and of what is left (8 bits); a product of pieces is exact in fp32.  Of the nine
+// products the six are taken whose sizes reach 2^-18 of the whole: with the rest rounded to nearest, what is left out is below 2^-26 of |x w|, of either sign.  The tensor
+// cores' sums of 64 columns, the first pieces' products apart from the others, go to fp32 registers and are added there, rounded to nearest, so the error does not grow with
+// what the tensor cores cut off a long sum.
+//
+// Features on the 128-row UMMA M axis, BN tokens on N.  TMA brings 32 columns of both operands at a time into a ring as they lie in memory; eight warps split them and
+// write the pieces in the 64-byte swizzle; one thread issues the products of two such blocks into an accumulator; eight warps add up the accumulators.  (Loads into the
+// splitting warps' registers, a block ahead, came in at a sixth of HBM's rate: what is in flight waits for room in the little L1 that is left beside the rings.)
+// Bound by shared memory: per block TMA writes, the split's reads and writes and the products' reads are 208 KB for 128 tokens, 1660 clocks, where the products take 768.
+// K is shared out over the CTAs of a cluster, as the weights' shape says, never the tokens': the order of a result's additions depends on M and K alone, so a row's result does
+// not depend on the batch it is in.
+// A result that is not finite is computed again in plain fp32 (an infinite operand times a piece that is zero would be NaN).
+#include <cuda_runtime.h>
+#include <stdio.h>
+
+#include "gemm_f32.cuh"
+#include "ops.h"
+
+using namespace sm100;
+using gemm_f32::F32Params;
+
+namespace {
+
+constexpr int kFeat = 128, kKB = 64, kHalf = 32;                                        // columns that are added up together, columns of a block
+constexpr int kAdders = 8, kSplitters = 8, kThreads = 32 * (kAdders + kSplitters + 2);
+
+template <int BN> struct Shape {
+  static constexpr int kRawBytes = (kFeat + BN) * kHalf * 4;                            // a block as it lies in memory: 32 / 24 / 20 / 18 KB
+  static constexpr int kPieceW = kFeat * kHalf * 2, kPieceX = BN * kHalf * 2;           // a piece of an operand
+  static constexpr int kStageBytes = 3 * (kPieceW + kPieceX);                           // 48 / 36 / 30 / 27 KB
+  static constexpr int kRaw = BN == 128 ? 3 : (BN == 64 ? 4 : 6), kStages = BN == 128 ? 2 : 3;
+  static constexpr int kSmem = kRaw * kRawBytes + kStages * kStageBytes + 1024;
+  static constexpr int kCols = 4 * BN;                                                  // TMEM columns of two accumulators, each of the largest products and of the others
+  static constexpr int kSides = BN >= 32 ? 2 : 1;                                       // warps that share a quarter's tokens
+  static constexpr int kUnits = (kFeat + BN + 63) / 64;                                 // groups of eight columns that a splitting thread has
+};
+
+struct SSmem {
+  unsigned long long raw_full[6], raw_empty[6], full[3], empty[3], acc_full[2], acc_empty[2];
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+// K-major operand tile with rows of 64 bytes in the 64-byte swizzle (8-row groups 512 bytes apart; tile base 512-aligned)
+__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t smem_addr) {
+  return uint64_t((smem_addr & 0x3FFFFu) >> 4) | uint64_t(1) << 16 | uint64_t(512 >> 4) << 32 | uint64_t(1) << 46 | uint64_t(4) << 61;
+}
+__device__ __forceinline__ float4 lds4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts4(uint32_t addr, const uint32_t* v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+
+// eight floats as three times eight bf16
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l, uint32_t& top) {
+  const __nv_bfloat162 h2 = __floats2bfloat162_rn(a, b);
+  h = *reinterpret_cast<const uint32_t*>(&h2);
+  const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
+  const __nv_bfloat162 m2 = __floats2bfloat162_rn(ra, rb);
+  m = *reinterpret_cast<const uint32_t*>(&m2);
+  const __nv_bfloat162 l2 = __floats2bfloat162_rn(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
+  l = *reinterpret_cast<const uint32_t*>(&l2);
+  top |= (h & 0x7f807f80u) + 0x00800080u;         // bits 15 and 31: an exponent of ones
+}
+// the same where a value is infinite, NaN or rounds to infinity
+__device__ __noinline__ void split_careful(const float* v, uint32_t* out12) {
+  for (int j = 0; j < 4; j++) {
+    uint32_t out[3] = {0, 0, 0};
+    for (int e = 0; e < 2; e++) {
+      const float x = v[2 * j + e];
+      uint32_t hb = __float_as_uint(x) >> 16, mb = 0, lb = 0;
+      if (x != x) {
+        hb = 0x7fffu;
+      } else if (!isinf(x)) {                     // the first piece is cut off, not rounded: the rest is at most 2^-7 of the value
+        const float r = x - __uint_as_float(hb << 16);
+        mb = __float_as_uint(r) >> 16;
+        lb = __float_as_uint(r - __uint_as_float(mb << 16)) >> 16;
+      }
+      out[0] |= hb << (16 * e); out[1] |= mb << (16 * e); out[2] |= lb << (16 * e);
+    }
+    out12[j] = out[0]; out12[4 + j] = out[1]; out12[8 + j] = out[2];
+  }
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+__device__ __noinline__ float plain_dot(const float* x, const float* w, int K) {
+  float sum = 0.f;
+  for (int k0 = 0; k0 < K; k0 += 16) {
+    float part = 0.f;
+    for (int k = k0; k < min(K, k0 + 16); k++) part = fmaf(x[k], w[k], part);
+    sum += part;
+  }
+  return sum;
+}
+
+template <int BN>
+__global__ void __launch_bounds__(kThreads, 1)
+k_gemm_f32_split(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ F32Params p, int splits, unsigned long long limit_ns,
+                 int* err) {
+  using S = Shape<BN>;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ SSmem s;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t raw0 = smem_u32(smem_raw), base = (raw0 + 1023u) & ~1023u, pieces = base + S::kRaw * S::kRawBytes;
+  const int split = splits > 1 ? int(cluster_ctarank()) : 0;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < S::kRaw; i++) {
+      mbar_init(smem_u32(&s.raw_full[i]), 1);
+      mbar_init(smem_u32(&s.raw_empty[i]), kSplitters);
+    }
+    for (int i = 0; i < S::kStages; i++) {
+      mbar_init(smem_u32(&s.full[i]), kSplitters);
+      mbar_init(smem_u32(&s.empty[i]), 1);
+    }
+    for (int i = 0; i < 2; i++) {
+      mbar_init(smem_u32(&s.acc_full[i]), 1);
+      mbar_init(smem_u32(&s.acc_empty[i]), 4 * S::kSides);
+    }
+    s.abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == kAdders + kSplitters + 1) {
+    tmem_alloc(smem_u32(&s.tmem_base), S::kCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl::launch_dependents();
+  pdl::grid_dependency_wait();
+  const gemm_f32::Where at = gemm_f32::f32_where(p, BN, kFeat);
+  const bool some = at.n0 < at.nend;              // a tile beyond a group's rows has nothing to do (the whole cluster)
+  const int kb_all = (p.K + kKB - 1) / kKB, kb_per = (kb_all + splits - 1) / splits, kb0 = split * kb_per;
+  const int nkb = some ? max(0, min(kb_per, kb_all - kb0)) : 0, blocks = 2 * nkb;
+  const float* w = p.w + (size_t(at.grp) * p.M + at.m0) * p.K;
+  const float* x = p.x + size_t(at.grp) * p.x_group + size_t(some ? at.n0 : 0) * p.ldx;
+  const int rows = min(BN, at.nend - at.n0), feats = min(kFeat, at.M - at.m0);
+  const uint32_t tmem0 = s.tmem_base;
+  volatile int* abortp = &s.abort_flag;
+  float* stage = reinterpret_cast<float*>(smem_raw + (base - raw0));    // [BN][128] results, after the rings have been read
+
+  if (warp < 4 * S::kSides) {
+    // ---- adders: thread = one feature, BN / kSides tokens ----
+    constexpr int kN = BN / S::kSides;
+    const int quarter = warp & 3, side = warp >> 2;
+    const uint32_t trow = tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t(side * kN);
+    float acc[kN];
+#pragma unroll
+    for (int j = 0; j < kN; j++) acc[j] = 0.f;
+    for (int i = 0; i < nkb; i++) {
+      const int buf = i & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s.acc_full[buf]), uint32_t(i >> 1) & 1u, abortp, limit_ns))) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < kN; c += 8) {
+        uint32_t r[8], q[8];
+        tmem_ld8(trow + uint32_t(2 * buf * BN + c), r);
+        tmem_ld8(trow + uint32_t((2 * buf + 1) * BN + c), q);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[c + j] += __uint_as_float(r[j]) + __uint_as_float(q[j]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&s.acc_empty[buf]));
+    }
+    // the products that read the rings are done: the last accumulator was committed behind them
+    if (nkb)
+#pragma unroll
+      for (int j = 0; j < kN; j++) stage[(side * kN + j) * kFeat + quarter * 32 + lane] = acc[j];
+  } else if (warp >= kAdders && warp < kAdders + kSplitters) {
+    // ---- splitters: eight columns of rows tid / 4, + 64, .. of the features, then of the tokens ----
+    const int tid = threadIdx.x - 32 * kAdders, c = tid & 3, r0 = tid >> 2;
+    int rs = 0, st = 0;
+    uint32_t rph = 0, ph = 0;
+    for (int i = 0; i < blocks; i++) {
+      const bool ok = mbar_wait(smem_u32(&s.raw_full[rs]), rph, abortp, limit_ns) && mbar_wait(smem_u32(&s.empty[st]), ph ^ 1u, abortp, limit_ns);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      const uint32_t from = base + rs * S::kRawBytes, to = pieces + st * S::kStageBytes;
+#pragma unroll
+      for (int u = 0; u < S::kUnits; u++) {
+        const int r = r0 + 64 * u;
+        const bool feat = u < kFeat / 64;
+        const int q = feat ? r : r - kFeat;
+        if (!feat && BN < 64 && q >= BN) continue;
+        const float4 a = lds4(from + r * 128 + (((2 * c) ^ (r & 7)) << 4)), b = lds4(from + r * 128 + (((2 * c + 1) ^ (r & 7)) << 4));
+        uint32_t h[4], m[4], l[4], top = 0;
+        split_pair(a.x, a.y, h[0], m[0], l[0], top);
+        split_pair(a.z, a.w, h[1], m[1], l[1], top);
+        split_pair(b.x, b.y, h[2], m[2], l[2], top);
+        split_pair(b.z, b.w, h[3], m[3], l[3], top);
+        if (top & 0x80008000u) {
+          const float e[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+          uint32_t out[12];                       // (arrays of their own: those above stay in registers)
+          split_careful(e, out);
+#pragma unroll
+          for (int j = 0; j < 4; j++) { h[j] = out[j]; m[j] = out[4 + j]; l[j] = out[8 + j]; }
+        }
+        constexpr int kW = S::kPieceW, kX = S::kPieceX;
+        const uint32_t dst = to + (feat ? 0 : 3 * kW) + q * 64 + ((c ^ ((q >> 1) & 3)) << 4);
+        sts4(dst, h);
+        sts4(dst + (feat ? kW : kX), m);
+        sts4(dst + 2 * (feat ? kW : kX), l);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(smem_u32(&s.full[st]));
+        mbar_arrive(smem_u32(&s.raw_empty[rs]));
+      }
+      if (++rs == S::kRaw) { rs = 0; rph ^= 1u; }
+      if (++st == S::kStages) { st = 0; ph ^= 1u; }
+    }
+  } else if (warp == kAdders + kSplitters && lane == 0) {
+    // ---- TMA producer ----
+    const uint64_t pol_x = policy_evict_last();
+    int rs = 0, issued = 0;
+    uint32_t rph = 0;
+    for (; issued < blocks; issued++) {
+      if (!mbar_wait(smem_u32(&s.raw_empty[rs]), rph ^ 1u, abortp, limit_ns)) break;
+      const uint32_t fb = smem_u32(&s.raw_full[rs]), to = base + rs * S::kRawBytes;
+      const int k = kb0 * kKB + issued * kHalf;
+      mbar_expect_tx(fb, S::kRawBytes);
+      tma_load_2d(to, &tmW, k, at.grp * p.M + at.m0, fb);
+      tma_load_2d_hint(to + kFeat * kHalf * 4, &tmX, at.grp * p.x_group + k, at.n0, fb, pol_x);
+      if (++rs == S::kRaw) { rs = 0; rph ^= 1u; }
+    }
+    if (*abortp) {
+      // gave up: let the copies already in flight land before this CTA's shared memory goes away
+      const unsigned long long t0 = globaltimer();
+      while (globaltimer() - t0 < 1000000ull) __nanosleep(1000);
+    }
+  } else if (warp == kAdders + kSplitters + 1 && lane == 0) {
+    // ---- products ----
+    const uint32_t idesc = umma_idesc_bf16(kFeat, BN);
+    int st = 0;
+    uint32_t ph = 0;
+    for (int i = 0; i < blocks; i++) {
+      const int buf = (i >> 1) & 1;
+      if (!(i & 1) && !mbar_wait(smem_u32(&s.acc_empty[buf]), (uint32_t(i >> 2) & 1u) ^ 1u, abortp, limit_ns)) break;
+      if (!mbar_wait(smem_u32(&s.full[st]), ph, abortp, limit_ns)) break;
+      tc_fence_after();
+      const uint32_t wb = pieces + st * S::kStageBytes, xb = wb + 3 * S::kPieceW, tmem_d = tmem0 + uint32_t(2 * buf * BN);
+      // the products of the first pieces apart from the others: what the tensor cores cut off a sum is small against the sum
+      constexpr int kPieces[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
+#pragma unroll
+      for (int t = 0; t < 6; t++) {
+        const uint64_t ad = umma_desc_sw64(wb + kPieces[t][0] * S::kPieceW), bd = umma_desc_sw64(xb + kPieces[t][1] * S::kPieceX);
+#pragma unroll
+        for (int k = 0; k < kHalf / 16; k++) umma_bf16(tmem_d + (t < 5 ? uint32_t(BN) : 0u), ad + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, (t % 5 | k | (i & 1)) != 0 ? 1u : 0u);
+      }
+      umma_commit(smem_u32(&s.empty[st]));
+      if (i & 1) umma_commit(smem_u32(&s.acc_full[buf]));
+      if (++st == S::kStages) { st = 0; ph ^= 1u; }
+    }
+  }
+
+  // ---- results: the cluster's sums in the order of K, CTA j the j-th share of the tokens ----
+  __syncwarp();
+  if (splits > 1) cluster_sync_all();
+  else __syncthreads();
+  if (nkb && warp < 4 * S::kSides) {
+    float* y = p.y + size_t(at.grp) * p.y_group;
+    const uint32_t stage_addr = smem_u32(stage);
+    const int share = BN / splits, t0 = split * share, t1 = min(rows, t0 + share);
+    const float* xr = x;
+    for (int idx = t0 * 32 + int(threadIdx.x); idx < t1 * 32; idx += 128 * S::kSides) {
+      const int t = idx >> 5, f = (idx & 31) * 4, m = at.m0 + f, n = at.n0 + t;
+      if (f >= feats) continue;
+      float v[4];
+      const float4 sum = splits > 1 ? dsmem_sum_f32x4(stage_addr + uint32_t((t * kFeat + f) * 4), splits) : *reinterpret_cast<const float4*>(stage + t * kFeat + f);
+      v[0] = sum.x; v[1] = sum.y; v[2] = sum.z; v[3] = sum.w;
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        if (f + e >= feats) continue;
+        if (!isfinite(v[e])) v[e] = plain_dot(xr + size_t(t) * p.ldx, w + size_t(f + e) * p.K, p.K);
+        if (p.bias) v[e] += p.bias[m + e];
+      }
+      if (p.epi == gemm::kEpiClampGlu) {
+#pragma unroll
+        for (int e = 0; e < 4; e += 2)
+          if (f + e + 1 < feats) y[size_t(n) * p.ldy + (m + e) / 2] = gemm_f32::f32_glu(p, v[e], v[e + 1]);
+      } else {
+        float* dst = y + size_t(n) * p.ldy + m;
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[e] = gemm_f32::f32_act(p, v[e], m + e);
+        if (f + 3 < feats && !(reinterpret_cast<uintptr_t>(dst) & 15)) {
+          *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; e++)
+            if (f + e < feats) dst[e] = v[e];
+        }
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  if (splits > 1) cluster_sync_all();             // nobody leaves while a peer may still read its shared memory
+  else __syncthreads();
+  if (warp == kAdders + kSplitters + 1) {
+    tc_fence_after();
+    tmem_dealloc(s.tmem_base, S::kCols);
+  }
+  if (threadIdx.x == 0 && s.abort_flag && err) atomicExch(err, 1);
+}
+
+template <int BN>
+cudaError_t launch(const F32Params& p, int x_rows, int splits, cudaStream_t st, int* map_rc) {
+  using S = Shape<BN>;
+  static std::atomic<unsigned> done{0};
+  const cudaError_t attr = pdl::allow_smem(k_gemm_f32_split<BN>, S::kSmem, done);
+  if (attr != cudaSuccess) return attr;
+  CUtensorMap tmW, tmX;
+  const int xg = p.groups - 1 + (p.m_last > 0);
+  *map_rc = tbvops::make_tensor_map_f32(&tmW, p.w, (unsigned long long)p.groups * p.M + p.m_last, p.K, p.K, kFeat) ||
+            tbvops::make_tensor_map_f32(&tmX, p.x, x_rows, (unsigned long long)xg * p.x_group + p.K, p.ldx, BN);
+  if (*map_rc) return cudaSuccess;
+  const dim3 grid(p.groups * ((p.M + kFeat - 1) / kFeat) + (p.m_last + kFeat - 1) / kFeat, (p.N + BN - 1) / BN, splits);
+  return pdl::launch(k_gemm_f32_split<BN>, grid, dim3(kThreads), S::kSmem, st, splits, tmW, tmX, p, splits, 2000000000ull, tbvops::gemm_err_flag());
+}
+
+// CTAs that share a tile's k-blocks: as many as find an SM when there is one tile of tokens, with four k-blocks or more each.
+int split_count(int M, int K, int groups, int m_last) {
+  const int kb = (K + kKB - 1) / kKB, tiles = groups * ((M + kFeat - 1) / kFeat) + (m_last + kFeat - 1) / kFeat;
+  int s = 1;
+  while (s < 8 && tiles * s * 2 <= 148 && kb / (s * 2) >= 4) s *= 2;
+  while (s > 1 && (kb + s - 1) / s * (s - 1) >= kb) s /= 2;          // every share has work
+  return s;
+}
+
+}  // namespace
+
+namespace tbvops {
+
+// By the weights' shape alone (see above).  With short K the start and the end of a tile weigh more than its products (us, here / on the CUDA cores: 130 tokens, 1024 x 520 19 / 14,
+// 512 x 512 17 / 13, 4096 x 128 17 / 13; 604 tokens, 1024 x 520 20 / 42, 4096 x 128 28 / 26); with long K it is faster at all numbers of tokens (8192 x 2048 at 1 / 16 / 130 / 604 tokens
+// 32 / 33 / 74 / 191 against 42 / 42 / 175 / 519, 2048 x 7168 54 / 55 / 94 / 197 against 92 / 94 / 326 / 607, 160 x 4096 18 / 18 / 23 / 24 against 49 / 49 / 50 / 70, 14336 x 2048
+// 56 / 56 / 128 / 266 against 109 / 111 / 266 / 906).  Relative error over such shapes 0.9 .. 1.3e-7 against 1.2 .. 2.8e-7 there.
+bool gemm_f32_split_takes(int M, int K, int groups, int m_last) { return K >= 1024 ? M >= 128 : K >= 512 && (long)M * groups >= 2048; }
+
+int gemm_f32_split_launch(const F32Params& p, int x_rows, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int splits = split_count(p.M, p.K, p.groups, p.m_last);
+  const int n = p.row_off ? min(p.N, (x_rows + p.groups - 1) / p.groups + 8) : p.N;      // rows that a tile should have room for
+  int map_rc = 0;
+  const cudaError_t e = n <= 16 ? launch<16>(p, x_rows, splits, st, &map_rc) : n <= 32 ? launch<32>(p, x_rows, splits, st, &map_rc) :
+                        n <= 64 ? launch<64>(p, x_rows, splits, st, &map_rc) : launch<128>(p, x_rows, splits, st, &map_rc);
+  if (map_rc) return -3;
+  if (e != cudaSuccess) {
+    fprintf(stderr, "[tbvops] fp32 gemm launch failed: %s (M=%d N=%d K=%d)\n", cudaGetErrorString(e), p.M, p.N, p.K);
+    return -1;
+  }
+  return 0;
+}
+
+}  // namespace tbvops

@@ -8,6 +8,7 @@ namespace gemm { struct Params; }
 namespace tbvops {
 int make_tensor_map_bf16(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned long long cols,
                          unsigned long long ld, unsigned box_rows, bool cache = true);
+int make_tensor_map_f32(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld, unsigned box_rows);
 int make_tensor_map_heads(CUtensorMap* out, const void* ptr, unsigned long long rows, unsigned heads, unsigned dim, unsigned long long ld, unsigned box_heads,
                           unsigned box_rows);
 int* gemm_err_flag();

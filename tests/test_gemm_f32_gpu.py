@@ -91,3 +91,82 @@ def test_more_rows_than_a_grid_has_small_tiles():
     ops.linear(x, w, out)
     want = x.double() @ w.double().t()
     assert ((out.double() - want).abs() <= limit(x, w)).all()
+
+
+# ---- the form on tensor cores: sums of three bf16 pieces (gemm_f32_split.cu) ----------------------------------------------------------------------------
+def split_limit(x, w):
+    # the products left out: 3 of 2^-26 of a product; sums of 64 columns: 4 accumulations of the first pieces' products, each cut off at 2^-23 of the products' sizes, the other products'
+    # 2^-8 of that; adding up the columns' sums: one rounding of 2^-24 per 64 columns, two for the parts of a cluster
+    return (x.abs().double() @ w.abs().double().t()) * (2.0 ** -24 + 5 * 2.0 ** -23 + (-(-x.shape[1] // 64) + 2) * 2.0 ** -24) + 1e-30
+
+
+@pytest.mark.parametrize("N", [1, 16, 17, 33, 64, 65, 129, 300])
+@pytest.mark.parametrize("M,K", [(128, 1024), (130, 1028), (257, 1092), (2050, 516), (1100, 2052)])
+def test_split_form(N, M, K):
+    """Remainders of tokens, features, blocks and cluster shares; strided operands; bias and activation, gated unit."""
+    from libtbvcoll_b200 import ops
+    x, w, b = rnd(N, K + 4, seed=1)[:, :K], rnd(M, K, seed=2), rnd(M, seed=3)
+    out = torch.full((N, M + 3), 7.0, device=DEV)
+    ops.linear(x, w, out[:, :M], bias=b)
+    want, e = x.double() @ w.double().t() + b.double(), split_limit(x, w)
+    assert not ops.gemm_error()
+    assert ((out[:, :M].double() - want).abs() <= e + 2.0 ** -23 * want.abs()).all() and (out[:, M:] == 7.0).all()
+    if M % 2 == 0:
+        glu = torch.zeros(N, M // 2, device=DEV)
+        ops.linear(x, w, glu, glu=(2.0, 1.7))
+        y = want - b.double()
+        g, u = y[:, 0::2].clamp(max=2.0), y[:, 1::2].clamp(-2.0, 2.0)
+        assert ((glu.double() - g * torch.sigmoid(1.7 * g) * (u + 1)).abs() <= 5 * (e[:, 0::2] + e[:, 1::2]) + 1e-5).all()
+
+
+def test_split_form_rows_do_not_depend_on_their_batch():
+    from libtbvcoll_b200 import ops
+    x, w = rnd(300, 1100, seed=1), rnd(260, 1100, seed=2)
+    whole = torch.empty(300, 260, device=DEV)
+    ops.linear(x, w, whole)
+    for n in (1, 20, 50, 129):
+        part = torch.empty(n, 260, device=DEV)
+        ops.linear(x[:n], w, part)
+        assert torch.equal(part, whole[:n])
+
+
+def test_split_form_groups():
+    from libtbvcoll_b200 import ops
+    G, M, K, last, N = 3, 130, 1032, 34, 40
+    x, w = rnd(N, G * 1036 + K, seed=1), rnd(G * M + last, K, seed=2)
+    out = torch.zeros(N, G * 136 + last, device=DEV)
+    ops.linear(x, w, out, groups=G, x_group=1036, y_group=136, last=last)
+    for g in range(G + 1):
+        rows, xs = (slice(g * M, g * M + (M if g < G else last)), x[:, g * 1036: g * 1036 + K])
+        want = xs.double() @ w[rows].double().t()
+        assert ((out[:, g * 136: g * 136 + want.shape[1]].double() - want).abs() <= split_limit(xs, w[rows])).all()
+    counts = [0, 70, 1, 0, 129, 33]
+    off = torch.tensor([0] + counts).cumsum(0).to(torch.int32).to(DEV)
+    x, w = rnd(sum(counts), K, seed=1), rnd(len(counts) * M, K, seed=2)
+    out = torch.zeros(sum(counts), M, device=DEV)
+    ops.linear_rows(x, w, out, off, len(counts), sum(counts))
+    for g in range(len(counts)):
+        a, b = int(off[g]), int(off[g + 1])
+        want = x[a:b].double() @ w[g * M: (g + 1) * M].double().t()
+        assert ((out[a:b].double() - want).abs() <= split_limit(x[a:b], w[g * M: (g + 1) * M])).all()
+    assert not ops.gemm_error()
+
+
+def test_split_form_with_values_that_are_not_finite_huge_or_tiny():
+    """As fp32 products give it: infinities keep their sign (also against weights whose lower pieces are zero), NaN stays in its row or feature, the largest values do not round to infinity."""
+    from libtbvcoll_b200 import ops
+    x, w = rnd(40, 1024, seed=1), rnd(128, 1024, seed=2).to(torch.bfloat16).float()
+    x[3, 7], x[9, 9], x[5, 1], x[11] = float("inf"), float("nan"), 3.4e38, 2.0 ** -120
+    x[5, :1], x[5, 2:] = 0.0, 0.0
+    w[5, 100], w[6, 1], w[6, 0] = -float("inf"), 0.5, 0.0
+    out = torch.zeros(40, 128, device=DEV)
+    ops.linear(x, w, out)
+    want = x.double() @ w.double().t()                                        # 64 bits overflow nowhere
+    fits = want.abs() < 3.0e38
+    assert torch.equal(out.isnan(), want.isnan())
+    assert torch.equal(out.isinf()[fits | want.isinf()], want.isinf()[fits | want.isinf()]) and torch.equal(torch.sign(out)[want.isinf()].double(), torch.sign(want)[want.isinf()])
+    ok = want.isfinite() & fits & (torch.arange(40, device=DEV) != 11)[:, None]
+    size = x.nan_to_num(0, 0, 0).abs().double() @ w.nan_to_num(0, 0, 0).abs().double().t()
+    assert ((out.double() - want).abs()[ok] <= (size * 2.0 ** -18)[ok] + 1e-30).all()
+    rel = (out[11].double() - want[11])[want[11].isfinite()].norm() / want[11][want[11].isfinite()].norm()
+    assert rel < 1e-5                                                         # pieces below the smallest bf16 are lost: 2^-133 of 2^-120
