@@ -25,6 +25,7 @@ namespace {
 
 using gemm::kEpiClampGlu;
 using gemm::kEpiF32;
+using gemm::kEpiResid;
 using gemm::kEpiSiluMul;
 using gemm::kEpiStore;
 
@@ -71,11 +72,26 @@ __device__ __forceinline__ void store_f32x4(const Params& p, int M, size_t off, 
   }
 }
 
+// Four consecutive sums of one token of a kEpiResid product: the residual stream, its gained copy; returns the squares' sum.
+__device__ __forceinline__ float resid4(const Params& p, size_t off, int m, float4 v) {
+  const uint2 hr = *reinterpret_cast<const uint2*>(p.h + off), gr = *reinterpret_cast<const uint2*>(p.gain + m);
+  const float2 h0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hr.x)), h1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hr.y));
+  const float2 g0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gr.x)), g1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gr.y));
+  __nv_bfloat162 a = __floats2bfloat162_rn(v.x + h0.x, v.y + h0.y), b = __floats2bfloat162_rn(v.z + h1.x, v.w + h1.y);
+  *reinterpret_cast<uint2*>(p.h + off) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+  const float2 f0 = __bfloat1622float2(a), f1 = __bfloat1622float2(b);
+  a = __floats2bfloat162_rn(f0.x * g0.x, f0.y * g0.y);
+  b = __floats2bfloat162_rn(f1.x * g1.x, f1.y * g1.y);
+  *reinterpret_cast<uint2*>(p.y + off) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+  return fmaf(f0.x, f0.x, f0.y * f0.y) + fmaf(f1.x, f1.x, f1.y * f1.y);
+}
+
 template <int EPI>
 __global__ void __launch_bounds__(gemm::kThreads, 1)
 k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ gemm::Smem s;
+  __shared__ float scale[EPI == kEpiStore || EPI == kEpiSiluMul ? 256 : 1], part[EPI == kEpiStore || EPI == kEpiSiluMul ? 128 : 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Launch order follows blockIdx.x.  With many token tiles the CTAs that share one 128-row weight tile
   // must run together, so that the weights stream from HBM once and the activations stay in L2.
@@ -112,6 +128,9 @@ k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
   if (warp >= 2) {
     const int quarter = warp & 3;             // TMEM lane quarter this warp may read
     const int ml = quarter * 32 + lane;       // feature row inside the tile
+    if (EPI == kEpiResid) pdl::grid_dependency_wait();     // this thread reads the stream
+    const bool scaled = (EPI == kEpiStore || EPI == kEpiSiluMul) && p.sq;
+    if (scaled) gemm::tile_scales(p, n0, rows, scale, part);
     bool ok = nkb > 0 ? mbar_wait(smem_u32(&s.accum), 0, abortp, p.limit_ns) : true;
     // lanes leave the polling loop at different times: reconverge before the warp-wide
     // (.sync.aligned) TMEM loads, and make the decision to load warp-uniform
@@ -130,7 +149,11 @@ k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
 #pragma unroll
         for (int j = 0; j < 16; j++) r[j] = 0u;
       }
-      if (S > 1) {
+      if (scaled && S == 1) {
+#pragma unroll
+        for (int j = 0; j < 16; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * (c + j < rows ? scale[c + j] : 0.f));
+      }
+      if (S > 1 || EPI == kEpiResid) {
 #pragma unroll
         for (int j = 0; j < 16; j++) stage_f[(c + j) * 128 + ml] = __uint_as_float(r[j]);
       } else if (EPI == kEpiF32) {
@@ -155,7 +178,16 @@ k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
         for (int j = 0; j < 16; j++) stage_h[(c + j) * 128 + ml] = __float2bfloat16_rn(__uint_as_float(r[j]) + bias);
       }
     }
-    if (S == 1 && EPI == kEpiF32) {
+    if (S == 1 && EPI == kEpiResid) {
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      // a warp per token: 32 lanes of four features (M is a multiple of 128)
+      for (int t = warp - 2; t < rows; t += 4) {
+        float sum = resid4(p, size_t(n0 + t) * p.ldy + m0 + lane * 4, m0 + lane * 4, *reinterpret_cast<const float4*>(stage_f + t * 128 + lane * 4));
+#pragma unroll
+        for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) p.sq_out[size_t(m0 / gemm::kBM) * p.N + n0 + t] = sum;
+      }
+    } else if (S == 1 && EPI == kEpiF32) {
       asm volatile("bar.sync 1, 128;" ::: "memory");
       const int te = threadIdx.x - 64;
       for (int idx = te; idx < rows * 32; idx += 128) {
@@ -192,10 +224,21 @@ k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
       const int fs = 128 / S;            // features per CTA
       const int q4 = fs / 4;             // float4 pieces per row
       const uint32_t stage_addr = smem_u32(sm);
-      for (int idx = te; idx < rows * q4; idx += 128) {
+      for (int idx = te; idx < (EPI == kEpiResid ? (rows * q4 + 127) / 128 * 128 : rows * q4); idx += 128) {
         const int t = idx / q4, f = split * fs + (idx % q4) * 4;
-        float4 acc = dsmem_sum_f32x4(stage_addr + uint32_t((t * 128 + f) * 4), S);
         const int m = m0 + f;
+        if constexpr (EPI == kEpiResid) {     // (all lanes stay for the sum over the token's q4 threads)
+          float sum = 0.f;
+          if (t < rows) sum = resid4(p, size_t(n0 + t) * p.ldy + m, m, dsmem_sum_f32x4(stage_addr + uint32_t((t * 128 + f) * 4), S));
+          for (int o = q4 >> 1; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+          if (t < rows && idx % q4 == 0) p.sq_out[size_t(m0 / gemm::kBM * S + split) * p.N + n0 + t] = sum;
+          continue;
+        }
+        float4 acc = dsmem_sum_f32x4(stage_addr + uint32_t((t * 128 + f) * 4), S);
+        if ((EPI == kEpiStore || EPI == kEpiSiluMul) && p.sq) {
+          const float sc = scale[t];
+          acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
+        }
         if (p.bias) {
           if (m + 0 < M) acc.x += __bfloat162float(p.bias[m + 0]);
           if (m + 1 < M) acc.y += __bfloat162float(p.bias[m + 1]);
@@ -443,7 +486,7 @@ int launch_decode_form(const void* w, const void* x, int ldx, Params& p, int epi
     const int avg = (p.x_rows + G - 1) / G, want = N < 2 * avg + 8 ? N : 2 * avg + 8;
     tbvops::gemm_config(M, want < 128 ? want : 128, K, splits_hint, &bn, &splits, &stages, G < p.x_rows ? G : p.x_rows, epi == kEpiF32);
   } else {
-    tbvops::gemm_config(M, N, K, splits_hint, &bn, &splits, &stages, G, epi == kEpiF32);
+    tbvops::gemm_config(M, N, K, splits_hint, &bn, &splits, &stages, G, epi == kEpiF32 || epi == kEpiResid);
   }
   CUtensorMap tmA, tmB;
   const int xg = G - 1 + (p.m_last > 0);
@@ -456,10 +499,11 @@ int launch_decode_form(const void* w, const void* x, int ldx, Params& p, int epi
   const size_t smem = size_t(stages) * (gemm::kATileBytes + bn * 128) + 1024;
   if (!g_attr_done) {
     // 227 KB per CTA in total; the kernel's static shared state comes out of the same budget
-    const cudaError_t a[4] = {cudaFuncSetAttribute(k_gemm<kEpiStore>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                              cudaFuncSetAttribute(k_gemm<kEpiSiluMul>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                              cudaFuncSetAttribute(k_gemm<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024),
-                              cudaFuncSetAttribute(k_gemm<kEpiClampGlu>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024)};
+    const cudaError_t a[5] = {cudaFuncSetAttribute(k_gemm<kEpiStore>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024),
+                              cudaFuncSetAttribute(k_gemm<kEpiSiluMul>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024),
+                              cudaFuncSetAttribute(k_gemm<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024),
+                              cudaFuncSetAttribute(k_gemm<kEpiClampGlu>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024),
+                              cudaFuncSetAttribute(k_gemm<kEpiResid>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024)};
     for (cudaError_t e : a)
       if (e != cudaSuccess) {
         fprintf(stderr, "[tbvops] cudaFuncSetAttribute(max dynamic smem) failed: %s\n", cudaGetErrorString(e));
@@ -475,6 +519,7 @@ int launch_decode_form(const void* w, const void* x, int ldx, Params& p, int epi
     case kEpiSiluMul: e = pdl::launch(k_gemm<kEpiSiluMul>, grid, blk, smem, st, splits, tmA, tmB, p); break;
     case kEpiF32: e = pdl::launch(k_gemm<kEpiF32>, grid, blk, smem, st, splits, tmA, tmB, p); break;
     case kEpiClampGlu: e = pdl::launch(k_gemm<kEpiClampGlu>, grid, blk, smem, st, splits, tmA, tmB, p); break;
+    case kEpiResid: e = pdl::launch(k_gemm<kEpiResid>, grid, blk, smem, st, splits, tmA, tmB, p); break;
     default: e = pdl::launch(k_gemm<kEpiStore>, grid, blk, smem, st, splits, tmA, tmB, p); break;
   }
   if (e != cudaSuccess) {
@@ -494,8 +539,7 @@ extern "C" {
 // predecessor in the stream (that is what hides the weight stream behind the previous kernel).  If w was
 // written by a kernel launched just before (a dequantised or copied weight, an activation used as w), add
 // TBV_GEMM_W_NOT_CONSTANT (0x100) to epi: the fetch then follows the dependency wait.
-int tbv_op_gemm(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi,
-                int splits_hint, void* stream) {
+static int run_gemm(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi, int splits_hint, const gemm::Params* norm, void* stream) {
   const int w_not_constant = (epi & 0x100) ? 1 : 0;
   epi &= 0xff;
   const char* pf_ptr = nullptr;   // an announcement holds for exactly one launch, whichever kernel that launch picks
@@ -506,12 +550,13 @@ int tbv_op_gemm(const void* w, const void* x, void* y, const void* bias, int M, 
   const int persist = tbvops::gemm_persist_mode();
   if (persist > 0 && splits_hint <= 0) {
     const int th = w_not_constant ? 0 : tbvops::gemm_tok_choose(M, N, K, ldy, epi, persist, tbvops::sm_count());   // the many-token kernel always prefetches w
-    if (th > 0) return tbvops::gemm_tok_launch(w, x, y, bias, M, N, K, ldx, ldy, epi, th, stream);
+    if (th > 0) return tbvops::gemm_tok_launch(w, x, y, bias, M, N, K, ldx, ldy, epi, th, norm, stream);
   }
   // Large weight matrices at decode batch sizes: the persistent kernel that splits the work evenly over the SMs.
-  if (tbvops::gemm_streamk_wants(M, N, K, epi, splits_hint, w_not_constant != 0))
+  if (!norm && tbvops::gemm_streamk_wants(M, N, K, epi, splits_hint, w_not_constant != 0))
     return tbvops::gemm_streamk_launch(w, x, y, bias, M, N, K, ldx, ldy, epi, stream);
   Params p{};
+  if (norm) p = *norm;
   p.M = M; p.N = N; p.K = K; p.ldy = ldy;
   p.a_after_wait = w_not_constant;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
@@ -519,6 +564,48 @@ int tbv_op_gemm(const void* w, const void* x, void* y, const void* bias, int M, 
   p.pf_ptr = pf_ptr;
   p.pf_bytes = pf_bytes;
   return launch_decode_form(w, x, ldx, p, epi, splits_hint, static_cast<cudaStream_t>(stream));
+}
+
+int tbv_op_gemm(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi,
+                int splits_hint, void* stream) {
+  return run_gemm(w, x, y, bias, M, N, K, ldx, ldy, epi, splits_hint, nullptr, stream);
+}
+
+// The GEMM behind a norm whose gain is in x already (tbv_op_gemm_resid, tbv_op_embed_gain): y = epilogue(scale[n] * (x w^T)), scale = 1 / rms of row rows[n] (null: n) of the
+// stream, whose squares lie in sq as `parts` sums per row, `sq_ld` floats apart.  hidden: features of the stream.
+int tbv_op_gemm_scaled(const void* w, const void* x, void* y, int M, int N, int K, int ldx, int ldy, int epi, const void* sq, const void* rows, int parts, int sq_ld, int hidden,
+                       float eps, void* stream) {
+  if (!sq || parts <= 0 || hidden <= 0 || (epi != kEpiStore && epi != kEpiSiluMul)) return -2;
+  Params n{};
+  n.sq = static_cast<const float*>(sq); n.sq_rows = static_cast<const long long*>(rows); n.sq_parts = parts; n.sq_ld = sq_ld;
+  n.sq_inv = 1.0f / float(hidden); n.sq_eps = eps;
+  return run_gemm(w, x, y, nullptr, M, N, K, ldx, ldy, epi, 0, &n, stream);
+}
+
+// Sums of squares per row that tbv_op_gemm_resid leaves for these sizes on the current device.
+int tbv_op_gemm_resid_parts(int M, int N, int K) {
+  const int persist = tbvops::gemm_persist_mode(), th = persist > 0 ? tbvops::gemm_tok_choose(M, N, K, M, kEpiStore, persist, tbvops::sm_count()) : 0;
+  if (th > 0) return tbvops::gemm_tok_resid_parts(M, N, K, th, tbvops::sm_count());
+  int bn, splits, stages;
+  tbvops::gemm_config(M, N, K, 0, &bn, &splits, &stages, 1, true);
+  return (M + 127) / 128 * splits;
+}
+// Row-parallel product, residual and the gain of the norm that follows: h += x w^T (rounded to bf16), y = bf16(h * gain), and the sums of h's squares by parts of a row to sq
+// [tbv_op_gemm_resid_parts][N].  h, y: [N, M] contiguous, 32-byte aligned; M % 128 == 0.
+int tbv_op_gemm_resid(const void* w, const void* x, void* h, const void* gain, void* y, void* sq, int M, int N, int K, int ldx, void* stream) {
+  const char* pf_ptr = nullptr;
+  const unsigned long long pf_bytes = tbvops::take_next_prefetch(&pf_ptr, (unsigned long long)(M > 0 ? M : 0) * (unsigned long long)(K > 0 ? K : 0) * 2ull);
+  if (M <= 0 || N <= 0 || K <= 0 || (M % 128) || (K % 8) || (ldx % 8) || ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(y)) & 31u) ||
+      (reinterpret_cast<uintptr_t>(gain) & 15u) || !sq)
+    return -2;
+  Params p{};
+  p.M = M; p.N = N; p.K = K; p.ldy = M;
+  p.y = static_cast<__nv_bfloat16*>(y); p.h = static_cast<__nv_bfloat16*>(h); p.gain = static_cast<const __nv_bfloat16*>(gain); p.sq_out = static_cast<float*>(sq);
+  const int persist = tbvops::gemm_persist_mode(), th = persist > 0 ? tbvops::gemm_tok_choose(M, N, K, M, kEpiStore, persist, tbvops::sm_count()) : 0;
+  if (th > 0) return tbvops::gemm_tok_launch_p(w, x, p, ldx, kEpiResid, th, stream);
+  p.pf_ptr = pf_ptr;
+  p.pf_bytes = pf_bytes;
+  return launch_decode_form(w, x, ldx, p, kEpiResid, 0, static_cast<cudaStream_t>(stream));
 }
 
 // The GEMM with the wider set of epilogues: fp32 output with an activation, clamped gated unit, grouped weights.

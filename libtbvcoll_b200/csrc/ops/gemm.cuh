@@ -68,11 +68,21 @@ struct Params {
   int* err;                     // device flag: set to 1 if a wait gave up
   Rope rope;                    // kEpiRope only
   int wide;                     // many-token kernels: rows of y are 32-byte aligned
+  // Norm in front of the product: x holds bf16(h * gain), its rows' scales 1 / rms(h) multiply the results (null: none).  sq: sums of squares of h by parts of a row,
+  // part i of row r at i * sq_ld + r; sq_rows: row of h of every row of x (null: the same).
+  const float* sq;
+  const long long* sq_rows;
+  int sq_parts, sq_ld;
+  float sq_inv, sq_eps;         // 1 / features of h
+  // kEpiResid: h += the product, y = bf16(h * gain), squares of the sums by parts of a row to sq_out (stride N)
+  __nv_bfloat16* h;
+  const __nv_bfloat16* gain;
+  float* sq_out;
   const char* pf_ptr;           // weights of the GEMM that runs next (or null): see the producer's last step
   unsigned long long pf_bytes;  // how much of them to ask into L2 (a multiple of 16), shared out over the CTAs
 };
 
-enum Epi : int { kEpiStore = 0, kEpiSiluMul = 1, kEpiF32 = 2, kEpiClampGlu = 3, kEpiRope = 4 };   // the last in the many-token kernel only
+enum Epi : int { kEpiStore = 0, kEpiSiluMul = 1, kEpiF32 = 2, kEpiClampGlu = 3, kEpiRope = 4, kEpiResid = 5 };   // kEpiRope in the many-token kernels only
 enum Act : int { kActNone = 0, kActSoftplus = 1, kActSoftcap = 2, kActSilu = 3, kActGelu = 4 };
 
 // tanh form of gelu: v / 2 * (1 + tanh(s / 2)) = v * sigmoid(s), s = 2 sqrt(2 / pi) (v + 0.044715 v^3)
@@ -90,6 +100,41 @@ __device__ __forceinline__ float clamp_glu(float g, float u, float limit, float 
   u = fminf(fmaxf(u, -limit), limit);
   if (isinf(slope)) return fmaxf(g, 0.f) * (u + shift);
   return g / (1.0f + __expf(-slope * g)) * (u + shift);
+}
+
+// 1 / rms of the row that belongs to row n of x
+__device__ __forceinline__ float row_scale(const Params& p, int n) {
+  const float* at = p.sq + (p.sq_rows ? p.sq_rows[n] : (long long)n);
+  float sum = 0.f;
+#pragma unroll 8
+  for (int i = 0; i < p.sq_parts; i++) sum += at[size_t(i) * p.sq_ld];
+  return rsqrtf(fmaf(sum, p.sq_inv, p.sq_eps));
+}
+// Decode form: the scales of a tile's rows into shared memory, by the 128 epilogue threads while the products run (behind the kernel that left the squares).  A row's parts are
+// shared out over the threads that its count leaves, so that their reads are under way together.
+__device__ __forceinline__ void tile_scales(const Params& p, int n0, int rows, float* scale, float* part) {
+  const int tid = threadIdx.x - 64;
+  pdl::grid_dependency_wait();
+  int span = 1;                                    // rows, rounded up to a power of two
+  while (span < rows && span < 128) span <<= 1;
+  const int step = 128 / span;
+  for (int r0 = 0; r0 < rows; r0 += span) {
+    const int r = r0 + (tid & (span - 1)), first = tid / span;
+    float sum = 0.f;
+    if (r < rows) {
+      const float* at = p.sq + (p.sq_rows ? p.sq_rows[n0 + r] : (long long)(n0 + r));
+#pragma unroll 8
+      for (int i = first; i < p.sq_parts; i += step) sum += at[size_t(i) * p.sq_ld];
+    }
+    part[tid] = sum;
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (tid < span && r < rows) {
+      sum = 0.f;
+      for (int i = 0; i < step; i++) sum += part[i * span + tid];
+      scale[r] = rsqrtf(fmaf(sum, p.sq_inv, p.sq_eps));
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+  }
 }
 
 struct Smem {  // static shared state of one CTA

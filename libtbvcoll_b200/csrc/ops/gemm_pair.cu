@@ -187,6 +187,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
     // ---- epilogue: thread = one token row of this CTA's 128, on one side of the features ----
     const int quarter = warp & 3, side = (warp - 2) >> 2;
     const uint32_t free0 = mapa_shared(smem_u32(&s.acc_empty[0]), 0);
+    if (EPI == gemm::kEpiResid || p.sq) pdl::grid_dependency_wait();     // these threads read what the kernel before wrote
     for (int t = 0; t < my_tiles; t++) {
       const int buf = t & 1, use = t >> 1;
       const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s.acc_full[buf]), uint32_t(use) & 1u, abortp, p.limit_ns));   // together, before the warp-wide TMEM loads
@@ -244,6 +245,7 @@ int gemm_pair_launch(const void* w, const void* x, const gemm::Params& p, int ld
     case gemm::kEpiSiluMul: e = launch<1>(w, x, p, ldx, st, &map_rc); break;
     case gemm::kEpiF32: e = launch<2>(w, x, p, ldx, st, &map_rc); break;
     case gemm::kEpiClampGlu: e = launch<3>(w, x, p, ldx, st, &map_rc); break;
+    case gemm::kEpiResid: e = launch<5>(w, x, p, ldx, st, &map_rc); break;
     case gemm::kEpiRope: e = launch<4>(w, x, p, ldx, st, &map_rc); break;
     default: e = launch<0>(w, x, p, ldx, st, &map_rc); break;
   }

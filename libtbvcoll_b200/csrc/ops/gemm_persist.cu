@@ -170,6 +170,7 @@ k_gemm_tok(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
   } else if (warp >= 2) {
     // ---- epilogue: thread = one token row of the tile ----
     const int quarter = warp & 3;
+    if (EPI == gemm::kEpiResid || p.sq) pdl::grid_dependency_wait();     // these threads read what the kernel before wrote
     for (int t = 0; t < my_tiles; t++) {
       const int buf = t & 1, use = t >> 1;
       const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s.acc_full[buf]), uint32_t(use) & 1u, abortp, p.limit_ns));   // together, before the warp-wide TMEM loads
@@ -275,9 +276,18 @@ static bool takes_pairs(const gemm::Params& p, int epi, int sms) {
   return pairs <= single && (epi == gemm::kEpiSiluMul || epi == gemm::kEpiClampGlu || single * p.kb_total >= 48);
 }
 
-int gemm_tok_launch(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi, int th,
-                    void* stream) {
+// Sums of squares per row that a kEpiResid product in form `th` leaves: one per features that a thread of the epilogue has.
+int gemm_tok_resid_parts(int M, int N, int K, int th, int sms) {
   gemm::Params p{};
+  p.M = M; p.N = N; p.kb_total = (K + 63) / 64;
+  const bool pairs = gemm_persist_mode() == 1 ? th != 3 && takes_pairs(p, gemm::kEpiResid, sms) : th == 2;
+  const int width = pairs || th == 3 ? 128 : 256;
+  return (M + width - 1) / width;
+}
+
+int gemm_tok_launch(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi, int th, const gemm::Params* norm, void* stream) {
+  gemm::Params p{};
+  if (norm) p = *norm;
   p.M = M; p.N = N; p.K = K; p.ldy = ldy;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.y = static_cast<__nv_bfloat16*>(y);
@@ -308,6 +318,7 @@ int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, in
     case gemm::kEpiClampGlu:
       e = th == 3 ? launch_tok<3, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<3, 256>(w, x, p, ldx, st, &map_rc);
       break;
+    case gemm::kEpiResid: e = th == 3 ? launch_tok<5, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<5, 256>(w, x, p, ldx, st, &map_rc); break;
     case gemm::kEpiRope:
       e = th == 3 ? launch_tok<4, 128>(w, x, p, ldx, st, &map_rc) : launch_tok<4, 256>(w, x, p, ldx, st, &map_rc); break;
     default:

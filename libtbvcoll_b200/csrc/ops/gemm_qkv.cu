@@ -27,6 +27,7 @@ __global__ void __launch_bounds__(gemm::kThreads, 1)
 k_gemm_qkv_rope(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const gemm::Params p, const gemm::Rope ra) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ gemm::Smem s;
+  __shared__ float scale[256], part[128];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = p.raster ? blockIdx.y : blockIdx.x, m0 = head * gemm::kBM, n0 = (p.raster ? blockIdx.x : blockIdx.y) * p.bn;
   const int S = p.splits;
@@ -68,6 +69,7 @@ k_gemm_qkv_rope(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
   if (warp >= 2) {
     const int quarter = warp & 3, ml = quarter * 32 + lane;
+    if (p.sq) gemm::tile_scales(p, n0, rows, scale, part);
     bool ok = nkb > 0 ? mbar_wait(smem_u32(&s.accum), 0, abortp, p.limit_ns) : true;
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
@@ -82,6 +84,10 @@ k_gemm_qkv_rope(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       } else {
 #pragma unroll
         for (int j = 0; j < 16; j++) r[j] = 0u;
+      }
+      if (p.sq && S == 1) {
+#pragma unroll
+        for (int j = 0; j < 16; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * (col + j < rows ? scale[col + j] : 0.f));
       }
       if (S > 1) {
 #pragma unroll
@@ -133,6 +139,11 @@ k_gemm_qkv_rope(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const float4 a = dsmem_sum_f32x4(stage_addr + uint32_t((t * 128 + d) * 4), S);
         const float4 b = dsmem_sum_f32x4(stage_addr + uint32_t((t * 128 + d + 64) * 4), S);
         float lo[4] = {a.x, a.y, a.z, a.w}, hi[4] = {b.x, b.y, b.z, b.w};
+        if (p.sq) {
+          const float sc = scale[t];
+#pragma unroll
+          for (int e = 0; e < 4; e++) { lo[e] *= sc; hi[e] *= sc; }
+        }
         const bool pre = pf_ok && idx == pf_idx;   // this thread's first piece: its position, cos / sin and slot are in registers
         int pos = pf_pos;
         float cs[4] = {pf_cos.x, pf_cos.y, pf_cos.z, pf_cos.w}, sn[4] = {pf_sin.x, pf_sin.y, pf_sin.z, pf_sin.w};
@@ -179,9 +190,8 @@ bool g_attr = false;
 
 }  // namespace
 
-extern "C" int tbv_op_gemm_qkv_rope(const void* w, const void* x, void* qkv, const void* bias, int M, int N, int K, int ldx, int ldy,
-                                    const void* positions, const void* cos_sin, const void* slot_mapping, void* k_cache, void* v_cache,
-                                    int nq, int nkv, int max_pos, int splits_hint, void* stream) {
+static int run_qkv(const void* w, const void* x, void* qkv, const void* bias, int M, int N, int K, int ldx, int ldy, const void* positions, const void* cos_sin,
+                   const void* slot_mapping, void* k_cache, void* v_cache, int nq, int nkv, int max_pos, int splits_hint, const gemm::Params* norm, void* stream) {
   const char* pf_ptr = nullptr;   // an announcement holds for exactly one launch
   const unsigned long long pf_bytes = tbvops::take_next_prefetch(&pf_ptr, (unsigned long long)(M > 0 ? M : 0) * (unsigned long long)(K > 0 ? K : 0) * 2ull);
   if (M != (nq + 2 * nkv) * 128 || N <= 0 || (K % 8) || (ldx % 8) || (ldy % 8)) return -2;
@@ -194,6 +204,7 @@ extern "C" int tbv_op_gemm_qkv_rope(const void* w, const void* x, void* qkv, con
     const int persist = tbvops::gemm_persist_mode(), th = persist > 0 ? tbvops::gemm_tok_choose(M, N, K, ldy, gemm::kEpiSiluMul, persist, tbvops::sm_count()) : 0;   // an epilogue that computes
     if (th > 0) {
       gemm::Params p{};
+      if (norm) p = *norm;
       p.M = M; p.N = N; p.K = K; p.ldy = ldy;
       p.bias = static_cast<const __nv_bfloat16*>(bias);
       p.y = static_cast<__nv_bfloat16*>(qkv);
@@ -207,6 +218,7 @@ extern "C" int tbv_op_gemm_qkv_rope(const void* w, const void* x, void* qkv, con
   if (tbvops::make_tensor_map_bf16(&tmA, w, M, K, K, 128) != 0) return -3;
   if (tbvops::make_tensor_map_bf16(&tmB, x, N, K, ldx, bn) != 0) return -3;
   gemm::Params p{};
+  if (norm) p = *norm;
   p.M = M; p.N = N; p.K = K; p.ldy = ldy; p.bn = bn; p.splits = splits; p.stages = stages;
   p.kb_total = (K + 63) / 64;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
@@ -216,7 +228,7 @@ extern "C" int tbv_op_gemm_qkv_rope(const void* w, const void* x, void* qkv, con
   p.pf_ptr = pf_ptr;
   p.pf_bytes = pf_bytes;
   if (!g_attr) {
-    if (cudaFuncSetAttribute(k_gemm_qkv_rope, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) return -1;
+    if (cudaFuncSetAttribute(k_gemm_qkv_rope, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024) != cudaSuccess) return -1;
     g_attr = true;
   }
   const size_t smem = size_t(stages) * (gemm::kATileBytes + bn * 128) + 1024;
@@ -229,4 +241,19 @@ extern "C" int tbv_op_gemm_qkv_rope(const void* w, const void* x, void* qkv, con
     return -1;
   }
   return 0;
+}
+
+extern "C" int tbv_op_gemm_qkv_rope(const void* w, const void* x, void* qkv, const void* bias, int M, int N, int K, int ldx, int ldy,
+                                    const void* positions, const void* cos_sin, const void* slot_mapping, void* k_cache, void* v_cache,
+                                    int nq, int nkv, int max_pos, int splits_hint, void* stream) {
+  return run_qkv(w, x, qkv, bias, M, N, K, ldx, ldy, positions, cos_sin, slot_mapping, k_cache, v_cache, nq, nkv, max_pos, splits_hint, nullptr, stream);
+}
+// The same behind a norm whose gain is in x already: see tbv_op_gemm_scaled.
+extern "C" int tbv_op_gemm_qkv_rope_scaled(const void* w, const void* x, void* qkv, const void* bias, int M, int N, int K, int ldx, int ldy, const void* positions,
+                                           const void* cos_sin, const void* slot_mapping, void* k_cache, void* v_cache, int nq, int nkv, int max_pos, const void* sq, int parts,
+                                           int sq_ld, int hidden, float eps, void* stream) {
+  if (!sq || parts <= 0 || hidden <= 0) return -2;
+  gemm::Params n{};
+  n.sq = static_cast<const float*>(sq); n.sq_parts = parts; n.sq_ld = sq_ld; n.sq_inv = 1.0f / float(hidden); n.sq_eps = eps;
+  return run_qkv(w, x, qkv, bias, M, N, K, ldx, ldy, positions, cos_sin, slot_mapping, k_cache, v_cache, nq, nkv, max_pos, 0, &n, stream);
 }

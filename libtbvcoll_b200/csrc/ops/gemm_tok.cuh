@@ -204,11 +204,66 @@ __device__ __forceinline__ void store_rope16(const gemm::Params& p, int n, int h
   }
 }
 
+__device__ __forceinline__ void ld_global_b32x8(const void* p, uint32_t* v) {
+  asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "l"(p) : "memory");
+}
+// One token row, 32 features from f on: the residual stream (`old`: as it was), its gained copy; returns the squares' sum
+__device__ __forceinline__ float store_resid32(const gemm::Params& p, int n, int f, const uint32_t* q, const uint32_t* old) {
+  uint32_t h[16], y[16];
+  float sum = 0.f;
+  const uint4* gain = reinterpret_cast<const uint4*>(p.gain + f);
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    const uint4 gq = __ldg(gain + u);
+    const uint32_t g[4] = {gq.x, gq.y, gq.z, gq.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int j = 4 * u + i;
+      h[j] = pack_bf16(__uint_as_float(q[2 * j]) + __uint_as_float(old[j] << 16), __uint_as_float(q[2 * j + 1]) + __uint_as_float(old[j] & 0xffff0000u));
+      const float a = __uint_as_float(h[j] << 16), b = __uint_as_float(h[j] & 0xffff0000u);
+      sum = fmaf(a, a, fmaf(b, b, sum));
+      y[j] = pack_bf16(a * __uint_as_float(g[i] << 16), b * __uint_as_float(g[i] & 0xffff0000u));
+    }
+  }
+  const size_t off = size_t(n) * p.ldy + f;
+  st_global_b32x8(p.h + off, h);
+  st_global_b32x8(p.h + off + 16, h + 8);
+  st_global_b32x8(p.y + off, y);
+  st_global_b32x8(p.y + off + 16, y + 8);
+  return sum;
+}
+
 // A warp's 32 rows of an accumulator of FEAT columns (`trow`: its TMEM address), token row n of this lane, features f0 ..; release(): called by the whole warp when the
 // accumulator has been read.
 template <int EPI, int FEAT, typename F>
 __device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok, int f0, uint32_t trow, F release) {
-  if constexpr (EPI == gemm::kEpiRope) {
+  // behind a norm: the row's scale
+  constexpr bool kScales = EPI == gemm::kEpiStore || EPI == gemm::kEpiSiluMul || EPI == gemm::kEpiRope;
+  const bool scaled = kScales && p.sq;
+  const float scale = scaled && row_ok ? gemm::row_scale(p, n) : 1.f;
+  if constexpr (EPI == gemm::kEpiResid) {
+    // the stream's old values are fetched 32 features ahead of their use (M is a multiple of 128)
+    const __nv_bfloat16* h = p.h + size_t(n) * p.ldy + f0;
+    const bool any = row_ok && f0 < p.M;
+    uint32_t old[2][16];
+    if (any) { ld_global_b32x8(h, old[0]); ld_global_b32x8(h + 16, old[0] + 8); }
+    float sum = 0.f;
+#pragma unroll
+    for (int c = 0; c < FEAT; c += 32) {
+      uint32_t r[32];
+      __syncwarp();
+      tmem_ld32(trow + uint32_t(c), r);
+      if (c + 32 < FEAT && row_ok && f0 + c + 32 < p.M) { ld_global_b32x8(h + c + 32, old[(c >> 5) + 1 & 1]); ld_global_b32x8(h + c + 48, old[(c >> 5) + 1 & 1] + 8); }
+      tmem_ld_wait();
+      if (c + 32 == FEAT) {
+        tc_fence_before();
+        __syncwarp();
+        release();
+      }
+      if (row_ok && f0 + c < p.M) sum += store_resid32(p, n, f0 + c, r, old[c >> 5 & 1]);
+    }
+    if (any) p.sq_out[size_t(f0 / FEAT) * p.N + n] = sum;
+  } else if constexpr (EPI == gemm::kEpiRope) {
     // rotation partners lie 64 columns apart: 16 channels of every head of the tile and their partners at a time, with the angles they share
     int pos = 0;
     long long slot = -1;
@@ -229,6 +284,10 @@ __device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok,
         tmem_ld16(trow + uint32_t(h + d), a);
         tmem_ld16(trow + uint32_t(h + d + 64), b);
         tmem_ld_wait();
+        if (scaled) {
+#pragma unroll
+          for (int j = 0; j < 16; j++) { a[j] = __float_as_uint(__uint_as_float(a[j]) * scale); b[j] = __float_as_uint(__uint_as_float(b[j]) * scale); }
+        }
         if (d == 48 && h + 128 == FEAT) {
           tc_fence_before();
           __syncwarp();
@@ -243,6 +302,10 @@ __device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok,
       __syncwarp();   // rows past the end skip the stores below: reconverge before the warp-wide load
       tmem_ld32(trow + uint32_t(c), r);
       tmem_ld_wait();
+      if (scaled) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * scale);
+      }
       if (c + 32 == FEAT) {
         // accumulator fully read by this warp: hand it back to the MMA warp before the last stores go out
         tc_fence_before();

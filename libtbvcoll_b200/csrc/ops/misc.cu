@@ -114,6 +114,41 @@ __global__ void k_embedding(const long long* __restrict__ ids, const __nv_bfloat
   for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) dst[i] = mine ? src[i] : make_uint4(0, 0, 0, 0);
 }
 
+// Embedding, its copy with the first norm's gain and the sum of its squares.
+__global__ void __launch_bounds__(256) k_embed_gain(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ table, const __nv_bfloat16* __restrict__ gain,
+                                                    __nv_bfloat16* __restrict__ h, __nv_bfloat16* __restrict__ y, float* __restrict__ sq, int hidden, long long vocab) {
+  __shared__ float part[8];
+  pdl::launch_dependents();
+  pdl::grid_dependency_wait();
+  const size_t t = blockIdx.x;
+  const long long id = ids[t];
+  const bool known = id >= 0 && id < vocab;
+  const uint4* src = reinterpret_cast<const uint4*>(table + size_t(known ? id : 0) * hidden);
+  float sum = 0.f;
+  for (int i = threadIdx.x; i < hidden / 8; i += 256) {
+    const uint4 raw = known ? src[i] : make_uint4(0, 0, 0, 0), gq = reinterpret_cast<const uint4*>(gain)[i];
+    uint4 out;
+    const uint32_t *v = &raw.x, *g = &gq.x;
+    uint32_t* o = &out.x;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(v + j)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(g + j));
+      sum = fmaf(a.x, a.x, fmaf(a.y, a.y, sum));
+      const __nv_bfloat162 y2 = __floats2bfloat162_rn(a.x * b.x, a.y * b.y);
+      o[j] = *reinterpret_cast<const uint32_t*>(&y2);
+    }
+    reinterpret_cast<uint4*>(h + t * hidden)[i] = raw;
+    reinterpret_cast<uint4*>(y + t * hidden)[i] = out;
+  }
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) sum += part[w];
+    sq[t] = sum;
+  }
+}
+
 // Greedy sampling over a vocab shard: per row the maximum logit and the smallest index
 // holding it.  Stage 1: `nblk` CTAs per row write partials; stage 2: the last CTA of a row
 // (atomic ticket) folds them in block order — deterministic, first index wins ties like
@@ -289,6 +324,15 @@ int tbv_op_embedding(const void* ids, const void* table, void* out, int tokens, 
   cudaError_t e = pdl::launch(k_embedding, dim3(tokens), dim3(256), 0, static_cast<cudaStream_t>(stream), 1,
                               static_cast<const long long*>(ids), static_cast<const __nv_bfloat16*>(table),
                               static_cast<__nv_bfloat16*>(out), hidden, vocab_start, vocab_end);
+  return e == cudaSuccess ? 0 : -1;
+}
+
+// Embedding rows to h, bf16(row * gain) to y and the rows' sums of squares to sq [tokens]: what a norm folded into the products around it starts from (tbv_op_gemm_resid).
+int tbv_op_embed_gain(const void* ids, const void* table, const void* gain, void* h, void* y, void* sq, int tokens, int hidden, long long vocab, void* stream) {
+  if (tokens <= 0 || hidden % 8) return -2;
+  cudaError_t e = pdl::launch(k_embed_gain, dim3(tokens), dim3(256), 0, static_cast<cudaStream_t>(stream), 1, static_cast<const long long*>(ids),
+                              static_cast<const __nv_bfloat16*>(table), static_cast<const __nv_bfloat16*>(gain), static_cast<__nv_bfloat16*>(h), static_cast<__nv_bfloat16*>(y),
+                              static_cast<float*>(sq), hidden, vocab);
   return e == cudaSuccess ? 0 : -1;
 }
 

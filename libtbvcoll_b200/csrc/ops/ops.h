@@ -23,8 +23,9 @@ void gemm_config(int M, int N, int K, int splits_hint, int* bn_out, int* splits_
 // many-token (prefill) persistent kernel, gemm_persist.cu
 int gemm_persist_mode();
 int gemm_tok_choose(int M, int N, int K, int ldy, int epi, int mode, int sms);
-int gemm_tok_launch(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi, int th,
+int gemm_tok_launch(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi, int th, const gemm::Params* norm,
                     void* stream);
+int gemm_tok_resid_parts(int M, int N, int K, int th, int sms);
 // the same for a filled parameter block (M, N, K, ldy, outputs, epilogue arguments)
 int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, int epi, int th, void* stream);
 // the same choice for row-grouped problems (x_rows rows over `groups` groups)

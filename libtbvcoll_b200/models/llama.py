@@ -81,6 +81,8 @@ class LlamaTP:
         self.v_cache = [torch.zeros(num_blocks * block_size, self.nkv, self.D, dtype=bf, device=dev) for _ in range(cfg.num_layers)]
 
         self.attn_ctas_per_row = self.nkv
+        # without tensor parallelism no sum over ranks stands between a product and the norm behind it: the norms are folded into the products (ops.gemm_resid, ops.gemm_scaled)
+        self.squares = ops.RowSquares(max_tokens, H, dev) if tp.world == 1 and H % 128 == 0 else None
 
     @staticmethod
     def load_weights(cfg: ModelConfig, source, tp: TPGroup, device, dtype):
@@ -105,8 +107,7 @@ class LlamaTP:
         for c0 in range(0, b.n_logits, self.max_batch):
             n = min(self.max_batch, b.n_logits - c0)
             if c0:
-                torch.index_select(self.xn[: b.T], 0, b.logit_rows[c0: c0 + n], out=self.xl[:n])
-                ops.gemm(self.xl[:n], self.w["lm_head"], out=self.logits[:n])
+                self._head(b.T, b.logit_rows[c0: c0 + n], n)
             shards = torch.empty(self.tp.world, n, self.vpr, dtype=self.logits.dtype, device=self.device)
             if self.tp.world == 1:
                 shards[0].copy_(self.logits[:n])
@@ -132,10 +133,16 @@ class LlamaTP:
         q_view = qkv.view(T, self.nq + 2 * self.nkv, self.D)[:, : self.nq]
         attn_view = attn.view(T, self.nq, self.D)
 
-        if layer_begin == 0:
+        sq, eps = self.squares, cfg.rms_eps
+        if sq is not None:
+            if layer_begin == 0:
+                ops.embed_gain(ids, w["embed"], w["layers.0.input_norm"], h, xn, sq)
+            else:
+                sq.left_by(ops.resid_parts(cfg.hidden_size, T, self.ipr), T)
+        elif layer_begin == 0:
             ops.embedding(ids, w["embed"], vocab_start=tp.rank * self.vpr, out=h)
             tp.all_reduce(h)
-            ops.rmsnorm(h, w["layers.0.input_norm"], cfg.rms_eps, out=xn)
+            ops.rmsnorm(h, w["layers.0.input_norm"], eps, out=xn)
         # Decode: every GEMM asks for the NEXT GEMM's weights to be brought into L2 while its own epilogue, the kernel
         # boundary and the attention / all-reduce kernel in between would leave HBM idle (ops.prefetch_next).
         pf = self.l2_prefetch if T <= 64 else 0
@@ -145,7 +152,7 @@ class LlamaTP:
             if pf & 1:
                 ops.prefetch_next(w[p + "o.weight"])
             ops.gemm_qkv_rope(xn, w[p + "qkv.weight"], qkv, positions, self.cos_sin, slot_mapping, self.k_cache[l], self.v_cache[l],
-                              self.nq, self.nkv, bias=w.get(p + "qkv.bias"))
+                              self.nq, self.nkv, bias=w.get(p + "qkv.bias"), sq=sq, eps=eps)
             if prefill_tiles is not None:
                 ops.prefill_attention(q_view, self.k_cache[l], self.v_cache[l], block_tables, ctx_lens, seq_of_query, prefill_tiles,
                                       attn_view, self.scale, self.block_size, ops.prefill_tile_rows(self.block_size, prefill_keys), prefill_keys)
@@ -154,24 +161,36 @@ class LlamaTP:
                                     self.block_size, seq_of_query=seq_of_query, splits=attn_splits, workspace=self.attn_ws)
             if pf & 2:
                 ops.prefetch_next(w[p + "gate_up.weight"])
-            tp.gemm_all_reduce_add_rmsnorm(attn, w[p + "o.weight"], h, w[p + "post_norm"], cfg.rms_eps, out=part)   # part := norm(h), h += sum
+            if sq is not None:
+                ops.gemm_resid(attn, w[p + "o.weight"], h, w[p + "post_norm"], part, sq)                            # h += sum, part := h * gain
+            else:
+                tp.gemm_all_reduce_add_rmsnorm(attn, w[p + "o.weight"], h, w[p + "post_norm"], eps, out=part)       # part := norm(h), h += sum
             if pf & 4:
                 ops.prefetch_next(w[p + "down.weight"])
-            ops.gemm(part, w[p + "gate_up.weight"], out=act, epi=ops.EPI_SILU_MUL)
+            if sq is not None:
+                ops.gemm_scaled(part, w[p + "gate_up.weight"], act, sq, eps, epi=ops.EPI_SILU_MUL)
+            else:
+                ops.gemm(part, w[p + "gate_up.weight"], out=act, epi=ops.EPI_SILU_MUL)
             nxt = w[f"layers.{l + 1}.input_norm"] if l + 1 < cfg.num_layers else w["norm"]
             if pf & 8:
                 ops.prefetch_next(w[f"layers.{l + 1}.qkv.weight"] if l + 1 < cfg.num_layers else w["lm_head"])
-            tp.gemm_all_reduce_add_rmsnorm(act, w[p + "down.weight"], h, nxt, cfg.rms_eps, out=xn)                  # xn := norm(h) for the next layer
+            if sq is not None:
+                ops.gemm_resid(act, w[p + "down.weight"], h, nxt, xn, sq)
+            else:
+                tp.gemm_all_reduce_add_rmsnorm(act, w[p + "down.weight"], h, nxt, eps, out=xn)                      # xn := norm(h) for the next layer
         if layer_end < cfg.num_layers:
             return None
-        if logit_rows is None:
-            xl = xn
-        else:
-            xl = self.xl[:n_logits]
-            torch.index_select(xn, 0, logit_rows, out=xl)
-        logits = self.logits[:n_logits]
-        ops.gemm(xl, w["lm_head"], out=logits)
-        return self.sample_greedy(logits, n_logits, out_tokens)
+        return self.sample_greedy(self._head(T, logit_rows, n_logits), n_logits, out_tokens)
+
+    def _head(self, T: int, rows: Optional[torch.Tensor], n: int) -> torch.Tensor:
+        """Logits of ``n`` rows (None: the first n) of the last pass over T rows."""
+        xl, logits = self.xn[:n], self.logits[:n]
+        if rows is not None:
+            xl = self.xl[:n]
+            torch.index_select(self.xn[:T], 0, rows, out=xl)
+        if self.squares is not None:
+            return ops.gemm_scaled(xl, self.w["lm_head"], logits, self.squares, self.cfg.rms_eps, rows=rows)
+        return ops.gemm(xl, self.w["lm_head"], out=logits)
 
     # -- sequence-parallel prefill --------------------------------------------------------------
     def sp_ok(self, T: int) -> bool:

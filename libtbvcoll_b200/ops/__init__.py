@@ -74,6 +74,11 @@ def lib():
     l.tbv_op_gemm_streamk_min_bytes.restype = None
     l.tbv_op_gemm_qkv_rope.argtypes = [c_vp, c_vp, c_vp, c_vp, I, I, I, I, I, c_vp, c_vp, c_vp, c_vp, c_vp, I, I, I, I, c_vp]
     l.tbv_op_gemm_qkv_rope.restype = I
+    l.tbv_op_gemm_scaled.argtypes = [c_vp] * 3 + [I] * 6 + [c_vp, c_vp, I, I, I, F, c_vp]
+    l.tbv_op_gemm_resid.argtypes = [c_vp] * 6 + [I] * 4 + [c_vp]
+    l.tbv_op_gemm_resid_parts.argtypes = [I] * 3
+    l.tbv_op_gemm_qkv_rope_scaled.argtypes = [c_vp] * 4 + [I] * 5 + [c_vp] * 5 + [I] * 3 + [c_vp, I, I, I, F, c_vp]
+    l.tbv_op_embed_gain.argtypes = [c_vp] * 6 + [I, I, LL, c_vp]
     l.tbv_op_gemm_ex_form.argtypes = [c_vp, c_vp] + [I] * 7
     l.tbv_op_gemm_config.argtypes = [I, I, I, I, ctypes.POINTER(I), ctypes.POINTER(I), ctypes.POINTER(I)]
     l.tbv_op_rmsnorm.argtypes = [c_vp, c_vp, c_vp, I, I, F, c_vp]
@@ -168,6 +173,57 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, b
     return out
 
 
+# ---- a norm folded into the products around it ------------------------------------------------------------------------------------------------
+# RMSNorm(h) * gain = (h * gain) * (1 / rms(h)): the product that writes h writes bf16(h * gain) and the sums of h's squares beside it, the product behind the norm multiplies its
+# results by the rows' scales.  No pass over the stream is left between them.
+class RowSquares:
+    """Sums of squares of a stream's rows, by parts of a row: ``sums`` fp32, part i of row r at i * ld + r."""
+
+    def __init__(self, tokens: int, hidden: int, device):
+        # few rows are split over clusters: up to two CTAs of 256 rows per SM, a part each
+        sms = torch.cuda.get_device_properties(device).multi_processor_count
+        self.sums = torch.zeros(max(2 * sms * 256, -(-hidden // 128) * tokens), dtype=torch.float32, device=device)
+        self.hidden, self.parts, self.ld = hidden, 0, 0
+
+    def left_by(self, parts: int, rows: int) -> None:
+        assert parts * rows <= self.sums.numel()
+        self.parts, self.ld = parts, rows
+
+
+def embed_gain(ids: torch.Tensor, table: torch.Tensor, gain: torch.Tensor, h: torch.Tensor, out: torch.Tensor, sq: RowSquares) -> None:
+    """h = table[ids] (zeros for ids outside it), out = bf16(h * gain), squares to ``sq``."""
+    T, H = h.shape
+    assert h.is_contiguous() and out.is_contiguous() and ids.shape[0] == T and table.shape[1] == H and ids.dtype is torch.int64
+    sq.left_by(1, T)
+    _chk(lib().tbv_op_embed_gain(_p(ids), _p(table), _p(gain), _p(h), _p(out), _p(sq.sums), T, H, table.shape[0], _st()), "tbv_op_embed_gain")
+    _count()
+
+
+def resid_parts(features: int, rows: int, k: int) -> int:
+    """Parts of a row whose squares ``gemm_resid`` sums up apart, for a product of these sizes."""
+    return lib().tbv_op_gemm_resid_parts(features, rows, k)
+
+
+def gemm_resid(x: torch.Tensor, w: torch.Tensor, h: torch.Tensor, gain: torch.Tensor, out: torch.Tensor, sq: RowSquares) -> None:
+    """h += x @ w^T (bf16), out = bf16(h * gain), squares of h to ``sq``.  w is a constant, as in ``gemm``."""
+    (N, K), M = x.shape, w.shape[0]
+    assert x.dtype is w.dtype is h.dtype is out.dtype is torch.bfloat16 and x.stride(1) == 1 and w.is_contiguous() and w.shape[1] == K
+    assert h.shape == out.shape == (N, M) and h.is_contiguous() and out.is_contiguous()
+    sq.left_by(resid_parts(M, N, K), N)
+    _chk(lib().tbv_op_gemm_resid(_p(w), _p(x), _p(h), _p(gain), _p(out), _p(sq.sums), M, N, K, x.stride(0), _st()), "tbv_op_gemm_resid")
+    _count()
+
+
+def gemm_scaled(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, sq: RowSquares, eps: float, epi: int = EPI_STORE, rows: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``gemm`` of rows that a norm stands in front of: x = bf16(h * gain), results times 1 / rms of the stream's row (``rows``: int64, the row of every row of x)."""
+    (N, K), M = x.shape, w.shape[0]
+    assert x.dtype is w.dtype is out.dtype is torch.bfloat16 and x.stride(1) == 1 and w.is_contiguous() and w.shape[1] == K and out.stride(1) == 1 and sq.parts
+    assert out.shape == (N, M // 2 if epi == EPI_SILU_MUL else M) and (rows is None or (rows.dtype is torch.int64 and rows.shape[0] == N))
+    _chk(lib().tbv_op_gemm_scaled(_p(w), _p(x), _p(out), M, N, K, x.stride(0), out.stride(0), epi, _p(sq.sums), _p(rows), sq.parts, sq.ld, sq.hidden, eps, _st()), "tbv_op_gemm_scaled")
+    _count()
+    return out
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None, act: int = ACT_NONE, act_arg: float = 0.0,
            glu: Optional[tuple] = None, copy: Optional[torch.Tensor] = None, groups: int = 1, x_group: int = 0, y_group: int = 0,
            last: int = 0, act_cols: int = 0) -> torch.Tensor:
@@ -221,13 +277,19 @@ def linear_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, row_off: to
 
 def gemm_qkv_rope(x: torch.Tensor, w: torch.Tensor, qkv: torch.Tensor, positions: torch.Tensor, cos_sin: torch.Tensor,
                   slot_mapping: Optional[torch.Tensor], k_cache: Optional[torch.Tensor], v_cache: Optional[torch.Tensor], nq: int, nkv: int,
-                  bias: Optional[torch.Tensor] = None, splits: int = 0) -> torch.Tensor:
+                  bias: Optional[torch.Tensor] = None, splits: int = 0, sq: Optional[RowSquares] = None, eps: float = 0.0) -> torch.Tensor:
     """qkv[N, (nq+2nkv)*128] = x @ w^T (+ bias) with RoPE applied to the q and k heads and the k, v
     heads written to the paged cache, all in the GEMM epilogue (head_dim 128).  Same bits as
-    ``gemm`` followed by ``rope_kv``."""
+    ``gemm`` followed by ``rope_kv``.  ``sq``: x = bf16(h * gain) of a norm folded in, as in ``gemm_scaled``."""
     N, K = x.shape
     M = w.shape[0]
     assert M == (nq + 2 * nkv) * 128 and qkv.shape == (N, M) and positions.dtype is torch.int32 and cos_sin.shape[1] == 128
+    if sq is not None:
+        assert splits == 0 and sq.parts
+        _chk(lib().tbv_op_gemm_qkv_rope_scaled(_p(w), _p(x), _p(qkv), _p(bias), M, N, K, x.stride(0), qkv.stride(0), _p(positions), _p(cos_sin), _p(slot_mapping), _p(k_cache),
+                                               _p(v_cache), nq, nkv, cos_sin.shape[0], _p(sq.sums), sq.parts, sq.ld, sq.hidden, eps, _st()), "tbv_op_gemm_qkv_rope_scaled")
+        _count()
+        return qkv
     _chk(lib().tbv_op_gemm_qkv_rope(_p(w), _p(x), _p(qkv), _p(bias), M, N, K, x.stride(0), qkv.stride(0), _p(positions), _p(cos_sin),
                                     _p(slot_mapping), _p(k_cache), _p(v_cache), nq, nkv, cos_sin.shape[0], splits, _st()),
          "tbv_op_gemm_qkv_rope")
