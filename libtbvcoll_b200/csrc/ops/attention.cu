@@ -634,11 +634,9 @@ size_t tbv_op_attn_workspace(int nq_rows, int nq_heads, int nkv, int max_splits)
 }
 
 // splits: 1..8 CTAs (one thread-block cluster) per (query row, kv head).
-int tbv_op_paged_attention(const void* q, const void* k_cache, const void* v_cache, const void* block_tables,
-                           const void* seq_of_query, const void* ctx_lens, void* out, void* workspace, int nq_rows, int nq_heads,
-                           int nkv, int head_dim, int ldq, int ldo, int block_size, int max_blocks, int splits, float scale,
-                           void* stream) {
-  (void)workspace;
+static int run_paged_attention(const void* q, const void* k_cache, const void* v_cache, const void* block_tables, const void* seq_of_query, const void* ctx_lens, void* out,
+                               int nq_rows, int nq_heads, int nkv, int head_dim, int ldq, int ldo, int block_size, int max_blocks, int splits, float scale, bool settled,
+                               void* stream) {
   if (nq_rows <= 0) return 0;
   if (head_dim != kD || nq_heads % nkv || (ldq % 8) || block_size <= 0) return -2;
   const int G = nq_heads / nkv;
@@ -666,7 +664,7 @@ int tbv_op_paged_attention(const void* q, const void* k_cache, const void* v_cac
     cudaFuncSetAttribute(k_paged_attn_mma<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem);
   }
   if (impl == 1 && (G == 1 || G == 2 || G == 4 || G == 8) && tbvops::attn_rows_takes(q, k_cache, v_cache, out, nq_heads, nkv, ldq, ldo, block_size))
-    return tbvops::attn_rows(q, k_cache, v_cache, p.block_tables, p.seq_of_query, p.ctx_lens, out, nq_rows, nq_heads, nkv, ldq, ldo, block_size, max_blocks, splits, scale, st);
+    return tbvops::attn_rows(q, k_cache, v_cache, p.block_tables, p.seq_of_query, p.ctx_lens, out, nq_rows, nq_heads, nkv, ldq, ldo, block_size, max_blocks, splits, scale, settled, st);
   if (impl == 1) {
     const dim3 blk(kMW * 32);
     switch (G) {
@@ -686,6 +684,21 @@ int tbv_op_paged_attention(const void* q, const void* k_cache, const void* v_cac
     default: return -2;
   }
   return e == cudaSuccess ? 0 : -1;
+}
+int tbv_op_paged_attention(const void* q, const void* k_cache, const void* v_cache, const void* block_tables,
+                           const void* seq_of_query, const void* ctx_lens, void* out, void* workspace, int nq_rows, int nq_heads,
+                           int nkv, int head_dim, int ldq, int ldo, int block_size, int max_blocks, int splits, float scale,
+                           void* stream) {
+  (void)workspace;
+  return run_paged_attention(q, k_cache, v_cache, block_tables, seq_of_query, ctx_lens, out, nq_rows, nq_heads, nkv, head_dim, ldq, ldo, block_size, max_blocks, splits, scale,
+                             false, stream);
+}
+// The same for row i = sequence i, where context lengths, tables and all cached tokens but each row's last were complete before the kernel launched last on the stream began (a
+// pass that starts with tbv_op_embed_gain): they are read while that kernel still runs.
+int tbv_op_paged_attention_settled(const void* q, const void* k_cache, const void* v_cache, const void* block_tables, const void* ctx_lens, void* out, int nq_rows, int nq_heads,
+                                   int nkv, int head_dim, int ldq, int ldo, int block_size, int max_blocks, int splits, float scale, void* stream) {
+  return run_paged_attention(q, k_cache, v_cache, block_tables, nullptr, ctx_lens, out, nq_rows, nq_heads, nkv, head_dim, ldq, ldo, block_size, max_blocks, splits, scale, true,
+                             stream);
 }
 
 

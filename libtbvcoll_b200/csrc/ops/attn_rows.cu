@@ -33,6 +33,7 @@ struct Params {
   const int *tables, *seq_of_row, *ctx_lens;
   int ldq, ldo, kv_heads, G, block_size, max_blocks, splits;
   float scale_log2;
+  int settled;               // 1: context lengths, tables and all cached tokens but each row's last were complete before the kernel in front of this one began
   int* err;
 };
 
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_attn_rows(const __grid_const
     sm100::mbar_fence_init();
   }
   __syncthreads();
-  pdl::grid_dependency_wait();
+  if (!p.settled) pdl::grid_dependency_wait();
   const int row = blockIdx.x, h = blockIdx.y, sp = blockIdx.z, S = p.splits, G = p.G;
   const int ctx = min(p.ctx_lens[row], p.max_blocks * p.block_size);   // never walk past the block table (a captured loop replayed beyond the reserved length)
   const int* bt = p.tables + size_t(p.seq_of_row ? p.seq_of_row[row] : row) * p.max_blocks;
@@ -78,8 +79,16 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_attn_rows(const __grid_const
     if (lane < 4)                         // keys, keys, values, values: 64 channels each
       sm100::tma_load_2d(ring + (i % kStages) * kUnit + lane * kBox, lane < 2 ? &tmK : &tmV, h * kD + (lane & 1) * 64, y, bar);
   };
+  if (p.settled) {
+    // units without the last token, which the kernel in front writes, are on their way before it has finished
+    int early = 0;
+    while (early < min(mine, kStages) && t0 + (warp + kWarps * early + 1) * kTok < ctx) issue(early++);
+    pdl::grid_dependency_wait();
+    for (; early < kStages; early++) issue(early);
+  } else {
 #pragma unroll
-  for (int i = 0; i < kStages; i++) issue(i);
+    for (int i = 0; i < kStages; i++) issue(i);
+  }
 
   // right operand of the scores: q^T, channels x heads
   uint32_t qf[kD / 16][2];
@@ -262,14 +271,14 @@ bool attn_rows_takes(const void* q, const void* k_cache, const void* v_cache, co
 }
 
 int attn_rows(const void* q, const void* k_cache, const void* v_cache, const int* tables, const int* seq_of_row, const int* ctx_lens, void* out, int rows, int heads,
-              int kv_heads, int ldq, int ldo, int block_size, int max_blocks, int splits, float scale, cudaStream_t st) {
+              int kv_heads, int ldq, int ldo, int block_size, int max_blocks, int splits, float scale, bool settled, cudaStream_t st) {
   static std::atomic<unsigned> done{0};
   if (pdl::allow_smem(k_attn_rows, kSmem, done) != cudaSuccess) return -1;
   const unsigned long long width = (unsigned long long)kv_heads * kD;
   CUtensorMap mk, mv;
   if (make_tensor_map_bf16(&mk, k_cache, kAnyCacheRows, width, width, kTok) != 0 || make_tensor_map_bf16(&mv, v_cache, kAnyCacheRows, width, width, kTok) != 0) return -3;
   const Params p{static_cast<const __nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(out), tables, seq_of_row, ctx_lens, ldq, ldo, kv_heads, heads / kv_heads, block_size,
-                 max_blocks, splits, scale * kLog2e, gemm_err_flag()};
+                 max_blocks, splits, scale * kLog2e, settled, gemm_err_flag()};
   const cudaError_t e = pdl::launch(k_attn_rows, dim3(rows, kv_heads, splits), dim3(kWarps * 32), kSmem, st, splits, mk, mv, p);
   if (e != cudaSuccess) fprintf(stderr, "[tbvops] paged attention launch failed: %s\n", cudaGetErrorString(e));
   return e == cudaSuccess ? 0 : -1;

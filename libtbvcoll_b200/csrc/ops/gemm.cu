@@ -72,9 +72,8 @@ __device__ __forceinline__ void store_f32x4(const Params& p, int M, size_t off, 
   }
 }
 
-// Four consecutive sums of one token of a kEpiResid product: the residual stream, its gained copy; returns the squares' sum.
-__device__ __forceinline__ float resid4(const Params& p, size_t off, int m, float4 v) {
-  const uint2 hr = *reinterpret_cast<const uint2*>(p.h + off), gr = *reinterpret_cast<const uint2*>(p.gain + m);
+// Four consecutive sums of one token of a kEpiResid product and what the stream and the gain have there: the residual stream, its gained copy; returns the squares' sum.
+__device__ __forceinline__ float resid4(const Params& p, size_t off, float4 v, uint2 hr, uint2 gr) {
   const float2 h0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hr.x)), h1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hr.y));
   const float2 g0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gr.x)), g1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gr.y));
   __nv_bfloat162 a = __floats2bfloat162_rn(v.x + h0.x, v.y + h0.y), b = __floats2bfloat162_rn(v.z + h1.x, v.w + h1.y);
@@ -125,10 +124,19 @@ k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
   const int rows = (nend - n0 < p.bn) ? (nend - n0) : p.bn;  // valid tokens in this tile
   constexpr int OUTW = kGlu ? 64 : 128;       // output features per tile
 
+  // The split form's first piece of this thread (four features of a token): the stream's values come in while the products run
+  uint2 ahead_h = make_uint2(0, 0), ahead_gain = make_uint2(0, 0);
   if (warp >= 2) {
     const int quarter = warp & 3;             // TMEM lane quarter this warp may read
     const int ml = quarter * 32 + lane;       // feature row inside the tile
-    if (EPI == kEpiResid) pdl::grid_dependency_wait();     // this thread reads the stream
+    if (EPI == kEpiResid) {
+      pdl::grid_dependency_wait();             // this thread reads the stream
+      const int q4 = 32 / S, t = (int(threadIdx.x) - 64) / q4, m = m0 + split * (128 / S) + (int(threadIdx.x) - 64) % q4 * 4;
+      if (S > 1 && t < rows) {
+        ahead_h = *reinterpret_cast<const uint2*>(p.h + size_t(n0 + t) * p.ldy + m);
+        ahead_gain = *reinterpret_cast<const uint2*>(p.gain + m);
+      }
+    }
     const bool scaled = (EPI == kEpiStore || EPI == kEpiSiluMul) && p.sq;
     if (scaled) gemm::tile_scales(p, n0, rows, scale, part);
     bool ok = nkb > 0 ? mbar_wait(smem_u32(&s.accum), 0, abortp, p.limit_ns) : true;
@@ -182,7 +190,9 @@ k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
       asm volatile("bar.sync 1, 128;" ::: "memory");
       // a warp per token: 32 lanes of four features (M is a multiple of 128)
       for (int t = warp - 2; t < rows; t += 4) {
-        float sum = resid4(p, size_t(n0 + t) * p.ldy + m0 + lane * 4, m0 + lane * 4, *reinterpret_cast<const float4*>(stage_f + t * 128 + lane * 4));
+        const size_t off = size_t(n0 + t) * p.ldy + m0 + lane * 4;
+        float sum = resid4(p, off, *reinterpret_cast<const float4*>(stage_f + t * 128 + lane * 4), *reinterpret_cast<const uint2*>(p.h + off),
+                           *reinterpret_cast<const uint2*>(p.gain + m0 + lane * 4));
 #pragma unroll
         for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (lane == 0) p.sq_out[size_t(m0 / gemm::kBM) * p.N + n0 + t] = sum;
@@ -224,17 +234,27 @@ k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
       const int fs = 128 / S;            // features per CTA
       const int q4 = fs / 4;             // float4 pieces per row
       const uint32_t stage_addr = smem_u32(sm);
-      for (int idx = te; idx < (EPI == kEpiResid ? (rows * q4 + 127) / 128 * 128 : rows * q4); idx += 128) {
+      const int pieces = EPI == kEpiResid ? (rows * q4 + 127) / 128 * 128 : rows * q4;
+      auto more = [&](int idx) { return idx + 128 < pieces; };
+      if (te >= pieces) cluster_arrive();
+      for (int idx = te; idx < pieces; idx += 128) {
         const int t = idx / q4, f = split * fs + (idx % q4) * 4;
         const int m = m0 + f;
         if constexpr (EPI == kEpiResid) {     // (all lanes stay for the sum over the token's q4 threads)
           float sum = 0.f;
-          if (t < rows) sum = resid4(p, size_t(n0 + t) * p.ldy + m, m, dsmem_sum_f32x4(stage_addr + uint32_t((t * 128 + f) * 4), S));
+          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (t < rows) acc = dsmem_sum_f32x4(stage_addr + uint32_t((t * 128 + f) * 4), S);
+          if (!more(idx)) cluster_arrive();
+          if (t < rows) {
+            const size_t off = size_t(n0 + t) * p.ldy + m;
+            sum = resid4(p, off, acc, idx == te ? ahead_h : *reinterpret_cast<const uint2*>(p.h + off), idx == te ? ahead_gain : *reinterpret_cast<const uint2*>(p.gain + m));
+          }
           for (int o = q4 >> 1; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
           if (t < rows && idx % q4 == 0) p.sq_out[size_t(m0 / gemm::kBM * S + split) * p.N + n0 + t] = sum;
           continue;
         }
         float4 acc = dsmem_sum_f32x4(stage_addr + uint32_t((t * 128 + f) * 4), S);
+        if (!more(idx)) cluster_arrive();     // (behind this thread's last read of its peers)
         if ((EPI == kEpiStore || EPI == kEpiSiluMul) && p.sq) {
           const float sc = scale[t];
           acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
@@ -271,8 +291,8 @@ k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
         }
       }
     }
-    __syncwarp();
-    cluster_sync_all();  // nobody leaves while a peer may still read its shared memory
+    if (warp < 2) cluster_arrive();
+    cluster_wait();      // nobody leaves while a peer may still read its shared memory
   }
   __syncwarp();
   gemm::teardown(p, s);
@@ -443,8 +463,10 @@ void gemm_config(int M, int N, int K, int splits_hint, int* bn_out, int* splits_
   if (splits_hint > 0) {
     splits = splits_hint;
   } else {
-    // a K range per CTA of at least `min_kb` 64-wide blocks (TBV_GEMM_MIN_KB, read once)
-    static const int min_kb = [] { const char* e = getenv("TBV_GEMM_MIN_KB"); int v = e ? atoi(e) : 8; return v < 1 ? 1 : v; }();
+    // a K range per CTA of at least `min_kb` 64-wide blocks (TBV_GEMM_MIN_KB, read once): with few rows the sum over the cluster is cheap against the blocks that wait for one another
+    // (Llama 2K decode step, one row: 658 us with eight, 640 with four), with more rows it is not
+    static const int env_kb = [] { const char* e = getenv("TBV_GEMM_MIN_KB"); int v = e ? atoi(e) : 0; return v < 1 ? 0 : v; }();
+    const int min_kb = env_kb ? env_kb : (bn <= 64 ? 4 : 8);
     // fp32 staging of a 256-token tile (128 KB) leaves room for one CTA per SM
     const int slots = f32_out && bn == 256 ? sms : 2 * sms;
     while (splits < 8 && tiles * splits * 2 <= slots && kb / (splits * 2) >= min_kb) splits *= 2;

@@ -134,10 +134,12 @@ k_gemm_qkv_rope(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       const int te = threadIdx.x - 64;
       const int half = 64 / S, q4 = half / 4 > 0 ? half / 4 : 1;
       const uint32_t stage_addr = smem_u32(sm);
+      if (te >= rows * q4) cluster_arrive();
       for (int idx = te; idx < rows * q4; idx += 128) {
         const int t = idx / q4, d = split * half + (idx % q4) * 4;
         const float4 a = dsmem_sum_f32x4(stage_addr + uint32_t((t * 128 + d) * 4), S);
         const float4 b = dsmem_sum_f32x4(stage_addr + uint32_t((t * 128 + d + 64) * 4), S);
+        if (idx + 128 >= rows * q4) cluster_arrive();               // (behind this thread's last read of its peers)
         float lo[4] = {a.x, a.y, a.z, a.w}, hi[4] = {b.x, b.y, b.z, b.w};
         if (p.sq) {
           const float sc = scale[t];
@@ -179,8 +181,8 @@ k_gemm_qkv_rope(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
       }
     }
-    __syncwarp();
-    cluster_sync_all();
+    if (warp < 2) cluster_arrive();
+    cluster_wait();
   }
   __syncwarp();
   gemm::teardown(p, s);

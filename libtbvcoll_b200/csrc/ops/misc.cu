@@ -118,7 +118,7 @@ __global__ void k_embedding(const long long* __restrict__ ids, const __nv_bfloat
 __global__ void __launch_bounds__(256) k_embed_gain(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ table, const __nv_bfloat16* __restrict__ gain,
                                                     __nv_bfloat16* __restrict__ h, __nv_bfloat16* __restrict__ y, float* __restrict__ sq, int hidden, long long vocab) {
   __shared__ float part[8];
-  pdl::launch_dependents();
+  // No early launch of the dependents: what a kernel of this pass reads ahead of its own dependency (paged attention of settled tokens) was complete before the pass began.
   pdl::grid_dependency_wait();
   const size_t t = blockIdx.x;
   const long long id = ids[t];

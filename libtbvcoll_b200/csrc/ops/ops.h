@@ -48,7 +48,7 @@ constexpr unsigned long long kAnyCacheRows = 0x7fffffffull;
 // attention of single rows, keys and values in caches of their own (attn_rows.cu)
 bool attn_rows_takes(const void* q, const void* k_cache, const void* v_cache, const void* out, int heads, int kv_heads, int ldq, int ldo, int block_size);
 int attn_rows(const void* q, const void* k_cache, const void* v_cache, const int* tables, const int* seq_of_row, const int* ctx_lens, void* out, int rows, int heads,
-              int kv_heads, int ldq, int ldo, int block_size, int max_blocks, int splits, float scale, cudaStream_t st);
+              int kv_heads, int ldq, int ldo, int block_size, int max_blocks, int splits, float scale, bool settled, cudaStream_t st);
 // attention of prompt rows on tcgen05, heads of 128 channels (attn_prefill.cu): keys and values in caches of their own, or side by side in cached rows
 bool attn_prefill_takes(const void* q, const void* kv, const void* out, int heads, int kv_heads, int ldq, int ldo, int block_size);
 int attn_prefill_split(const void* q, const void* k_cache, const void* v_cache, const int* tables, const int* seq_of_row, const int* ctx_lens, const int* tiles,

@@ -158,7 +158,8 @@ class LlamaTP:
                                       attn_view, self.scale, self.block_size, ops.prefill_tile_rows(self.block_size, prefill_keys), prefill_keys)
             else:
                 ops.paged_attention(q_view, self.k_cache[l], self.v_cache[l], block_tables, ctx_lens, attn_view, self.scale,
-                                    self.block_size, seq_of_query=seq_of_query, splits=attn_splits, workspace=self.attn_ws)
+                                    self.block_size, seq_of_query=seq_of_query, splits=attn_splits, workspace=self.attn_ws,
+                                    settled=sq is not None and seq_of_query is None)
             if pf & 2:
                 ops.prefetch_next(w[p + "gate_up.weight"])
             if sq is not None:

@@ -103,6 +103,7 @@ def lib():
     l.tbv_op_attn_workspace.argtypes = [I, I, I, I]
     l.tbv_op_attn_workspace.restype = SZ
     l.tbv_op_paged_attention.argtypes = [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, I, I, I, I, I, I, I, I, I, F, c_vp]
+    l.tbv_op_paged_attention_settled.argtypes = [c_vp] * 6 + [I] * 9 + [F, c_vp]
     for n in ("tbv_op_gemm", "tbv_op_rmsnorm", "tbv_op_add_rmsnorm", "tbv_op_rope_kv", "tbv_op_silu_mul", "tbv_op_embedding",
               "tbv_op_argmax", "tbv_op_argmax_merge", "tbv_op_paged_attention"):
         getattr(l, n).restype = I
@@ -469,14 +470,22 @@ def attn_workspace(nq_rows: int, nq_heads: int, nkv: int, max_splits: int, devic
 
 def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_tables: torch.Tensor, ctx_lens: torch.Tensor,
                     out: torch.Tensor, scale: float, block_size: int, seq_of_query: Optional[torch.Tensor] = None, splits: int = 1,
-                    workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
+                    workspace: Optional[torch.Tensor] = None, settled: bool = False) -> torch.Tensor:
     """q: [Nq, nq, D] (a strided view into the qkv buffer is fine), caches [slots, nkv, D],
     block_tables [nseq, max_blocks] int32, ctx_lens [Nq] int32 = keys visible to each query
-    row, seq_of_query [Nq] int32 (None = row i is sequence i).  Writes out [Nq, nq, D]."""
+    row, seq_of_query [Nq] int32 (None = row i is sequence i).  Writes out [Nq, nq, D].
+    ``settled`` (row i = sequence i): tables, context lengths and all cached tokens but each row's last were complete before the kernel launched last began, as they are in a pass
+    that starts with ``embed_gain``; they are then read while that kernel still runs."""
     Nq, nq, D = q.shape
     nkv = k_cache.shape[-2]
     assert q.stride(2) == 1 and q.stride(1) == D and out.stride(2) == 1 and out.stride(1) == D
     assert block_tables.dtype is torch.int32 and ctx_lens.dtype is torch.int32
+    if settled:
+        assert seq_of_query is None
+        _chk(lib().tbv_op_paged_attention_settled(_p(q), _p(k_cache), _p(v_cache), _p(block_tables), _p(ctx_lens), _p(out), Nq, nq, nkv, D, q.stride(0), out.stride(0), block_size,
+                                                  block_tables.shape[1], splits, scale, _st()), "tbv_op_paged_attention_settled")
+        _count()
+        return out
     _chk(lib().tbv_op_paged_attention(_p(q), _p(k_cache), _p(v_cache), _p(block_tables), _p(seq_of_query), _p(ctx_lens), _p(out),
                                       _p(workspace), Nq, nq, nkv, D, q.stride(0), out.stride(0), block_size, block_tables.shape[1],
                                       splits, scale, _st()), "tbv_op_paged_attention")

@@ -98,3 +98,26 @@ def test_fp32_rows_of_many_heads_equal_few(paired, H, G, window, chunk, cap):
     whole = run(0, n)
     for i in (0, 127, 128, 139, 140, 150, 299):
         assert torch.equal(run(i, i + 1)[0], whole[i]) and torch.isfinite(whole[i]).all() and whole[i].any()
+
+
+@pytest.mark.parametrize("rows,nq,nkv,splits", [(1, 16, 4, 1), (3, 4, 4, 2), (9, 32, 8, 4), (2, 8, 1, 8)])
+def test_settled_tokens_are_read_ahead_of_the_one_being_written(rows, nq, nkv, splits):
+    """Behind the projection that writes each row's last token, without a wait between them: the bits of the plain call behind a wait.  Last tokens that begin a unit, a split, a context."""
+    from libtbvcoll_b200 import ops
+    bs, K, longest = 16, 1024, 400
+    kc, vc = (rnd((rows * longest // bs + 1) * bs, nkv, D, seed=s) for s in (1, 2))
+    tables = torch.arange(rows * longest // bs, dtype=torch.int32, device=DEV).view(rows, -1)
+    w, cs = rnd((nq + 2 * nkv) * D, K, seed=3), ops.rope_cos_sin(D, longest, 5e5, DEV)
+    for step, last in enumerate((0, 15, 16, 63, 64, 255, 257, 383)):
+        pos = torch.tensor([max(0, last - 5 * i) for i in range(rows)], dtype=torch.int32, device=DEV)
+        ctx, slots = pos + 1, torch.arange(rows, device=DEV) * longest + pos.long()
+        x, qkv = rnd(rows, K, seed=10 + step), torch.zeros(rows, (nq + 2 * nkv) * D, dtype=torch.bfloat16, device=DEV)
+        q = qkv.view(rows, -1, D)[:, :nq]
+        got, want = torch.zeros(rows, nq, D, dtype=torch.bfloat16, device=DEV), torch.zeros(rows, nq, D, dtype=torch.bfloat16, device=DEV)
+        torch.cuda.synchronize()
+        ops.gemm_qkv_rope(x, w, qkv, pos, cs, slots, kc, vc, nq, nkv)
+        ops.paged_attention(q, kc, vc, tables, ctx, got, 0.1, bs, splits=splits, settled=True)
+        torch.cuda.synchronize()
+        ops.paged_attention(q, kc, vc, tables, ctx, want, 0.1, bs, splits=splits)
+        torch.cuda.synchronize()
+        assert not ops.gemm_error() and torch.equal(got, want)
