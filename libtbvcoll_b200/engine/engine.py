@@ -177,30 +177,46 @@ class Engine:
         """Device arrays of one pass over ``parts`` (blocks reserved, tables on the device)."""
         m, dev = self.model, self.device
         hb = lay_out(parts, self._tables_np, self.block_size, m.rows_form_max, getattr(m, "context_window", 0))
-        put = lambda a, dt: torch.from_numpy(np.ascontiguousarray(a.astype(dt, copy=False))).to(dev)
         T = int(hb.ids.size)
-        b = StepBatch(T=T, ids=put(hb.ids, np.int64), positions=put(hb.pos, np.int32), slots=put(hb.slots, np.int64), tables=self.bm.tables,
-                      ctx=put(hb.pos + 1, np.int32), n_logits=int(hb.want_rows.size), seq_of_row=put(hb.seq, np.int32),
-                      logit_rows=put(hb.want_rows, np.int64), out_tokens=out_tokens, logits_out=logits_out, n_rows_form=hb.n_rows_form)
+        host = {"ids": (hb.ids, np.int64), "positions": (hb.pos, np.int32), "slots": (hb.slots, np.int64), "ctx": (hb.pos + 1, np.int32), "seq_of_row": (hb.seq, np.int32),
+                "logit_rows": (hb.want_rows, np.int64)}
+        more = {}
         if m.uses_state:
-            b.segs = put(hb.segs, np.int32)
+            host["segs"] = (hb.segs, np.int32)
             if T > len(hb.segs):                   # otherwise one row per sequence: the models' one-token forms
-                b.seg_of_row = put(hb.seg, np.int32)
+                host["seg_of_row"] = (hb.seg, np.int32)
                 rows = m.scan_group_rows(hb.segs[:, 1])
                 if rows:
                     groups = scan_groups(hb.segs, rows)
-                    b.scan_groups, b.scan_cut = put(groups, np.int32), len(groups) > len(hb.segs)
+                    host["scan_groups"], more["scan_cut"] = (groups, np.int32), len(groups) > len(hb.segs)
         if m.rows_form_max:
             if hb.n_rows_form:
-                b.attn_splits = self.attn_splits_for(hb.n_rows_form, int(hb.pos[: hb.n_rows_form].max()) + 1)
+                more["attn_splits"] = self.attn_splits_for(hb.n_rows_form, int(hb.pos[: hb.n_rows_form].max()) + 1)
             if hb.n_rows_form < T:
-                b.dense_tiles = put(hb.dense_tiles, np.int32)
+                host["dense_tiles"] = (hb.dense_tiles, np.int32)
                 if m.expands_context:
-                    b.dense_slots = put(hb.dense_slots, np.int64)
+                    host["dense_slots"] = (hb.dense_slots, np.int64)
         elif self.tiled_prefill_attention:
-            b.tile_keys = int(hb.pos.max()) + 1
-            b.tiles = ops.prefill_tiles(torch.from_numpy(hb.seq.astype(np.int32)), m.nq // m.nkv, ops.prefill_tile_rows(self.block_size, b.tile_keys)).to(dev)
-        return b
+            more["tile_keys"] = int(hb.pos.max()) + 1
+            tiles = ops.prefill_tiles(torch.from_numpy(hb.seq.astype(np.int32)), m.nq // m.nkv, ops.prefill_tile_rows(self.block_size, more["tile_keys"]))
+            host["tiles"] = (tiles.numpy(), np.int32)
+        return StepBatch(T=T, tables=self.bm.tables, n_logits=int(hb.want_rows.size), out_tokens=out_tokens, logits_out=logits_out, n_rows_form=hb.n_rows_form, **more,
+                         **self._to_device(host))
+
+    def _to_device(self, host: Dict[str, tuple]) -> Dict[str, torch.Tensor]:
+        """Arrays (name -> array, its type on the device) in ONE copy from pinned memory, each at a multiple of 256 bytes.  A copy each from pageable memory took the host 50 us and
+        waited for everything on the stream; here the host goes on while the pass before still runs (torch keeps the pinned block until its copy is done)."""
+        arrays = {k: np.ascontiguousarray(a, dtype=dt) for k, (a, dt) in host.items()}
+        at, offsets = 0, {}
+        for k, a in arrays.items():
+            offsets[k] = at
+            at += (a.nbytes + 255) // 256 * 256
+        pinned = torch.empty(max(at, 1), dtype=torch.uint8, pin_memory=self.device.type == "cuda")
+        raw = pinned.numpy()
+        for k, a in arrays.items():
+            raw[offsets[k]: offsets[k] + a.nbytes] = a.reshape(-1).view(np.uint8)
+        packed = pinned.to(self.device, non_blocking=True)
+        return {k: packed[offsets[k]: offsets[k] + a.nbytes].view(torch.from_numpy(a[:0]).dtype).view(a.shape) for k, a in arrays.items()}
 
     # ---- one mixed step ---------------------------------------------------------------------------
     def step(self, entries, end=(), sample: bool = False):

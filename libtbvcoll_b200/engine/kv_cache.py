@@ -18,8 +18,8 @@ class BlockManager:
         self.num_blocks, self.block_size = num_blocks, block_size
         self.max_batch, self.max_blocks_per_seq = max_batch, max_blocks_per_seq
         self.free: List[int] = list(range(num_blocks - 1, 0, -1))   # block 0 reserved
-        self.tables_host = torch.zeros(max_batch, max_blocks_per_seq, dtype=torch.int32).pin_memory() \
-            if torch.cuda.is_available() else torch.zeros(max_batch, max_blocks_per_seq, dtype=torch.int32)
+        self.tables_host = torch.zeros(max_batch, max_blocks_per_seq, dtype=torch.int32)
+        self._tables_np = self.tables_host.numpy()             # the same memory: a block at a time through torch cost 4 us, a millisecond for a prompt batch of 4096 tokens
         self.tables = torch.zeros(max_batch, max_blocks_per_seq, dtype=torch.int32, device=device)
         self.owned: List[List[int]] = [[] for _ in range(max_batch)]
 
@@ -32,17 +32,19 @@ class BlockManager:
         if need > self.max_blocks_per_seq:
             raise ValueError(f"sequence of {tokens} tokens exceeds max_seq_len")
         have = self.owned[row]
-        while len(have) < need:
-            if not self.free:
-                raise RuntimeError("KV cache is out of blocks")
-            b = self.free.pop()
-            self.tables_host[row, len(have)] = b
-            have.append(b)
+        take = min(need - len(have), len(self.free))
+        if take > 0:
+            new = self.free[: -take - 1: -1]                   # from the end, last first
+            del self.free[-take:]
+            self._tables_np[row, len(have): len(have) + take] = new
+            have.extend(new)
+        if len(have) < need:
+            raise RuntimeError("KV cache is out of blocks")
 
     def release(self, row: int) -> None:
         self.free.extend(reversed(self.owned[row]))
         self.owned[row] = []
-        self.tables_host[row].zero_()
+        self._tables_np[row] = 0
 
     def release_all(self) -> None:
         for r in range(self.max_batch):
@@ -53,7 +55,13 @@ class BlockManager:
         return int(self.tables_host[row, pos // self.block_size]) * self.block_size + pos % self.block_size
 
     def sync_to_device(self) -> None:
-        self.tables.copy_(self.tables_host, non_blocking=True)
+        """Behind what the stream still has to do, from a copy of its own: the tables on the host may change at once."""
+        if self.tables.is_cuda:
+            now = torch.empty(self.tables_host.shape, dtype=torch.int32, pin_memory=True)        # (torch keeps the block until the copy is done)
+            now.copy_(self.tables_host)
+            self.tables.copy_(now, non_blocking=True)
+        else:
+            self.tables.copy_(self.tables_host)
 
 
 class Request(NamedTuple):
