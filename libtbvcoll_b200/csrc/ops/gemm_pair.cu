@@ -54,9 +54,9 @@ __device__ __forceinline__ void umma2_bf16(uint32_t tmem_d, uint64_t adesc, uint
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// one arrival at the barrier of that offset in both CTAs, when the products issued so far have finished
-__device__ __forceinline__ void umma2_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)3) : "memory");
+// one arrival at the barrier of that offset in both CTAs of the pair that begins with rank `lead`, when the products issued so far have finished
+__device__ __forceinline__ void umma2_commit(uint32_t bar, int lead) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)(3 << lead)) : "memory");
 }
 // into this CTA's shared memory; `bar` (shared::cluster) may be the other CTA's
 __device__ __forceinline__ void tma2_load(uint32_t smem_dst, const CUtensorMap* m, int x, int y, uint32_t bar) {
@@ -77,16 +77,20 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
   return true;
 }
 
-template <int EPI, bool ROWS>
+// SPLIT: clusters of two pairs with a tile each, one for the first half of K and one for the second.  A pair hands the half of the features that the other finishes over through its
+// (then free) ring: 64 KB per CTA, read over distributed shared memory.
+template <int EPI, bool ROWS, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 k_gemm_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ gemm::Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ PSmem s;
   __shared__ typename std::conditional<ROWS, RowGroups, int>::type groups;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = int(cluster_ctarank()), pair = int(blockIdx.x) >> 1, pairs = int(gridDim.x) >> 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cluster_rank = int(cluster_ctarank()), rank = cluster_rank & 1, lead = cluster_rank & ~1,
+            half = SPLIT ? cluster_rank >> 1 : 0, pair = int(blockIdx.x) >> (SPLIT ? 2 : 1), pairs = int(gridDim.x) >> (SPLIT ? 2 : 1);
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;                  // the same offset in both CTAs
-  const int tok_tiles = (p.N + kTok - 1) / kTok, feat_tiles = (p.M + kFeat - 1) / kFeat, nkb = p.kb_total;
+  const int tok_tiles = (p.N + kTok - 1) / kTok, feat_tiles = (p.M + kFeat - 1) / kFeat, kb0 = SPLIT ? half * ((p.kb_total + 1) / 2) : 0,
+            nkb = SPLIT ? (half ? p.kb_total / 2 : (p.kb_total + 1) / 2) : p.kb_total;      // k-blocks of this pair
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; i++) {
@@ -126,21 +130,22 @@ k_gemm_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
   };
   const uint32_t tmem0 = s.tmem_base;
   volatile int* abortp = &s.abort_flag;
+  bool all_ok = false;                           // SPLIT: this thread's accumulator is there
 
   if (warp == 0 && lane == 0) {
     // ---- TMA producer of this CTA: one flat sequence of k-blocks over all of the pair's tiles ----
     const uint64_t pol_x = policy_evict_last();
-    const uint32_t full0 = mapa_shared(smem_u32(&s.full[0]), 0);              // barriers of the first CTA
+    const uint32_t full0 = mapa_shared(smem_u32(&s.full[0]), lead);           // barriers of the pair's first CTA
     // Weights are never written by a kernel: the first ring fill of weight tiles goes out before the
     // preceding kernel has finished; the activations follow once it has.
     const int pre = my_tiles ? min(kStages, nkb) : 0;
     At at = my_tiles ? locate(pair) : At{};
     for (int i = 0; i < pre; i++) {
       if (rank == 0) mbar_expect_tx(smem_u32(&s.full[i]), 2 * kStageBytes);
-      tma2_load(base + i * kStageBytes + kXBytes, &tmW, i * gemm::kBK, at.w0 + rank * kFeat / 2, full0 + 8u * i);
+      tma2_load(base + i * kStageBytes + kXBytes, &tmW, (kb0 + i) * gemm::kBK, at.w0 + rank * kFeat / 2, full0 + 8u * i);
     }
     pdl::grid_dependency_wait();
-    for (int i = 0; i < pre; i++) tma2_load_hint(base + i * kStageBytes, &tmX, i * gemm::kBK, at.n0 + rank * 128, full0 + 8u * i, pol_x);
+    for (int i = 0; i < pre; i++) tma2_load_hint(base + i * kStageBytes, &tmX, (kb0 + i) * gemm::kBK, at.n0 + rank * 128, full0 + 8u * i, pol_x);
     int st = pre == kStages ? 0 : pre;
     uint32_t ph = pre == kStages ? 1u : 0u;   // of the ring's current round
     bool ok = true;
@@ -150,8 +155,8 @@ k_gemm_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
         // (the first CTA's wait for this round stands behind the products that read the stage, so the other CTA's bytes cannot meet an older round's count)
         if (!mbar_wait(smem_u32(&s.empty[st]), ph ^ 1u, abortp, p.limit_ns)) { ok = false; break; }
         if (rank == 0) mbar_expect_tx(smem_u32(&s.full[st]), 2 * kStageBytes);
-        tma2_load_hint(base + st * kStageBytes, &tmX, kb * gemm::kBK, at.n0 + rank * 128, full0 + 8u * st, pol_x);
-        tma2_load(base + st * kStageBytes + kXBytes, &tmW, kb * gemm::kBK, at.w0 + rank * kFeat / 2, full0 + 8u * st);
+        tma2_load_hint(base + st * kStageBytes, &tmX, (kb0 + kb) * gemm::kBK, at.n0 + rank * 128, full0 + 8u * st, pol_x);
+        tma2_load(base + st * kStageBytes + kXBytes, &tmW, (kb0 + kb) * gemm::kBK, at.w0 + rank * kFeat / 2, full0 + 8u * st);
         if (++st == kStages) { st = 0; ph ^= 1u; }
       }
     }
@@ -178,25 +183,61 @@ k_gemm_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
         const uint64_t ad = umma_desc_sw128(base + st * kStageBytes), bd = umma_desc_sw128(base + st * kStageBytes + kXBytes);
 #pragma unroll
         for (int k = 0; k < gemm::kBK / 16; k++) umma2_bf16(tmem_d, ad + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
-        umma2_commit(smem_u32(&s.empty[st]));
+        umma2_commit(smem_u32(&s.empty[st]), lead);
         if (++st == kStages) { st = 0; ph ^= 1u; }
       }
-      if (ok) umma2_commit(smem_u32(&s.acc_full[buf]));
+      if (ok) umma2_commit(smem_u32(&s.acc_full[buf]), lead);
     }
   } else if (warp >= 2) {
     // ---- epilogue: thread = one token row of this CTA's 128, on one side of the features ----
     const int quarter = warp & 3, side = (warp - 2) >> 2;
-    const uint32_t free0 = mapa_shared(smem_u32(&s.acc_empty[0]), 0);
+    const uint32_t free0 = mapa_shared(smem_u32(&s.acc_empty[0]), lead);
     if (EPI == gemm::kEpiResid || p.sq) pdl::grid_dependency_wait();     // these threads read what the kernel before wrote
     for (int t = 0; t < my_tiles; t++) {
       const int buf = t & 1, use = t >> 1;
       const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s.acc_full[buf]), uint32_t(use) & 1u, abortp, p.limit_ns));   // together, before the warp-wide TMEM loads
       if (!ok) break;
       tc_fence_after();
+      if constexpr (SPLIT) {
+        // the features that the other pair finishes, [feature][row of this CTA]
+        const uint32_t from = tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t(buf * kFeat + (half ^ 1) * kSide + side * 64), to = base + uint32_t(side * 64 * 128 + quarter * 32 + lane) * 4u;
+#pragma unroll
+        for (int c = 0; c < 64; c += 32) {
+          uint32_t r[32];
+          tmem_ld32(from + uint32_t(c), r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; j++) asm volatile("st.shared.b32 [%0], %1;" ::"r"(to + uint32_t((c + j) * 512)), "r"(r[j]) : "memory");
+        }
+        all_ok = true;
+        break;
+      }
       const At at = locate(pair + t * pairs);
       const int n = at.n0 + rank * 128 + quarter * 32 + lane;   // token row
       drain<EPI, kSide>(p, n, n < at.nend, at.f0 + side * kSide, tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t(buf * kFeat + side * kSide), [&] {
         if (lane == 0) mbar_arrive_cluster(free0 + 8u * buf);
+      });
+    }
+  }
+
+  if constexpr (SPLIT) {
+    __syncwarp();
+    tc_fence_before();
+    cluster_sync_all();
+    if (warp >= 2 && warp < 6 && all_ok) {
+      tc_fence_after();
+      const int quarter = warp & 3;
+      const uint32_t there = mapa_shared(base + uint32_t(quarter * 32 + lane) * 4u, uint32_t(cluster_rank ^ 2));
+      const At at = locate(pair);
+      const int n = at.n0 + rank * 128 + quarter * 32 + lane;
+      drain<EPI, kSide>(p, n, n < at.nend, at.f0 + half * kSide, tmem0 + (uint32_t(quarter * 32) << 16) + uint32_t(half * kSide), [] {}, [&](int c, int cnt, uint32_t* r) {
+        float v[32];                             // all on their way before the first is used
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+          if (j < cnt) v[j] = ld_dsmem_f32(there + uint32_t((c + j) * 512));
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+          if (j < cnt) r[j] = __float_as_uint(__uint_as_float(r[j]) + v[j]);
       });
     }
   }
@@ -212,7 +253,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
   if (threadIdx.x == 0 && s.abort_flag && p.err) atomicExch(p.err, 1);
 }
 
-template <int EPI, bool ROWS = false>
+template <int EPI, bool ROWS = false, bool SPLIT = false>
 cudaError_t launch(const void* w, const void* x, const gemm::Params& p, int ldx, cudaStream_t st, int* map_rc) {
   CUtensorMap tmX, tmW;
   *map_rc = 0;
@@ -223,11 +264,12 @@ cudaError_t launch(const void* w, const void* x, const gemm::Params& p, int ldx,
   }
   constexpr size_t smem = size_t(kStages) * kStageBytes + 1024;
   static std::atomic<unsigned> done{0};
-  const cudaError_t attr = pdl::allow_smem(k_gemm_pair<EPI, ROWS>, smem, done);
+  const cudaError_t attr = pdl::allow_smem(k_gemm_pair<EPI, ROWS, SPLIT>, smem, done);
   if (attr != cudaSuccess) return attr;
   const int tiles = (ROWS ? p.x_rows / 256 + p.groups : (p.N + 255) / 256) * ((p.M + kFeat - 1) / kFeat);   // ROWS: at most
+  if (SPLIT) return pdl::launch_clusters(k_gemm_pair<EPI, ROWS, SPLIT>, dim3(4 * tiles), dim3(kThreads), smem, st, dim3(4), tmX, tmW, p);
   const int pairs = tbvops::sm_count() / 2;
-  return pdl::launch_clusters(k_gemm_pair<EPI, ROWS>, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kThreads), smem, st, dim3(2), tmX, tmW, p);   // (pairs lie along x)
+  return pdl::launch_clusters(k_gemm_pair<EPI, ROWS, SPLIT>, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kThreads), smem, st, dim3(2), tmX, tmW, p);   // (pairs lie along x)
 }
 
 }  // namespace
@@ -235,11 +277,14 @@ cudaError_t launch(const void* w, const void* x, const gemm::Params& p, int ldx,
 namespace tbvops {
 
 // p is filled (gemm_tok_launch_p)
-int gemm_pair_launch(const void* w, const void* x, const gemm::Params& p, int ldx, int epi, void* stream) {
+int gemm_pair_launch(const void* w, const void* x, const gemm::Params& p, int ldx, int epi, bool split, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int map_rc = 0;
   cudaError_t e;
-  if (p.row_off) {
+  if (split) {
+    e = epi == gemm::kEpiResid ? launch<5, false, true>(w, x, p, ldx, st, &map_rc) : epi == gemm::kEpiF32 ? launch<2, false, true>(w, x, p, ldx, st, &map_rc) :
+        launch<0, false, true>(w, x, p, ldx, st, &map_rc);
+  } else if (p.row_off) {
     e = epi == gemm::kEpiClampGlu ? launch<3, true>(w, x, p, ldx, st, &map_rc) : launch<0, true>(w, x, p, ldx, st, &map_rc);
   } else switch (epi) {
     case gemm::kEpiSiluMul: e = launch<1>(w, x, p, ldx, st, &map_rc); break;

@@ -263,23 +263,30 @@ int gemm_tok_rows_choose(int M, int x_rows, int groups, int K, int epi, int mode
   return K > 4096 && x_rows / groups >= 768 && tiles >= 3l * sms ? 2 : 1;
 }
 
-// Whether the 256-feature tiles of a problem go to pairs of SMs (gemm_pair.cu): where that needs no more rounds and the pair's start and end (a cluster's launch, two barriers: some
+// Whether the 256-feature tiles of a problem go to pairs of SMs (gemm_pair.cu), a round of which takes 0.92 of one here: where that is no longer and the pair's start and end (a cluster's launch, two barriers: some
 // 2 us) are small beside them.  A gated unit's long epilogue gains by the pair's twice as many warps in any case.
 // us, alone / in pairs: 4096 tokens, 6144 x 4096 with rotation 158 / 148, 4096 x 4096 102 / 94, 14336 x 2048 with the SiLU unit 186 / 165, 2048 x 7168 101 / 91, 8192 x 2048 98 / 92;
-// 1024 tokens, 14336 x 2048 with the SiLU unit 68 / 58, 28672 x 4096 190 / 172, 4096 x 14336 99 / 87; the other side: 1024 tokens, 3072 x 2048 27 / 28, 2048 x 2048 17.6 / 18.4,
+// 1024 tokens, 14336 x 2048 with the SiLU unit 68 / 58, 28672 x 4096 190 / 172, 4096 x 14336 99 / 87; 3903 tokens, whose 31 tiles of 128 make 16 of 256, 28672 x 4096 675 / 660 (25 rounds against 24); the other side: 1024 tokens, 3072 x 2048 27 / 28, 2048 x 2048 17.6 / 18.4,
 // 2048 tokens, 2048 x 2048 20 / 22, 4096 tokens, 4096 x 128 26 / 30.  Groups of rows, whose last tiles are half empty on average: 8 groups of about 700, 7168 x 2048 gated 174 / 153,
 // 2048 x 3584 87 / 78, of about 1024 206 / 197 and 114 / 102; of about 512 137 / 135 and 67 / 84.
 static bool takes_pairs(const gemm::Params& p, int epi, int sms) {
   if (sms < 2) return false;
   if (p.row_off) return p.x_rows / p.groups >= 640;
   const long f256 = (p.M + 255) / 256, single = ((p.N + 127l) / 128 * f256 + sms - 1) / sms, pairs = ((p.N + 255l) / 256 * f256 + sms / 2 - 1) / (sms / 2);
-  return pairs <= single && (epi == gemm::kEpiSiluMul || epi == gemm::kEpiClampGlu || single * p.kb_total >= 48);
+  return 11 * pairs <= 12 * single && (epi == gemm::kEpiSiluMul || epi == gemm::kEpiClampGlu || single * p.kb_total >= 48);
+}
+
+// Whether a plain product goes to clusters of two pairs that share out K: where all of its 256 x 256 tiles find one, and K is long against the exchange of half the results.
+// us, before / in split pairs: 384 tokens, 2048 x 7168 36 / 24, 1024 tokens 37 / 26, 2048 x 4096 23 / 19, 512 tokens, 4096 x 14336 69 / 47, 2048 tokens, 1024 x 7168 37 / 26.
+static bool takes_split(const gemm::Params& p, int epi, int sms) {
+  return !p.row_off && (epi == gemm::kEpiStore || epi == gemm::kEpiF32 || epi == gemm::kEpiResid) && p.kb_total >= 64 && (p.N + 255l) / 256 * ((p.M + 255) / 256) <= sms / 4;
 }
 
 // Sums of squares per row that a kEpiResid product in form `th` leaves: one per features that a thread of the epilogue has.
 int gemm_tok_resid_parts(int M, int N, int K, int th, int sms) {
   gemm::Params p{};
   p.M = M; p.N = N; p.kb_total = (K + 63) / 64;
+  if (gemm_persist_mode() == 1 && takes_split(p, gemm::kEpiResid, sms)) return (M + 127) / 128;
   const bool pairs = gemm_persist_mode() == 1 ? th != 3 && takes_pairs(p, gemm::kEpiResid, sms) : th == 2;
   const int width = pairs || th == 3 ? 128 : 256;
   return (M + width - 1) / width;
@@ -301,8 +308,9 @@ int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, in
   p.limit_ns = 2000000000ull;
   p.err = gemm_err_flag();
   const int mode = gemm_persist_mode();
+  if (mode == 1 && takes_split(p, epi, sm_count())) return gemm_pair_launch(w, x, p, ldx, epi, true, stream);
   if (mode == 1 && th == 2 && p.kb_total <= 4 && epi == gemm::kEpiF32) th = 3;    // all epilogue: more CTAs for it (4096 tokens, 4096 x 128 23.6 us against 26)
-  if (mode == 1 ? th != 3 && takes_pairs(p, epi, sm_count()) : th == 2) return gemm_pair_launch(w, x, p, ldx, epi, stream);
+  if (mode == 1 ? th != 3 && takes_pairs(p, epi, sm_count()) : th == 2) return gemm_pair_launch(w, x, p, ldx, epi, false, stream);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int map_rc = 0;
   cudaError_t e;

@@ -233,10 +233,11 @@ __device__ __forceinline__ float store_resid32(const gemm::Params& p, int n, int
   return sum;
 }
 
+struct NoMore { __device__ __forceinline__ void operator()(int, int, uint32_t*) const {} };
 // A warp's 32 rows of an accumulator of FEAT columns (`trow`: its TMEM address), token row n of this lane, features f0 ..; release(): called by the whole warp when the
-// accumulator has been read.
-template <int EPI, int FEAT, typename F>
-__device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok, int f0, uint32_t trow, F release) {
+// accumulator has been read; more(c, n, r): adds what others have of columns c .. c + n - 1.
+template <int EPI, int FEAT, typename F, typename G = NoMore>
+__device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok, int f0, uint32_t trow, F release, G more = G{}) {
   // behind a norm: the row's scale
   constexpr bool kScales = EPI == gemm::kEpiStore || EPI == gemm::kEpiSiluMul || EPI == gemm::kEpiRope;
   const bool scaled = kScales && p.sq;
@@ -255,6 +256,7 @@ __device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok,
       tmem_ld32(trow + uint32_t(c), r);
       if (c + 32 < FEAT && row_ok && f0 + c + 32 < p.M) { ld_global_b32x8(h + c + 32, old[(c >> 5) + 1 & 1]); ld_global_b32x8(h + c + 48, old[(c >> 5) + 1 & 1] + 8); }
       tmem_ld_wait();
+      more(c, 32, r);
       if (c + 32 == FEAT) {
         tc_fence_before();
         __syncwarp();
@@ -284,6 +286,8 @@ __device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok,
         tmem_ld16(trow + uint32_t(h + d), a);
         tmem_ld16(trow + uint32_t(h + d + 64), b);
         tmem_ld_wait();
+        more(h + d, 16, a);
+        more(h + d + 64, 16, b);
         if (scaled) {
 #pragma unroll
           for (int j = 0; j < 16; j++) { a[j] = __float_as_uint(__uint_as_float(a[j]) * scale); b[j] = __float_as_uint(__uint_as_float(b[j]) * scale); }
@@ -302,6 +306,7 @@ __device__ __forceinline__ void drain(const gemm::Params& p, int n, bool row_ok,
       __syncwarp();   // rows past the end skip the stores below: reconverge before the warp-wide load
       tmem_ld32(trow + uint32_t(c), r);
       tmem_ld_wait();
+      more(c, 32, r);
       if (scaled) {
 #pragma unroll
         for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * scale);

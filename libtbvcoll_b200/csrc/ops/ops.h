@@ -31,7 +31,7 @@ int gemm_tok_launch_p(const void* w, const void* x, gemm::Params& p, int ldx, in
 // the same choice for row-grouped problems (x_rows rows over `groups` groups)
 int gemm_tok_rows_choose(int M, int x_rows, int groups, int K, int epi, int mode, int sms);
 // its form on pairs of SMs, gemm_pair.cu
-int gemm_pair_launch(const void* w, const void* x, const gemm::Params& p, int ldx, int epi, void* stream);
+int gemm_pair_launch(const void* w, const void* x, const gemm::Params& p, int ldx, int epi, bool split, void* stream);
 // evenly-split (stream-K) decode GEMM, gemm_streamk.cu
 bool gemm_streamk_wants(int M, int N, int K, int epi, int splits_hint, bool w_not_constant);
 int gemm_streamk_launch(const void* w, const void* x, void* y, const void* bias, int M, int N, int K, int ldx, int ldy, int epi,

@@ -144,3 +144,25 @@ def test_gated_row_groups_on_pairs_of_sms(counts, M, K):
     finally:
         ops.gemm_persist_mode(None)
     assert not ops.gemm_error() and torch.equal(*got)
+
+
+@pytest.mark.parametrize("N,M,K", [(384, 2048, 7168), (513, 2064, 4104), (1000, 2048, 4160), (1024, 2304, 8200), (1153, 1800, 6152)])
+def test_long_k_shared_out_over_two_pairs(N, M, K):
+    """Tiles that find a cluster each: odd numbers of k-blocks, remainders of tokens and features; every epilogue that goes there."""
+    from libtbvcoll_b200 import ops
+    x, w, b = rnd(N, K, seed=1), rnd(M, K, seed=2, scale=K ** -0.5), rnd(M, seed=3)
+    want, e = x.double() @ w.double().t(), (x.double().abs() @ w.double().abs().t()) * K * 2.0 ** -24     # K fp32 additions
+    f32, copy = torch.zeros(N, M, device=DEV), torch.zeros(N, M, dtype=torch.bfloat16, device=DEV)
+    ops.linear(x, w, f32, bias=b, copy=copy)
+    out, plain = torch.zeros(N, M, dtype=torch.bfloat16, device=DEV), ops.gemm(x, w)
+    ops.linear(x, w, out, act=ops.ACT_SILU, act_cols=32)
+    assert not ops.gemm_error()
+    assert ((f32.double() - want - b.double()).abs() <= e + want.abs() * 2.0 ** -23).all() and torch.equal(copy, f32.to(torch.bfloat16))
+    assert ((plain.double() - want).abs() <= e + want.abs() * 2.0 ** -8).all() and torch.equal(out[:, 32:], plain[:, 32:])
+    if M % 128 == 0:
+        h0, gain, sq = rnd(N, M, seed=4), rnd(M, seed=5), ops.RowSquares(N, M, DEV)
+        h, y = h0.clone(), torch.zeros(N, M, dtype=torch.bfloat16, device=DEV)
+        ops.gemm_resid(x, w, h, gain, y, sq)
+        assert ((h.double() - want - h0.double()).abs() <= e + (want + h0.double()).abs() * 2.0 ** -8).all() and torch.equal(y, (h.float() * gain.float()).to(torch.bfloat16))
+        got = sq.sums[: sq.parts * sq.ld].view(sq.parts, sq.ld).double().sum(0)
+        assert not ops.gemm_error() and ((got - h.double().pow(2).sum(1)).abs() <= h.double().pow(2).sum(1) * M * 2.0 ** -24).all()
