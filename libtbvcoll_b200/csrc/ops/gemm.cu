@@ -467,9 +467,10 @@ void gemm_config(int M, int N, int K, int splits_hint, int* bn_out, int* splits_
     // (Llama 2K decode step, one row: 658 us with eight, 640 with four), with more rows it is not
     static const int env_kb = [] { const char* e = getenv("TBV_GEMM_MIN_KB"); int v = e ? atoi(e) : 0; return v < 1 ? 0 : v; }();
     const int min_kb = env_kb ? env_kb : (bn <= 64 ? 4 : 8);
-    // fp32 staging of a 256-token tile (128 KB) leaves room for one CTA per SM
-    const int slots = f32_out && bn == 256 ? sms : 2 * sms;
-    while (splits < 8 && tiles * splits * 2 <= slots && kb / (splits * 2) >= min_kb) splits *= 2;
+    // CTAs that find a place at once: two per SM, but the fp32 staging of a 256-token tile (128 KB), which every split one has, leaves room for one, and then clusters of eight find four
+    // fifths of the SMs (us with a second wave of CTAs / without: 512 tokens, 2048 x 4096 40 / 18, 300 tokens, 2048 x 7168 40 / 22, 129 tokens, 4096 x 14336 61 / 31, 14336 x 2048 36 / 20)
+    auto slots = [&](int s) { return bn < 256 ? 2 * sms : (s < 8 ? sms : sms * 4 / 5); };
+    while (splits < 8 && tiles * splits * 2 <= slots(splits * 2) && kb / (splits * 2) >= min_kb) splits *= 2;
   }
   while (splits > 1 && (kb + splits - 1) / splits * (splits - 1) >= kb) splits /= 2;  // every split gets work
   const int stage_bytes = gemm::kATileBytes + bn * 128;
