@@ -138,8 +138,9 @@ struct RowsParams {
 enum RowKind { kLatent, kShared, kPaired };
 
 // fp32: HP heads (of one cache head) of a row per CTA, tiles of 128 keys.  A thread multiplies one key with the queries of all HP heads and sums up to KA result
-// columns, one in 128, for all of them, so that a cached row passes once for HP heads.  Bound by those passes through L2: four heads at a time instead of one take
-// 575 instead of 1210 us (rows of prompts of 101 and 503 tokens, 16 heads, latents of 512 + 64).  Exponents are taken of differences of natural-unit scores: a score of hundreds loses nothing to a multiplication by log2 e.
+// columns, one in 128, for all of them, so that a cached row passes once for HP heads.  With several heads the keys come in by 32 columns through shared memory, rows 144 bytes
+// apart (a key per lane straight from memory touched 32 sectors per load), and a value meets the weights of all heads at once.  Rows of prompts of 101 and 503 tokens, 16 heads,
+// latents of 512 + 64: one head at a time 1210 us, four 530, eight 430 without and 375 with the staging.  Exponents are taken of differences of natural-unit scores: a score of hundreds loses nothing to a multiplication by log2 e.
 template <RowKind KIND, int HP, int KA>
 __global__ void __launch_bounds__(128) k_latent_rows_f32(const RowsParams p) {
   extern __shared__ __align__(16) float sm[];
@@ -151,6 +152,8 @@ __global__ void __launch_bounds__(128) k_latent_rows_f32(const RowsParams p) {
   float* sq = sm;                 // [HP][kd]
   float* sp = sm + HP * kd;       // [128][HP]
   int* sl = reinterpret_cast<int*>(sp + 128 * HP);
+  constexpr int kCols = 32, kPitch = kCols + 4;                // HP > 1: two stages of 32 columns of 128 keys
+  float* sk = reinterpret_cast<float*>(sl + 128);
   const float* qa = static_cast<const float*>(p.qa) + (size_t(row) * p.heads + h0) * (kd + kRowPad);
 #pragma unroll
   for (int e = 0; e < HP; e++)
@@ -173,7 +176,49 @@ __global__ void __launch_bounds__(128) k_latent_rows_f32(const RowsParams p) {
     float s[HP];
 #pragma unroll
     for (int e = 0; e < HP; e++) s[e] = kNegBig;
-    if (tid < n) {
+    if constexpr (HP > 1) {
+      if (tid < n) {
+        const int tok = t0 + tid;
+        sl[tid] = (bt[tok / p.block_size] * G + g) * p.block_size + tok % p.block_size;
+      }
+      __syncthreads();
+      auto stage = [&](int c0, int buf) {                        // 16 bytes of rows tid / 8, + 16, ..
+        const int c = (tid & 7) * 4;
+        if (c0 + c < kd)
+#pragma unroll
+          for (int r = tid >> 3; r < 128; r += 16)
+            if (r < n) cp_async16(smem_addr(sk + (buf * 128 + r) * kPitch + c), cache + size_t(sl[r]) * (Dk + kRowPad) + c0 + c);
+        cp_async_commit();
+      };
+      float4 a[HP];
+#pragma unroll
+      for (int e = 0; e < HP; e++) a[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+      stage(0, 0);
+      for (int c0 = 0, buf = 0; c0 < kd; c0 += kCols, buf ^= 1) {
+        stage(c0 + kCols, buf ^ 1);
+        cp_async_wait<1>();
+        __syncthreads();
+        const float4* kr = reinterpret_cast<const float4*>(sk + (buf * 128 + tid) * kPitch);
+        const int cols = min(kCols, kd - c0) / 4;                // (rows behind the last key hold anything: their sums are not used)
+#pragma unroll 4
+        for (int i = 0; i < cols; i++) {
+          const float4 k = kr[i];
+#pragma unroll
+          for (int e = 0; e < HP; e++) {
+            const float4 q = reinterpret_cast<const float4*>(sq + e * kd + c0)[i];
+            a[e].x = fmaf(q.x, k.x, a[e].x); a[e].y = fmaf(q.y, k.y, a[e].y); a[e].z = fmaf(q.z, k.z, a[e].z); a[e].w = fmaf(q.w, k.w, a[e].w);
+          }
+        }
+        __syncthreads();
+      }
+      if (tid < n)
+#pragma unroll
+        for (int e = 0; e < HP; e++) {
+          s[e] = ((a[e].x + a[e].y) + (a[e].z + a[e].w)) * p.scale;
+          if (KIND == kShared) s[e] *= cache[size_t(sl[tid]) * (Dk + kRowPad) + Dk];
+          if (KIND != kLatent && p.softcap > 0.f) s[e] = p.softcap * tanhf(s[e] / p.softcap);
+        }
+    } else if (tid < n) {
       const int tok = t0 + tid, slot = (bt[tok / p.block_size] * G + g) * p.block_size + tok % p.block_size;
       sl[tid] = slot;
       const float4* kr = reinterpret_cast<const float4*>(cache + size_t(slot) * (Dk + kRowPad));
@@ -221,6 +266,36 @@ __global__ void __launch_bounds__(128) k_latent_rows_f32(const RowsParams p) {
     __syncthreads();
 #pragma unroll
     for (int e = 0; e < HP; e++) l[e] = l[e] * corr[e] + (red[e][0] + red[e][1] + red[e][2] + red[e][3]);
+    if constexpr (HP > 1) {
+      float acc[HP][KA];
+#pragma unroll
+      for (int e = 0; e < HP; e++)
+#pragma unroll
+        for (int k = 0; k < KA; k++) acc[e][k] = 0.f;
+#pragma unroll 4
+      for (int t = 0; t < n; t++) {
+        const float* at = cache + size_t(sl[t]) * (Dk + kRowPad) + voff + tid;
+        float v[KA];
+#pragma unroll
+        for (int k = 0; k < KA; k++) v[k] = tid + k * 128 < p.R ? at[k * 128] : 0.f;
+        float4 w[HP / 4];
+#pragma unroll
+        for (int e = 0; e < HP / 4; e++) w[e] = reinterpret_cast<const float4*>(sp + t * HP)[e];
+#pragma unroll
+        for (int e = 0; e < HP / 4; e++)
+#pragma unroll
+          for (int k = 0; k < KA; k++) {
+            acc[4 * e][k] = fmaf(w[e].x, v[k], acc[4 * e][k]);
+            acc[4 * e + 1][k] = fmaf(w[e].y, v[k], acc[4 * e + 1][k]);
+            acc[4 * e + 2][k] = fmaf(w[e].z, v[k], acc[4 * e + 2][k]);
+            acc[4 * e + 3][k] = fmaf(w[e].w, v[k], acc[4 * e + 3][k]);
+          }
+      }
+#pragma unroll
+      for (int e = 0; e < HP; e++)
+#pragma unroll
+        for (int k = 0; k < KA; k++) o[e][k] = fmaf(o[e][k], corr[e], acc[e][k]);
+    } else
 #pragma unroll
     for (int k = 0; k < KA; k++) {
       const int d = tid + k * 128;
@@ -263,7 +338,7 @@ template <RowKind KIND, int HP, int KA>
 cudaError_t launch_rows_f32(const RowsParams& p, int rows, cudaStream_t st) {
   static std::atomic<unsigned> done{0};
   const int kd = KIND == kPaired ? p.rotp : p.Rp + p.rotp;
-  const size_t smem = size_t(HP) * (kd + 128) * 4 + 128 * 4;
+  const size_t smem = size_t(HP) * (kd + 128) * 4 + 128 * 4 + (HP > 1 ? 2 * 128 * 36 * 4 : 0);
   const cudaError_t e = smem > 32 * 1024 ? pdl::allow_smem(k_latent_rows_f32<KIND, HP, KA>, kMaxSmem, done) : cudaSuccess;   // 48 KB need no opt-in
   return e != cudaSuccess ? e : pdl::launch(k_latent_rows_f32<KIND, HP, KA>, dim3(rows, p.heads / HP), dim3(128), smem, st, 1, p);
 }
@@ -766,9 +841,10 @@ int rows_form(RowsParams& p, int rows, int bf16, cudaStream_t st) {
   if (!bf16) {
     p.splits = 1;
     if (p.Rp > 2048) return -2;
-    // four heads at a time where a cache head has a multiple of four and their CTAs fill the GPU; a single row's heads spread over SMs instead
-    const bool four = p.heads / p.kv_heads % 4 == 0 && p.Rp <= 512 && rows * p.heads / 4 >= tbvops::sm_count();
-    e = four ? launch_rows_f32<KIND, 4, 4>(p, rows, st) : launch_rows_f32<KIND, 1, 16>(p, rows, st);
+    // eight or four heads at a time where a cache head has a multiple of them and their CTAs fill the GPU; a single row's heads spread over SMs instead
+    const int per = p.heads / p.kv_heads;
+    auto fills = [&](int heads) { return per % heads == 0 && p.Rp <= 512 && rows * p.heads / heads >= tbvops::sm_count(); };
+    e = fills(8) ? launch_rows_f32<KIND, 8, 4>(p, rows, st) : fills(4) ? launch_rows_f32<KIND, 4, 4>(p, rows, st) : launch_rows_f32<KIND, 1, 16>(p, rows, st);
     return e == cudaSuccess ? 0 : -1;
   }
   p.splits = p.splits < 1 ? 1 : (p.splits > kMaxSplits ? kMaxSplits : p.splits);
