@@ -347,7 +347,7 @@ namespace tbvops {
 // By the weights' shape alone (see above).  With short K the start and the end of a tile weigh more than its products (us, here / on the CUDA cores: 130 tokens, 1024 x 520 19 / 14,
 // 512 x 512 17 / 13, 4096 x 128 17 / 13; 604 tokens, 1024 x 520 20 / 42, 4096 x 128 28 / 26); with long K it is faster at all numbers of tokens (8192 x 2048 at 1 / 16 / 130 / 604 tokens
 // 32 / 33 / 74 / 191 against 42 / 42 / 175 / 519, 2048 x 7168 54 / 55 / 94 / 197 against 92 / 94 / 326 / 607, 160 x 4096 18 / 18 / 23 / 24 against 49 / 49 / 50 / 70, 14336 x 2048
-// 56 / 56 / 128 / 266 against 109 / 111 / 266 / 906).  Relative error over such shapes 0.9 .. 1.3e-7 against 1.2 .. 2.8e-7 there.
+// 56 / 56 / 128 / 266 against 109 / 111 / 266 / 906; 256 x 1024 at 130 tokens 15.9 against 15.1).  Relative error over such shapes 0.9 .. 1.3e-7 against 1.2 .. 2.8e-7 there.
 bool gemm_f32_split_takes(int M, int K, int groups, int m_last) { return K >= 1024 ? M >= 128 : K >= 512 && (long)M * groups >= 2048; }
 
 int gemm_f32_split_launch(const F32Params& p, int x_rows, void* stream) {

@@ -15,6 +15,7 @@ programmatic dependent launch so that each GEMM streams its weights while the co
 ``TBV_FUSE_GEMM_AR=1`` folds each row-parallel GEMM into its collective (one kernel whose epilogue stores LL
 packets into the peers' memory; 5 launches per layer, same bits); it is not the default because it measures
 slower (see ``parallel/tp.py``).
+With one rank the norms are folded into the GEMMs beside them (``ops.gemm_resid``, ``ops.gemm_scaled``): 5 launches per layer.
 All buffers are preallocated so a decode step can be captured in a CUDA graph.
 """
 from __future__ import annotations

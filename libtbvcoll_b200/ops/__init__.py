@@ -126,7 +126,7 @@ def _chk(rc: int, name: str):
 
 def gemm_persist_mode(mode: Optional[int]) -> None:
     """Selection of the many-token (persistent) GEMM: 0 never, 1 where it is estimated faster, 2 / 3 / 4 force
-    its 128 x 256 / 256 x 256 / 128 x 128 tile; None = read ``TBV_GEMM_PERSIST`` again (the library reads it once)."""
+    its 128 x 256 / 256 x 256 (on pairs of SMs) / 128 x 128 tile; None = read ``TBV_GEMM_PERSIST`` again (the library reads it once)."""
     lib().tbv_op_gemm_persist_mode(-1 if mode is None else int(mode))
 
 
@@ -228,7 +228,8 @@ def gemm_scaled(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, sq: RowSqua
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None, act: int = ACT_NONE, act_arg: float = 0.0,
            glu: Optional[tuple] = None, copy: Optional[torch.Tensor] = None, groups: int = 1, x_group: int = 0, y_group: int = 0,
            last: int = 0, act_cols: int = 0) -> torch.Tensor:
-    """out[N, M] = epilogue(x[N, K] @ w[M, K]^T + bias) for bf16 operands (tcgen05) or fp32 operands (CUDA cores, full 32-bit).
+    """out[N, M] = epilogue(x[N, K] @ w[M, K]^T + bias) for bf16 operands (tcgen05) or fp32 operands (three bf16 pieces each on
+    tcgen05, or the CUDA cores for short K: no larger error than fp32 sums).
 
     The output dtype is ``out``'s: fp32 results take an activation (``ACT_SOFTPLUS``, ``ACT_SOFTCAP`` with its limit in ``act_arg``, ``ACT_SILU``, ``ACT_GELU``)
     and, from bf16 operands, an optional bf16 ``copy`` with the same row stride; ``act_cols`` > 0 (a multiple of 16; results of the operands' dtype): the
