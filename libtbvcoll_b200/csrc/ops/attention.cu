@@ -720,7 +720,7 @@ int tbv_op_prefill_attention(const void* q, const void* k_cache, const void* v_c
   if (!few && scale > 0.f && tile_rows <= 128 && !(reinterpret_cast<uintptr_t>(v_cache) & 15) && tbvops::attn_prefill_takes(q, k_cache, out, nq_heads, nkv, ldq, ldo, block_size))
     return tbvops::attn_prefill_split(q, k_cache, v_cache, static_cast<const int*>(block_tables), static_cast<const int*>(seq_of_query),
                                       static_cast<const int*>(ctx_lens), static_cast<const int*>(tiles), out, nq_rows, ntiles, nq_heads, nkv, ldq, ldo, block_size,
-                                      max_blocks, scale, static_cast<cudaStream_t>(stream));
+                                      max_blocks, keys, scale, static_cast<cudaStream_t>(stream));
   if (tile_rows > 64) return -2;
   PrefillParams pp{};
   AttnParams& p = pp.a;

@@ -14,6 +14,7 @@
 // What bounds it: 16384 exponentials per tile take 1024 clocks of the SM's exponential units (three times that with a soft cap), its two products 1024 clocks of the
 // tensor cores.  Measured (32 query heads, 8 key heads, causal; before: warp-level products, 64 rows per CTA): 8 x 512 tokens 50 us (was 128), 1 x 4096 tokens
 // 155 us (was 868; 0.53 of the measured bf16 burst rate), rows that hold both 50 and 157 us (were 148 and 848); 1 x 4096, 16 heads, soft cap 50: 4 layers take 0.9 ms less.
+// With few units the chain of one CTA is all there is: two CTAs of a cluster then take every other tile (rule and figures at attn_prefill_split).
 // Set-up and one tile take some 7 us, so few keys are better served elsewhere: tbv_op_prefill_attention sends up to 64 of them to the 64-row form.  Rows that hold both
 // stay here: one token 7.1 us (7.2 before), 64 tokens 7.3 (8.1), but 5 tokens with a soft cap 8.5 (7.4).
 //
@@ -60,6 +61,7 @@ struct Smem {
   unsigned long long q_full, k_full, k_empty, v_full, v_empty, s_full, p_ready;
   uint32_t tmem_base;
   int abort_flag;
+  float m[kRows], l[kRows];        // TWO: for the other CTA
 };
 
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, int x, int y, int z, uint32_t bar) {
@@ -102,6 +104,7 @@ __device__ __forceinline__ uint64_t desc_channels_contiguous(uint32_t addr) {
   d |= uint64_t(2) << 61;                          // 128-byte swizzle
   return d;
 }
+__device__ __forceinline__ void st_shared_f32(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
 __device__ __forceinline__ float exp2_ftz(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -116,7 +119,8 @@ __device__ __forceinline__ void st_global_32(void* p, const uint32_t* v) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 
-template <bool PAIR, bool CAP>
+// TWO: the two CTAs of a cluster take every other tile of keys of one unit and add up what they have, each for half of the channels
+template <bool PAIR, bool CAP, bool TWO>
 __global__ void __launch_bounds__(192, 2)
 k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -148,7 +152,8 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
   // which rows: a tile of the list and a key head (PAIR: and a part of the tile)
   const int hpk = p.hpk, per = kRows / hpk;                       // tokens per CTA
-  const int unit = blockIdx.x, head = unit % p.kv_heads, rest = unit / p.kv_heads;
+  const int part = TWO ? int(blockIdx.x & 1) : 0, step = TWO ? 2 : 1;
+  const int unit = TWO ? int(blockIdx.x >> 1) : int(blockIdx.x), head = unit % p.kv_heads, rest = unit / p.kv_heads;
   const int tile = PAIR ? rest / p.parts : p.ntiles - 1 - rest;   // a prompt's last rows see most keys: they start first (PAIR: the list is in that order)
   const int t0 = PAIR ? rest % p.parts * per : 0;
   const int* tl = p.tiles + tile * (PAIR ? 4 : 2);
@@ -159,9 +164,16 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   // keys that the first and the last row see, and the first key that the first row sees
   const int see_first = any ? min(PAIR ? tl[3] + t0 : p.ctx_lens[row0], cap) : 0, see_last = any ? min(PAIR ? tl[3] + t0 + nrows - 1 : p.ctx_lens[row0 + nrows - 1], cap) : 0;
   const int j0 = PAIR ? attn_mma::first_visible(see_first, p.window, p.chunk) / kKeys : 0;
-  const int j1 = (see_last + kKeys - 1) / kKeys, n = any ? max(0, j1 - j0) : 0;
+  const int j1 = (see_last + kKeys - 1) / kKeys, n_all = any ? max(0, j1 - j0) : 0, n = (n_all + step - 1 - part) / step;
   const uint32_t tm_s = s.tmem_base, tm_o = tm_s + 128u;
   volatile int* abortp = &s.abort_flag;
+
+  // a row's weights: what the thread that owns it holds
+  const int r = threadIdx.x, t = r / hpk, g = r - t * hpk;
+  const bool mine = t < nrows;
+  const uint32_t lanes = uint32_t(warp * 32) << 16;
+  float m = kFloor, l = 0.f;
+  bool ok = true;
 
   if (warp == 4) {
     // ---- copies: lane i takes half i & 1 of the 16 tokens i >> 1 of a tile ----
@@ -172,11 +184,10 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     }
     const int piece = lane >> 1, half = lane & 1;
     int entry = 0;
-    bool ok = true;
     int k_issued = 0, v_issued = 0;
     for (int i = 0; i < n && ok; i++) {
-      const int tok = (j0 + i) * kKeys + piece * 16;
-      const int pieces = min(8, (see_last - (j0 + i) * kKeys + 15) >> 4);
+      const int tok = (j0 + i * step + part) * kKeys + piece * 16;
+      const int pieces = min(8, (see_last - (j0 + i * step + part) * kKeys + 15) >> 4);
       int x = half * 64, y = 0;
       if (piece < pieces) {
         entry = bt[tok / p.block_size];
@@ -208,7 +219,7 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       // ---- products ----
       const uint32_t id_s = umma_idesc_bf16(kRows, kKeys), id_o = umma_idesc_bf16(kRows, kD) | (1u << 16);   // bit 16: channels of V contiguous
       const uint64_t qd = umma_desc_sw128(sq), kd = umma_desc_sw128(sk), vd = desc_channels_contiguous(sv);
-      bool ok = mbar_wait(bq, 0, abortp, p.limit_ns);
+      ok = mbar_wait(bq, 0, abortp, p.limit_ns);
       for (int i = 0; i < n && ok; i++) {
         const uint32_t ph = uint32_t(i) & 1u;
         // the scores replace the weights of the tile before: those must have been used (which also settles the sums before anyone rescales them)
@@ -232,19 +243,14 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     }
   } else if (n > 0) {
     // ---- weights: thread = row (token, query head) ----
-    const int r = threadIdx.x, t = r / hpk, g = r - t * hpk;
-    const bool mine = t < nrows;
     const int see = !mine ? 0 : min(PAIR ? see_first + t : p.ctx_lens[row0 + t], cap);
     const int lo = PAIR ? attn_mma::first_visible(see, p.window, p.chunk) : 0;
     const int lo_last = PAIR ? attn_mma::first_visible(see_last, p.window, p.chunk) : 0;
-    const uint32_t lanes = uint32_t(warp * 32) << 16;
     const float sc = CAP ? 1.f : p.scale_log2;
     const float cap_a = CAP ? 2.f * attn_mma::kLog2e / p.softcap : 0.f, cap_c = p.softcap * attn_mma::kLog2e, cap_b = -2.f * cap_c;
-    float m = kFloor, l = 0.f;
-    bool ok = true;
     for (int i = 0; i < n; i++) {
       const uint32_t ph = uint32_t(i) & 1u;
-      const int key0 = (j0 + i) * kKeys;
+      const int key0 = (j0 + i * step + part) * kKeys;
       ok = __all_sync(0xffffffffu, mbar_wait(bsf, ph, abortp, p.limit_ns));
       if (!ok) break;
       tc_fence_after();
@@ -319,54 +325,95 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       if (lane == 0) mbar_arrive(bpr);
     }
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bve, uint32_t(n - 1) & 1u, abortp, p.limit_ns));
-    if (ok) {
-      tc_fence_after();
-      const float f = l > 0.f ? 1.f / l : 0.f;
-      const size_t col = size_t(head * hpk + g) * kD;
-      __nv_bfloat16* dst = p.out + size_t(row0 + (mine ? t : 0)) * p.ldo + col;
-      const __nv_bfloat16* gate = PAIR && p.gate ? p.gate + size_t(row0 + (mine ? t : 0)) * p.ldg + col : nullptr;
-#pragma unroll 1
-      for (int c = 0; c < kD; c += 32) {
+    if (ok) tc_fence_after();
+  } else if (any && n_all == 0 && part == 0) {
+    // no visible key at all: nothing to sum
+    if (mine)
+      for (int c = 0; c < kD; c += 8) *reinterpret_cast<uint4*>(p.out + size_t(row0 + t) * p.ldo + size_t(head * hpk + g) * kD + c) = make_uint4(0, 0, 0, 0);
+  }
+
+  // ---- results ----
+  float own = 1.f, other = 0.f;                                   // factors of this CTA's sums and of the other one's
+  if constexpr (TWO) {
+    if (warp < 4 && n_all > 0) {
+      // the half of the channels that the other CTA finishes, [channel][row], where keys and values were: all products that read those are complete
+      for (int c = 0; c < kD / 2; c += 32) {
         float o[32];
+        if (n > 0) {
+          tmem_ld32(tm_o + lanes + uint32_t((part ^ 1) * (kD / 2) + c), o);
+          tmem_ld_wait();
+        }
+        if (ok) {
+#pragma unroll
+          for (int e = 0; e < 32; e++) st_shared_f32(sk + uint32_t(((c + e) * kRows + r) * 4), n > 0 ? o[e] : 0.f);
+        }
+      }
+      s.m[r] = m;
+      s.l[r] = l;
+    }
+    __syncwarp();
+    cluster_sync_all();
+    if (warp < 4 && n_all > 0) {
+      const float m2 = ld_dsmem_f32(mapa_shared(smem_u32(&s.m[r]), uint32_t(part ^ 1))), l2 = ld_dsmem_f32(mapa_shared(smem_u32(&s.l[r]), uint32_t(part ^ 1)));
+      const float top = fmaxf(m, m2);
+      own = exp2_ftz(m - top);
+      other = exp2_ftz(m2 - top);
+      l = part ? fmaf(l2, other, l * own) : fmaf(l, own, l2 * other);
+    }
+  }
+  if (warp < 4 && n_all > 0 && ok) {
+    const float f = l > 0.f ? 1.f / l : 0.f;
+    own *= f;
+    other *= f;
+    const size_t col = size_t(head * hpk + g) * kD;
+    __nv_bfloat16* dst = p.out + size_t(row0 + (mine ? t : 0)) * p.ldo + col;
+    const __nv_bfloat16* gate = PAIR && p.gate ? p.gate + size_t(row0 + (mine ? t : 0)) * p.ldg + col : nullptr;
+    const int c0 = TWO ? part * (kD / 2) : 0;
+    const uint32_t far = TWO ? mapa_shared(sk + uint32_t(r * 4), uint32_t(part ^ 1)) : 0u;
+#pragma unroll 1
+    for (int c = c0; c < (TWO ? c0 + kD / 2 : kD); c += 32) {
+      float o[32];
+      if (!TWO || n > 0) {
         tmem_ld32(tm_o + lanes + uint32_t(c), o);
         tmem_ld_wait();
-        if (mine) {
-          uint32_t w[16];
-#pragma unroll
-          for (int e = 0; e < 32; e += 8) {
-            float a[8];
-#pragma unroll
-            for (int q = 0; q < 8; q++) a[q] = o[e + q] * f;
-            if (gate) {
-              float gt[8];
-              vec::load8(gate + c + e, gt);
-#pragma unroll
-              for (int q = 0; q < 8; q++) a[q] *= vec::sigmoid<__nv_bfloat16>(gt[q]);
-            }
-#pragma unroll
-            for (int q = 0; q < 8; q += 2) w[(e + q) >> 1] = attn_mma::pack_bf16(a[q], a[q + 1]);
-          }
-          if (p.wide) {                            // a whole sector at a time
-            st_global_32(dst + c, w);
-            st_global_32(dst + c + 16, w + 8);
-          } else {
-#pragma unroll
-            for (int q = 0; q < 4; q++) *reinterpret_cast<uint4*>(dst + c + 8 * q) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-          }
-        }
-        __syncwarp();
       }
+#pragma unroll
+      for (int e = 0; e < 32; e++) {
+        if constexpr (TWO) o[e] = fmaf(ld_dsmem_f32(far + uint32_t((c - c0 + e) * kRows * 4)), other, n > 0 ? o[e] * own : 0.f);
+        else o[e] *= own;
+      }
+      if (mine) {
+        uint32_t w[16];
+#pragma unroll
+        for (int e = 0; e < 32; e += 8) {
+          float a[8];
+#pragma unroll
+          for (int q = 0; q < 8; q++) a[q] = o[e + q];
+          if (gate) {
+            float gt[8];
+            vec::load8(gate + c + e, gt);
+#pragma unroll
+            for (int q = 0; q < 8; q++) a[q] *= vec::sigmoid<__nv_bfloat16>(gt[q]);
+          }
+#pragma unroll
+          for (int q = 0; q < 8; q += 2) w[(e + q) >> 1] = attn_mma::pack_bf16(a[q], a[q + 1]);
+        }
+        if (p.wide) {                              // a whole sector at a time
+          st_global_32(dst + c, w);
+          st_global_32(dst + c + 16, w + 8);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; q++) *reinterpret_cast<uint4*>(dst + c + 8 * q) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+        }
+      }
+      __syncwarp();
     }
-  } else if (any) {
-    // no visible key at all: nothing to sum
-    const int r = threadIdx.x, t = r / hpk, g = r - t * hpk;
-    if (t < nrows)
-      for (int c = 0; c < kD; c += 8) *reinterpret_cast<uint4*>(p.out + size_t(row0 + t) * p.ldo + size_t(head * hpk + g) * kD + c) = make_uint4(0, 0, 0, 0);
   }
 
   __syncwarp();
   tc_fence_before();
   __syncthreads();
+  if constexpr (TWO) cluster_sync_all();                          // nobody leaves while the other CTA may still read its shared memory
   if (warp == 5) {
     tc_fence_after();
     tmem_dealloc(s.tmem_base, 256);
@@ -374,12 +421,13 @@ k_attn_prefill(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   if (threadIdx.x == 0 && s.abort_flag && p.err) atomicExch(p.err, 1);
 }
 
-template <bool PAIR, bool CAP>
+template <bool PAIR, bool CAP, bool TWO = false>
 cudaError_t launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const Params& p, cudaStream_t st) {
   static std::atomic<unsigned> done{0};
-  const cudaError_t attr = pdl::allow_smem(k_attn_prefill<PAIR, CAP>, kSmem, done);
+  const cudaError_t attr = pdl::allow_smem(k_attn_prefill<PAIR, CAP, TWO>, kSmem, done);
   if (attr != cudaSuccess) return attr;
-  return pdl::launch(k_attn_prefill<PAIR, CAP>, dim3(unsigned(p.ntiles) * p.parts * p.kv_heads), dim3(192), kSmem, st, 1, q, k, v, p);
+  const unsigned units = unsigned(p.ntiles) * p.parts * p.kv_heads;
+  return pdl::launch_clusters(k_attn_prefill<PAIR, CAP, TWO>, dim3(TWO ? 2 * units : units), dim3(192), kSmem, st, dim3(TWO ? 2 : 1), q, k, v, p);
 }
 
 int report(cudaError_t e) {
@@ -397,7 +445,7 @@ bool attn_prefill_takes(const void* q, const void* kv, const void* out, int head
 }
 
 int attn_prefill_split(const void* q, const void* k_cache, const void* v_cache, const int* tables, const int* seq_of_row, const int* ctx_lens, const int* tiles,
-                       void* out, int rows, int ntiles, int heads, int kv_heads, int ldq, int ldo, int block_size, int max_blocks, float scale, cudaStream_t st) {
+                       void* out, int rows, int ntiles, int heads, int kv_heads, int ldq, int ldo, int block_size, int max_blocks, int keys, float scale, cudaStream_t st) {
   Params p{};
   p.tiles = tiles; p.seq_of_row = seq_of_row; p.ctx_lens = ctx_lens; p.tables = tables; p.out = static_cast<__nv_bfloat16*>(out);
   p.ntiles = ntiles; p.kv_heads = kv_heads; p.hpk = heads / kv_heads; p.parts = 1; p.block_size = block_size; p.max_blocks = max_blocks; p.ldo = ldo;
@@ -407,7 +455,11 @@ int attn_prefill_split(const void* q, const void* k_cache, const void* v_cache, 
   const unsigned long long width = (unsigned long long)kv_heads * kD;
   if (make_tensor_map_heads(&mq, q, rows, heads, kD, ldq, p.hpk, kRows / p.hpk) != 0 || make_tensor_map_bf16(&mk, k_cache, kAnyCacheRows, width, width, 16) != 0 ||
       make_tensor_map_bf16(&mv, v_cache, kAnyCacheRows, width, width, 16) != 0) return -3;
-  return report(launch<false, false>(mq, mk, mv, p, st));
+  // Shared out over two CTAs where both of every unit find a place at once (two per SM) and the longest context is known to be long against the exchange.  16 query heads on 4
+  // key heads, us, one CTA / two: 256 tokens behind 256 13.2 / 11.2, 1024 tokens 22.5 / 18.2, 128 behind 1024 21.9 / 16.3, 256 behind 1800 36.6 / 25.3, 4 x 100 behind 300
+  // 14.9 / 13.3; 384 tokens 11.2 / 11.2, but 10.8 / 11.7 with 8 key heads and 12.0 / 13.0 with 32 on 8.
+  const bool two = ntiles * kv_heads <= sm_count() && keys > 3 * kKeys;
+  return report(two ? launch<false, false, true>(mq, mk, mv, p, st) : launch<false, false>(mq, mk, mv, p, st));
 }
 
 int attn_prefill_paired(const void* q, const void* cache, const int* tables, const int* seq_of_row, const int* tiles, const void* gate, void* out, int rows,

@@ -52,7 +52,7 @@ int attn_rows(const void* q, const void* k_cache, const void* v_cache, const int
 // attention of prompt rows on tcgen05, heads of 128 channels (attn_prefill.cu): keys and values in caches of their own, or side by side in cached rows
 bool attn_prefill_takes(const void* q, const void* kv, const void* out, int heads, int kv_heads, int ldq, int ldo, int block_size);
 int attn_prefill_split(const void* q, const void* k_cache, const void* v_cache, const int* tables, const int* seq_of_row, const int* ctx_lens, const int* tiles,
-                       void* out, int rows, int ntiles, int heads, int kv_heads, int ldq, int ldo, int block_size, int max_blocks, float scale, cudaStream_t st);
+                       void* out, int rows, int ntiles, int heads, int kv_heads, int ldq, int ldo, int block_size, int max_blocks, int keys, float scale, cudaStream_t st);
 int attn_prefill_paired(const void* q, const void* cache, const int* tables, const int* seq_of_row, const int* tiles, const void* gate, void* out, int rows,
                         int ntiles, int heads, int kv_heads, int ldq, int ldo, int ldg, int row_len, int block_size, int max_blocks, float softcap, int window, int chunk,
                         cudaStream_t st);

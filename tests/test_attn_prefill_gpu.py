@@ -89,6 +89,24 @@ def test_split_caches(ops, nq, nkv, bs, tile_rows, off, keys):
     assert (around[:, :off] == 7).all()
 
 
+# both CTAs of a cluster at work on a unit: one tile of keys (nothing for the second CTA), the edges of two and three, contexts before the prompt; 37 and 38
+# tiles of 4 key heads are the last grid that is shared out on 148 SMs and the first that is not.  The stated longest context only chooses the kernel.
+@pytest.mark.parametrize("nq,nkv,rows,before", [(4, 1, 1, 0), (4, 1, 128, 0), (4, 1, 129, 0), (8, 2, 256, 0), (8, 2, 257, 0), (8, 1, 40, 345), (4, 4, 385, 127), (16, 4, 1184, 0), (16, 4, 1216, 0)])
+def test_keys_shared_out_over_two_ctas(ops, nq, nkv, rows, before):
+    n, bs = rows + before, 16
+    q, kc, vc = rnd(rows, nq, D, seed=8), rnd(n + 16, nkv, D, seed=9), rnd(n + 16, nkv, D, seed=10)
+    kc[n:], vc[n:] = float("nan"), float("nan")
+    tables = torch.arange(n // bs + 1, dtype=torch.int32)[None].to(DEV)
+    see = torch.arange(before + 1, n + 1, device=DEV)
+    seq = torch.zeros(rows, dtype=torch.int32)
+    tiles = ops.prefill_tiles(seq, nq // nkv, 128).to(DEV)
+    out = torch.full_like(q, float("nan"))
+    ops.prefill_attention(q, kc, vc, tables, see.to(torch.int32), seq.to(DEV), tiles, out, 0.2, bs, 128, 2000)
+    torch.cuda.synchronize()
+    assert not ops.gemm_error()
+    check(out, *plain(q, kc[:n], vc[:n], 0.2, see, torch.zeros_like(see)))
+
+
 def test_growing_and_huge_scores(ops):
     """Keys whose scores grow by more than the rescaling threshold from tile to tile, fall again, and single keys that take all of the weight."""
     n, bs = 700, 16
