@@ -90,6 +90,9 @@ __global__ void __launch_bounds__(gemm::kThreads, 1)
 k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ gemm::Smem s;
+  // Where a Llama layer's chain waits for them, threads report their last read of a peer when it has been made; with fp32 results and clamped units one barrier of whole warps at the
+  // end is the quicker (decode steps, one row, early / at the end: Bobarax 955 / 946 us, Nubosun 934 / 924).  The same for stores that no norm scales was no gain (952 / 927).
+  constexpr bool kEarly = EPI == kEpiResid || EPI == kEpiStore || EPI == kEpiSiluMul;
   __shared__ float scale[EPI == kEpiStore || EPI == kEpiSiluMul ? 256 : 1], part[EPI == kEpiStore || EPI == kEpiSiluMul ? 128 : 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Launch order follows blockIdx.x.  With many token tiles the CTAs that share one 128-row weight tile
@@ -236,7 +239,7 @@ k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
       const uint32_t stage_addr = smem_u32(sm);
       const int pieces = EPI == kEpiResid ? (rows * q4 + 127) / 128 * 128 : rows * q4;
       auto more = [&](int idx) { return idx + 128 < pieces; };
-      if (te >= pieces) cluster_arrive();
+      if (kEarly && te >= pieces) cluster_arrive();
       for (int idx = te; idx < pieces; idx += 128) {
         const int t = idx / q4, f = split * fs + (idx % q4) * 4;
         const int m = m0 + f;
@@ -254,7 +257,7 @@ k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
           continue;
         }
         float4 acc = dsmem_sum_f32x4(stage_addr + uint32_t((t * 128 + f) * 4), S);
-        if (!more(idx)) cluster_arrive();     // (behind this thread's last read of its peers)
+        if (kEarly && !more(idx)) cluster_arrive();     // (behind this thread's last read of its peers)
         if ((EPI == kEpiStore || EPI == kEpiSiluMul) && p.sq) {
           const float sc = scale[t];
           acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
@@ -291,8 +294,13 @@ k_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
         }
       }
     }
-    if (warp < 2) cluster_arrive();
-    cluster_wait();      // nobody leaves while a peer may still read its shared memory
+    if constexpr (kEarly) {
+      if (warp < 2) cluster_arrive();
+      cluster_wait();    // nobody leaves while a peer may still read its shared memory
+    } else {
+      __syncwarp();
+      cluster_sync_all();
+    }
   }
   __syncwarp();
   gemm::teardown(p, s);
